@@ -58,7 +58,7 @@ struct AdjBlock {
 
 // The backward wave's camera: the forward's camera rays again, and each slot's radiance still to
 // come set to the radiance the forward pass found (left in P.sum).
-__global__ void k_adjoint_camera(SceneDev S, WaveDesc w, PathBuffers P, AdjointDev A) {
+__global__ void k_adjoint_camera(const __grid_constant__ SceneDev S, WaveDesc w, PathBuffers P, AdjointDev A) {
     float all = 0.0f;
     for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < w.n; slot += gridDim.x * blockDim.x) {
         uint32_t x, y, index;
@@ -391,7 +391,7 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
 
 // Eight blocks per SM (64 registers, with spills) rather than the compiler's 168 registers: as for
 // k_shade, more warps hide the scattered loads (512^2 adjoint iteration 51.4 -> 48.9 ms).
-__global__ void __launch_bounds__(128, RTG_SHADE_MIN_BLOCKS) k_shade_adjoint(SceneDev S, const LightsDev* __restrict__ Lg, PathBuffers P, int cur, uint32_t bounce,
+__global__ void __launch_bounds__(128, RTG_SHADE_MIN_BLOCKS) k_shade_adjoint(const __grid_constant__ SceneDev S, const LightsDev* __restrict__ Lg, PathBuffers P, int cur, uint32_t bounce,
                                                        WaveDesc w, AdjointDev A) {
     __shared__ float s_grad[MAX_ADJOINT_PARAMS];
     AdjBlock blk{s_grad};
@@ -426,7 +426,7 @@ __device__ __forceinline__ void adjoint_unblocked(const PathBuffers& P, const Ad
     }
 }
 
-__global__ void __launch_bounds__(TRACE_THREADS) k_shadow_adjoint(SceneDev S, PathBuffers P, WaveDesc w, AdjointDev A) {
+__global__ void __launch_bounds__(TRACE_THREADS) k_shadow_adjoint(const __grid_constant__ SceneDev S, PathBuffers P, WaveDesc w, AdjointDev A) {
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
     __shared__ float s_grad[MAX_ADJOINT_PARAMS];
     uint64_t deep[STACK_CAP - SHORT_STACK];
@@ -464,7 +464,12 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_shadow_adjoint(SceneDev S, Pa
         }
         if (busy) {
             bool blocked = false;
-            if (trav_step<true>(S, T, stack, &err, blocked)) {
+            const auto src = [&](V3& ro, V3& rd) {
+                const float4 o = P.sh_o[ray], d = P.sh_d[ray];
+                ro = v3(o.x, o.y, o.z);
+                rd = v3(d.x, d.y, d.z);
+            };
+            if (trav_step<true, true>(S, T, 1.0e-3f, stack, &err, blocked, src)) {
                 busy = false;
                 if (!blocked) adjoint_unblocked(P, A, w, s_grad, ray);
             }

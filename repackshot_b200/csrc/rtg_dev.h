@@ -11,33 +11,35 @@ namespace rtg {
 
 constexpr uint32_t NODE_EMPTY = 0xffffffffu;
 constexpr uint32_t NODE_LEAF = 1u << 31;
-// Leaf reference: NODE_LEAF | first << 4 | (count - 1), count in 1..16.
-RTG_HD uint32_t make_leaf(uint32_t first, uint32_t count) { return NODE_LEAF | (first << 4) | (count - 1); }
+// Leaf reference: NODE_LEAF | the leaf's first triangle (in a top-level tree: its BlasInst).
+RTG_HD uint32_t make_leaf(uint32_t first) { return NODE_LEAF | first; }
 
-// An 8-wide BVH node with child boxes quantised to 8 bits per plane (96 bytes, six 16-byte
-// loads). A child box decodes as p + q * 2^e per axis; the builder checks that every decoded box
-// (computed with the same IEEE operations as the kernels) contains the child's exact box, so the
-// slab test never drops a hit that the exact box keeps. A flat child at the node's lower corner
-// (a floor under the rest of the scene) decodes to its exact plane, so a ray starting within
-// t_min of it is culled exactly where the reference's box culls it.
-struct alignas(16) QNode {
-    float px, py, pz;
-    uint8_t ex, ey, ez;   // biased exponents of the per-axis scales 2^(e-127)
-    uint8_t nchild;
+// An 8-wide BVH node with child boxes quantised to 8 bits per plane (96 bytes: three 32-byte loads,
+// a sector each). Plane q of an axis lies at p + q s, s = scale 2^-15 a power of two; the builder
+// checks that every child's box lies inside its planes, in exact arithmetic. The children are the
+// `inner` nodes at node_base + off, then leaves at leaf_base + off. A slot without a child has an
+// inverted box; should a ray pass it by rounding, it leads to a leaf of this node (or to a
+// triangle that nothing hits), which changes no answer.
+struct alignas(32) QNode {
+    float p[3];
+    float scale[3];
+    uint32_t node_base, leaf_base;
     uint8_t qlo[3][8];
     uint8_t qhi[3][8];
-    uint32_t child[8];    // inner node index, leaf reference or NODE_EMPTY
+    uint8_t off[8];
+    uint32_t inner, pad;
 };
 static_assert(sizeof(QNode) == 96, "QNode must be 96 bytes");
 
 // A leaf triangle (48 bytes): corners in its BLAS's space; w lanes carry the triangle's index in
 // its mesh, its instance (0xffffffff: the BLAS instance's) and flags (bit 0 one-sided, bit 1
-// hidden to camera rays).
+// hidden to camera rays, bit 2 the last of its leaf, the leaf's index from bit 3 on).
 struct alignas(16) TriRec {
     float v0[3]; uint32_t tri;
     float v1[3]; uint32_t inst;
     float v2[3]; uint32_t flags;
 };
+constexpr uint32_t TRI_LAST = 4u, TRI_LEAF_SHIFT = 3u;
 
 // A TLAS leaf: one bottom-level tree placed in the world.
 struct alignas(16) BlasInst {
@@ -46,6 +48,7 @@ struct alignas(16) BlasInst {
     uint32_t identity;    // the BLAS is in world space
     uint32_t instance;    // instance id for BLAS records that carry 0xffffffff
     uint32_t flags;       // bit 0 one-sided, bit 1 hidden to camera rays
+    float box[8];         // its world box: lower corner in [0, 3), upper in [4, 7)
 };
 
 // Per instance, what hit details and shading read.
@@ -154,6 +157,7 @@ struct SceneDev {
     const QNode* nodes;
     const TriRec* tris;
     const BlasInst* blas;
+    const float* leaf_boxes;  // 8 floats per leaf: its triangles' box, lower corner in [0, 3), upper in [4, 7)
     const DevInstance* instances;
     const float4* positions;  // xyz per vertex (global)
     const float4* normals;    // xyz per vertex (global)
@@ -162,7 +166,10 @@ struct SceneDev {
     // Bsdf::surface of every material seen from outside (2 m) and from inside (2 m + 1), and the
     // floor's Lambert lobe (2 n_materials): built once on the host, the same bits.
     const Bsdf* bsdfs;
-    uint32_t tlas_root, n_instances, n_materials, stack_need;
+    // The root of the walk: the top-level tree's, or, when the scene is one world-space tree, that
+    // tree's (single_blas 0; otherwise 0xffffffff).
+    uint32_t tlas_root, single_blas;
+    uint32_t n_instances, n_materials, stack_need;
     EnergyTables energy;
     // The section view (geometry/section.rs): the plane n . p = d removes the side n points to from
     // every query; with section_cap the closed solids it cuts are capped (their instances' `solid`),

@@ -249,7 +249,8 @@ uint32_t upload_geometry(const Flat& F, BufSet& set, SceneDev& S, size_t* hot_by
         if (b_blas) S.blas = (const BlasInst*)(p + round(b_nodes) + round(b_tris));
     }
     uint32_t st;
-    if ((st = upload(set, pos, S.positions)) || (st = upload(set, nrm, S.normals)) || (st = upload(set, ti, S.tri_index)))
+    if ((st = upload(set, pos, S.positions)) || (st = upload(set, nrm, S.normals)) || (st = upload(set, ti, S.tri_index)) ||
+        (st = upload(set, F.leaf_boxes, S.leaf_boxes)))
         return st;
     return RTG_STATUS_OK;
 }
@@ -307,9 +308,9 @@ void keep_shading(Scene& sc, const HScene& hs, const Flat& F) {
 // The scene constants of `F` with the device pointers and tree fields of `geom` and `shade`.
 SceneDev compose(const SceneDev& constants, const SceneDev& geom, const SceneDev& shade) {
     SceneDev S = constants;
-    S.nodes = geom.nodes; S.tris = geom.tris; S.blas = geom.blas;
+    S.nodes = geom.nodes; S.tris = geom.tris; S.blas = geom.blas; S.leaf_boxes = geom.leaf_boxes;
     S.positions = geom.positions; S.normals = geom.normals; S.tri_index = geom.tri_index;
-    S.tlas_root = geom.tlas_root; S.stack_need = geom.stack_need;
+    S.tlas_root = geom.tlas_root; S.single_blas = geom.single_blas; S.stack_need = geom.stack_need;
     S.instances = shade.instances; S.materials = shade.materials; S.bsdfs = shade.bsdfs; S.plate = shade.plate;
     S.exempt_boxes = shade.exempt_boxes;
     S.energy = g_energy;
@@ -904,9 +905,11 @@ uint32_t rtg_scene_update(uint32_t handle, const uint8_t* bytes, uint32_t len) {
     }
     if (same_geometry) {
         geom.tlas_root = sc->S.tlas_root;
+        geom.single_blas = sc->S.single_blas;
         geom.stack_need = sc->S.stack_need;
     } else {
         geom.tlas_root = F.scene.tlas_root;
+        geom.single_blas = F.scene.single_blas;
         geom.stack_need = F.scene.stack_need;
         set_sort_box(*sc, F);
         sc->hot_bytes = hot;

@@ -116,7 +116,7 @@ __device__ __forceinline__ void add_clamped(float4& sum, Rgb c, bool indirect, f
 // ---- camera generation ---------------------------------------------------------------------------
 // BATCH: the slots belong to the jobs of a batched wave, each with its own camera.
 template <bool BATCH>
-__global__ void k_camera(SceneDev S, WaveDesc w, PathBuffers P) {
+__global__ void k_camera(const __grid_constant__ SceneDev S, WaveDesc w, PathBuffers P) {
     for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < w.n; slot += gridDim.x * blockDim.x) {
         uint32_t x, y, index;
         V3 o, d;
@@ -237,7 +237,7 @@ __global__ void k_key_scatter(const uint32_t* __restrict__ list, const uint32_t*
 // (one atomic per warp on counters[4]) while the rest of the warp keeps traversing, so no lane idles
 // until the slowest ray of its warp is done.
 // `order`: the active queue in the order to trace it (P.queue[cur], or its ray-sorted copy).
-__global__ void RTG_TRACE_BOUNDS k_extend(SceneDev S, PathBuffers P, int cur, const uint32_t* __restrict__ order) {
+__global__ void RTG_TRACE_BOUNDS k_extend(const __grid_constant__ SceneDev S, PathBuffers P, int cur, const uint32_t* __restrict__ order) {
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
     uint64_t deep[STACK_CAP - SHORT_STACK];
     SplitStack stack{s_stack + threadIdx.x, deep, TRACE_THREADS};
@@ -276,7 +276,12 @@ __global__ void RTG_TRACE_BOUNDS k_extend(SceneDev S, PathBuffers P, int cur, co
         }
         if (busy) {
             bool got = false;
-            if (trav_step<false>(S, T, stack, &err, got)) {
+            const auto src = [&](V3& ro, V3& rd) {
+                const float4 o = P.o[slot], d = P.d[slot];
+                ro = v3(o.x, o.y, o.z);
+                rd = v3(d.x, d.y, d.z);
+            };
+            if (trav_step<false, true>(S, T, 1.0e-3f, stack, &err, got, src)) {
                 busy = false;
                 P.hit[slot] = got ? make_uint4(T.best_i, T.best_tri, __float_as_uint(T.best_t), 1u)
                                   : make_uint4(0xffffffffu, 0xffffffffu, 0u, 0u);
@@ -575,7 +580,7 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
 // frame: 369 -> 383 Mpaths/s; 5, 6 and 7 blocks measured 367, 379 and 372).
 // `order`: the active queue in the order to shade it (material-sorted, or as traced).
 template <bool BATCH>
-__global__ void __launch_bounds__(128, RTG_SHADE_MIN_BLOCKS) k_shade(SceneDev S, const LightsDev* __restrict__ Lg, PathBuffers P, int cur, WaveDesc w,
+__global__ void __launch_bounds__(128, RTG_SHADE_MIN_BLOCKS) k_shade(const __grid_constant__ SceneDev S, const LightsDev* __restrict__ Lg, PathBuffers P, int cur, WaveDesc w,
                                                   const uint32_t* __restrict__ order, RaySort R) {
     uint32_t n = *(volatile uint32_t*)&P.counters[cur];
     uint32_t rays_local = 0, shadow_local = 0;
@@ -610,7 +615,7 @@ __device__ __forceinline__ void shadow_unblocked(const PathBuffers& P, uint32_t 
 }
 
 // `perm` (may be null): the shadow queue in the order to trace it.
-__global__ void RTG_TRACE_BOUNDS k_shadow(SceneDev S, PathBuffers P, const uint32_t* __restrict__ perm) {
+__global__ void RTG_TRACE_BOUNDS k_shadow(const __grid_constant__ SceneDev S, PathBuffers P, const uint32_t* __restrict__ perm) {
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
     uint64_t deep[STACK_CAP - SHORT_STACK];
     SplitStack stack{s_stack + threadIdx.x, deep, TRACE_THREADS};
@@ -643,7 +648,12 @@ __global__ void RTG_TRACE_BOUNDS k_shadow(SceneDev S, PathBuffers P, const uint3
         }
         if (busy) {
             bool blocked = false;
-            if (trav_step<true>(S, T, stack, &err, blocked)) {
+            const auto src = [&](V3& ro, V3& rd) {
+                const float4 o = P.sh_o[ray], d = P.sh_d[ray];
+                ro = v3(o.x, o.y, o.z);
+                rd = v3(d.x, d.y, d.z);
+            };
+            if (trav_step<true, true>(S, T, 1.0e-3f, stack, &err, blocked, src)) {
                 busy = false;
                 if (!blocked) shadow_unblocked(P, ray);
             }
@@ -657,7 +667,7 @@ __global__ void RTG_TRACE_BOUNDS k_shadow(SceneDev S, PathBuffers P, const uint3
 // plane, the studio on the removed side), so the lane refill of the plain kernels does not apply.
 // Launched instead of them for a scene with a section; they write the same records (a cap is a hit
 // with triangle CAP_TRIANGLE).
-__global__ void __launch_bounds__(TRACE_THREADS) k_extend_section(SceneDev S, PathBuffers P, int cur, const uint32_t* __restrict__ order) {
+__global__ void __launch_bounds__(TRACE_THREADS) k_extend_section(const __grid_constant__ SceneDev S, PathBuffers P, int cur, const uint32_t* __restrict__ order) {
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
     uint64_t deep[STACK_CAP - SHORT_STACK];
     SplitStack stack{s_stack + threadIdx.x, deep, TRACE_THREADS};
@@ -678,7 +688,7 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_extend_section(SceneDev S, Pa
     if (err) atomicOr(&P.counters[3], err);
 }
 
-__global__ void __launch_bounds__(TRACE_THREADS) k_shadow_section(SceneDev S, PathBuffers P, const uint32_t* __restrict__ perm) {
+__global__ void __launch_bounds__(TRACE_THREADS) k_shadow_section(const __grid_constant__ SceneDev S, PathBuffers P, const uint32_t* __restrict__ perm) {
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
     uint64_t deep[STACK_CAP - SHORT_STACK];
     SplitStack stack{s_stack + threadIdx.x, deep, TRACE_THREADS};
@@ -699,7 +709,7 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_shadow_section(SceneDev S, Pa
 // behind it, up to 32 crossings; any other surface blocks it. One thread per ray: only scenes with
 // passable instances run it, instead of k_shadow. BATCH: each ray's job gives its materials.
 template <bool BATCH>
-__global__ void __launch_bounds__(TRACE_THREADS) k_shadow_walk(SceneDev S, PathBuffers P, WaveDesc w, const uint32_t* __restrict__ perm) {
+__global__ void __launch_bounds__(TRACE_THREADS) k_shadow_walk(const __grid_constant__ SceneDev S, PathBuffers P, WaveDesc w, const uint32_t* __restrict__ perm) {
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
     uint64_t deep[STACK_CAP - SHORT_STACK];
     SplitStack stack{s_stack + threadIdx.x, deep, TRACE_THREADS};
@@ -763,7 +773,7 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_shadow_walk(SceneDev S, PathB
 // of a chain of launches, each as long as its slowest ray. k_tail_end then empties the queue, so
 // the later rounds' launches find no work. Scenes with passable surfaces (shadow walks) and
 // batched waves keep the wavefront.
-__global__ void __launch_bounds__(TRACE_THREADS) k_tail(SceneDev S, const LightsDev* __restrict__ Lg, PathBuffers P, int cur, WaveDesc w, uint32_t rounds_left,
+__global__ void __launch_bounds__(TRACE_THREADS) k_tail(const __grid_constant__ SceneDev S, const LightsDev* __restrict__ Lg, PathBuffers P, int cur, WaveDesc w, uint32_t rounds_left,
                                         uint32_t limit) {
     const uint32_t n = *(volatile uint32_t*)&P.counters[cur];
     if (n == 0 || n > limit) return;
@@ -780,7 +790,7 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_tail(SceneDev S, const Lights
             const uint32_t pf = P.flags[slot];
             TraceResult res;
             const bool got = !(pf & PF_NOTHING) &&
-                             traverse<false>(S, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 1.0e-3f, f_inf(), (pf & PF_PRIMARY) != 0, res, &err, stack);
+                             traverse<false, true>(S, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 1.0e-3f, f_inf(), (pf & PF_PRIMARY) != 0, res, &err, stack);
             P.hit[slot] = got ? make_uint4(res.inst, res.tri, __float_as_uint(res.t), 1u) : make_uint4(0xffffffffu, 0xffffffffu, 0u, 0u);
             TailShadow sh;
             sh.on = false;
@@ -788,7 +798,7 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_tail(SceneDev S, const Lights
                                           rays_local, shadow_local, &sh);
             if (sh.on) {
                 TraceResult unused;
-                if (!traverse<true>(S, v3(sh.o.x, sh.o.y, sh.o.z), v3(sh.d.x, sh.d.y, sh.d.z), 1.0e-3f, sh.o.w, false, unused, &err, stack)) {
+                if (!traverse<true, true>(S, v3(sh.o.x, sh.o.y, sh.o.z), v3(sh.d.x, sh.d.y, sh.d.z), 1.0e-3f, sh.o.w, false, unused, &err, stack)) {
                     float4 sum = P.sum[slot];  // shadow_unblocked's addition
                     sum.x = sum.x + sh.c.x;
                     sum.y = sum.y + sh.c.y;
@@ -895,7 +905,7 @@ __global__ void k_accumulate_edges(WaveDesc w, PathBuffers P, FilmDev F) {
 // What the centre ray of a pixel meets first (render.rs:503 centre_ray, integrator/mod.rs:911
 // first_hit, passes.rs:168 Exact::of): x = part (instance + 1, 0xffffffff the floor, 0 the
 // background), y = material (+ 1, the same codes), z = depth along the view axis (bits).
-__global__ void __launch_bounds__(TRACE_THREADS) k_edge_exact(SceneDev S, const LightsDev* __restrict__ Lg, uint4* exact) {
+__global__ void __launch_bounds__(TRACE_THREADS) k_edge_exact(const __grid_constant__ SceneDev S, const LightsDev* __restrict__ Lg, uint4* exact) {
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
     uint64_t deep[STACK_CAP - SHORT_STACK];
     SplitStack stack{s_stack + threadIdx.x, deep, TRACE_THREADS};
@@ -949,7 +959,7 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_edge_exact(SceneDev S, const 
 // albedo (passes.rs:209: the material's base colour, the default material's for an index out of
 // range, the floor's colour, black for the background).
 // `sees`: false for a panoramic camera's ray that sees nothing (an empty interval: the background).
-__device__ void first_hit_passes(const SceneDev& S, const LightsDev& L, V3 o, V3 d, bool sees, SplitStack& stack, uint32_t* err, uint4& e,
+static __device__ __noinline__ void first_hit_passes(const SceneDev& S, const LightsDev& L, V3 o, V3 d, bool sees, SplitStack& stack, uint32_t* err, uint4& e,
                                  V3& normal, Rgb& albedo) {
     TraceResult res;
     const bool got = sees && trace_q<false>(S, o, d, 1.0e-3f, f_inf(), true, res, err, stack);
@@ -991,7 +1001,7 @@ __device__ void first_hit_passes(const SceneDev& S, const LightsDev& L, V3 o, V3
 __device__ __forceinline__ bool first_hit_covers(uint4 e) { return e.x != 0u && e.x != 0xffffffffu; }
 
 // The exact passes of the centre rays of a rectangle (render.rs:529), background outside the image.
-__global__ void __launch_bounds__(TRACE_THREADS) k_exact_passes(SceneDev S, const LightsDev* __restrict__ Lg, uint32_t x0, uint32_t y0,
+__global__ void __launch_bounds__(TRACE_THREADS) k_exact_passes(const __grid_constant__ SceneDev S, const LightsDev* __restrict__ Lg, uint32_t x0, uint32_t y0,
                                                                  uint32_t w, uint32_t h, float* normal, float* depth, uint32_t* part,
                                                                  uint32_t* material) {
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
@@ -1024,7 +1034,7 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_exact_passes(SceneDev S, cons
 // an edge pixel (`edge`, the image's mask, may be null) adds the mean of its k sub-samples. With
 // `alpha` (may be null) the coverage of the same first hits is added likewise (passes.rs:221
 // coverage_of: 1 for a surface of an instance, 0 for the floor, a light panel or the background).
-__global__ void __launch_bounds__(TRACE_THREADS) k_albedo_pass(SceneDev S, const LightsDev* __restrict__ Lg, const uint8_t* __restrict__ edge,
+__global__ void __launch_bounds__(TRACE_THREADS) k_albedo_pass(const __grid_constant__ SceneDev S, const LightsDev* __restrict__ Lg, const uint8_t* __restrict__ edge,
                                                                 uint32_t x0, uint32_t y0, uint32_t w, uint32_t h, uint32_t first,
                                                                 uint32_t count, float* sum, float* weight, float* alpha) {
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
@@ -1077,7 +1087,7 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_albedo_pass(SceneDev S, const
 // The albedo of each camera ray's first hit from the wave's first extend (the ray in P.o / P.d,
 // the hit in P.hit): first_hit_passes without its traversal, which the extend has done with the
 // same ray, class and interval.
-__global__ void k_albedo_hits(SceneDev S, const LightsDev* __restrict__ Lg, WaveDesc w, PathBuffers P) {
+__global__ void k_albedo_hits(const __grid_constant__ SceneDev S, const LightsDev* __restrict__ Lg, WaveDesc w, PathBuffers P) {
     const LightsDev& L = *Lg;
     for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < w.n; slot += gridDim.x * blockDim.x) {
         const float4 of = P.o[slot], df = P.d[slot];
@@ -1167,7 +1177,7 @@ __global__ void k_accumulate_albedo(WaveDesc w, FilmDev F) {
 
 // A pixel is an edge when a neighbour inside the image sees another part, another material, or
 // a depth more than 2 % away (two background pixels never differ).
-__global__ void k_edge_mask(SceneDev S, const uint4* __restrict__ exact, uint8_t* mask) {
+__global__ void k_edge_mask(const __grid_constant__ SceneDev S, const uint4* __restrict__ exact, uint8_t* mask) {
     const uint32_t w = S.width, h = S.height, n = w * h;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
         const uint32_t x = p % w, y = p / w;
@@ -1236,7 +1246,7 @@ __global__ void k_film_encode(FilmDev F, float gain, uint32_t kind, AgxMatrices 
 }
 
 // ---- ray batches for the traversal parity harness ---------------------------------------------------
-__global__ void __launch_bounds__(TRACE_THREADS) k_trace_batch(SceneDev S, const float* __restrict__ rays, uint32_t n, uint32_t mode, uint32_t* out,
+__global__ void __launch_bounds__(TRACE_THREADS) k_trace_batch(const __grid_constant__ SceneDev S, const float* __restrict__ rays, uint32_t n, uint32_t mode, uint32_t* out,
                                                      uint32_t* counters) {
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
     uint64_t deep[STACK_CAP - SHORT_STACK];

@@ -467,123 +467,155 @@ struct SahBuilder {
     }
 };
 
-// ---- 8-wide collapse (bvh.rs:439) and quantisation -------------------------------------------------
-// The decoded lower/upper plane of a child, with the kernels' operations.
-inline float decode(float p, uint32_t q, float scale) { return p + (float)q * scale; }
-
+// ---- 8-wide collapse and quantisation ---------------------------------------------------------------
+// The binary tree's leaves are the wide tree's; which of its inner nodes become wide nodes is chosen
+// for the smallest total surface area of the wide nodes, the expected number of node steps of a ray
+// (the dynamic program of Ylitie, Karras and Laine, "Efficient Incoherent Ray Traversal on GPUs
+// Through Compressed Wide BVHs", HPG 2017, section 3). The greedy widest-child collapse left 60% of
+// the product scene's nodes with two children.
 struct Flattener {
     Flat& F;
     const std::vector<BNode>* bn = nullptr;
     const std::vector<uint32_t>* order = nullptr;
-    // emit(prims) -> leaf reference
-    std::function<uint32_t(const uint32_t*, uint32_t)> emit;
+    // Appends a leaf's primitives: the index of the first.
+    std::function<uint32_t(const uint32_t*, uint32_t, const Box&)> emit;
     uint32_t max_depth = 0;
-    // The top level: a child box that is flat on an axis but not at its node's lower corner
-    // there (a floor under instances whose rotated boxes reach below it) is wrapped into a node
-    // of its own, whose origin is the box itself, so that it decodes to the exact plane and the
-    // slab test drops the hits just before t_min as the reference's tree does.
-    bool exact_flat = false;
-    bool wrapped = false;
+    uint32_t dummy = 0;  // what the empty slots of a node without leaves lead to
+    // Always open the child with the largest box instead: a shallower tree where the least area goes
+    // too deep for the traversal stack.
+    bool widest = false;
+    struct Choice {
+        float cost[7];     // [i - 1]: least cost of the subtree as at most i subtrees
+        uint8_t split[8];  // [i - 1]: subtrees the left child gets of i (0: the choice of i - 1)
+    };
+    std::vector<Choice> choice;
 
-    void quantise(QNode& q, const Box* kids, int nk) {
+    void choose() {
+        const std::vector<BNode>& B = *bn;
+        choice.assign(B.size(), Choice());  // a binary leaf costs no node step, whatever its share
+        for (size_t n = B.size(); n-- > 0;) {  // children come after their parents
+            if (B[n].count > 0) continue;
+            const Choice &l = choice[B[n].left], &r = choice[B[n].right];
+            Choice& c = choice[n];
+            auto distribute = [&](int j, uint8_t& split) {
+                float best = f_inf();
+                split = 1;
+                for (int k = 1; k < j; ++k) {
+                    if (k > 7 || j - k > 7) continue;
+                    const float cost = l.cost[k - 1] + r.cost[j - k - 1];
+                    if (cost < best) { best = cost; split = (uint8_t)k; }
+                }
+                return best;
+            };
+            c.cost[0] = B[n].box.area() + distribute(8, c.split[7]);
+            c.split[0] = 0;
+            for (int i = 2; i <= 7; ++i) {
+                c.cost[i - 1] = distribute(i, c.split[i - 1]);
+                if (c.cost[i - 2] <= c.cost[i - 1]) { c.cost[i - 1] = c.cost[i - 2]; c.split[i - 1] = 0; }
+            }
+        }
+    }
+    // The roots of the subtrees that inner node n becomes with `slots` of them.
+    void gather(uint32_t n, int slots, uint32_t* kids, int& nk) {
+        const int left = choice[n].split[slots - 1];
+        const uint32_t child[2] = {(*bn)[n].left, (*bn)[n].right};
+        for (int s = 0; s < 2; ++s) {
+            int i = s == 0 ? left : slots - left;
+            if ((*bn)[child[s]].count > 0) { kids[nk++] = child[s]; continue; }
+            while (i > 1 && choice[child[s]].split[i - 1] == 0) --i;
+            if (i == 1) kids[nk++] = child[s];
+            else gather(child[s], i, kids, nk);
+        }
+    }
+
+    void open_widest(uint32_t n, uint32_t* kids, int& nk) {
+        kids[0] = (*bn)[n].left;
+        kids[1] = (*bn)[n].right;
+        for (nk = 2; nk < 8; ++nk) {
+            int at = -1;
+            for (int s = 0; s < nk; ++s)
+                if ((*bn)[kids[s]].count == 0 && (at < 0 || (*bn)[kids[s]].box.area() > (*bn)[kids[at]].box.area())) at = s;
+            if (at < 0) break;
+            kids[nk] = (*bn)[kids[at]].right;
+            kids[at] = (*bn)[kids[at]].left;
+        }
+    }
+
+    static void quantise(QNode& q, const Box* kids, int nk) {
         Box nb;
         for (int k = 0; k < nk; ++k) nb = nb.uni(kids[k]);
-        float p[3] = {nb.lo.x, nb.lo.y, nb.lo.z};
-        q.px = p[0]; q.py = p[1]; q.pz = p[2];
-        uint8_t* es[3] = {&q.ex, &q.ey, &q.ez};
         for (int a = 0; a < 3; ++a) {
-            float extent = comp(nb.hi, a) - p[a];
+            const float p = comp(nb.lo, a);
+            q.p[a] = p;
+            const float extent = comp(nb.hi, a) - p;
             int e = 1;  // biased exponent, 2^(e-127); at least the smallest normal
             if (extent > 0.0f) {
                 int ex;
                 std::frexp((double)extent / 255.0, &ex);  // extent/255 < 2^ex
-                e = ex + 127;
-                if (e < 1) e = 1;
+                e = std::max(1, ex + 127);
             }
             for (;; ++e) {
                 if (e > 254) e = 254;
-                float scale = bitsf((uint32_t)e << 23);
+                const double scale = std::ldexp(1.0, e - 127);
                 bool ok = true;
                 uint8_t lo[8], hi[8];
                 for (int k = 0; k < nk && ok; ++k) {
-                    float clo = comp(kids[k].lo, a), chi = comp(kids[k].hi, a);
-                    double ql = std::floor(((double)clo - (double)p[a]) / (double)scale);
-                    double qh = std::ceil(((double)chi - (double)p[a]) / (double)scale);
-                    long a0 = (long)std::max(0.0, ql), a1 = (long)std::min(255.0, std::max(0.0, qh));
-                    while (a0 > 0 && decode(p[a], (uint32_t)a0, scale) > clo) --a0;
-                    while (a1 < 255 && decode(p[a], (uint32_t)a1, scale) < chi) ++a1;
-                    if (decode(p[a], (uint32_t)a0, scale) > clo || decode(p[a], (uint32_t)a1, scale) < chi) ok = false;
-                    lo[k] = (uint8_t)a0;
-                    hi[k] = (uint8_t)a1;
+                    const double clo = (double)comp(kids[k].lo, a) - (double)p, chi = (double)comp(kids[k].hi, a) - (double)p;
+                    const double l = std::floor(clo / scale), h = std::ceil(chi / scale);
+                    ok = l >= 0.0 && h <= 255.0;
+                    lo[k] = (uint8_t)(ok ? l : 0.0);
+                    hi[k] = (uint8_t)(ok ? h : 0.0);
                 }
                 if (ok || e == 254) {
-                    *es[a] = (uint8_t)e;
+                    q.scale[a] = e + 15 <= 254 ? bitsf((uint32_t)(e + 15) << 23) : f_inf();  // inf: the axis culls nothing
                     for (int k = 0; k < 8; ++k) {
-                        q.qlo[a][k] = k < nk ? lo[k] : 255;
-                        q.qhi[a][k] = k < nk ? hi[k] : 0;
+                        q.qlo[a][k] = k < nk ? (ok ? lo[k] : 0) : 255;
+                        q.qhi[a][k] = k < nk ? (ok ? hi[k] : 255) : 0;
                     }
                     break;
                 }
             }
         }
-        q.nchild = (uint8_t)nk;
     }
-    // Reference of the subtree replacing binary node b (Collapser::reference).
-    uint32_t reference(uint32_t b, uint32_t depth) {
-        const BNode& node = (*bn)[b];
-        if (node.count > 0) return emit(order->data() + node.first, node.count);
-        if (depth + 1 > max_depth) max_depth = depth + 1;
-        uint32_t index = (uint32_t)F.nodes.size();
+    // Emits the tree under binary node 0: the reference of its root.
+    uint32_t flatten() {
+        max_depth = 0;
+        if ((*bn)[0].count > 0) return make_leaf(emit(order->data() + (*bn)[0].first, (*bn)[0].count, (*bn)[0].box));
+        if (!widest) choose();
+        const uint32_t root = (uint32_t)F.nodes.size();
         F.nodes.push_back(QNode());
-        uint32_t kids[8] = {};
-        kids[0] = node.left;
-        kids[1] = node.right;
-        int n = 2;
-        while (n < 8) {
-            int widest = -1;
-            float warea = 0;
-            for (int s = 0; s < n; ++s) {
-                const BNode& k = (*bn)[kids[s]];
-                if (k.count == 0) {
-                    float a = k.box.area();
-                    if (widest < 0 || a > warea) { widest = s; warea = a; }
-                }
-            }
-            if (widest < 0) break;
-            BNode opened = (*bn)[kids[widest]];
-            for (int s = n - 1; s >= widest + 1; --s) kids[s + 1] = kids[s];
-            kids[widest] = opened.left;
-            kids[widest + 1] = opened.right;
-            ++n;
-        }
+        node(0, root, 1);
+        return root;
+    }
+    // Emits inner binary node b as wide node `index`: its inner children side by side, its leaves'
+    // primitives side by side.
+    void node(uint32_t b, uint32_t index, uint32_t depth) {
+        max_depth = std::max(max_depth, depth);
+        uint32_t kids[8];
+        int nk = 0;
+        if (widest) open_widest(b, kids, nk);
+        else gather(b, 8, kids, nk);
+        std::stable_partition(kids, kids + nk, [&](uint32_t k) { return (*bn)[k].count == 0; });
         Box boxes[8];
-        for (int s = 0; s < n; ++s) boxes[s] = (*bn)[kids[s]].box;
-        uint32_t refs[8];
-        for (int s = 0; s < n; ++s) refs[s] = reference(kids[s], depth + 1);
-        if (exact_flat) {
-            Box nb;
-            for (int s = 0; s < n; ++s) nb = nb.uni(boxes[s]);
-            for (int s = 0; s < n; ++s)
-                for (int a = 0; a < 3; ++a) {
-                    const float lo = comp(boxes[s].lo, a);
-                    if (lo != comp(boxes[s].hi, a) || lo == comp(nb.lo, a)) continue;
-                    QNode qw;
-                    std::memset(&qw, 0, sizeof(qw));
-                    quantise(qw, &boxes[s], 1);
-                    qw.child[0] = refs[s];
-                    for (int k = 1; k < 8; ++k) qw.child[k] = NODE_EMPTY;
-                    refs[s] = (uint32_t)F.nodes.size();
-                    F.nodes.push_back(qw);
-                    wrapped = true;
-                    break;
-                }
-        }
+        for (int s = 0; s < nk; ++s) boxes[s] = (*bn)[kids[s]].box;
         QNode q;
         std::memset(&q, 0, sizeof(q));
-        quantise(q, boxes, n);
-        for (int s = 0; s < 8; ++s) q.child[s] = s < n ? refs[s] : NODE_EMPTY;
+        quantise(q, boxes, nk);
+        q.node_base = (uint32_t)F.nodes.size();
+        q.leaf_base = dummy;
+        for (int s = 0; s < nk; ++s) {
+            const BNode& k = (*bn)[kids[s]];
+            if (k.count == 0) {
+                q.off[q.inner++] = (uint8_t)s;
+                continue;
+            }
+            const uint32_t first = emit(order->data() + k.first, k.count, k.box);
+            if (s == (int)q.inner) q.leaf_base = first;
+            q.off[s] = (uint8_t)(first - q.leaf_base);
+        }
+        F.nodes.resize(F.nodes.size() + q.inner);
         F.nodes[index] = q;
-        return index;
+        for (uint32_t s = 0; s < q.inner; ++s) node(kids[s], q.node_base + s, depth + 1);
     }
 };
 }  // namespace
@@ -927,7 +959,7 @@ std::string geometry_key(const HScene& s) {
     return k;
 }
 
-bool flatten_scene(const HScene& s, Flat& F, std::string& error, bool geometry) {
+static bool flatten(const HScene& s, Flat& F, std::string& error, bool geometry, bool widest) {
     auto t0 = std::chrono::steady_clock::now();
     F = Flat();
     const size_t ni = s.instances.size();
@@ -1059,9 +1091,44 @@ bool flatten_scene(const HScene& s, Flat& F, std::string& error, bool geometry) 
         // nearest hit does not depend on the tree, so they can share one), one object-space tree per
         // mesh used by a transformed instance.
         Flattener fl{F};
+        fl.widest = widest;
         uint32_t blas_depth = 0;
-        std::vector<BlasInst> tlas_leaves;
+        std::vector<BlasInst> placed;
         std::vector<Box> tlas_boxes;
+        // Triangle 0 has no area, so nothing hits it: where the empty slots of a node without
+        // leaves lead.
+        TriRec none;
+        std::memset(&none, 0, sizeof(none));
+        none.flags = TRI_LAST;
+        F.tris.push_back(none);
+        auto put_box = [](float* to, const Box& b) {
+            const float v[8] = {b.lo.x, b.lo.y, b.lo.z, 0.0f, b.hi.x, b.hi.y, b.hi.z, 0.0f};
+            std::memcpy(to, v, sizeof(v));
+        };
+        F.leaf_boxes.assign(8, 0.0f);
+        // Appends the leaf of the triangles `p` as record(p) gives them.
+        auto emit_leaf = [&](const uint32_t* p, uint32_t n, const Box& box, auto&& record) {
+            const uint32_t first = (uint32_t)F.tris.size(), leaf = (uint32_t)(F.leaf_boxes.size() / 8);
+            F.leaf_boxes.resize(F.leaf_boxes.size() + 8);
+            put_box(&F.leaf_boxes[8 * (size_t)leaf], box);
+            for (uint32_t k = 0; k < n; ++k) {
+                TriRec r = record(p[k]);
+                r.flags |= (leaf << TRI_LEAF_SHIFT) | (k + 1 == n ? TRI_LAST : 0u);
+                F.tris.push_back(r);
+            }
+            return first;
+        };
+        auto triangle = [](const HMesh& M, uint32_t t, uint32_t inst, uint32_t flags) {
+            TriRec r;
+            const V3& a = M.positions[M.indices[3 * t]];
+            const V3& b = M.positions[M.indices[3 * t + 1]];
+            const V3& c = M.positions[M.indices[3 * t + 2]];
+            r.v0[0] = a.x; r.v0[1] = a.y; r.v0[2] = a.z; r.tri = t;
+            r.v1[0] = b.x; r.v1[1] = b.y; r.v1[2] = b.z; r.inst = inst;
+            r.v2[0] = c.x; r.v2[1] = c.y; r.v2[2] = c.z; r.flags = flags;
+            return r;
+        };
+        auto seen = [&](uint32_t i) { return (s.instances[i].flags & 1u) | ((s.instances[i].flags & 4u) ? 2u : 0u); };
         {
             std::vector<std::pair<uint32_t, uint32_t>> prims;  // (instance, triangle)
             for (size_t i = 0; i < ni; ++i)
@@ -1085,32 +1152,19 @@ bool flatten_scene(const HScene& s, Flat& F, std::string& error, bool geometry) 
                 sb.build(0, prims.size(), 0);
                 fl.bn = &sb.nodes;
                 fl.order = &sb.order;
-                fl.max_depth = 0;
-                fl.emit = [&](const uint32_t* p, uint32_t n) {
-                    uint32_t first = (uint32_t)F.tris.size();
-                    for (uint32_t k = 0; k < n; ++k) {
-                        uint32_t inst = prims[p[k]].first, t = prims[p[k]].second;
-                        const HMesh& M = s.meshes[s.instances[inst].mesh];
-                        TriRec r;
-                        const V3& a = M.positions[M.indices[3 * t]];
-                        const V3& b = M.positions[M.indices[3 * t + 1]];
-                        const V3& c = M.positions[M.indices[3 * t + 2]];
-                        r.v0[0] = a.x; r.v0[1] = a.y; r.v0[2] = a.z; r.tri = t;
-                        r.v1[0] = b.x; r.v1[1] = b.y; r.v1[2] = b.z; r.inst = inst;
-                        r.v2[0] = c.x; r.v2[1] = c.y; r.v2[2] = c.z;
-                        r.flags = (s.instances[inst].flags & 1u) | ((s.instances[inst].flags & 4u) ? 2u : 0u);
-                        F.tris.push_back(r);
-                    }
-                    return make_leaf(first, n);
+                fl.emit = [&](const uint32_t* p, uint32_t n, const Box& box) {
+                    return emit_leaf(p, n, box, [&](uint32_t k) {
+                        return triangle(s.meshes[s.instances[prims[k].first].mesh], prims[k].second, prims[k].first, seen(prims[k].first));
+                    });
                 };
-                uint32_t root = fl.reference(0, 0);
-                blas_depth = std::max(blas_depth, fl.max_depth);
                 BlasInst bi;
                 std::memset(&bi, 0, sizeof(bi));
-                bi.root = root;
+                bi.root = fl.flatten();
+                blas_depth = std::max(blas_depth, fl.max_depth);
                 bi.identity = 1;
                 bi.instance = 0xffffffffu;
-                tlas_leaves.push_back(bi);
+                put_box(bi.box, all);
+                placed.push_back(bi);
                 tlas_boxes.push_back(all);
             }
         }
@@ -1133,23 +1187,10 @@ bool flatten_scene(const HScene& s, Flat& F, std::string& error, bool geometry) 
                 sb.build(0, n, 0);
                 fl.bn = &sb.nodes;
                 fl.order = &sb.order;
-                fl.max_depth = 0;
-                fl.emit = [&](const uint32_t* p, uint32_t cnt) {
-                    uint32_t first = (uint32_t)F.tris.size();
-                    for (uint32_t k = 0; k < cnt; ++k) {
-                        uint32_t t = p[k];
-                        TriRec r;
-                        const V3& a = M.positions[M.indices[3 * t]];
-                        const V3& b = M.positions[M.indices[3 * t + 1]];
-                        const V3& c = M.positions[M.indices[3 * t + 2]];
-                        r.v0[0] = a.x; r.v0[1] = a.y; r.v0[2] = a.z; r.tri = t;
-                        r.v1[0] = b.x; r.v1[1] = b.y; r.v1[2] = b.z; r.inst = 0xffffffffu;
-                        r.v2[0] = c.x; r.v2[1] = c.y; r.v2[2] = c.z; r.flags = 0;
-                        F.tris.push_back(r);
-                    }
-                    return make_leaf(first, cnt);
+                fl.emit = [&](const uint32_t* p, uint32_t cnt, const Box& box) {
+                    return emit_leaf(p, cnt, box, [&](uint32_t t) { return triangle(M, t, 0xffffffffu, 0u); });
                 };
-                mesh_root[m] = fl.reference(0, 0);
+                mesh_root[m] = fl.flatten();
                 blas_depth = std::max(blas_depth, fl.max_depth);
             }
             BlasInst bi;
@@ -1158,14 +1199,19 @@ bool flatten_scene(const HScene& s, Flat& F, std::string& error, bool geometry) 
             bi.root = mesh_root[m];
             bi.identity = 0;
             bi.instance = (uint32_t)i;
-            bi.flags = (s.instances[i].flags & 1u) | ((s.instances[i].flags & 4u) ? 2u : 0u);
-            tlas_leaves.push_back(bi);
-            tlas_boxes.push_back(instance_box(s.meshes[m], xf[i]));
+            bi.flags = seen((uint32_t)i);
+            const Box world = instance_box(s.meshes[m], xf[i]);
+            put_box(bi.box, world);
+            placed.push_back(bi);
+            tlas_boxes.push_back(world);
         }
-        // Top level over the placed trees (one per leaf).
-        F.blas = tlas_leaves;
+        // Top level over the placed trees (one per leaf), or just the one world-space tree.
         uint32_t tlas_depth = 0;
-        if (!tlas_leaves.empty()) {
+        if (placed.size() == 1 && placed[0].identity) {
+            F.blas = placed;
+            F.tlas_root = placed[0].root;
+            F.single_blas = 0;
+        } else if (!placed.empty()) {
             std::vector<V3> cents(tlas_boxes.size());
             for (size_t k = 0; k < cents.size(); ++k) cents[k] = tlas_boxes[k].centroid();
             SahBuilder sb{tlas_boxes, cents, 1, 1, {}, {}};
@@ -1174,15 +1220,15 @@ bool flatten_scene(const HScene& s, Flat& F, std::string& error, bool geometry) 
             sb.build(0, tlas_boxes.size(), 0);
             fl.bn = &sb.nodes;
             fl.order = &sb.order;
-            fl.max_depth = 0;
-            fl.emit = [&](const uint32_t* p, uint32_t) { return make_leaf(p[0], 1); };
-            fl.exact_flat = true;
-            fl.wrapped = false;
-            F.tlas_root = fl.reference(0, 0);
-            fl.exact_flat = false;
-            tlas_depth = fl.max_depth + (fl.wrapped ? 1 : 0);  // a wrapper adds one level
+            fl.emit = [&](const uint32_t* p, uint32_t, const Box&) {
+                F.blas.push_back(placed[p[0]]);
+                return (uint32_t)F.blas.size() - 1;
+            };
+            F.tlas_root = fl.flatten();
+            tlas_depth = fl.max_depth;
         }
         F.stack_need = 7 * (tlas_depth + blas_depth) + 2;
+        if (F.stack_need > 96 && !widest) return flatten(s, F, error, geometry, true);
         if (F.stack_need > 96) { error = "unsupported: BVH too deep for the traversal stack"; return false; }
         if (F.tris.size() >= (1u << 27) - 16) { error = "unsupported: more than 2^27 triangles"; return false; }
     }
@@ -1278,11 +1324,14 @@ bool flatten_scene(const HScene& s, Flat& F, std::string& error, bool geometry) 
     S.floor_z = s.floor_z;
     for (int c = 0; c < 3; ++c) S.floor_color[c] = s.floor_color[c];
     S.tlas_root = F.tlas_root;
+    S.single_blas = F.single_blas;
     S.n_instances = (uint32_t)ni;
     S.n_materials = (uint32_t)s.materials.size();
     S.stack_need = F.stack_need;
     F.build_seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     return true;
 }
+
+bool flatten_scene(const HScene& s, Flat& F, std::string& error, bool geometry) { return flatten(s, F, error, geometry, false); }
 
 }  // namespace rtg

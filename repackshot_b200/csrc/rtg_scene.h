@@ -142,6 +142,7 @@ struct Flat {
     std::vector<QNode> nodes;
     std::vector<TriRec> tris;
     std::vector<BlasInst> blas;
+    std::vector<float> leaf_boxes;  // 8 per leaf
     std::vector<DevInstance> instances;
     std::vector<float> positions, normals;  // 4 floats per vertex
     std::vector<uint32_t> tri_index;        // 4 per triangle
@@ -149,7 +150,7 @@ struct Flat {
     std::vector<Bsdf> bsdfs;  // 2 per material (entering, leaving), then the floor's
     LightsDev lights;
     SceneDev scene;  // pointers left null
-    uint32_t tlas_root = NODE_EMPTY;
+    uint32_t tlas_root = NODE_EMPTY, single_blas = 0xffffffffu;
     uint32_t stack_need = 0;
     float box_lo[3] = {0, 0, 0}, box_hi[3] = {0, 0, 0};  // the ray sort's box (empty: lo > hi)
     uint64_t instanced_triangles = 0;
