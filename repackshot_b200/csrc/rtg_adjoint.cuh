@@ -170,8 +170,7 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
     Sel from;
     from.p = v3(sel4.x, sel4.y, sel4.z);
     from.by_flux = !(L.per_point && L.n_entries > 0);
-    from.total = 0.0f;
-    if (has_pdf && !from.by_flux) from = select_at(L, from.p);
+    from.total = sel4.w;
     // crossed_from, light by light, in its order
     Rgb crossed = splat(0.0f);
     for (int i = 0; i < L.n_areas; ++i) {
@@ -261,20 +260,27 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
             }
         }
         V3 wo = to_local(fr, -rd);
+        if (wo.z <= 0.0f) break;  // below the surface the BSDF is zero and has no samples
         V3 ng = s_geom;
         V3 origin = offset_origin(s_point, ng);
         uint32_t dims = bounce_dim(bounce);
         uint64_t key = sample_key(S, x, y, index);
-        Sel selection = select_at(L, s_point);
+        const BsdfWo bo = bsdf_wo(S.energy, b, wo);
+        const LobeWeights lobe_w = lobe_weights(b, bo, wo);
+        float weights[SEL_KEPT];
+        Sel selection = select_at(L, s_point, weights);
         LightSample ls;
-        if (sample_light(L, selection, sample1(c_sobol, key, index, dims + OFF_LIGHT_SELECT), sample1(c_sobol, key, index, dims + OFF_LIGHT),
-                         sample1(c_sobol, key, index, dims + OFF_LIGHT + 1), ls)) {
+        if (sample_light(L, selection, weights, sample_at(S, c_sobol, key, index, dims + OFF_LIGHT_SELECT), sample_at(S, c_sobol, key, index, dims + OFF_LIGHT),
+                         sample_at(S, c_sobol, key, index, dims + OFF_LIGHT + 1), ls)) {
             V3 wi = to_local(fr, ls.wi);
             const LobesSel lobes = ls.glossy ? LOBES_ALL : LOBES_DIFFUSE;
-            Rgb f = bsdf_eval(S.energy, b, wo, wi, lobes);
+            const bool mis = ls.glossy && !ls.delta;
+            Rgb f;
+            float bsdf_density = 0.0f;
+            bsdf_eval_pdf(S.energy, b, bo, &lobe_w, wo, wi, lobes, f, mis ? &bsdf_density : nullptr);
             if (peak(f) > 0.0f) {
                 V3 from_p = wi.z < 0.0f ? offset_origin(s_hit, -ng) : origin;
-                float weight = (ls.delta || !ls.glossy) ? 1.0f : power_heuristic(ls.pdf, bsdf_pdf(S.energy, b, wo, wi));
+                float weight = mis ? power_heuristic(ls.pdf, bsdf_density) : 1.0f;
                 float kscale = absf(wi.z) * weight / ls.pdf;
                 Rgb c = thr * f * ls.radiance * kscale;
                 bool finite_c = finitef(c.r) && finitef(c.g) && finitef(c.b);
@@ -328,7 +334,7 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
             }
         }
         BsdfSample bs;
-        if (!bsdf_sample(S.energy, b, wo, sample1(c_sobol, key, index, dims + OFF_BSDF), sample1(c_sobol, key, index, dims + OFF_BSDF + 1), bs))
+        if (!bsdf_sample(S.energy, b, bo, lobe_w, wo, sample_at(S, c_sobol, key, index, dims + OFF_BSDF), sample_at(S, c_sobol, key, index, dims + OFF_BSDF + 1), bs))
             break;
         bool transmitted = bs.wi.z < 0.0f;
         V3 wi = bs.straight ? rd : normalize(to_world(fr, bs.wi));
@@ -340,7 +346,7 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
         thr = thr * bs.weight;
         if (bounce >= 2) {
             float survive = rclamp(peak(thr), 0.05f, 1.0f);
-            if (sample1(c_sobol, key, index, dims + OFF_ROULETTE) >= survive) break;
+            if (sample_at(S, c_sobol, key, index, dims + OFF_ROULETTE) >= survive) break;
             thr = thr / survive;
         }
         float pk = peak(thr);
@@ -349,7 +355,8 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
         // applied when the next vertex knows rem.
         if (mat && !bs.straight) {
             const uint32_t k = 2 * m + side;
-            Rgb f = bsdf_eval(S.energy, b, wo, bs.wi, LOBES_ALL);
+            Rgb f;
+            bsdf_eval_pdf(S.energy, b, bo, nullptr, wo, bs.wi, LOBES_ALL, f, nullptr);
             Rgb fa = rgb_sub(bsdf_eval(S.energy, A.albedo_plus[k], wo, bs.wi, LOBES_ALL), bsdf_eval(S.energy, A.albedo_minus[k], wo, bs.wi, LOBES_ALL)) *
                      A.inv_2h_albedo;
             Rgb fr2 = rgb_sub(bsdf_eval(S.energy, A.alpha_plus[k], wo, bs.wi, LOBES_ALL), bsdf_eval(S.energy, A.alpha_minus[k], wo, bs.wi, LOBES_ALL)) *
@@ -365,7 +372,7 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
             flags |= PF_HAS_PDF;
             flags &= ~PF_PRIMARY;
             pdf = bs.pdf;
-            P.sel[slot] = make_float4(s_point.x, s_point.y, s_point.z, 0.0f);
+            P.sel[slot] = make_float4(s_point.x, s_point.y, s_point.z, selection.total);
             offset = 0.0f;
             if (transmitted) {
                 if (s_outside && mat && mat->has_medium) {

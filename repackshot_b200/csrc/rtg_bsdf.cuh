@@ -78,14 +78,6 @@ RTG_HD float ggx_L(const Ggx& g, V3 w) {
     float x = g.ax * w.x, y = g.ay * w.y;
     return (sqrt_(1.0f + (x * x + y * y) / cos2) - 1.0f) * 0.5f;
 }
-RTG_HD float ggx_reflection_pdf(const Ggx& g, V3 wo, V3 h) {
-    float g1 = 1.0f / (1.0f + ggx_L(g, wo));
-    return g1 * ggx_D(g, h) / (4.0f * wo.z);
-}
-RTG_HD float ggx_microfacet(const Ggx& g, V3 wo, V3 wi, V3 h) {
-    float g2 = 1.0f / (1.0f + ggx_L(g, wo) + ggx_L(g, wi));
-    return ggx_D(g, h) * g2 / (4.0f * wo.z * wi.z);
-}
 RTG_HD float schlick(float f0, float f90, float cos) {
     float m = rclamp(1.0f - cos, 0.0f, 1.0f);
     float m2 = m * m;
@@ -134,24 +126,36 @@ RTG_HD void locate(float x, int n, int& i, float& w) {
     i = (int)(ti < (uint32_t)(n - 2) ? ti : (uint32_t)(n - 2));
     w = t - (float)i;
 }
-RTG_HD float tab(const uint16_t* t, int idx) {
+// Where a cosine or an alpha lies on its axis of the tables (both have 32 nodes at square roots):
+// the node below and the way to the next. A vertex finds its cosines' once, and a BSDF's alphas'
+// are found when it is built.
+static_assert(NODES_MU == NODES_ROUGHNESS, "one node count for both axes");
+struct TabAt { int i; float w; };
+RTG_HD TabAt tab_at(float x) {
+    TabAt t;
+    locate(sqrt_(rmax(x, 0.0f)), NODES_MU, t.i, t.w);
+    return t;
+}
+// The four u16 corners of a cell. On the device the tables are stored cell by cell (device_cells),
+// so that a lookup is one 8-byte load.
+RTG_HD void tab_cell(const uint16_t* t, int slice, int j, int i, float v[4]) {
 #ifdef __CUDA_ARCH__
-    return (float)__ldg(t + idx) * (1.0f / 65535.0f);
+    const ushort4 c = __ldg(reinterpret_cast<const ushort4*>(t) + (slice * NODES_ROUGHNESS + j) * NODES_MU + i);
+    const uint16_t q[4] = {c.x, c.y, c.z, c.w};
 #else
-    return (float)t[idx] * (1.0f / 65535.0f);
+    t += (slice * NODES_ROUGHNESS + j) * NODES_MU + i;
+    const uint16_t q[4] = {t[0], t[1], t[NODES_MU], t[NODES_MU + 1]};
 #endif
+    for (int k = 0; k < 4; ++k) v[k] = (float)q[k] * (1.0f / 65535.0f);
 }
-RTG_HD float table_lookup(const uint16_t* table, float mu, float alpha) {
-    int i, j;
-    float u, v;
-    locate(sqrt_(rmax(mu, 0.0f)), NODES_MU, i, u);
-    locate(sqrt_(rmax(alpha, 0.0f)), NODES_ROUGHNESS, j, v);
-    float a00 = tab(table, j * NODES_MU + i), a01 = tab(table, j * NODES_MU + i + 1);
-    float a10 = tab(table, (j + 1) * NODES_MU + i), a11 = tab(table, (j + 1) * NODES_MU + i + 1);
-    float low = a00 + (a01 - a00) * u;
-    float high = a10 + (a11 - a10) * u;
-    return low + (high - low) * v;
+RTG_HD float table_lookup(const uint16_t* table, int slice, TabAt mu, TabAt alpha) {
+    float v[4];
+    tab_cell(table, slice, alpha.i, mu.i, v);
+    float low = v[0] + (v[1] - v[0]) * mu.w;
+    float high = v[2] + (v[3] - v[2]) * mu.w;
+    return low + (high - low) * alpha.w;
 }
+RTG_HD float table_lookup(const uint16_t* table, float mu, float alpha) { return table_lookup(table, 0, tab_at(mu), tab_at(alpha)); }
 RTG_HD float avg_lookup(const float* t, float alpha) {
     int j; float v;
     locate(sqrt_(rmax(alpha, 0.0f)), NODES_ROUGHNESS, j, v);
@@ -162,28 +166,32 @@ RTG_HD float multiple_fresnel(float f_avg, float e_avg) {
     float d = 1.0f - f_avg * (1.0f - e_avg);
     return d > 0.0f ? f_avg * f_avg * e_avg / d : 0.0f;
 }
-RTG_HD float clear_albedo(const EnergyTables& E, float mu, float alpha, float eta) {
+RTG_HD float clear_albedo(const EnergyTables& E, TabAt mu, TabAt alpha, float eta) {
     const uint16_t* table = eta >= 1.0f ? E.clear_in : E.clear_out;
     float ior = eta >= 1.0f ? eta : 1.0f / eta;
     const float MAX_X = (3.0f - 1.0f) / (3.0f + 1.0f);
     float x = (ior - 1.0f) / (ior + 1.0f);
     int k; float w;
     locate(x / MAX_X, NODES_IOR, k, w);
-    const int slice = NODES_MU * NODES_ROUGHNESS;
-    float a = table_lookup(table + k * slice, mu, alpha);
-    float b = table_lookup(table + (k + 1) * slice, mu, alpha);
+    float a = table_lookup(table, k, mu, alpha);
+    float b = table_lookup(table, k + 1, mu, alpha);
     return a + (b - a) * w;
 }
 
 struct Layer {
     float f0, f90, strength, alpha, ms, norm;
     bool rough;
+    TabAt at;  // alpha's place in the tables
 };
-RTG_HD Layer layer_clear() { Layer l; l.f0 = 0; l.f90 = 0; l.strength = 0; l.alpha = 0; l.ms = 0; l.norm = 1.0f; l.rough = false; return l; }
+RTG_HD Layer layer_clear() {
+    Layer l;
+    l.f0 = 0; l.f90 = 0; l.strength = 0; l.alpha = 0; l.ms = 0; l.norm = 1.0f; l.rough = false; l.at = tab_at(0.0f);
+    return l;
+}
 RTG_HD Layer make_layer(const EnergyTables& E, float f0, float f90, float strength, float alpha, float ms) {
     if (strength != strength || strength <= 0.0f || (f90 <= 0.0f && f0 <= 0.0f)) return layer_clear();
     Layer l;
-    l.f0 = f0; l.f90 = f90; l.strength = strength; l.alpha = alpha; l.ms = ms;
+    l.f0 = f0; l.f90 = f90; l.strength = strength; l.alpha = alpha; l.ms = ms; l.at = tab_at(alpha);
     l.rough = alpha >= MIN_COMPENSATED_ALPHA;
     float avg;
     if (l.rough) {
@@ -196,11 +204,11 @@ RTG_HD Layer make_layer(const EnergyTables& E, float f0, float f90, float streng
     l.norm = 1.0f / (1.0f - rmin(avg, 0.999f));
     return l;
 }
-RTG_HD float layer_passes(const EnergyTables& E, const Layer& l, float mu) {
+RTG_HD float layer_passes(const EnergyTables& E, const Layer& l, float mu, TabAt at) {  // at: mu's place
     float e;
     if (l.rough) {
-        float ee = table_lookup(E.albedo, mu, l.alpha);
-        e = l.f0 * ee + (l.f90 - l.f0) * table_lookup(E.schlick, mu, l.alpha) + l.ms * (1.0f - ee);
+        float ee = table_lookup(E.albedo, 0, at, l.at);
+        e = l.f0 * ee + (l.f90 - l.f0) * table_lookup(E.schlick, 0, at, l.at) + l.ms * (1.0f - ee);
     } else {
         float m = rclamp(1.0f - mu, 0.0f, 1.0f);
         float m2 = m * m;
@@ -208,9 +216,9 @@ RTG_HD float layer_passes(const EnergyTables& E, const Layer& l, float mu) {
     }
     return 1.0f - rclamp(e * l.strength, 0.0f, 1.0f);
 }
-struct MsLobe { float alpha, norm, e_avg; bool on; };
+struct MsLobe { float alpha, norm, e_avg; bool on; TabAt at; };
 RTG_HD MsLobe make_lobe(const EnergyTables& E, float alpha) {
-    MsLobe l; l.on = false; l.alpha = 0; l.norm = 0; l.e_avg = 0;
+    MsLobe l; l.on = false; l.alpha = 0; l.norm = 0; l.e_avg = 0; l.at = tab_at(alpha);
     if (alpha != alpha || alpha < MIN_COMPENSATED_ALPHA) return l;
     float e_avg = avg_lookup(E.albedo_avg, alpha);
     float lost = 1.0f - e_avg;
@@ -218,7 +226,7 @@ RTG_HD MsLobe make_lobe(const EnergyTables& E, float alpha) {
     l.on = true; l.alpha = alpha; l.norm = FRAC_1_PI / lost; l.e_avg = e_avg;
     return l;
 }
-RTG_HD float lobe_lost(const EnergyTables& E, const MsLobe& l, float mu) { return rmax(1.0f - table_lookup(E.albedo, mu, l.alpha), 0.0f); }
+RTG_HD float lobe_lost(const EnergyTables& E, const MsLobe& l, TabAt mu) { return rmax(1.0f - table_lookup(E.albedo, 0, mu, l.at), 0.0f); }
 
 enum LobesSel { LOBES_ALL = 0, LOBES_DIFFUSE = 1 };
 struct BsdfSample { V3 wi; Rgb weight; float pdf; bool straight; };
@@ -235,7 +243,7 @@ struct Bsdf {
     bool thin;
     bool ms_spec_on; MsLobe ms_spec_lobe; Rgb ms_spec_colour;
     bool ms_coat_on; MsLobe ms_coat_lobe; float ms_coat_c;
-    bool ms_clear_on; float ms_clear_alpha;
+    bool ms_clear_on; float ms_clear_alpha; TabAt ms_clear_at;
     Layer base_layer, coat_layer;
     float diffuse_norm;
 };
@@ -248,7 +256,7 @@ RTG_HD float joint_norm(const EnergyTables& E, const Layer& below, const Layer& 
                            {0.40828268f, 0.18134189f},  {0.5917173f, 0.18134189f},  {0.7627662f, 0.15685332f},
                            {0.8983332f, 0.11119052f},   {0.9801449f, 0.05061427f}};
     float sum = 0.0f;
-    for (int i = 0; i < 8; ++i) sum = sum + G[i][1] * 2.0f * G[i][0] * layer_passes(E, below, G[i][0]) * layer_passes(E, above, G[i][0]);
+    for (int i = 0; i < 8; ++i) sum = sum + G[i][1] * 2.0f * G[i][0] * layer_passes(E, below, G[i][0], tab_at(G[i][0])) * layer_passes(E, above, G[i][0], tab_at(G[i][0]));
     return 1.0f / rmax(sum, 0.001f);
 }
 
@@ -263,7 +271,8 @@ RTG_HD Bsdf bsdf_lambert(Rgb a) {
     b.clear = 0.0f; b.eta = 1.0f; b.tint = splat(1.0f); b.thin = false;
     b.ms_spec_on = false; b.ms_coat_on = false; b.ms_clear_on = false;
     b.ms_spec_lobe.on = false; b.ms_coat_lobe.on = false;
-    b.ms_spec_colour = splat(0.0f); b.ms_coat_c = 0.0f; b.ms_clear_alpha = 0.0f;
+    b.ms_spec_colour = splat(0.0f); b.ms_coat_c = 0.0f; b.ms_clear_alpha = 0.0f; b.ms_clear_at = tab_at(0.0f);
+    b.ms_spec_lobe.at = b.ms_coat_lobe.at = tab_at(0.0f);
     b.base_layer = layer_clear(); b.coat_layer = layer_clear();
     b.diffuse_norm = 1.0f;
     return b;
@@ -301,7 +310,7 @@ RTG_HD Bsdf bsdf_surface(const EnergyTables& E, const DevMaterial& m, bool enter
     // multiple_scattering
     float alpha = b.spec.iso ? b.spec.ax : sqrt_(b.spec.ax * b.spec.ay);
     b.ms_spec_on = false; b.ms_coat_on = false; b.ms_clear_on = false;
-    b.ms_spec_colour = splat(0.0f); b.ms_coat_c = 0.0f; b.ms_clear_alpha = 0.0f;
+    b.ms_spec_colour = splat(0.0f); b.ms_coat_c = 0.0f; b.ms_clear_alpha = 0.0f; b.ms_clear_at = tab_at(alpha);
     b.ms_spec_lobe.on = false; b.ms_coat_lobe.on = false;
     MsLobe lobe = make_lobe(E, alpha);
     if (lobe.on && has_specular(b)) {
@@ -354,9 +363,9 @@ RTG_HD float reflect_probability(const Bsdf& b, float cos) { return rmin(clear_f
 RTG_HD float reflect_chance(const Bsdf& b, float mu_o, float cos_h) {
     return b.ms_clear_on ? clear_fresnel(b, cos_h) : reflect_probability(b, mu_o);
 }
-RTG_HD bool clear_compensation(const EnergyTables& E, const Bsdf& b, float mu_o, float& k) {
+RTG_HD bool clear_compensation(const EnergyTables& E, const Bsdf& b, TabAt mu_o, float& k) {
     if (!b.ms_clear_on) return false;
-    float e = clear_albedo(E, mu_o, b.ms_clear_alpha, b.eta);
+    float e = clear_albedo(E, mu_o, b.ms_clear_at, b.eta);
     k = 1.0f / rmax(e, 0.05f);
     return true;
 }
@@ -367,15 +376,33 @@ RTG_HD Rgb straight_transmittance(const Bsdf& b, float cos) {
     return b.tint * (b.clear * (1.0f - coat_fresnel(b, cos)) * t);
 }
 
-RTG_HD LobeWeights lobe_weights(const EnergyTables& E, const Bsdf& b, V3 wo) {
+// What evaluation, density and sampling at one vertex all take from the outgoing direction alone.
+// wo.z > 0 (below, everything is zero).
+struct BsdfWo {
+    TabAt at;                                  // wo.z's place in the tables
+    float pass_base, pass_coat;                // layer_passes of the two layers
+    float lost_spec, lost_coat;                // lobe_lost of the two multiple-scattering lobes (0: off)
+    float lambda;                              // ggx_L of the specular distribution
+};
+RTG_HD BsdfWo bsdf_wo(const EnergyTables& E, const Bsdf& b, V3 wo) {
+    BsdfWo o;
+    o.at = tab_at(wo.z);
+    o.pass_base = layer_passes(E, b.base_layer, wo.z, o.at);
+    o.pass_coat = layer_passes(E, b.coat_layer, wo.z, o.at);
+    o.lost_spec = b.ms_spec_on ? lobe_lost(E, b.ms_spec_lobe, o.at) : 0.0f;
+    o.lost_coat = b.ms_coat_on ? lobe_lost(E, b.ms_coat_lobe, o.at) : 0.0f;
+    o.lambda = ggx_L(b.spec, wo);
+    return o;
+}
+RTG_HD LobeWeights lobe_weights(const Bsdf& b, const BsdfWo& o, V3 wo) {
     float c = coat_fresnel(b, wo.z);
     float below = 1.0f - c;
     float specular = has_specular(b) ? below * rmax(luminance(specular_fresnel(b, wo.z)), 0.0f) : 0.0f;
-    float diff = below * luminance(b.diffuse) * layer_passes(E, b.base_layer, wo.z);
+    float diff = below * luminance(b.diffuse) * o.pass_base;
     float cl = below * b.clear;
     float ms = 0.0f;
-    if (b.ms_spec_on) ms += below * rmax(luminance(b.ms_spec_colour), 0.0f) * lobe_lost(E, b.ms_spec_lobe, wo.z);
-    if (b.ms_coat_on) ms += b.ms_coat_c * lobe_lost(E, b.ms_coat_lobe, wo.z);
+    if (b.ms_spec_on) ms += below * rmax(luminance(b.ms_spec_colour), 0.0f) * o.lost_spec;
+    if (b.ms_coat_on) ms += b.ms_coat_c * o.lost_coat;
     float total = c + specular + diff + cl + ms;
     LobeWeights w;
     if (total > 0.0f) {
@@ -394,101 +421,129 @@ RTG_HD bool refraction_half(const Bsdf& b, V3 wo, V3 wi, V3& h, float& co, float
     ci = dot(wi, h);
     return co > 0.0f && ci < 0.0f && len2(h) > 0.5f;
 }
-RTG_HD Rgb eval_refraction(const EnergyTables& E, const Bsdf& b, V3 wo, V3 wi) {
+// Value (`f`, when not null) and density (`pdf`, when not null, with the lobe weights `w`) of the
+// refraction wo -> wi, wi.z < 0.
+RTG_HD void refraction_eval_pdf(const EnergyTables& E, const Bsdf& b, const BsdfWo& o, const LobeWeights* w, V3 wo, V3 wi, Rgb* f, float* pdf) {
+    if (f) *f = splat(0.0f);
+    if (pdf) *pdf = 0.0f;
     V3 h; float co, ci;
-    if (!refraction_half(b, wo, wi, h, co, ci)) return splat(0.0f);
-    float f = fresnel_dielectric(co, b.eta);
+    if (!refraction_half(b, wo, wi, h, co, ci)) return;
+    const float D = ggx_D(b.spec, h);
     float denom = co + b.eta * ci;
-    float g2 = 1.0f / (1.0f + ggx_L(b.spec, wo) + ggx_L(b.spec, wi));
-    float value = (1.0f - f) * ggx_D(b.spec, h) * g2 * (-ci) * co / (-wi.z * wo.z * denom * denom);
-    float k;
-    if (clear_compensation(E, b, wo.z, k)) value *= k;
-    float attenuation = layer_passes(E, b.coat_layer, wo.z);
-    return b.tint * (b.clear * attenuation * value);
-}
-RTG_HD_NI Rgb bsdf_eval(const EnergyTables& E, const Bsdf& b, V3 wo, V3 wi, int lobes) {
-    if (wo.z <= 0.0f) return splat(0.0f);
-    if (wi.z <= 0.0f) {
-        if (wi.z < 0.0f && lobes == LOBES_ALL && b.clear > 0.0f && !b.thin) return eval_refraction(E, b, wo, wi);
-        return splat(0.0f);
-    }
-    float attenuation = layer_passes(E, b.coat_layer, wo.z) * layer_passes(E, b.coat_layer, wi.z);
-    Rgb diff = b.diffuse * (FRAC_1_PI * layer_passes(E, b.base_layer, wo.z) * layer_passes(E, b.base_layer, wi.z) * b.diffuse_norm);
-    if (lobes == LOBES_DIFFUSE) return diff * attenuation;
-    V3 h = normalize(wo + wi);
-    float cos_h = rmax(dot(wo, h), 0.0f);
-    Rgb below = diff;
-    if (has_specular(b)) below = below + specular_fresnel(b, cos_h) * ggx_microfacet(b.spec, wo, wi, h);
-    if (b.ms_spec_on) below = below + b.ms_spec_colour * (lobe_lost(E, b.ms_spec_lobe, wo.z) * lobe_lost(E, b.ms_spec_lobe, wi.z) * b.ms_spec_lobe.norm);
-    if (b.clear > 0.0f) {
-        float cl = b.clear * clear_fresnel(b, cos_h) * ggx_microfacet(b.spec, wo, wi, h);
+    if (f) {
+        float fr = fresnel_dielectric(co, b.eta);
+        float g2 = 1.0f / (1.0f + o.lambda + ggx_L(b.spec, wi));
+        float value = (1.0f - fr) * D * g2 * (-ci) * co / (-wi.z * wo.z * denom * denom);
         float k;
-        if (clear_compensation(E, b, wo.z, k)) cl *= k;
-        below = below + splat(cl);
+        if (clear_compensation(E, b, o.at, k)) value *= k;
+        *f = b.tint * (b.clear * o.pass_coat * value);
     }
-    Rgb f = below * attenuation;
-    if (b.coat > 0.0f) f = f + splat(coat_fresnel(b, cos_h) * ggx_microfacet(b.coat_ggx, wo, wi, h));
-    if (b.ms_coat_on) f = f + splat(b.ms_coat_c * (lobe_lost(E, b.ms_coat_lobe, wo.z) * lobe_lost(E, b.ms_coat_lobe, wi.z) * b.ms_coat_lobe.norm));
-    return f;
+    if (pdf && !(w->clear != w->clear || w->clear <= 0.0f)) {
+        float g1 = 1.0f / (1.0f + o.lambda);
+        float visible = g1 * D * co / wo.z;
+        float jacobian = b.eta * b.eta * (-ci) / (denom * denom);
+        *pdf = w->clear * (1.0f - reflect_chance(b, wo.z, co)) * visible * jacobian;
+    }
 }
-RTG_HD float pdf_with(const Bsdf& b, const LobeWeights& w, V3 wo, V3 wi) {
-    float p = (w.diffuse + w.ms) * wi.z * FRAC_1_PI;
-    if (w.specular > 0.0f || w.coat > 0.0f || w.clear > 0.0f) {
-        V3 h = normalize(wo + wi);
-        if (dot(wo, h) > 0.0f) {
-            if (w.specular > 0.0f) p += w.specular * ggx_reflection_pdf(b.spec, wo, h);
-            if (w.coat > 0.0f) p += w.coat * ggx_reflection_pdf(b.coat_ggx, wo, h);
-            if (w.clear > 0.0f) p += w.clear * reflect_chance(b, wo.z, dot(wo, h)) * ggx_reflection_pdf(b.spec, wo, h);
+// Value of the BSDF for the lobes asked for and (with `w`, when `pdf` is not null) the density of
+// its sampling, for wo.z > 0: the half vector, the distribution and the terms of wo are shared.
+RTG_HD_NI void bsdf_eval_pdf(const EnergyTables& E, const Bsdf& b, const BsdfWo& o, const LobeWeights* w, V3 wo, V3 wi, int lobes, Rgb& f, float* pdf) {
+    f = splat(0.0f);
+    if (pdf) *pdf = 0.0f;
+    if (wi.z <= 0.0f) {
+        if (wi.z < 0.0f && b.clear > 0.0f && !b.thin) refraction_eval_pdf(E, b, o, w, wo, wi, lobes == LOBES_ALL ? &f : nullptr, pdf);
+        return;
+    }
+    const TabAt at = tab_at(wi.z);
+    float attenuation = o.pass_coat * layer_passes(E, b.coat_layer, wi.z, at);
+    Rgb diff = b.diffuse * (FRAC_1_PI * o.pass_base * layer_passes(E, b.base_layer, wi.z, at) * b.diffuse_norm);
+    if (lobes == LOBES_DIFFUSE) {
+        f = diff * attenuation;
+        if (!pdf) return;
+    }
+    V3 h = normalize(wo + wi);
+    const float wo_h = dot(wo, h);
+    float cos_h = rmax(wo_h, 0.0f);
+    const bool spec_on = has_specular(b) || b.clear > 0.0f;
+    float D = 0.0f, micro = 0.0f, refl = 0.0f, refl_coat = 0.0f, micro_coat = 0.0f;
+    if (spec_on) {
+        D = ggx_D(b.spec, h);
+        float g2 = 1.0f / (1.0f + o.lambda + ggx_L(b.spec, wi));
+        micro = D * g2 / (4.0f * wo.z * wi.z);
+        if (pdf) {
+            float g1 = 1.0f / (1.0f + o.lambda);
+            refl = g1 * D / (4.0f * wo.z);
         }
     }
-    return p;
-}
-RTG_HD float refraction_pdf(const Bsdf& b, const LobeWeights& w, V3 wo, V3 wi) {
-    if (w.clear != w.clear || w.clear <= 0.0f) return 0.0f;
-    V3 h; float co, ci;
-    if (!refraction_half(b, wo, wi, h, co, ci)) return 0.0f;
-    float g1 = 1.0f / (1.0f + ggx_L(b.spec, wo));
-    float visible = g1 * ggx_D(b.spec, h) * co / wo.z;
-    float denom = co + b.eta * ci;
-    float jacobian = b.eta * b.eta * (-ci) / (denom * denom);
-    return w.clear * (1.0f - reflect_chance(b, wo.z, co)) * visible * jacobian;
-}
-RTG_HD_NI float bsdf_pdf(const EnergyTables& E, const Bsdf& b, V3 wo, V3 wi) {
-    if (wo.z <= 0.0f) return 0.0f;
-    if (wi.z <= 0.0f) {
-        if (wi.z < 0.0f && b.clear > 0.0f && !b.thin) return refraction_pdf(b, lobe_weights(E, b, wo), wo, wi);
-        return 0.0f;
+    if (b.coat > 0.0f) {
+        const float Dc = ggx_D(b.coat_ggx, h), lo = ggx_L(b.coat_ggx, wo);
+        float g2 = 1.0f / (1.0f + lo + ggx_L(b.coat_ggx, wi));
+        micro_coat = Dc * g2 / (4.0f * wo.z * wi.z);
+        float g1 = 1.0f / (1.0f + lo);
+        refl_coat = g1 * Dc / (4.0f * wo.z);
     }
-    return pdf_with(b, lobe_weights(E, b, wo), wo, wi);
+    if (pdf) {  // pdf_with (bsdf.rs:776)
+        float p = (w->diffuse + w->ms) * wi.z * FRAC_1_PI;
+        if ((w->specular > 0.0f || w->coat > 0.0f || w->clear > 0.0f) && wo_h > 0.0f) {
+            if (w->specular > 0.0f) p += w->specular * refl;
+            if (w->coat > 0.0f) p += w->coat * refl_coat;
+            if (w->clear > 0.0f) p += w->clear * reflect_chance(b, wo.z, wo_h) * refl;
+        }
+        *pdf = p;
+    }
+    if (lobes == LOBES_DIFFUSE) return;
+    Rgb below = diff;
+    if (has_specular(b)) below = below + specular_fresnel(b, cos_h) * micro;
+    if (b.ms_spec_on) below = below + b.ms_spec_colour * (o.lost_spec * lobe_lost(E, b.ms_spec_lobe, at) * b.ms_spec_lobe.norm);
+    if (b.clear > 0.0f) {
+        float cl = b.clear * clear_fresnel(b, cos_h) * micro;
+        float k;
+        if (clear_compensation(E, b, o.at, k)) cl *= k;
+        below = below + splat(cl);
+    }
+    f = below * attenuation;
+    if (b.coat > 0.0f) f = f + splat(coat_fresnel(b, cos_h) * micro_coat);
+    if (b.ms_coat_on) f = f + splat(b.ms_coat_c * (o.lost_coat * lobe_lost(E, b.ms_coat_lobe, at) * b.ms_coat_lobe.norm));
+}
+// The value alone.
+RTG_HD Rgb bsdf_eval(const EnergyTables& E, const Bsdf& b, V3 wo, V3 wi, int lobes) {
+    Rgb f = splat(0.0f);
+    if (!(wo.z <= 0.0f)) bsdf_eval_pdf(E, b, bsdf_wo(E, b, wo), nullptr, wo, wi, lobes, f, nullptr);
+    return f;
 }
 
-RTG_HD bool finish_reflection(const EnergyTables& E, const Bsdf& b, const LobeWeights& w, V3 wo, V3 wi, BsdfSample& out) {
+RTG_HD bool finish_reflection(const EnergyTables& E, const Bsdf& b, const BsdfWo& o, const LobeWeights& w, V3 wo, V3 wi, BsdfSample& out) {
     if (wi.z <= 0.0f) return false;
-    float p = pdf_with(b, w, wo, wi);
+    Rgb f;
+    float p;
+    bsdf_eval_pdf(E, b, o, &w, wo, wi, LOBES_ALL, f, &p);
     if (!(p > 0.0f && finitef(p))) return false;
-    out.weight = bsdf_eval(E, b, wo, wi, LOBES_ALL) * (wi.z / p);
+    out.weight = f * (wi.z / p);
     out.wi = wi; out.pdf = p; out.straight = false;
     return true;
 }
-RTG_HD bool finish_refraction(const EnergyTables& E, const Bsdf& b, const LobeWeights& w, V3 wo, V3 h, BsdfSample& out) {
+RTG_HD bool finish_refraction(const EnergyTables& E, const Bsdf& b, const BsdfWo& o, const LobeWeights& w, V3 wo, V3 h, BsdfSample& out) {
     V3 wi;
     if (!refract(wo, h, b.eta, wi)) return false;
     if (wi.z >= 0.0f) return false;
-    float p = refraction_pdf(b, w, wo, wi);
+    Rgb f;
+    float p;
+    bsdf_eval_pdf(E, b, o, &w, wo, wi, LOBES_ALL, f, &p);
     if (!(p > 0.0f && finitef(p))) return false;
-    out.weight = eval_refraction(E, b, wo, wi) * (-wi.z / p);
+    out.weight = f * (-wi.z / p);
     out.wi = wi; out.pdf = p; out.straight = false;
     return true;
 }
-RTG_HD_NI bool bsdf_sample(const EnergyTables& E, const Bsdf& b, V3 wo, float u0, float u1, BsdfSample& out) {  // bsdf.rs:833
-    if (wo.z <= 0.0f) return false;
-    LobeWeights w = lobe_weights(E, b, wo);
-    V3 wi;
+// A direction for wo (wo.z > 0) with its value and density. A reflection ends in one evaluation, at
+// the bottom, and a refraction in another, so their code is there once each.
+RTG_HD_NI bool bsdf_sample(const EnergyTables& E, const Bsdf& b, const BsdfWo& o, const LobeWeights& w, V3 wo, float u0, float u1, BsdfSample& out) {  // bsdf.rs:833
+    V3 wi, h;
+    bool through = false;
     if (u0 < w.coat) {
-        V3 h = sample_vndf(wo, b.coat_ggx.ax, b.coat_ggx.ay, u0 / w.coat, u1);
+        h = sample_vndf(wo, b.coat_ggx.ax, b.coat_ggx.ay, u0 / w.coat, u1);
         wi = h * (2.0f * dot(wo, h)) - wo;
     } else if (u0 < w.coat + w.specular) {
-        V3 h = sample_vndf(wo, b.spec.ax, b.spec.ay, (u0 - w.coat) / w.specular, u1);
+        h = sample_vndf(wo, b.spec.ax, b.spec.ay, (u0 - w.coat) / w.specular, u1);
         wi = h * (2.0f * dot(wo, h)) - wo;
     } else if (w.diffuse + w.ms > 0.0f && (w.clear <= 0.0f || u0 < w.coat + w.specular + (w.diffuse + w.ms))) {
         float start = w.coat + w.specular;
@@ -500,32 +555,28 @@ RTG_HD_NI bool bsdf_sample(const EnergyTables& E, const Bsdf& b, V3 wo, float u0
         float uc = rclamp((u0 - start) / w.clear, 0.0f, 0.99999994f);
         if (b.ms_clear_on) {
             // sample_rough_clear (bsdf.rs:947)
-            V3 h = sample_vndf(wo, b.spec.ax, b.spec.ay, uc, u1);
+            h = sample_vndf(wo, b.spec.ax, b.spec.ay, uc, u1);
             float fr = clear_fresnel(b, dot(wo, h));
             uint64_t key = ((uint64_t)fbits(uc) << 32) | (uint64_t)fbits(u1);
             float choice = (float)(mix64(key ^ 0x9e3779b97f4a7c15ULL) >> 40) * (1.0f / 16777216.0f);
-            if (choice < fr) return finish_reflection(E, b, w, wo, h * (2.0f * dot(wo, h)) - wo, out);
-            return finish_refraction(E, b, w, wo, h, out);
+            through = !(choice < fr);
+        } else {
+            float pr = reflect_probability(b, wo.z);
+            through = !(uc < pr);
+            if (through && b.thin) {
+                float chance = w.clear * (1.0f - pr);
+                if (chance != chance || chance <= 0.0f) return false;
+                out.weight = straight_transmittance(b, wo.z) / chance;
+                out.wi = -wo; out.pdf = chance; out.straight = true;
+                return true;
+            }
+            h = sample_vndf(wo, b.spec.ax, b.spec.ay, through ? rclamp((uc - pr) / (1.0f - pr), 0.0f, 0.99999994f) : uc / pr, u1);
         }
-        float pr = reflect_probability(b, wo.z);
-        if (uc < pr) {
-            V3 h = sample_vndf(wo, b.spec.ax, b.spec.ay, uc / pr, u1);
-            return finish_reflection(E, b, w, wo, h * (2.0f * dot(wo, h)) - wo, out);
-        }
-        if (b.thin) {
-            float chance = w.clear * (1.0f - pr);
-            if (chance != chance || chance <= 0.0f) return false;
-            out.weight = straight_transmittance(b, wo.z) / chance;
-            out.wi = -wo; out.pdf = chance; out.straight = true;
-            return true;
-        }
-        float ut = rclamp((uc - pr) / (1.0f - pr), 0.0f, 0.99999994f);
-        V3 h = sample_vndf(wo, b.spec.ax, b.spec.ay, ut, u1);
-        return finish_refraction(E, b, w, wo, h, out);
+        wi = h * (2.0f * dot(wo, h)) - wo;
     } else {
         return false;
     }
-    return finish_reflection(E, b, w, wo, wi, out);
+    return through ? finish_refraction(E, b, o, w, wo, h, out) : finish_reflection(E, b, o, w, wo, wi, out);
 }
 
 }  // namespace rtg

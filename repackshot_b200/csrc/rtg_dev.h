@@ -138,6 +138,9 @@ struct SceneDev {
     // Sample indices from split_b on are scrambled with seed_b instead of seed (sample_key). A
     // render keeps split_b = 0xffffffff; the decorrelated adjoint draws its second half with it.
     uint32_t seed_b, split_b;
+    uint64_t seed_key, seed_key_b;  // seed_key() of the two seeds
+    // Per dimension below 64: the XOR of its generator's columns over the bits of 0..255.
+    const uint32_t* sobol;
     float clamp_indirect;
     const float* filter_table;  // the Blackman-Harris inverse CDF, 256 points (pixel filter 3)
     uint32_t edge_k;            // samples per sample index of an edge pixel (1: no edge samples)

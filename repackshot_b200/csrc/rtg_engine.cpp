@@ -34,6 +34,7 @@ std::string g_error;
 bool g_device_ready = false;
 void* g_energy_dev = nullptr;
 EnergyTables g_energy{};
+const uint32_t* g_sobol_low = nullptr;  // SceneDev::sobol
 const float* g_filter_table = nullptr;  // the Blackman-Harris inverse CDF on the device
 int g_sms = 148;
 
@@ -179,29 +180,47 @@ uint32_t device_init() {
     RTG_CHECK(cudaDeviceSynchronize());
     set_sobol(sob, 0);
     RTG_CHECK(cudaGetLastError());
+    // The energy tables cell by cell (table_lookup reads a cell's four corners in one load), their
+    // averages, the Blackman-Harris table and the Sobol columns summed over a low byte.
     const EnergyData& E = energy_data();
-    size_t n16 = E.albedo.size() + E.schlick.size() + E.clear_in.size() + E.clear_out.size();
-    size_t bytes = n16 * 2 + 64 * 4 + 256 * 4;
-    RTG_CHECK(cudaMalloc(&g_energy_dev, bytes));
-    std::vector<uint8_t> host(bytes);
-    uint8_t* p = host.data();
-    auto put = [&](const void* src, size_t n) { std::memcpy(p, src, n); p += n; };
-    put(E.albedo.data(), E.albedo.size() * 2);
-    put(E.schlick.data(), E.schlick.size() * 2);
-    put(E.clear_in.data(), E.clear_in.size() * 2);
-    put(E.clear_out.data(), E.clear_out.size() * 2);
-    put(E.albedo_avg.data(), 32 * 4);
-    put(E.schlick_avg.data(), 32 * 4);
-    put(blackman_harris_table(), 256 * 4);
-    RTG_CHECK(cudaMemcpy(g_energy_dev, host.data(), bytes, cudaMemcpyHostToDevice));
+    auto cells = [](const std::vector<uint16_t>& t) {
+        std::vector<uint16_t> c(t.size() * 4);
+        for (size_t k = 0; k < t.size(); ++k) {
+            const size_t i = k % NODES_MU, j = k / NODES_MU % NODES_ROUGHNESS, slice = k - i - j * NODES_MU;
+            const size_t i1 = std::min<size_t>(i + 1, NODES_MU - 1), j1 = std::min<size_t>(j + 1, NODES_ROUGHNESS - 1);
+            c[4 * k] = t[k];
+            c[4 * k + 1] = t[slice + j * NODES_MU + i1];
+            c[4 * k + 2] = t[slice + j1 * NODES_MU + i];
+            c[4 * k + 3] = t[slice + j1 * NODES_MU + i1];
+        }
+        return c;
+    };
+    std::vector<uint32_t> low(64 * 256);
+    for (uint32_t d = 0; d < 64; ++d)
+        for (uint32_t v = 0; v < 256; ++v)
+            for (uint32_t bit = 0; bit < 8; ++bit)
+                if (v >> bit & 1u) low[d << 8 | v] ^= sob.m[sob.layout[d]][bit];
+    std::vector<uint8_t> host;
+    auto put = [&](const void* src, size_t n) {
+        const size_t at = host.size();
+        host.resize(at + n);
+        std::memcpy(host.data() + at, src, n);
+        return at;
+    };
+    auto put_cells = [&](const std::vector<uint16_t>& t) {
+        const std::vector<uint16_t> c = cells(t);
+        return put(c.data(), c.size() * 2);
+    };
+    const size_t albedo = put_cells(E.albedo), schlick = put_cells(E.schlick), clear_in = put_cells(E.clear_in), clear_out = put_cells(E.clear_out);
+    const size_t albedo_avg = put(E.albedo_avg.data(), 32 * 4), schlick_avg = put(E.schlick_avg.data(), 32 * 4);
+    const size_t filter = put(blackman_harris_table(), 256 * 4), sobol = put(low.data(), low.size() * 4);
+    RTG_CHECK(cudaMalloc(&g_energy_dev, host.size()));
+    RTG_CHECK(cudaMemcpy(g_energy_dev, host.data(), host.size(), cudaMemcpyHostToDevice));
     const uint8_t* d = (const uint8_t*)g_energy_dev;
-    g_energy.albedo = (const uint16_t*)d;
-    g_energy.schlick = g_energy.albedo + E.albedo.size();
-    g_energy.clear_in = g_energy.schlick + E.schlick.size();
-    g_energy.clear_out = g_energy.clear_in + E.clear_in.size();
-    g_energy.albedo_avg = (const float*)(g_energy.clear_out + E.clear_out.size());
-    g_energy.schlick_avg = g_energy.albedo_avg + 32;
-    g_filter_table = g_energy.schlick_avg + 32;
+    g_energy = EnergyTables{(const uint16_t*)(d + albedo), (const uint16_t*)(d + schlick), (const uint16_t*)(d + clear_in),
+                            (const uint16_t*)(d + clear_out), (const float*)(d + albedo_avg), (const float*)(d + schlick_avg)};
+    g_filter_table = (const float*)(d + filter);
+    g_sobol_low = (const uint32_t*)(d + sobol);
     RTG_CHECK(cudaDeviceSynchronize());
     g_device_ready = true;
     return RTG_STATUS_OK;
@@ -315,6 +334,7 @@ SceneDev compose(const SceneDev& constants, const SceneDev& geom, const SceneDev
     S.exempt_boxes = shade.exempt_boxes;
     S.energy = g_energy;
     S.filter_table = g_filter_table;
+    S.sobol = g_sobol_low;
     return S;
 }
 
@@ -1129,6 +1149,8 @@ void pack_waves(const std::vector<std::unique_ptr<QueueJob>>& jobs, uint64_t cap
                 continue;
             }
             g.slot_begin = (uint32_t)used;
+            g.by_pixels = divisor(g.w * g.h);
+            g.by_width = divisor(g.w);
             uint64_t seg_pix = (uint64_t)g.w * g.h;
             g.pix_begin = cur.empty() ? 0 : cur.back().pix_begin + cur.back().w * cur.back().h;
             cur.push_back(g);
@@ -1367,9 +1389,9 @@ uint32_t rtg_render_adjoint(uint32_t scene, uint32_t film, const float* target, 
     struct SplitSeeds {
         SceneDev& S;
         SplitSeeds(SceneDev& s_, bool on, uint32_t split) : S(s_) {
-            if (on) { S.split_b = split; S.seed_b = ~S.seed; }
+            if (on) { S.split_b = split; S.seed_b = ~S.seed; S.seed_key_b = seed_key(S.seed_b); }
         }
-        ~SplitSeeds() { S.split_b = 0xffffffffu; S.seed_b = S.seed; }
+        ~SplitSeeds() { S.split_b = 0xffffffffu; S.seed_b = S.seed; S.seed_key_b = S.seed_key; }
     } split_seeds(sc->S, halves, first_sample + count / 2);
     // Forward: every path of the call in one wave, into the cleared film.
     RTG_CHECK(cudaMemsetAsync(f->mem.p, 0, f->mem.bytes, s));

@@ -27,11 +27,32 @@ cudaError_t launch_albedo_pass(const SceneDev& S, const LightsDev* L, const uint
 cudaError_t launch_edge_list(const uint8_t* mask, uint32_t stride, uint32_t x0, uint32_t y0, uint32_t w, uint32_t h, uint32_t* list,
                              uint32_t* count, cudaStream_t st, int grid);
 
+// Division of slots (below 2^31) by a divisor of the whole launch: the high word of a product with
+// 2^(31 + shift) / d rounded up, shift = ceil(log2 d), and a shift (Granlund and Montgomery,
+// "Division by invariant integers using multiplication", PLDI 1994): three instructions for the
+// twenty of a division by a variable. mul 0: divides by 1.
+struct Divisor {
+    uint32_t mul = 0, shift = 0;
+#ifdef __CUDACC__
+    __device__ __forceinline__ uint32_t of(uint32_t n) const { return mul ? __umulhi(n, mul) >> shift : n; }
+#endif
+};
+inline Divisor divisor(uint32_t d) {
+    Divisor v;
+    if (d < 2) return v;
+    uint32_t bits = 0;
+    while ((1ull << bits) < d) ++bits;
+    v.mul = (uint32_t)(((1ull << (31 + bits)) + d - 1) / d);
+    v.shift = bits - 1;
+    return v;
+}
+
 // A segment of a batched wave: samples [first, first + ns) of the full-width rows [y0, y0 + h) of
 // one job's image. Its slots start at slot_begin (sample-major, then row-major pixels); its pixels
 // start at pix_begin in the wave's accumulation order.
 struct SegDev {
     uint32_t job, y0, w, h, first, ns, slot_begin, pix_begin;
+    Divisor by_pixels, by_width;
 };
 
 // A wave of path slots: either the pixels of the rectangle (x0, y0, w, h) for the sample
@@ -63,7 +84,15 @@ struct WaveDesc {
     float4* alb;
     float* guide_sum;
     float* guide_weight;
+    Divisor by_pixels, by_width, by_ek, by_ne;  // of w h, w, ek and ne (with_divisors)
 };
+inline WaveDesc with_divisors(WaveDesc w) {
+    w.by_pixels = divisor(w.w * w.h);
+    w.by_width = divisor(w.w);
+    w.by_ek = divisor(w.ek);
+    w.by_ne = divisor(w.ne);
+    return w;
+}
 
 // Structure-of-arrays path state of one wave (device pointers).
 struct PathBuffers {

@@ -304,20 +304,9 @@ constexpr uint32_t OFF_LIGHT_SELECT = 0, OFF_LIGHT = 1, OFF_BSDF = 3, OFF_ROULET
 // from a table the caller provides (constant memory on the device).
 struct SobolTable { uint32_t m[64][32]; uint32_t layout[64]; };
 
-RTG_HD uint64_t pixel_key(uint32_t seed, uint32_t x, uint32_t y) {  // sampler.rs:339
-    uint64_t pixel = ((uint64_t)y << 32) | (uint64_t)x;
-    return mix64(pixel ^ mix64((uint64_t)seed ^ 0x5851f42d4c957f2dULL));
-}
-RTG_HD float sample1(const SobolTable& T, uint64_t key, uint32_t index, uint32_t dim) {  // sampler.rs:353
-    uint64_t seed = mix64(key ^ ((uint64_t)(dim + 1) * 0x9e3779b97f4a7c15ULL));
-    if (dim < 64) {
-        const uint32_t* col = T.m[T.layout[dim]];
-        uint32_t bits = index, x = 0;
-        while (bits) { x ^= col[ctz32(bits)]; bits &= bits - 1; }
-        return to_unit(owen_scramble(x, (uint32_t)(seed >> 32)));
-    }
-    return to_unit((uint32_t)(mix64(seed ^ (uint64_t)index) >> 32));
-}
+RTG_HD uint64_t seed_key(uint32_t seed) { return mix64((uint64_t)seed ^ 0x5851f42d4c957f2dULL); }  // sampler.rs:339
+RTG_HD uint64_t pixel_key(uint64_t seed_key, uint32_t x, uint32_t y) { return mix64((((uint64_t)y << 32) | (uint64_t)x) ^ seed_key); }
+RTG_HD uint64_t sample_seed(uint64_t key, uint32_t dim) { return mix64(key ^ ((uint64_t)(dim + 1) * 0x9e3779b97f4a7c15ULL)); }  // sampler.rs:353
 
 // ---- warp.rs ------------------------------------------------------------------------------------
 RTG_HD void concentric_disk(float u0, float u1, float& ox, float& oy) {

@@ -1256,6 +1256,7 @@ static bool flatten(const HScene& s, Flat& F, std::string& error, bool geometry,
     S.projection = panoramic ? s.projection : 0;
     S.fov_x_deg = s.fov_x; S.fov_y_deg = s.fov_y;
     S.width = s.width; S.height = s.height; S.seed = s.seed; S.seed_b = s.seed; S.split_b = 0xffffffffu;
+    S.seed_key = S.seed_key_b = seed_key(s.seed);
     S.max_depth = s.max_depth == 0 ? 8 : (s.max_depth < 1024 ? s.max_depth : 1024);
     S.pixel_filter = s.pixel_filter;
     S.edge_k = s.edge_supersample < 1 ? 1 : (s.edge_supersample > 16 ? 16 : s.edge_supersample);  // RenderSettings::edge_factor

@@ -163,8 +163,10 @@ RTG_D Rgb backdrop(const SceneDev& S, float su, float sv) {
 }
 
 // The selection at a vertex (light.rs:495): its point, the sum of the weights there and whether
-// it is the static one. Weights are recomputed from the point with the same operations.
+// it is the static one. The path keeps the point and the sum for its next vertex; a weight is
+// computed again from the point, with the same operations.
 struct Sel { V3 p; float total; bool by_flux; };
+constexpr int SEL_KEPT = 8;  // weights that select_at leaves for the pick at the same vertex
 RTG_D float entry_weight(const LightsDev& L, int e, V3 x) {  // light.rs:1014
     int a = L.entries[e];
     if (a < 0) return L.env_base;
@@ -174,13 +176,17 @@ RTG_D float entry_weight(const LightsDev& L, int e, V3 x) {  // light.rs:1014
     if (l.kind == LIGHT_MESH) return mesh_weight(l, x);
     return sphere_weight(l, x);
 }
-RTG_D Sel select_at(const LightsDev& L, V3 x) {
+RTG_D Sel select_at(const LightsDev& L, V3 x, float* weights) {
     Sel s;
     s.p = x;
     s.total = 0.0f;
     s.by_flux = !(L.per_point && L.n_entries > 0);
     if (!s.by_flux)
-        for (int e = 0; e < L.n_entries; ++e) s.total += entry_weight(L, e, x);
+        for (int e = 0; e < L.n_entries; ++e) {
+            const float w = entry_weight(L, e, x);
+            if (e < SEL_KEPT) weights[e] = w;
+            s.total += w;
+        }
     return s;
 }
 RTG_D float pmf_of(const LightsDev& L, uint32_t entry, const Sel& s) {
@@ -208,7 +214,7 @@ RTG_D float emitter_weight(const LightsDev& L, uint32_t emitter, float pdf, cons
 // light: index into lights[], -1 the environment; delta: no other technique finds it
 struct LightSample { V3 wi; float distance; Rgb radiance; float pdf; bool glossy, shadow, delta; int light; };
 
-RTG_D_NI bool sample_light(const LightsDev& L, const Sel& s, float u_select, float u0, float u1, LightSample& out) {  // light.rs:1150
+RTG_D_NI bool sample_light(const LightsDev& L, const Sel& s, const float* weights, float u_select, float u0, float u1, LightSample& out) {  // light.rs:1150
     int n = L.n_entries;
     if (n == 0) return false;
     int index = 0;
@@ -226,7 +232,7 @@ RTG_D_NI bool sample_light(const LightsDev& L, const Sel& s, float u_select, flo
         float acc = 0.0f, lo = 0.0f;
         int last = n - 1;
         for (int e = 0; e <= last; ++e) {
-            float w = entry_weight(L, e, s.p);
+            float w = e < SEL_KEPT ? weights[e] : entry_weight(L, e, s.p);
             acc += w;
             float hi = e == last ? 1.0f : acc / s.total;
             if (hi > u_select || e == last) {
@@ -444,14 +450,27 @@ RTG_D float filter_offset(const SceneDev& S, float u) {
 // The scramble key of a pixel's sample (sampler.rs:339 with the render's seed): indices from
 // S.split_b on take S.seed_b. Every render has split_b = 0xffffffff, so its keys are the seed's.
 RTG_D uint64_t sample_key(const SceneDev& S, uint32_t x, uint32_t y, uint32_t index) {
-    return pixel_key(index >= S.split_b ? S.seed_b : S.seed, x, y);
+    return pixel_key(index >= S.split_b ? S.seed_key_b : S.seed_key, x, y);
+}
+// Dimension `dim` of sample `index` (sample1): the generator columns of the index's low byte come
+// summed from a table of 256 entries a dimension (a path's first 256 samples need no other), the
+// higher bits' one by one.
+RTG_D float sample_at(const SceneDev& S, const SobolTable& T, uint64_t key, uint32_t index, uint32_t dim) {
+    const uint64_t seed = sample_seed(key, dim);
+    if (dim >= 64) return to_unit((uint32_t)(mix64(seed ^ (uint64_t)index) >> 32));
+    uint32_t x = __ldg(S.sobol + (dim << 8 | (index & 255u)));
+    if (index >> 8) {
+        const uint32_t* col = T.m[T.layout[dim]];
+        for (uint32_t bits = index & ~255u; bits; bits &= bits - 1) x ^= col[ctz32(bits)];
+    }
+    return to_unit(owen_scramble(x, (uint32_t)(seed >> 32)));
 }
 // The screen position (u, v) in [0, 1]^2 of a camera sample (render.rs:96).
 RTG_D void screen_of(const SceneDev& S, const SobolTable& T, uint32_t x, uint32_t y, uint32_t index, float& su, float& sv) {
     uint32_t width = S.width ? S.width : 1, height = S.height ? S.height : 1;
     uint64_t key = sample_key(S, x, y, index);
-    float du = filter_offset(S, sample1(T, key, index, DIM_CAMERA));
-    float dv = filter_offset(S, sample1(T, key, index, DIM_CAMERA + 1));
+    float du = filter_offset(S, sample_at(S, T, key, index, DIM_CAMERA));
+    float dv = filter_offset(S, sample_at(S, T, key, index, DIM_CAMERA + 1));
     su = rclamp(((float)x + du) / (float)width, 0.0f, 1.0f);
     sv = rclamp(((float)y + dv) / (float)height, 0.0f, 1.0f);
 }
@@ -510,13 +529,13 @@ RTG_D bool camera_ray_at(const SceneDev& S, float u, float v, float lx, float ly
 RTG_D bool camera_ray(const SceneDev& S, const SobolTable& T, uint32_t x, uint32_t y, uint32_t index, V3& o, V3& d) {
     uint32_t width = S.width ? S.width : 1, height = S.height ? S.height : 1;
     uint64_t key = sample_key(S, x, y, index);
-    float du = filter_offset(S, sample1(T, key, index, DIM_CAMERA));
-    float dv = filter_offset(S, sample1(T, key, index, DIM_CAMERA + 1));
+    float du = filter_offset(S, sample_at(S, T, key, index, DIM_CAMERA));
+    float dv = filter_offset(S, sample_at(S, T, key, index, DIM_CAMERA + 1));
     float u = ((float)x + du) / (float)width;
     float v = ((float)y + dv) / (float)height;
     float lx = 0.0f, ly = 0.0f;
     if (!S.ortho && S.lens_radius > 0.0f)
-        concentric_disk(sample1(T, key, index, DIM_LENS), sample1(T, key, index, DIM_LENS + 1), lx, ly);
+        concentric_disk(sample_at(S, T, key, index, DIM_LENS), sample_at(S, T, key, index, DIM_LENS + 1), lx, ly);
     return camera_ray_at(S, u, v, lx, ly, o, d);
 }
 
