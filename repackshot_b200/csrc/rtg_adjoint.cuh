@@ -119,6 +119,7 @@ __device__ __noinline__ Rgb adjoint_spheres(const LightsDev& L, Rgb crossed, V3 
     return crossed;
 }
 
+template <bool PLAIN>
 __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const LightsDev& L, const PathBuffers& P, const AdjointDev& A, float* g,
                                                    uint32_t slot, int cur, uint32_t bounce, const WaveDesc& w) {
     float4 o4 = P.o[slot], d4 = P.d[slot], thr4 = P.thr[slot];
@@ -147,12 +148,12 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
     }
     float t_geometry = hit.w ? __uint_as_float(hit.z) : f_inf();
     float t_floor = f_inf();
-    if ((S.floor_mode == 1) && rd.z != 0.0f) {
+    if (!PLAIN && S.floor_mode == 1 && rd.z != 0.0f) {
         float t = (S.floor_z - ro.z) / rd.z;
         if (t > 1.0e-3f && t < f_inf()) t_floor = t;
     }
     float t_nearest = rmin(t_geometry, t_floor);
-    if ((flags & PF_MEDIUM) && finitef(t_nearest)) {
+    if (!PLAIN && (flags & PF_MEDIUM) && finitef(t_nearest)) {
         const uint32_t medium = P.medium[slot];
         const DevMaterial& mm = S.materials[medium];
         thr = thr * rgb(fexp(-mm.sigma[0] * t_nearest), fexp(-mm.sigma[1] * t_nearest), fexp(-mm.sigma[2] * t_nearest));
@@ -181,14 +182,14 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
         float wgt = 1.0f;
         if (has_pdf) {
             float dd = offset + t;
-            float light_pdf = pmf_of(L, l.entry, from) * dd * dd / (l.area * cos);
+            float light_pdf = pmf_of<PLAIN>(L, l.entry, from) * dd * dd / (l.area * cos);
             wgt = power_heuristic(pdf, light_pdf);
         }
         Rgb term = area_radiance(l, cos) * wgt;
         crossed = crossed + term;
         adj_add(g, base_light + i, adj_dot(dl, thr * term));
     }
-    if (L.n_spheres) crossed = adjoint_spheres(L, crossed, ro, rd, t_nearest, has_pdf, pdf, from, offset, thr, dl, g, base_light);
+    if (!PLAIN && L.n_spheres) crossed = adjoint_spheres(L, crossed, ro, rd, t_nearest, has_pdf, pdf, from, offset, thr, dl, g, base_light);
     {
         float4 c4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         add_clamped(c4, thr * crossed, bounce >= 2, S.clamp_indirect);
@@ -198,16 +199,16 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
     do {
         if (t_nearest == f_inf()) {
             if (primary && S.background == 0) {
-                Rgb seen = escaped(L, rd, false, 0.0f, from);
+                Rgb seen = escaped<PLAIN>(L, rd, false, 0.0f, from);
                 rem = rgb_sub(rem, thr * (S.exterior == 1.0f ? seen : seen * S.exterior));
-                if (L.n_suns) adjoint_suns(L, rd, false, 0.0f, from, thr * S.exterior, dl, g, base_light);
+                if (!PLAIN && L.n_suns) adjoint_suns(L, rd, false, 0.0f, from, thr * S.exterior, dl, g, base_light);
             } else if (primary && S.background == 1) {
                 rem = rgb_sub(rem, thr * rgb(S.background_color[0], S.background_color[1], S.background_color[2]));
             } else if (!(primary && S.background == 2)) {
                 float4 c4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                add_clamped(c4, thr * escaped(L, rd, has_pdf, pdf, from), bounce >= 2, S.clamp_indirect);
+                add_clamped(c4, thr * escaped<PLAIN>(L, rd, has_pdf, pdf, from), bounce >= 2, S.clamp_indirect);
                 rem = rgb_sub(rem, rgb(c4.x, c4.y, c4.z));
-                if (L.n_suns) adjoint_suns(L, rd, has_pdf, pdf, from, thr, dl, g, base_light);
+                if (!PLAIN && L.n_suns) adjoint_suns(L, rd, has_pdf, pdf, from, thr, dl, g, base_light);
             }
             break;
         }
@@ -215,7 +216,7 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
         bool s_inst = false, s_outside = true;
         const DevInstance* I = nullptr;
         const DevMaterial* mat = nullptr;
-        if (t_floor < t_geometry) {
+        if (!PLAIN && t_floor < t_geometry) {
             V3 pp = ro + rd * t_floor;
             V3 point = v3(pp.x, pp.y, S.floor_z);
             V3 nn = v3(0.0f, 0.0f, rd.z < 0.0f ? 1.0f : -1.0f);
@@ -223,7 +224,7 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
         } else {
             HitInfo h;
             uint4 idx;
-            if (!hit_details(S, ro, rd, 1.0e-3f, f_inf(), hit.x, hit.y, __uint_as_float(hit.z), h, I, idx)) break;
+            if (!hit_details<PLAIN>(S, ro, rd, 1.0e-3f, f_inf(), hit.x, hit.y, __uint_as_float(hit.z), h, I, idx)) break;
             V3 ng = h.geometric, nrm = h.normal;
             if (dot(nrm, ng) < 0.0f) nrm = -nrm;
             if (dot(nrm, rd) >= -1.0e-4f) nrm = ng;
@@ -234,7 +235,7 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
             s_inst = true;
             s_outside = h.outside;
             mat = S.materials + I->material;
-            if (mat->kind == MATERIAL_EMISSIVE) {
+            if (!PLAIN && mat->kind == MATERIAL_EMISSIVE) {
                 if (h.front || !(I->flags & 1u)) {
                     const float wgt = has_pdf ? emitter_weight(L, I->emitter, pdf, from, offset + t_geometry, dot(ng, rd)) : 1.0f;
                     float4 c4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -248,7 +249,7 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
         const uint32_t m = mat ? I->material : 0, side = s_outside ? 0 : 1;
         const Bsdf& b = S.bsdfs[mat ? 2 * m + side : 2 * S.n_materials];
         Frame fr = frame_from_normal(s_normal);
-        if (s_inst && I->tangent_on) {
+        if (!PLAIN && s_inst && I->tangent_on) {
             V3 cands[2] = {cross(ld3(I->tan_axis), s_point - ld3(I->tan_centre)), ld3(I->tan_x)};
             for (int k = 0; k < 2; ++k) {
                 V3 t = cands[k] - s_normal * dot(s_normal, cands[k]);
@@ -265,19 +266,19 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
         V3 origin = offset_origin(s_point, ng);
         uint32_t dims = bounce_dim(bounce);
         uint64_t key = sample_key(S, x, y, index);
-        const BsdfWo bo = bsdf_wo(S.energy, b, wo);
-        const LobeWeights lobe_w = lobe_weights(b, bo, wo);
+        const BsdfWo bo = bsdf_wo<PLAIN>(S.energy, b, wo);
+        const LobeWeights lobe_w = lobe_weights<PLAIN>(b, bo, wo);
         float weights[SEL_KEPT];
-        Sel selection = select_at(L, s_point, weights);
+        Sel selection = select_at<PLAIN>(L, s_point, weights);
         LightSample ls;
-        if (sample_light(L, selection, weights, sample_at(S, c_sobol, key, index, dims + OFF_LIGHT_SELECT), sample_at(S, c_sobol, key, index, dims + OFF_LIGHT),
+        if (sample_light<PLAIN>(L, selection, weights, sample_at(S, c_sobol, key, index, dims + OFF_LIGHT_SELECT), sample_at(S, c_sobol, key, index, dims + OFF_LIGHT),
                          sample_at(S, c_sobol, key, index, dims + OFF_LIGHT + 1), ls)) {
             V3 wi = to_local(fr, ls.wi);
             const LobesSel lobes = ls.glossy ? LOBES_ALL : LOBES_DIFFUSE;
             const bool mis = ls.glossy && !ls.delta;
             Rgb f;
             float bsdf_density = 0.0f;
-            bsdf_eval_pdf(S.energy, b, bo, &lobe_w, wo, wi, lobes, f, mis ? &bsdf_density : nullptr);
+            bsdf_eval_pdf<PLAIN>(S.energy, b, bo, &lobe_w, wo, wi, lobes, f, mis ? &bsdf_density : nullptr);
             if (peak(f) > 0.0f) {
                 V3 from_p = wi.z < 0.0f ? offset_origin(s_hit, -ng) : origin;
                 float weight = mis ? power_heuristic(ls.pdf, bsdf_density) : 1.0f;
@@ -297,9 +298,9 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
                 if (mat && finite_c) {
                     Rgb K = thr * ls.radiance * (kscale * clamp_scale);
                     const uint32_t k = 2 * m + side;
-                    Rgb fa = rgb_sub(bsdf_eval(S.energy, A.albedo_plus[k], wo, wi, lobes), bsdf_eval(S.energy, A.albedo_minus[k], wo, wi, lobes)) *
+                    Rgb fa = rgb_sub(bsdf_eval<PLAIN>(S.energy, A.albedo_plus[k], wo, wi, lobes), bsdf_eval<PLAIN>(S.energy, A.albedo_minus[k], wo, wi, lobes)) *
                              A.inv_2h_albedo;
-                    Rgb fr2 = rgb_sub(bsdf_eval(S.energy, A.alpha_plus[k], wo, wi, lobes), bsdf_eval(S.energy, A.alpha_minus[k], wo, wi, lobes)) *
+                    Rgb fr2 = rgb_sub(bsdf_eval<PLAIN>(S.energy, A.alpha_plus[k], wo, wi, lobes), bsdf_eval<PLAIN>(S.energy, A.alpha_minus[k], wo, wi, lobes)) *
                               A.inv_2h_alpha;
                     mg = make_float4(dl.r * K.r * fa.r, dl.g * K.g * fa.g, dl.b * K.b * fa.b,
                                      dl.r * K.r * fr2.r + dl.g * K.g * fr2.g + dl.b * K.b * fr2.b);
@@ -318,7 +319,7 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
                 } else {
                     float tmax = finitef(ls.distance) ? ls.distance * (1.0f - 1.0e-4f) : f_inf();
                     bool floor_blocks = false;
-                    if (S.floor_mode == 1 && ls.wi.z != 0.0f) {
+                    if (!PLAIN && S.floor_mode == 1 && ls.wi.z != 0.0f) {
                         float t = (S.floor_z - from_p.z) / ls.wi.z;
                         floor_blocks = t > 1.0e-3f && t < tmax;
                     }
@@ -334,10 +335,10 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
             }
         }
         BsdfSample bs;
-        if (!bsdf_sample(S.energy, b, bo, lobe_w, wo, sample_at(S, c_sobol, key, index, dims + OFF_BSDF), sample_at(S, c_sobol, key, index, dims + OFF_BSDF + 1), bs))
+        if (!bsdf_sample<PLAIN>(S.energy, b, bo, lobe_w, wo, sample_at(S, c_sobol, key, index, dims + OFF_BSDF), sample_at(S, c_sobol, key, index, dims + OFF_BSDF + 1), bs))
             break;
         bool transmitted = bs.wi.z < 0.0f;
-        V3 wi = bs.straight ? rd : normalize(to_world(fr, bs.wi));
+        V3 wi = !PLAIN && bs.straight ? rd : normalize(to_world(fr, bs.wi));
         if (transmitted) {
             if (dot(wi, ng) >= 0.0f) break;
         } else if (dot(wi, ng) <= 0.0f) {
@@ -356,17 +357,17 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
         if (mat && !bs.straight) {
             const uint32_t k = 2 * m + side;
             Rgb f;
-            bsdf_eval_pdf(S.energy, b, bo, nullptr, wo, bs.wi, LOBES_ALL, f, nullptr);
-            Rgb fa = rgb_sub(bsdf_eval(S.energy, A.albedo_plus[k], wo, bs.wi, LOBES_ALL), bsdf_eval(S.energy, A.albedo_minus[k], wo, bs.wi, LOBES_ALL)) *
+            bsdf_eval_pdf<PLAIN>(S.energy, b, bo, nullptr, wo, bs.wi, LOBES_ALL, f, nullptr);
+            Rgb fa = rgb_sub(bsdf_eval<PLAIN>(S.energy, A.albedo_plus[k], wo, bs.wi, LOBES_ALL), bsdf_eval<PLAIN>(S.energy, A.albedo_minus[k], wo, bs.wi, LOBES_ALL)) *
                      A.inv_2h_albedo;
-            Rgb fr2 = rgb_sub(bsdf_eval(S.energy, A.alpha_plus[k], wo, bs.wi, LOBES_ALL), bsdf_eval(S.energy, A.alpha_minus[k], wo, bs.wi, LOBES_ALL)) *
+            Rgb fr2 = rgb_sub(bsdf_eval<PLAIN>(S.energy, A.alpha_plus[k], wo, bs.wi, LOBES_ALL), bsdf_eval<PLAIN>(S.energy, A.alpha_minus[k], wo, bs.wi, LOBES_ALL)) *
                       A.inv_2h_alpha;
             A.pend[slot] = m;
             A.pend_albedo[slot] = make_float4(f.r > 0.0f ? fa.r / f.r : 0.0f, f.g > 0.0f ? fa.g / f.g : 0.0f, f.b > 0.0f ? fa.b / f.b : 0.0f, 0.0f);
             A.pend_alpha[slot] = make_float4(f.r > 0.0f ? fr2.r / f.r : 0.0f, f.g > 0.0f ? fr2.g / f.g : 0.0f, f.b > 0.0f ? fr2.b / f.b : 0.0f, 0.0f);
         }
         V3 next_origin = transmitted ? offset_origin(s_hit, -ng) : origin;
-        if (bs.straight) {
+        if (!PLAIN && bs.straight) {
             offset += dot(next_origin - ro, rd);
         } else {
             flags |= PF_HAS_PDF;
@@ -374,7 +375,7 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
             pdf = bs.pdf;
             P.sel[slot] = make_float4(s_point.x, s_point.y, s_point.z, selection.total);
             offset = 0.0f;
-            if (transmitted) {
+            if (!PLAIN && transmitted) {
                 if (s_outside && mat && mat->has_medium) {
                     flags |= PF_MEDIUM;
                     P.medium[slot] = I->material;
@@ -398,6 +399,7 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
 
 // Eight blocks per SM (64 registers, with spills) rather than the compiler's 168 registers: as for
 // k_shade, more warps hide the scattered loads (512^2 adjoint iteration 51.4 -> 48.9 ms).
+template <bool PLAIN>
 __global__ void __launch_bounds__(128, RTG_SHADE_MIN_BLOCKS) k_shade_adjoint(const __grid_constant__ SceneDev S, const LightsDev* __restrict__ Lg, PathBuffers P, int cur, uint32_t bounce,
                                                        WaveDesc w, AdjointDev A) {
     __shared__ float s_grad[MAX_ADJOINT_PARAMS];
@@ -406,7 +408,7 @@ __global__ void __launch_bounds__(128, RTG_SHADE_MIN_BLOCKS) k_shade_adjoint(con
     blk.begin(n_params);
     uint32_t n = *(volatile uint32_t*)&P.counters[cur];
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        shade_adjoint_slot(S, *Lg, P, A, s_grad, P.sorted[i], cur, bounce, w);
+        shade_adjoint_slot<PLAIN>(S, *Lg, P, A, s_grad, P.sorted[i], cur, bounce, w);
     blk.end(n_params, A.grads);
 }
 

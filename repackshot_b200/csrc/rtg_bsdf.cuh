@@ -64,15 +64,19 @@ RTG_HD Ggx make_ggx(float alpha, float anisotropy) {
     }
     return g;
 }
+// `P` (here and below): the BSDF is known to be plain, with an isotropic distribution, no coat and
+// no thin wall (SceneDev::plain); the rest of the code falls away.
+template <bool P = false>
 RTG_HD float ggx_D(const Ggx& g, V3 h) {
-    if (g.iso) return ggx_d(h, g.a2);
+    if (P || g.iso) return ggx_d(h, g.a2);
     float x = h.x / g.ax, y = h.y / g.ay;
     float t = x * x + y * y + h.z * h.z;
     if (t <= 0.0f) return 0.0f;
     return 1.0f / (PI * g.ax * g.ay * t * t);
 }
+template <bool P = false>
 RTG_HD float ggx_L(const Ggx& g, V3 w) {
-    if (g.iso) return ggx_lambda(w, g.a2);
+    if (P || g.iso) return ggx_lambda(w, g.a2);
     float cos2 = w.z * w.z;
     if (cos2 <= 0.0f) return f_inf();
     float x = g.ax * w.x, y = g.ay * w.y;
@@ -357,11 +361,15 @@ RTG_HD Rgb specular_fresnel(const Bsdf& b, float cos) {
                     schlick(b.metal_f0.b, b.metal_f90.b, cos));
     return splat(d) * b.dielectric + metal * b.metallic;
 }
-RTG_HD float coat_fresnel(const Bsdf& b, float cos) { return b.coat <= 0.0f ? 0.0f : b.coat * schlick(COAT_F0, 1.0f, cos); }
-RTG_HD float clear_fresnel(const Bsdf& b, float cos) { return b.thin ? thin_reflectance(cos, b.eta) : fresnel_dielectric(cos, b.eta); }
-RTG_HD float reflect_probability(const Bsdf& b, float cos) { return rmin(clear_fresnel(b, cos), MAX_REFLECT_PROBABILITY); }
+template <bool P = false>
+RTG_HD float coat_fresnel(const Bsdf& b, float cos) { return P || b.coat <= 0.0f ? 0.0f : b.coat * schlick(COAT_F0, 1.0f, cos); }
+template <bool P = false>
+RTG_HD float clear_fresnel(const Bsdf& b, float cos) { return !P && b.thin ? thin_reflectance(cos, b.eta) : fresnel_dielectric(cos, b.eta); }
+template <bool P = false>
+RTG_HD float reflect_probability(const Bsdf& b, float cos) { return rmin(clear_fresnel<P>(b, cos), MAX_REFLECT_PROBABILITY); }
+template <bool P = false>
 RTG_HD float reflect_chance(const Bsdf& b, float mu_o, float cos_h) {
-    return b.ms_clear_on ? clear_fresnel(b, cos_h) : reflect_probability(b, mu_o);
+    return b.ms_clear_on ? clear_fresnel<P>(b, cos_h) : reflect_probability<P>(b, mu_o);
 }
 RTG_HD bool clear_compensation(const EnergyTables& E, const Bsdf& b, TabAt mu_o, float& k) {
     if (!b.ms_clear_on) return false;
@@ -376,6 +384,12 @@ RTG_HD Rgb straight_transmittance(const Bsdf& b, float cos) {
     return b.tint * (b.clear * (1.0f - coat_fresnel(b, cos)) * t);
 }
 
+// layer_passes of the coat; without one it is 1 (a NaN stays one).
+template <bool P = false>
+RTG_HD float coat_passes(const EnergyTables& E, const Bsdf& b, float mu, TabAt at) {
+    if (P) return mu == mu ? 1.0f : mu;
+    return layer_passes(E, b.coat_layer, mu, at);
+}
 // What evaluation, density and sampling at one vertex all take from the outgoing direction alone.
 // wo.z > 0 (below, everything is zero).
 struct BsdfWo {
@@ -384,25 +398,27 @@ struct BsdfWo {
     float lost_spec, lost_coat;                // lobe_lost of the two multiple-scattering lobes (0: off)
     float lambda;                              // ggx_L of the specular distribution
 };
+template <bool P = false>
 RTG_HD BsdfWo bsdf_wo(const EnergyTables& E, const Bsdf& b, V3 wo) {
     BsdfWo o;
     o.at = tab_at(wo.z);
     o.pass_base = layer_passes(E, b.base_layer, wo.z, o.at);
-    o.pass_coat = layer_passes(E, b.coat_layer, wo.z, o.at);
+    o.pass_coat = coat_passes<P>(E, b, wo.z, o.at);
     o.lost_spec = b.ms_spec_on ? lobe_lost(E, b.ms_spec_lobe, o.at) : 0.0f;
-    o.lost_coat = b.ms_coat_on ? lobe_lost(E, b.ms_coat_lobe, o.at) : 0.0f;
-    o.lambda = ggx_L(b.spec, wo);
+    o.lost_coat = !P && b.ms_coat_on ? lobe_lost(E, b.ms_coat_lobe, o.at) : 0.0f;
+    o.lambda = ggx_L<P>(b.spec, wo);
     return o;
 }
+template <bool P = false>
 RTG_HD LobeWeights lobe_weights(const Bsdf& b, const BsdfWo& o, V3 wo) {
-    float c = coat_fresnel(b, wo.z);
+    float c = coat_fresnel<P>(b, wo.z);
     float below = 1.0f - c;
     float specular = has_specular(b) ? below * rmax(luminance(specular_fresnel(b, wo.z)), 0.0f) : 0.0f;
     float diff = below * luminance(b.diffuse) * o.pass_base;
     float cl = below * b.clear;
     float ms = 0.0f;
     if (b.ms_spec_on) ms += below * rmax(luminance(b.ms_spec_colour), 0.0f) * o.lost_spec;
-    if (b.ms_coat_on) ms += b.ms_coat_c * o.lost_coat;
+    if (!P && b.ms_coat_on) ms += b.ms_coat_c * o.lost_coat;
     float total = c + specular + diff + cl + ms;
     LobeWeights w;
     if (total > 0.0f) {
@@ -423,16 +439,17 @@ RTG_HD bool refraction_half(const Bsdf& b, V3 wo, V3 wi, V3& h, float& co, float
 }
 // Value (`f`, when not null) and density (`pdf`, when not null, with the lobe weights `w`) of the
 // refraction wo -> wi, wi.z < 0.
+template <bool P = false>
 RTG_HD void refraction_eval_pdf(const EnergyTables& E, const Bsdf& b, const BsdfWo& o, const LobeWeights* w, V3 wo, V3 wi, Rgb* f, float* pdf) {
     if (f) *f = splat(0.0f);
     if (pdf) *pdf = 0.0f;
     V3 h; float co, ci;
     if (!refraction_half(b, wo, wi, h, co, ci)) return;
-    const float D = ggx_D(b.spec, h);
+    const float D = ggx_D<P>(b.spec, h);
     float denom = co + b.eta * ci;
     if (f) {
         float fr = fresnel_dielectric(co, b.eta);
-        float g2 = 1.0f / (1.0f + o.lambda + ggx_L(b.spec, wi));
+        float g2 = 1.0f / (1.0f + o.lambda + ggx_L<P>(b.spec, wi));
         float value = (1.0f - fr) * D * g2 * (-ci) * co / (-wi.z * wo.z * denom * denom);
         float k;
         if (clear_compensation(E, b, o.at, k)) value *= k;
@@ -442,20 +459,21 @@ RTG_HD void refraction_eval_pdf(const EnergyTables& E, const Bsdf& b, const Bsdf
         float g1 = 1.0f / (1.0f + o.lambda);
         float visible = g1 * D * co / wo.z;
         float jacobian = b.eta * b.eta * (-ci) / (denom * denom);
-        *pdf = w->clear * (1.0f - reflect_chance(b, wo.z, co)) * visible * jacobian;
+        *pdf = w->clear * (1.0f - reflect_chance<P>(b, wo.z, co)) * visible * jacobian;
     }
 }
 // Value of the BSDF for the lobes asked for and (with `w`, when `pdf` is not null) the density of
 // its sampling, for wo.z > 0: the half vector, the distribution and the terms of wo are shared.
+template <bool P = false>
 RTG_HD_NI void bsdf_eval_pdf(const EnergyTables& E, const Bsdf& b, const BsdfWo& o, const LobeWeights* w, V3 wo, V3 wi, int lobes, Rgb& f, float* pdf) {
     f = splat(0.0f);
     if (pdf) *pdf = 0.0f;
     if (wi.z <= 0.0f) {
-        if (wi.z < 0.0f && b.clear > 0.0f && !b.thin) refraction_eval_pdf(E, b, o, w, wo, wi, lobes == LOBES_ALL ? &f : nullptr, pdf);
+        if (wi.z < 0.0f && b.clear > 0.0f && (P || !b.thin)) refraction_eval_pdf<P>(E, b, o, w, wo, wi, lobes == LOBES_ALL ? &f : nullptr, pdf);
         return;
     }
     const TabAt at = tab_at(wi.z);
-    float attenuation = o.pass_coat * layer_passes(E, b.coat_layer, wi.z, at);
+    float attenuation = o.pass_coat * coat_passes<P>(E, b, wi.z, at);
     Rgb diff = b.diffuse * (FRAC_1_PI * o.pass_base * layer_passes(E, b.base_layer, wi.z, at) * b.diffuse_norm);
     if (lobes == LOBES_DIFFUSE) {
         f = diff * attenuation;
@@ -467,15 +485,15 @@ RTG_HD_NI void bsdf_eval_pdf(const EnergyTables& E, const Bsdf& b, const BsdfWo&
     const bool spec_on = has_specular(b) || b.clear > 0.0f;
     float D = 0.0f, micro = 0.0f, refl = 0.0f, refl_coat = 0.0f, micro_coat = 0.0f;
     if (spec_on) {
-        D = ggx_D(b.spec, h);
-        float g2 = 1.0f / (1.0f + o.lambda + ggx_L(b.spec, wi));
+        D = ggx_D<P>(b.spec, h);
+        float g2 = 1.0f / (1.0f + o.lambda + ggx_L<P>(b.spec, wi));
         micro = D * g2 / (4.0f * wo.z * wi.z);
         if (pdf) {
             float g1 = 1.0f / (1.0f + o.lambda);
             refl = g1 * D / (4.0f * wo.z);
         }
     }
-    if (b.coat > 0.0f) {
+    if (!P && b.coat > 0.0f) {
         const float Dc = ggx_D(b.coat_ggx, h), lo = ggx_L(b.coat_ggx, wo);
         float g2 = 1.0f / (1.0f + lo + ggx_L(b.coat_ggx, wi));
         micro_coat = Dc * g2 / (4.0f * wo.z * wi.z);
@@ -484,10 +502,10 @@ RTG_HD_NI void bsdf_eval_pdf(const EnergyTables& E, const Bsdf& b, const BsdfWo&
     }
     if (pdf) {  // pdf_with (bsdf.rs:776)
         float p = (w->diffuse + w->ms) * wi.z * FRAC_1_PI;
-        if ((w->specular > 0.0f || w->coat > 0.0f || w->clear > 0.0f) && wo_h > 0.0f) {
+        if ((w->specular > 0.0f || (!P && w->coat > 0.0f) || w->clear > 0.0f) && wo_h > 0.0f) {
             if (w->specular > 0.0f) p += w->specular * refl;
-            if (w->coat > 0.0f) p += w->coat * refl_coat;
-            if (w->clear > 0.0f) p += w->clear * reflect_chance(b, wo.z, wo_h) * refl;
+            if (!P && w->coat > 0.0f) p += w->coat * refl_coat;
+            if (w->clear > 0.0f) p += w->clear * reflect_chance<P>(b, wo.z, wo_h) * refl;
         }
         *pdf = p;
     }
@@ -496,39 +514,42 @@ RTG_HD_NI void bsdf_eval_pdf(const EnergyTables& E, const Bsdf& b, const BsdfWo&
     if (has_specular(b)) below = below + specular_fresnel(b, cos_h) * micro;
     if (b.ms_spec_on) below = below + b.ms_spec_colour * (o.lost_spec * lobe_lost(E, b.ms_spec_lobe, at) * b.ms_spec_lobe.norm);
     if (b.clear > 0.0f) {
-        float cl = b.clear * clear_fresnel(b, cos_h) * micro;
+        float cl = b.clear * clear_fresnel<P>(b, cos_h) * micro;
         float k;
         if (clear_compensation(E, b, o.at, k)) cl *= k;
         below = below + splat(cl);
     }
     f = below * attenuation;
-    if (b.coat > 0.0f) f = f + splat(coat_fresnel(b, cos_h) * micro_coat);
-    if (b.ms_coat_on) f = f + splat(b.ms_coat_c * (o.lost_coat * lobe_lost(E, b.ms_coat_lobe, at) * b.ms_coat_lobe.norm));
+    if (!P && b.coat > 0.0f) f = f + splat(coat_fresnel(b, cos_h) * micro_coat);
+    if (!P && b.ms_coat_on) f = f + splat(b.ms_coat_c * (o.lost_coat * lobe_lost(E, b.ms_coat_lobe, at) * b.ms_coat_lobe.norm));
 }
 // The value alone.
+template <bool P = false>
 RTG_HD Rgb bsdf_eval(const EnergyTables& E, const Bsdf& b, V3 wo, V3 wi, int lobes) {
     Rgb f = splat(0.0f);
-    if (!(wo.z <= 0.0f)) bsdf_eval_pdf(E, b, bsdf_wo(E, b, wo), nullptr, wo, wi, lobes, f, nullptr);
+    if (!(wo.z <= 0.0f)) bsdf_eval_pdf<P>(E, b, bsdf_wo<P>(E, b, wo), nullptr, wo, wi, lobes, f, nullptr);
     return f;
 }
 
+template <bool P = false>
 RTG_HD bool finish_reflection(const EnergyTables& E, const Bsdf& b, const BsdfWo& o, const LobeWeights& w, V3 wo, V3 wi, BsdfSample& out) {
     if (wi.z <= 0.0f) return false;
     Rgb f;
     float p;
-    bsdf_eval_pdf(E, b, o, &w, wo, wi, LOBES_ALL, f, &p);
+    bsdf_eval_pdf<P>(E, b, o, &w, wo, wi, LOBES_ALL, f, &p);
     if (!(p > 0.0f && finitef(p))) return false;
     out.weight = f * (wi.z / p);
     out.wi = wi; out.pdf = p; out.straight = false;
     return true;
 }
+template <bool P = false>
 RTG_HD bool finish_refraction(const EnergyTables& E, const Bsdf& b, const BsdfWo& o, const LobeWeights& w, V3 wo, V3 h, BsdfSample& out) {
     V3 wi;
     if (!refract(wo, h, b.eta, wi)) return false;
     if (wi.z >= 0.0f) return false;
     Rgb f;
     float p;
-    bsdf_eval_pdf(E, b, o, &w, wo, wi, LOBES_ALL, f, &p);
+    bsdf_eval_pdf<P>(E, b, o, &w, wo, wi, LOBES_ALL, f, &p);
     if (!(p > 0.0f && finitef(p))) return false;
     out.weight = f * (-wi.z / p);
     out.wi = wi; out.pdf = p; out.straight = false;
@@ -536,10 +557,11 @@ RTG_HD bool finish_refraction(const EnergyTables& E, const Bsdf& b, const BsdfWo
 }
 // A direction for wo (wo.z > 0) with its value and density. A reflection ends in one evaluation, at
 // the bottom, and a refraction in another, so their code is there once each.
+template <bool P = false>
 RTG_HD_NI bool bsdf_sample(const EnergyTables& E, const Bsdf& b, const BsdfWo& o, const LobeWeights& w, V3 wo, float u0, float u1, BsdfSample& out) {  // bsdf.rs:833
     V3 wi, h;
     bool through = false;
-    if (u0 < w.coat) {
+    if (!P && u0 < w.coat) {
         h = sample_vndf(wo, b.coat_ggx.ax, b.coat_ggx.ay, u0 / w.coat, u1);
         wi = h * (2.0f * dot(wo, h)) - wo;
     } else if (u0 < w.coat + w.specular) {
@@ -556,14 +578,14 @@ RTG_HD_NI bool bsdf_sample(const EnergyTables& E, const Bsdf& b, const BsdfWo& o
         if (b.ms_clear_on) {
             // sample_rough_clear (bsdf.rs:947)
             h = sample_vndf(wo, b.spec.ax, b.spec.ay, uc, u1);
-            float fr = clear_fresnel(b, dot(wo, h));
+            float fr = clear_fresnel<P>(b, dot(wo, h));
             uint64_t key = ((uint64_t)fbits(uc) << 32) | (uint64_t)fbits(u1);
             float choice = (float)(mix64(key ^ 0x9e3779b97f4a7c15ULL) >> 40) * (1.0f / 16777216.0f);
             through = !(choice < fr);
         } else {
-            float pr = reflect_probability(b, wo.z);
+            float pr = reflect_probability<P>(b, wo.z);
             through = !(uc < pr);
-            if (through && b.thin) {
+            if (!P && through && b.thin) {
                 float chance = w.clear * (1.0f - pr);
                 if (chance != chance || chance <= 0.0f) return false;
                 out.weight = straight_transmittance(b, wo.z) / chance;
@@ -576,7 +598,7 @@ RTG_HD_NI bool bsdf_sample(const EnergyTables& E, const Bsdf& b, const BsdfWo& o
     } else {
         return false;
     }
-    return through ? finish_refraction(E, b, o, w, wo, h, out) : finish_reflection(E, b, o, w, wo, wi, out);
+    return through ? finish_refraction<P>(E, b, o, w, wo, h, out) : finish_reflection<P>(E, b, o, w, wo, wi, out);
 }
 
 }  // namespace rtg

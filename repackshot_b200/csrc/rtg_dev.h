@@ -153,6 +153,10 @@ struct SceneDev {
     // Some instance lets shadow rays through (a cut-out or a thin wall); some material is a cut-out
     // (paths then pass surfaces without a vertex, and waves run extra rounds).
     uint32_t any_passable, any_cutout;
+    // The common scene: area lights and the ramp environment only; no emissive, cut-out, absorbing,
+    // thin, coated or anisotropic material; no floor plane, background image or section. The shade
+    // kernels have a variant for it (scene_plain).
+    uint32_t plain;
     uint32_t floor_mode;
     float floor_z;
     float floor_color[3];

@@ -1184,6 +1184,7 @@ uint32_t rtg_queue_run(uint32_t queue, uint32_t flags, uint64_t* rays) {
         Sw.max_depth = std::max(Sw.max_depth, J.constants.max_depth);
         Sw.any_cutout |= J.constants.any_cutout;
         Sw.any_passable |= J.constants.any_passable;
+        Sw.plain &= J.constants.plain;
         total += (uint64_t)J.width * J.height * J.count;
     }
     if (total == 0) {

@@ -328,13 +328,14 @@ __global__ void k_scatter(PathBuffers P, int cur, const uint32_t* __restrict__ i
 // the path's pixel and sample index (the sampler's key).
 // With P.rbins set, each surviving path's next ray gets its coherence key (in P.key) and is counted
 // in the histogram; with P.sbins set, each shadow ray likewise (in P.sh_key).
+// PLAIN: the scene is plain (SceneDev::plain); what it cannot hold falls away from the code.
 // With `tail` (the tail kernel), the shadow ray goes to *tail instead of the shadow queue and the
 // surviving path to no queue. Returns whether the path goes on.
 struct TailShadow {
     bool on;
     float4 o, d, c;
 };
-template <class XYI>
+template <bool PLAIN, class XYI>
 __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L, const PathBuffers& P, const RaySort& R, uint32_t slot, int cur,
                                            XYI xyi, uint32_t& rays_local, uint32_t& shadow_local, TailShadow* tail = nullptr) {
     float4 o4 = P.o[slot], d4 = P.d[slot], thr4 = P.thr[slot], sum = P.sum[slot];
@@ -350,12 +351,12 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
     float t_geometry = hit.w ? __uint_as_float(hit.z) : f_inf();
     // floor_t (integrator/mod.rs:493)
     float t_floor = f_inf();
-    if ((S.floor_mode == 1) && rd.z != 0.0f && !(flags & PF_NOTHING)) {
+    if (!PLAIN && S.floor_mode == 1 && rd.z != 0.0f && !(flags & PF_NOTHING)) {
         float t = (S.floor_z - ro.z) / rd.z;
         if (t > 1.0e-3f && t < f_inf()) t_floor = t;
     }
     float t_nearest = rmin(t_geometry, t_floor);
-    if ((flags & PF_MEDIUM) && finitef(t_nearest)) {
+    if (!PLAIN && (flags & PF_MEDIUM) && finitef(t_nearest)) {
         const DevMaterial& mm = S.materials[P.medium[slot]];
         thr = thr * rgb(fexp(-mm.sigma[0] * t_nearest), fexp(-mm.sigma[1] * t_nearest), fexp(-mm.sigma[2] * t_nearest));
     }
@@ -364,16 +365,16 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
     from.p = v3(sel4.x, sel4.y, sel4.z);
     from.by_flux = !(L.per_point && L.n_entries > 0);
     from.total = sel4.w;
-    Rgb crossed = crossed_from(L, ro, rd, 1.0e-3f, t_nearest, has_pdf, pdf, from, offset);
+    Rgb crossed = crossed_from<PLAIN>(L, ro, rd, 1.0e-3f, t_nearest, has_pdf, pdf, from, offset);
     add_clamped(sum, thr * crossed, bounce >= 2, S.clamp_indirect);
     bool alive = false;
     do {
         if (t_nearest == f_inf()) {
             if (primary && S.background == 0) {
-                Rgb seen = escaped(L, rd, false, 0.0f, from);
+                Rgb seen = escaped<PLAIN>(L, rd, false, 0.0f, from);
                 Rgb c = thr * (S.exterior == 1.0f ? seen : seen * S.exterior);
                 sum.x = sum.x + c.r; sum.y = sum.y + c.g; sum.z = sum.z + c.b;
-            } else if (primary && (S.background == 1 || S.background == 3)) {
+            } else if (primary && (S.background == 1 || (!PLAIN && S.background == 3))) {
                 uint32_t x, y, index;
                 xyi(x, y, index);
                 float su, sv;
@@ -383,7 +384,7 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
             } else if (primary && S.background == 2) {
                 alpha = peak(crossed) > 0.0f ? 1.0f : 0.0f;
             } else {
-                add_clamped(sum, thr * escaped(L, rd, has_pdf, pdf, from), bounce >= 2, S.clamp_indirect);
+                add_clamped(sum, thr * escaped<PLAIN>(L, rd, has_pdf, pdf, from), bounce >= 2, S.clamp_indirect);
             }
             break;
         }
@@ -392,7 +393,7 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
         uint32_t inst = 0;
         const DevInstance* I = nullptr;
         const DevMaterial* mat = nullptr;
-        if (t_floor < t_geometry) {
+        if (!PLAIN && t_floor < t_geometry) {
             V3 pp = ro + rd * t_floor;
             V3 point = v3(pp.x, pp.y, S.floor_z);
             V3 nn = v3(0.0f, 0.0f, rd.z < 0.0f ? 1.0f : -1.0f);
@@ -400,7 +401,7 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
         } else {
             HitInfo h;
             uint4 idx;
-            if (!hit_details(S, ro, rd, 1.0e-3f, f_inf(), hit.x, hit.y, __uint_as_float(hit.z), h, I, idx)) break;
+            if (!hit_details<PLAIN>(S, ro, rd, 1.0e-3f, f_inf(), hit.x, hit.y, __uint_as_float(hit.z), h, I, idx)) break;
             // bevel.rs:232 shading_point without a bevel
             V3 ng = h.geometric, nrm = h.normal;
             if (dot(nrm, ng) < 0.0f) nrm = -nrm;
@@ -413,7 +414,7 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
             inst = hit.x;
             s_outside = h.outside;
             mat = S.materials + I->material;
-            if (mat->kind == MATERIAL_EMISSIVE) {
+            if (!PLAIN && mat->kind == MATERIAL_EMISSIVE) {
                 // A BSDF-sampled ray that finds a mesh light weighs it against the light's own
                 // sample (integrator/mod.rs:1556); other emitters and camera rays weigh 1.
                 if (h.front || !(I->flags & 1u)) {
@@ -426,7 +427,7 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
             // direction, density and selection; the path goes back to the extension queue
             // (integrator/mod.rs:1571).
             const uint32_t cut = (flags & PF_CUT_MASK) >> PF_CUT_SHIFT;
-            if (S.any_cutout && mat->opacity < 1.0f && cut < MAX_CUTOUTS) {
+            if (!PLAIN && S.any_cutout && mat->opacity < 1.0f && cut < MAX_CUTOUTS) {
                 uint32_t x, y, index;
                 xyi(x, y, index);
                 const float u = sample_at(S, c_sobol, sample_key(S, x, y, index), index, cutout_dim(bounce, cut));
@@ -442,10 +443,10 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
             }
         }
         if (bounce >= S.max_depth) break;
-        const Bsdf& b = S.bsdfs[mat ? 2 * I->material + (s_outside ? 0 : 1) : 2 * S.n_materials];
+        const Bsdf& b = S.bsdfs[PLAIN || mat ? 2 * I->material + (s_outside ? 0 : 1) : 2 * S.n_materials];
         // Prepared::frame (integrator/mod.rs:833)
         Frame fr = frame_from_normal(s_normal);
-        if (s_inst && I->tangent_on) {
+        if (!PLAIN && s_inst && I->tangent_on) {
             V3 cands[2] = {cross(ld3(I->tan_axis), s_point - ld3(I->tan_centre)), ld3(I->tan_x)};
             for (int k = 0; k < 2; ++k) {
                 V3 t = cands[k] - s_normal * dot(s_normal, cands[k]);
@@ -465,25 +466,25 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
         xyi(x, y, index);
         uint64_t key = sample_key(S, x, y, index);
         // Next-event estimation: one light; the shadow ray goes to the shadow queue.
-        const BsdfWo bo = bsdf_wo(S.energy, b, wo);
-        const LobeWeights lobes = lobe_weights(b, bo, wo);
+        const BsdfWo bo = bsdf_wo<PLAIN>(S.energy, b, wo);
+        const LobeWeights lobes = lobe_weights<PLAIN>(b, bo, wo);
         float weights[SEL_KEPT];
-        Sel selection = select_at(L, s_point, weights);
+        Sel selection = select_at<PLAIN>(L, s_point, weights);
         LightSample ls;
-        if (sample_light(L, selection, weights, sample_at(S, c_sobol, key, index, dims + OFF_LIGHT_SELECT), sample_at(S, c_sobol, key, index, dims + OFF_LIGHT),
+        if (sample_light<PLAIN>(L, selection, weights, sample_at(S, c_sobol, key, index, dims + OFF_LIGHT_SELECT), sample_at(S, c_sobol, key, index, dims + OFF_LIGHT),
                          sample_at(S, c_sobol, key, index, dims + OFF_LIGHT + 1), ls)) {
             V3 wi = to_local(fr, ls.wi);
             const bool mis = ls.glossy && !ls.delta;
             Rgb f;
             float bsdf_density = 0.0f;
-            bsdf_eval_pdf(S.energy, b, bo, &lobes, wo, wi, ls.glossy ? LOBES_ALL : LOBES_DIFFUSE, f, mis ? &bsdf_density : nullptr);
+            bsdf_eval_pdf<PLAIN>(S.energy, b, bo, &lobes, wo, wi, ls.glossy ? LOBES_ALL : LOBES_DIFFUSE, f, mis ? &bsdf_density : nullptr);
             if (peak(f) > 0.0f) {
                 V3 from_p = wi.z < 0.0f ? offset_origin(s_hit, -ng) : origin;
                 float weight = mis ? power_heuristic(ls.pdf, bsdf_density) : 1.0f;
                 Rgb c = thr * f * ls.radiance * (absf(wi.z) * weight / ls.pdf);
                 bool finite_c = finitef(c.r) && finitef(c.g) && finitef(c.b);
                 // The clamp applies to what arrives: after the shadow walk when it may attenuate.
-                const bool walk = ls.shadow && S.any_passable;
+                const bool walk = !PLAIN && ls.shadow && S.any_passable;
                 if (finite_c && bounce >= 1 && S.clamp_indirect > 0.0f && !walk) {
                     float p = rmax(rmax(c.r, c.g), c.b);
                     if (p > S.clamp_indirect) c = c * (S.clamp_indirect / p);
@@ -494,7 +495,7 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
                     shadow_local += 1;
                     float tmax = finitef(ls.distance) ? ls.distance * (1.0f - 1.0e-4f) : f_inf();
                     bool floor_blocks = false;
-                    if (S.floor_mode == 1 && ls.wi.z != 0.0f) {
+                    if (!PLAIN && S.floor_mode == 1 && ls.wi.z != 0.0f) {
                         float t = (S.floor_z - from_p.z) / ls.wi.z;
                         floor_blocks = t > 1.0e-3f && t < tmax;
                     }
@@ -524,10 +525,10 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
         }
         // The next direction.
         BsdfSample bs;
-        if (!bsdf_sample(S.energy, b, bo, lobes, wo, sample_at(S, c_sobol, key, index, dims + OFF_BSDF), sample_at(S, c_sobol, key, index, dims + OFF_BSDF + 1), bs))
+        if (!bsdf_sample<PLAIN>(S.energy, b, bo, lobes, wo, sample_at(S, c_sobol, key, index, dims + OFF_BSDF), sample_at(S, c_sobol, key, index, dims + OFF_BSDF + 1), bs))
             break;
         bool transmitted = bs.wi.z < 0.0f;
-        V3 wi = bs.straight ? rd : normalize(to_world(fr, bs.wi));
+        V3 wi = !PLAIN && bs.straight ? rd : normalize(to_world(fr, bs.wi));
         if (transmitted) {
             if (dot(wi, ng) >= 0.0f) break;
         } else if (dot(wi, ng) <= 0.0f) {
@@ -542,7 +543,7 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
         float pk = peak(thr);
         if (!(pk > 0.0f && finitef(pk))) break;
         V3 next_origin = transmitted ? offset_origin(s_hit, -ng) : origin;
-        if (bs.straight) {
+        if (!PLAIN && bs.straight) {
             offset += dot(next_origin - ro, rd);
         } else {
             flags |= PF_HAS_PDF;
@@ -550,7 +551,7 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
             pdf = bs.pdf;
             P.sel[slot] = make_float4(s_point.x, s_point.y, s_point.z, selection.total);
             offset = 0.0f;
-            if (transmitted) {
+            if (!PLAIN && transmitted) {
                 if (s_outside && mat && mat->has_medium) {
                     flags |= PF_MEDIUM;
                     P.medium[slot] = I->material;
@@ -581,16 +582,20 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
 
 // BATCH: the slots belong to the jobs of a batched wave, each with its own constants and lights.
 // Eight blocks per SM (64 registers, with some spills) beat the 128 registers the compiler would
-// use on its own: the kernel waits on scattered hit-detail loads, and more warps hide them (1080p
-// frame: 369 -> 383 Mpaths/s; 5, 6 and 7 blocks measured 367, 379 and 372).
+// use on its own: the kernel waits on scattered hit-detail loads, and more warps hide them.
 // Instruction fetch and issue weigh as much as the loads (4,200 instructions a vertex before), so a
 // vertex computes nothing twice: the BSDF's terms of wo and the half vector's are shared by value,
 // density and sampling, the light weights by sum and pick, the selection's sum is kept for the next
 // vertex's MIS weights, sampler columns and table cells come summed and packed from tables, and
 // slots are divided by multiplication. 1080p frame 229.0 -> 210.8 ms, studio still 32.1 -> 23.9 ms,
 // 512^2 fit iteration 47.3 -> 39.3 ms (the last two with the shorter node steps), films bit-equal.
+// PLAIN: the variant for plain scenes (SceneDev::plain). A vertex of one still went past the code of
+// every light, environment and material, and the kernel's size is what its instruction fetch stalls
+// on (3.4-7.4 of some 18 stall cycles an issue): 1080p frame 210.8 -> 192.6 ms, 512^2 fit iteration
+// 39.3 -> 32.8 ms. Other scenes take the general kernel, as before. At 4, 5, 6, 7, 8 and 10 blocks an
+// SM the frame takes 195.4, 198.4, 199.7, 197.7, 192.7 and 202.2 ms.
 // `order`: the active queue in the order to shade it (material-sorted, or as traced).
-template <bool BATCH>
+template <bool BATCH, bool PLAIN>
 __global__ void __launch_bounds__(128, RTG_SHADE_MIN_BLOCKS) k_shade(const __grid_constant__ SceneDev S, const LightsDev* __restrict__ Lg, PathBuffers P, int cur, WaveDesc w,
                                                   const uint32_t* __restrict__ order, RaySort R) {
     uint32_t n = *(volatile uint32_t*)&P.counters[cur];
@@ -601,10 +606,10 @@ __global__ void __launch_bounds__(128, RTG_SHADE_MIN_BLOCKS) k_shade(const __gri
             uint32_t job, x, y, index;
             batch_slot(w, slot, job, x, y, index);
             const JobDev& J = w.jobs[job];
-            shade_slot(J.S, *J.lights, P, R, slot, cur, [&](uint32_t& xx, uint32_t& yy, uint32_t& ii) { xx = x; yy = y; ii = index; },
+            shade_slot<PLAIN>(J.S, *J.lights, P, R, slot, cur, [&](uint32_t& xx, uint32_t& yy, uint32_t& ii) { xx = x; yy = y; ii = index; },
                        rays_local, shadow_local);
         } else {
-            shade_slot(S, *Lg, P, R, slot, cur, [&](uint32_t& xx, uint32_t& yy, uint32_t& ii) { wave_slot(w, slot, xx, yy, ii); },
+            shade_slot<PLAIN>(S, *Lg, P, R, slot, cur, [&](uint32_t& xx, uint32_t& yy, uint32_t& ii) { wave_slot(w, slot, xx, yy, ii); },
                        rays_local, shadow_local);
         }
     }
@@ -784,6 +789,7 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_shadow_walk(const __grid_cons
 // of a chain of launches, each as long as its slowest ray. k_tail_end then empties the queue, so
 // the later rounds' launches find no work. Scenes with passable surfaces (shadow walks) and
 // batched waves keep the wavefront.
+template <bool PLAIN>
 __global__ void __launch_bounds__(TRACE_THREADS) k_tail(const __grid_constant__ SceneDev S, const LightsDev* __restrict__ Lg, PathBuffers P, int cur, WaveDesc w, uint32_t rounds_left,
                                         uint32_t limit) {
     const uint32_t n = *(volatile uint32_t*)&P.counters[cur];
@@ -805,7 +811,7 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_tail(const __grid_constant__ 
             P.hit[slot] = got ? make_uint4(res.inst, res.tri, __float_as_uint(res.t), 1u) : make_uint4(0xffffffffu, 0xffffffffu, 0u, 0u);
             TailShadow sh;
             sh.on = false;
-            const bool alive = shade_slot(S, *Lg, P, R, slot, cur, [&](uint32_t& xx, uint32_t& yy, uint32_t& ii) { wave_slot(w, slot, xx, yy, ii); },
+            const bool alive = shade_slot<PLAIN>(S, *Lg, P, R, slot, cur, [&](uint32_t& xx, uint32_t& yy, uint32_t& ii) { wave_slot(w, slot, xx, yy, ii); },
                                           rays_local, shadow_local, &sh);
             if (sh.on) {
                 TraceResult unused;
@@ -1340,7 +1346,7 @@ void launch_wave(const SceneDev& S, const LightsDev* L, const WaveDesc& wave, co
                  int grid, WaveTiming* timing, const RaySort& order) {
     static const int ext_resident = resident_blocks((const void*)k_extend, TRACE_THREADS);
     static const int sh_resident = resident_blocks((const void*)k_shadow, TRACE_THREADS);
-    static const int tail_resident = resident_blocks((const void*)k_tail, TRACE_THREADS);
+    static const int tail_resident = resident_blocks((const void*)k_tail<false>, TRACE_THREADS);
     const WaveDesc w = with_divisors(wave);
     const int g = grid;
     const int g_ext = ext_resident > 0 && ext_resident < g ? ext_resident : g;
@@ -1356,7 +1362,7 @@ void launch_wave(const SceneDev& S, const LightsDev* L, const WaveDesc& wave, co
     const bool tail = tail_on(S, order, batch);
     for (uint32_t round = 0; round < rounds; ++round) {
         if (tail && round >= TAIL_FIRST_ROUND) {
-            k_tail<<<tail_resident > 0 ? tail_resident : g, TRACE_THREADS, 0, st>>>(S, L, P, cur, w, rounds - round, order.tail_paths);
+            (S.plain ? k_tail<true> : k_tail<false>)<<<tail_resident > 0 ? tail_resident : g, TRACE_THREADS, 0, st>>>(S, L, P, cur, w, rounds - round, order.tail_paths);
             k_tail_end<<<1, 1, 0, st>>>(P, cur, order.tail_paths);
         }
         // The camera rays are traced in pixel order; later rounds' rays in coherence order.
@@ -1386,8 +1392,8 @@ void launch_wave(const SceneDev& S, const LightsDev* L, const WaveDesc& wave, co
         PathBuffers Q = P;
         Q.rbins = rsort && round + 1 < rounds ? P.rbins : nullptr;
         Q.sbins = ssort ? P.sbins : nullptr;
-        if (batch) k_shade<true><<<g, 128, 0, st>>>(S, L, Q, cur, w, shaded, order);
-        else k_shade<false><<<g, 128, 0, st>>>(S, L, Q, cur, w, shaded, order);
+        (batch ? (S.plain ? k_shade<true, true> : k_shade<true, false>) : (S.plain ? k_shade<false, true> : k_shade<false, false>))
+            <<<g, 128, 0, st>>>(S, L, Q, cur, w, shaded, order);
         // queue[cur] is free once shade has read its list: it holds the shadow rays' order.
         const uint32_t* perm = nullptr;
         if (ssort) {
@@ -1447,7 +1453,7 @@ void launch_adjoint_wave(const SceneDev& S, const LightsDev* L, const WaveDesc& 
         k_extend<<<g_ext, TRACE_THREADS, 0, st>>>(S, P, cur, P.queue[cur]);
         k_scan<<<1, 32, 0, st>>>(P);
         k_scatter<<<g, 256, 0, st>>>(P, cur, P.queue[cur], P.sorted);
-        k_shade_adjoint<<<g, 128, 0, st>>>(S, L, P, cur, bounce, w, A);
+        (S.plain ? k_shade_adjoint<true> : k_shade_adjoint<false>)<<<g, 128, 0, st>>>(S, L, P, cur, bounce, w, A);
         k_shadow_adjoint<<<g_sh, TRACE_THREADS, 0, st>>>(S, P, w, A);
         k_next_round<<<1, 1, 0, st>>>(P, cur);
         cur ^= 1;

@@ -1321,6 +1321,10 @@ static bool flatten(const HScene& s, Flat& F, std::string& error, bool geometry,
         const HMaterial& m = s.materials[in.material_id];
         if (m.kind != MATERIAL_EMISSIVE && m.opacity < 1.0f) S.any_cutout = 1;
     }
+    S.plain = s.floor_mode == 0 && S.background != 3 && !S.section_on && !S.any_cutout && !S.any_passable && !F.lights.env_is_map;
+    for (uint32_t i = 0; i < F.lights.n_lights; ++i) S.plain &= F.lights.lights[i].kind == LIGHT_AREA;
+    for (const DevMaterial& d : F.materials) S.plain &= d.kind != MATERIAL_EMISSIVE && !d.has_medium;
+    for (const Bsdf& b : F.bsdfs) S.plain &= b.coat == 0.0f && !b.ms_coat_on && !(b.thin && b.clear > 0.0f) && b.spec.iso;
     S.floor_mode = s.floor_mode;
     S.floor_z = s.floor_z;
     for (int c = 0; c < 3; ++c) S.floor_color[c] = s.floor_color[c];

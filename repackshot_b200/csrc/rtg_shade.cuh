@@ -132,10 +132,14 @@ RTG_D bool ramp_sample(const LightsDev& L, float u0, float u1, V3& dir, float& p
     return pdf > 0.0f;
 }
 // EnvLight (environment.rs:333): the map or the ramp.
-RTG_D Rgb env_radiance(const LightsDev& L, V3 dir) { return L.env_is_map ? map_radiance(L.env_map, dir) : splat(env_value(L, dir.z)); }
-RTG_D float env_pdf(const LightsDev& L, V3 dir) { return L.env_is_map ? map_pdf(L.env_map, dir) : ramp_pdf(L, dir); }
+// `P` (here and below): a plain scene (SceneDev::plain): area lights and the ramp only.
+template <bool P = false>
+RTG_D Rgb env_radiance(const LightsDev& L, V3 dir) { return !P && L.env_is_map ? map_radiance(L.env_map, dir) : splat(env_value(L, dir.z)); }
+template <bool P = false>
+RTG_D float env_pdf(const LightsDev& L, V3 dir) { return !P && L.env_is_map ? map_pdf(L.env_map, dir) : ramp_pdf(L, dir); }
+template <bool P = false>
 RTG_D bool env_sample(const LightsDev& L, float u0, float u1, V3& dir, float& pdf) {
-    return L.env_is_map ? map_sample(L.env_map, u0, u1, dir, pdf) : ramp_sample(L, u0, u1, dir, pdf);
+    return !P && L.env_is_map ? map_sample(L.env_map, u0, u1, dir, pdf) : ramp_sample(L, u0, u1, dir, pdf);
 }
 
 // ---- background image (integrator/mod.rs:199-232) -----------------------------------------------------
@@ -167,15 +171,17 @@ RTG_D Rgb backdrop(const SceneDev& S, float su, float sv) {
 // computed again from the point, with the same operations.
 struct Sel { V3 p; float total; bool by_flux; };
 constexpr int SEL_KEPT = 8;  // weights that select_at leaves for the pick at the same vertex
+template <bool P = false>
 RTG_D float entry_weight(const LightsDev& L, int e, V3 x) {  // light.rs:1014
     int a = L.entries[e];
     if (a < 0) return L.env_base;
     const LightDev& l = L.lights[a];
-    if (l.kind == LIGHT_AREA) return area_weight(l, x);
+    if (P || l.kind == LIGHT_AREA) return area_weight(l, x);
     if (l.kind == LIGHT_SUN) return l.base;
     if (l.kind == LIGHT_MESH) return mesh_weight(l, x);
     return sphere_weight(l, x);
 }
+template <bool P = false>
 RTG_D Sel select_at(const LightsDev& L, V3 x, float* weights) {
     Sel s;
     s.p = x;
@@ -183,17 +189,18 @@ RTG_D Sel select_at(const LightsDev& L, V3 x, float* weights) {
     s.by_flux = !(L.per_point && L.n_entries > 0);
     if (!s.by_flux)
         for (int e = 0; e < L.n_entries; ++e) {
-            const float w = entry_weight(L, e, x);
+            const float w = entry_weight<P>(L, e, x);
             if (e < SEL_KEPT) weights[e] = w;
             s.total += w;
         }
     return s;
 }
+template <bool P = false>
 RTG_D float pmf_of(const LightsDev& L, uint32_t entry, const Sel& s) {
     if ((int)entry >= L.n_entries) return 0.0f;
     if (s.by_flux) return L.flux_pmf[entry];
     if (!(s.total > 0.0f && finitef(s.total))) return 0.0f;
-    return entry_weight(L, (int)entry, s.p) / s.total;
+    return entry_weight<P>(L, (int)entry, s.p) / s.total;
 }
 RTG_D float power_heuristic(float pa, float pb) {
     if (!(pa > 0.0f)) return 0.0f;
@@ -214,6 +221,7 @@ RTG_D float emitter_weight(const LightsDev& L, uint32_t emitter, float pdf, cons
 // light: index into lights[], -1 the environment; delta: no other technique finds it
 struct LightSample { V3 wi; float distance; Rgb radiance; float pdf; bool glossy, shadow, delta; int light; };
 
+template <bool P = false>
 RTG_D_NI bool sample_light(const LightsDev& L, const Sel& s, const float* weights, float u_select, float u0, float u1, LightSample& out) {  // light.rs:1150
     int n = L.n_entries;
     if (n == 0) return false;
@@ -223,7 +231,7 @@ RTG_D_NI bool sample_light(const LightsDev& L, const Sel& s, const float* weight
         int k = 0;
         while (k < n && L.cdf[k] <= u_select) ++k;
         index = k < n - 1 ? k : n - 1;
-        pmf = pmf_of(L, (uint32_t)index, s);
+        pmf = pmf_of<P>(L, (uint32_t)index, s);
         const float lo = index == 0 ? 0.0f : L.cdf[index - 1], width = L.cdf[index] - lo;
         rest = width > 0.0f ? rclamp((u_select - lo) / width, 0.0f, 0.99999994f) : 0.0f;
     } else {
@@ -232,7 +240,7 @@ RTG_D_NI bool sample_light(const LightsDev& L, const Sel& s, const float* weight
         float acc = 0.0f, lo = 0.0f;
         int last = n - 1;
         for (int e = 0; e <= last; ++e) {
-            float w = e < SEL_KEPT ? weights[e] : entry_weight(L, e, s.p);
+            float w = e < SEL_KEPT ? weights[e] : entry_weight<P>(L, e, s.p);
             acc += w;
             float hi = e == last ? 1.0f : acc / s.total;
             if (hi > u_select || e == last) {
@@ -249,7 +257,7 @@ RTG_D_NI bool sample_light(const LightsDev& L, const Sel& s, const float* weight
     int a = L.entries[index];
     out.light = a;
     out.delta = false;
-    if (a >= 0 && L.lights[a].kind == LIGHT_SUN) {  // light.rs:1197
+    if (!P && a >= 0 && L.lights[a].kind == LIGHT_SUN) {  // light.rs:1197
         const LightDev& l = L.lights[a];
         out.distance = f_inf();
         out.radiance = rgb(l.radiance[0], l.radiance[1], l.radiance[2]);
@@ -265,7 +273,7 @@ RTG_D_NI bool sample_light(const LightsDev& L, const Sel& s, const float* weight
             out.wi = normalize(to_world(f, uniform_cone(u0, u1, l.one_minus_cos_max)));
             out.pdf = pmf / l.solid_angle;
         }
-    } else if (a >= 0 && L.lights[a].kind == LIGHT_SPHERE) {  // light.rs:1224
+    } else if (!P && a >= 0 && L.lights[a].kind == LIGHT_SPHERE) {  // light.rs:1224
         const LightDev& l = L.lights[a];
         float m = sphere_mask(l, s.p);
         V3 d = ld3(l.centre) - s.p;
@@ -293,7 +301,7 @@ RTG_D_NI bool sample_light(const LightsDev& L, const Sel& s, const float* weight
             out.radiance = rgb(l.radiance[0], l.radiance[1], l.radiance[2]) * m;
             out.pdf = pmf / (TAU * omc);
         }
-    } else if (a >= 0 && L.lights[a].kind == LIGHT_MESH) {  // light.rs:1270: a triangle by area, a point uniformly
+    } else if (!P && a >= 0 && L.lights[a].kind == LIGHT_MESH) {  // light.rs:1270: a triangle by area, a point uniformly
         const LightDev& l = L.lights[a];
         uint32_t k = 0;
         while (k < l.n_tris && __ldg(&l.tris[4 * k].w) <= rest) ++k;
@@ -337,10 +345,10 @@ RTG_D_NI bool sample_light(const LightsDev& L, const Sel& s, const float* weight
     } else {
         V3 wi;
         float p;
-        if (!env_sample(L, u0, u1, wi, p)) return false;
+        if (!env_sample<P>(L, u0, u1, wi, p)) return false;
         out.wi = wi;
         out.distance = f_inf();
-        out.radiance = env_radiance(L, wi);
+        out.radiance = env_radiance<P>(L, wi);
         out.pdf = pmf * p;
         out.glossy = true;
         out.shadow = true;
@@ -378,6 +386,7 @@ RTG_D bool sun_seen(const LightsDev& L, const LightDev& l, V3 dir, bool has_pdf,
 }
 
 // Lights::crossed_from (light.rs:1329): the area lights, then the spheres, a ray crosses before t_max.
+template <bool P = false>
 RTG_D_NI Rgb crossed_from(const LightsDev& L, V3 o, V3 d, float tmin, float tmax, bool has_pdf, float pdf, const Sel& from, float offset) {
     Rgb sum = splat(0.0f);
     for (int i = 0; i < L.n_areas; ++i) {
@@ -388,11 +397,12 @@ RTG_D_NI Rgb crossed_from(const LightsDev& L, V3 o, V3 d, float tmin, float tmax
         float w = 1.0f;
         if (has_pdf) {
             float dd = offset + t;
-            float light_pdf = pmf_of(L, l.entry, from) * dd * dd / (l.area * cos);
+            float light_pdf = pmf_of<P>(L, l.entry, from) * dd * dd / (l.area * cos);
             w = power_heuristic(pdf, light_pdf);
         }
         sum = sum + area_radiance(l, cos) * w;
     }
+    if (P) return sum;
     const int first_sphere = L.n_areas + (int)L.n_suns;
     for (int i = first_sphere; i < first_sphere + (int)L.n_spheres; ++i) {
         Rgb c;
@@ -424,10 +434,11 @@ RTG_D bool camera_sees_panel(const LightsDev& L, V3 o, V3 d, float t_max) {
     return false;
 }
 // Lights::escaped (light.rs:1502): the ramp environment, then the sun discs.
+template <bool P = false>
 RTG_D Rgb escaped(const LightsDev& L, V3 dir, bool has_pdf, float pdf, const Sel& from) {
-    Rgb sum = env_radiance(L, dir);
-    if (has_pdf && L.env_is_entry) sum = sum * power_heuristic(pdf, pmf_of(L, L.env_entry, from) * env_pdf(L, dir));
-    return L.n_suns ? add_suns(L, sum, dir, has_pdf, pdf, from) : sum;
+    Rgb sum = env_radiance<P>(L, dir);
+    if (has_pdf && L.env_is_entry) sum = sum * power_heuristic(pdf, pmf_of<P>(L, L.env_entry, from) * env_pdf<P>(L, dir));
+    return !P && L.n_suns ? add_suns(L, sum, dir, has_pdf, pdf, from) : sum;
 }
 
 // ---- camera (render.rs:79, scene/mod.rs:280) -------------------------------------------------------

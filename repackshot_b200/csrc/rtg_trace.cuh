@@ -649,14 +649,15 @@ struct HitInfo {
     bool cap;  // on a section's cap: no triangle, the plane's normal
 };
 
-// geometry/mod.rs:731 hit_details for an instance hit.
+// geometry/mod.rs:731 hit_details for an instance hit. `P`: a plain scene (SceneDev::plain), no section.
+template <bool P = false>
 RTG_D_NI bool hit_details(const SceneDev& S, V3 o, V3 d, float tmin, float tmax, uint32_t inst, uint32_t tri, float t_hit,
                        HitInfo& h, const DevInstance*& I_out, uint4& idx_out) {
     if (inst >= S.n_instances) return false;
     const DevInstance* I = S.instances + inst;
     I_out = I;
     if (!I->active) return false;
-    h.cap = tri == CAP_TRIANGLE;
+    h.cap = !P && tri == CAP_TRIANGLE;
     if (h.cap) {  // Section::cap_details (section.rs:424-448): on the plane, facing where the ray came from
         if (!S.section_on) return false;
         const V3 n = v3(S.section_n[0], S.section_n[1], S.section_n[2]);
