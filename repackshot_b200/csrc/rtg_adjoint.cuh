@@ -6,7 +6,7 @@
 // A forward wave renders every path of the call and leaves each path's radiance L in its slot.
 // k_adjoint_delta turns the film and the target image into the loss and, per pixel, the loss's
 // derivative with respect to one path's radiance. The backward wave (k_adjoint_camera, the forward's
-// k_extend, k_scan and k_scatter, then k_shade_adjoint and k_shadow_adjoint per bounce) runs every
+// k_extend and k_material_sort, then k_shade_adjoint and k_shadow_adjoint per bounce) runs every
 // path again from its pixel and sample index (the sampler makes it the same path), carrying
 // L_rem = L - (the contributions met so far), which is the radiance still to come. At each vertex:
 // - a contribution c of area light i adds <dL, c> to light i's scale gradient, and when c is a
@@ -58,7 +58,7 @@ struct AdjBlock {
 
 // The backward wave's camera: the forward's camera rays again, and each slot's radiance still to
 // come set to the radiance the forward pass found (left in P.sum).
-__global__ void k_adjoint_camera(const __grid_constant__ SceneDev S, WaveDesc w, PathBuffers P, AdjointDev A) {
+__global__ void k_adjoint_camera(const __grid_constant__ SceneDev S, WaveDesc w, PathBuffers P, AdjointDev A, uint32_t rounds) {
     float all = 0.0f;
     for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < w.n; slot += gridDim.x * blockDim.x) {
         uint32_t x, y, index;
@@ -80,16 +80,7 @@ __global__ void k_adjoint_camera(const __grid_constant__ SceneDev S, WaveDesc w,
     }
     for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
     if ((threadIdx.x & 31) == 0) atomicAdd(A.residual + 1, all);
-    if (blockIdx.x == 0) {
-        for (uint32_t k = threadIdx.x; k < 512; k += blockDim.x) P.bins[k] = 0;
-        if (threadIdx.x == 0) {
-            P.counters[0] = w.n;
-            P.counters[1] = 0;
-            P.counters[2] = 0;
-            P.counters[4] = 0;
-            P.counters[5] = 0;
-        }
-    }
+    start_rounds(P, rounds, w.n);
 }
 
 // One vertex of the backward wave: the forward's shading (shade_slot) step for step, taking every
@@ -121,7 +112,7 @@ __device__ __noinline__ Rgb adjoint_spheres(const LightsDev& L, Rgb crossed, V3 
 
 template <bool PLAIN>
 __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const LightsDev& L, const PathBuffers& P, const AdjointDev& A, float* g,
-                                                   uint32_t slot, int cur, uint32_t bounce, const WaveDesc& w) {
+                                                   uint32_t slot, uint32_t bounce, const WaveDesc& w) {
     float4 o4 = P.o[slot], d4 = P.d[slot], thr4 = P.thr[slot];
     uint32_t flags = P.flags[slot];
     uint4 hit = P.hit[slot];
@@ -324,7 +315,7 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
                         floor_blocks = t > 1.0e-3f && t < tmax;
                     }
                     if (finite_c && !floor_blocks) {
-                        uint32_t k = atomicAdd(&P.counters[2], 1u);
+                        uint32_t k = atomicAdd(&P.counters[round_counter(bounce, COUNT_SHADOW)], 1u);
                         P.sh_o[k] = make_float4(from_p.x, from_p.y, from_p.z, tmax);
                         P.sh_d[k] = make_float4(ls.wi.x, ls.wi.y, ls.wi.z, 0.0f);
                         P.sh_c[k] = make_float4(c.r, c.g, c.b, __uint_as_float(slot));
@@ -392,23 +383,22 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
     P.thr[slot] = make_float4(thr.r, thr.g, thr.b, thr4.w);
     A.rem[slot] = make_float4(rem.r, rem.g, rem.b, 0.0f);
     if (alive) {
-        uint32_t k = atomicAdd(&P.counters[cur ^ 1], 1u);
-        P.queue[cur ^ 1][k] = slot;
+        uint32_t k = atomicAdd(&P.counters[round_counter(bounce + 1, COUNT_PATHS)], 1u);
+        P.queue[(bounce + 1) & 1][k] = slot;
     }
 }
 
 // Eight blocks per SM (64 registers, with spills) rather than the compiler's 168 registers: as for
 // k_shade, more warps hide the scattered loads (512^2 adjoint iteration 51.4 -> 48.9 ms).
 template <bool PLAIN>
-__global__ void __launch_bounds__(128, RTG_SHADE_MIN_BLOCKS) k_shade_adjoint(const __grid_constant__ SceneDev S, const LightsDev* __restrict__ Lg, PathBuffers P, int cur, uint32_t bounce,
+__global__ void __launch_bounds__(128, RTG_SHADE_MIN_BLOCKS) k_shade_adjoint(const __grid_constant__ SceneDev S, const LightsDev* __restrict__ Lg, PathBuffers P, uint32_t bounce,
                                                        WaveDesc w, AdjointDev A) {
     __shared__ float s_grad[MAX_ADJOINT_PARAMS];
     AdjBlock blk{s_grad};
     const uint32_t n_params = 4 * A.n_materials + A.n_lights;
     blk.begin(n_params);
-    uint32_t n = *(volatile uint32_t*)&P.counters[cur];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        shade_adjoint_slot<PLAIN>(S, *Lg, P, A, s_grad, P.sorted[i], cur, bounce, w);
+    for_each_path(P, P.sorted, round_paths(P, bounce, 0), bounce,
+                  [&](uint32_t slot) { shade_adjoint_slot<PLAIN>(S, *Lg, P, A, s_grad, slot, bounce, w); });
     blk.end(n_params, A.grads);
 }
 
@@ -435,7 +425,7 @@ __device__ __forceinline__ void adjoint_unblocked(const PathBuffers& P, const Ad
     }
 }
 
-__global__ void __launch_bounds__(TRACE_THREADS) k_shadow_adjoint(const __grid_constant__ SceneDev S, PathBuffers P, WaveDesc w, AdjointDev A) {
+__global__ void __launch_bounds__(TRACE_THREADS) k_shadow_adjoint(const __grid_constant__ SceneDev S, PathBuffers P, uint32_t bounce, WaveDesc w, AdjointDev A) {
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
     __shared__ float s_grad[MAX_ADJOINT_PARAMS];
     uint64_t deep[STACK_CAP - SHORT_STACK];
@@ -443,23 +433,23 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_shadow_adjoint(const __grid_c
     AdjBlock blk{s_grad};
     const uint32_t n_params = 4 * A.n_materials + A.n_lights;
     blk.begin(n_params);
-    const uint32_t n = *(volatile uint32_t*)&P.counters[2];
-    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t n = *(volatile uint32_t*)&P.counters[round_counter(bounce, COUNT_SHADOW)];
+    uint32_t* position = &P.counters[round_counter(bounce, NEXT_SHADOW)];
+    const uint32_t lane = threadIdx.x & 31u, lanes = lanes_for(n), enough = min(lanes, (uint32_t)RTG_SHADOW_REFILL_MIN);
     uint32_t err = 0, ray = 0;
     bool busy = false, drained = false;
     Trav T;
     for (;;) {
         if (!drained) {
-            const uint32_t idle = __ballot_sync(0xffffffffu, !busy);
-            // k_shadow's refill threshold (RTG_SHADOW_REFILL_MIN idle lanes, or all of them)
-            if (idle && (RTG_SHADOW_REFILL_MIN <= 1 || __popc(idle) >= RTG_SHADOW_REFILL_MIN || idle == 0xffffffffu)) {
+            const uint32_t idle = __ballot_sync(0xffffffffu, !busy && lane < lanes);
+            if ((uint32_t)__popc(idle) >= enough) {
                 const int leader = __ffs((int)idle) - 1;
                 uint32_t base = 0;
-                if ((int)lane == leader) base = atomicAdd(&P.counters[5], (uint32_t)__popc(idle));
+                if ((int)lane == leader) base = atomicAdd(position, (uint32_t)__popc(idle));
                 base = __shfl_sync(0xffffffffu, base, leader);
                 if (base + (uint32_t)__popc(idle) >= n) drained = true;
                 const uint32_t i = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
-                if (!busy && i < n) {
+                if (!busy && lane < lanes && i < n) {
                     ray = i;
                     const float4 o = P.sh_o[i], d = P.sh_d[i];
                     busy = trav_init(S, T, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 1.0e-3f, o.w, false);

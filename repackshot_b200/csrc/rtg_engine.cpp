@@ -432,7 +432,7 @@ uint32_t ensure_capacity(Scene& sc, uint32_t paths) {
     sc.path_mem.release();
     sc.capacity = 0;
     size_t n = paths;
-    size_t bytes = n * PATH_BYTES + 17 * 256 + 256 + 512 * 4 + SORT_BINS_BYTES;
+    size_t bytes = n * PATH_BYTES + 17 * 256 + COUNTERS_BYTES + 2 * KEY_BINS * 4 + 256 + SORT_BINS_BYTES;
     RTG_CHECK(cudaMalloc(&sc.path_mem.p, bytes));
     sc.path_mem.bytes = bytes;
     uint8_t* p = (uint8_t*)sc.path_mem.p;
@@ -451,7 +451,7 @@ uint32_t ensure_capacity(Scene& sc, uint32_t paths) {
     sc.P.sorted = (uint32_t*)take(4);
     sc.P.key = (uint32_t*)take(4);
     sc.P.bins = (uint32_t*)p;
-    p += 512 * 4;
+    p += 2 * KEY_BINS * 4;
     sc.P.sh_o = (float4*)take(16);
     sc.P.sh_d = (float4*)take(16);
     sc.P.sh_c = (float4*)take(16);
@@ -461,7 +461,7 @@ uint32_t ensure_capacity(Scene& sc, uint32_t paths) {
     p += SORT_BINS_BYTES;
     RTG_CHECK(cudaMemsetAsync(sc.P.rbins, 0, SORT_BINS_BYTES, sc.stream));  // histograms start at zero
     sc.P.counters = (uint32_t*)p;
-    p += 64;
+    p += COUNTERS_BYTES;
     sc.P.rays = (unsigned long long*)p;
     p += 64;
     if ((size_t)(p - (uint8_t*)sc.path_mem.p) > bytes) { g_error = "internal: path buffer layout"; return RTG_STATUS_CUDA_ERROR; }
@@ -1042,7 +1042,7 @@ uint32_t rtg_render_progressive_noalloc(uint32_t handle, uint32_t film, uint32_t
     const char* why = "";
     uint32_t st = noalloc_render(job, res, &why);
     if (st) { g_error = why; return st; }
-    sc->launches += res.waves * (2 + 6 * (uint64_t)wave_rounds(sc->S) + (job.guide_sum ? 2 : 0));
+    sc->launches += res.waves * (wave_launches(sc->S, RaySort(), PathBuffers{}, false) + (job.guide_sum ? 2 : 0));
     sc->rays += res.extend_rays + res.shadow_rays;
     sc->extend_rays += res.extend_rays;
     sc->shadow_rays += res.shadow_rays;
@@ -1412,7 +1412,7 @@ uint32_t rtg_render_adjoint(uint32_t scene, uint32_t film, const float* target, 
                  (float4*)(base + off_shg), (uint32_t*)(base + off_shi)};
     launch_adjoint_wave(sc->S, sc->d_lights, wd, sc->P, A, s, grid_for((uint32_t)paths, 128));
     RTG_CHECK(cudaGetLastError());
-    sc->launches += 3 + 6 * (uint64_t)(sc->S.max_depth + 1);
+    sc->launches += 3 + 4 * (uint64_t)(sc->S.max_depth + 1);
     uint64_t rays = 0;
     st = finish(*sc, &rays);
     if (st) return st;

@@ -5,6 +5,8 @@
 // sample order (integrator/mod.rs:1140-1891, render.rs:388-497, image.rs:82-93).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "rtg_image.cuh"
 #include "rtg_kernels.h"
 #include "rtg_shade.cuh"
@@ -27,6 +29,10 @@ constexpr int TRACE_THREADS = 128;
 // at 4, 312 at 16).
 #ifndef RTG_SHADOW_REFILL_MIN
 #define RTG_SHADOW_REFILL_MIN 8
+#endif
+// RTG_MIN_LANES (build setting): the fewest lanes of a warp that a thin round fills (lanes_for).
+#ifndef RTG_MIN_LANES
+#define RTG_MIN_LANES 1u
 #endif
 // RTG_TRACE_MIN_BLOCKS (build setting): blocks per SM the traversal kernels (k_extend, k_shadow)
 // are compiled for (0: the compiler's choice of registers, 76). At 8 (64 registers, no spills in
@@ -112,10 +118,30 @@ __device__ __forceinline__ void add_clamped(float4& sum, Rgb c, bool indirect, f
     sum.z = sum.z + c.b;
 }
 
+// The counts of a wave's rounds and the key bins at its start: n paths in round 0.
+__device__ __forceinline__ void start_rounds(const PathBuffers& P, uint32_t rounds, uint32_t n) {
+    if (blockIdx.x) return;
+    for (uint32_t k = threadIdx.x; k < 4 * (rounds + 1); k += blockDim.x) P.counters[ROUND_COUNTERS + k] = k == COUNT_PATHS ? n : 0;
+    for (uint32_t k = threadIdx.x; k < 2 * KEY_BINS; k += blockDim.x) P.bins[k] = 0;
+}
+// The paths a round's kernels work on: none where the tail kernel takes the round (its queue holds
+// at most `tail` paths) or an earlier one, which leaves it empty.
+__device__ __forceinline__ uint32_t round_paths(const PathBuffers& P, uint32_t round, uint32_t tail) {
+    const uint32_t n = *(volatile uint32_t*)&P.counters[round_counter(round, COUNT_PATHS)];
+    return round >= TAIL_FIRST_ROUND && n <= tail ? 0 : n;
+}
+// Lanes of each warp that n units of work fill when every resident warp takes its share: a thin
+// round is as long as its slowest ray, and a ray in a warp of its own does not wait for the leaves
+// and nodes of 31 others.
+__device__ __forceinline__ uint32_t lanes_for(uint32_t n) {
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    return min(32u, max(RTG_MIN_LANES, (n + warps - 1) / warps));
+}
+
 // ---- camera generation ---------------------------------------------------------------------------
 // BATCH: the slots belong to the jobs of a batched wave, each with its own camera.
 template <bool BATCH>
-__global__ void k_camera(const __grid_constant__ SceneDev S, WaveDesc w, PathBuffers P) {
+__global__ void k_camera(const __grid_constant__ SceneDev S, WaveDesc w, PathBuffers P, uint32_t rounds) {
     for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < w.n; slot += gridDim.x * blockDim.x) {
         uint32_t x, y, index;
         V3 o, d;
@@ -135,16 +161,7 @@ __global__ void k_camera(const __grid_constant__ SceneDev S, WaveDesc w, PathBuf
         P.flags[slot] = PF_PRIMARY | (sees ? 0u : PF_NOTHING);
         P.queue[0][slot] = slot;
     }
-    if (blockIdx.x == 0) {
-        for (uint32_t k = threadIdx.x; k < 512; k += blockDim.x) P.bins[k] = 0;
-        if (threadIdx.x == 0) {
-            P.counters[0] = w.n;
-            P.counters[1] = 0;
-            P.counters[2] = 0;
-            P.counters[4] = 0;
-            P.counters[5] = 0;
-        }
-    }
+    start_rounds(P, rounds, w.n);
 }
 
 // Material key of a path's next vertex, for the material-sorted shade.
@@ -233,29 +250,32 @@ __global__ void k_key_scatter(const uint32_t* __restrict__ list, const uint32_t*
 
 // ---- extend: nearest hit of every active path ------------------------------------------------------------
 // Persistent warps over the active queue: a lane whose ray has finished takes the next queue entry
-// (one atomic per warp on counters[4]) while the rest of the warp keeps traversing, so no lane idles
-// until the slowest ray of its warp is done.
-// `order`: the active queue in the order to trace it (P.queue[cur], or its ray-sorted copy).
-__global__ void RTG_TRACE_BOUNDS k_extend(const __grid_constant__ SceneDev S, PathBuffers P, int cur, const uint32_t* __restrict__ order) {
+// (one atomic per warp on the round's position) while the rest of the warp keeps traversing, so no
+// lane idles until the slowest ray of its warp is done. In a thin round only lanes_for lanes take rays.
+// `order`: the active queue in the order to trace it (the round's queue, or its ray-sorted copy).
+__global__ void RTG_TRACE_BOUNDS k_extend(const __grid_constant__ SceneDev S, PathBuffers P, uint32_t round, const uint32_t* __restrict__ order, uint32_t tail) {
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
     uint64_t deep[STACK_CAP - SHORT_STACK];
     SplitStack stack{s_stack + threadIdx.x, deep, TRACE_THREADS};
-    const uint32_t n = *(volatile uint32_t*)&P.counters[cur];
-    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t n = round_paths(P, round, tail);
+    if (n == 0) return;
+    uint32_t* position = &P.counters[round_counter(round, NEXT_PATH)];
+    uint32_t* bins = P.bins + KEY_BINS * (round & 1);
+    const uint32_t lane = threadIdx.x & 31u, lanes = lanes_for(n), enough = min(lanes, (uint32_t)RTG_REFILL_MIN);
     uint32_t err = 0, slot = 0;
     bool busy = false, drained = false;
     Trav T;
     for (;;) {
         if (!drained) {
-            const uint32_t idle = __ballot_sync(0xffffffffu, !busy);
-            if (idle && (RTG_REFILL_MIN <= 1 || __popc(idle) >= RTG_REFILL_MIN || idle == 0xffffffffu)) {
+            const uint32_t idle = __ballot_sync(0xffffffffu, !busy && lane < lanes);
+            if ((uint32_t)__popc(idle) >= enough) {
                 const int leader = __ffs((int)idle) - 1;
                 uint32_t base = 0;
-                if ((int)lane == leader) base = atomicAdd(&P.counters[4], (uint32_t)__popc(idle));
+                if ((int)lane == leader) base = atomicAdd(position, (uint32_t)__popc(idle));
                 base = __shfl_sync(0xffffffffu, base, leader);
                 if (base + (uint32_t)__popc(idle) >= n) drained = true;
                 const uint32_t i = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
-                if (!busy && i < n) {
+                if (!busy && lane < lanes && i < n) {
                     slot = order[i];
                     const float4 o = P.o[slot], d = P.d[slot];
                     const uint32_t pf = P.flags[slot];
@@ -264,7 +284,7 @@ __global__ void RTG_TRACE_BOUNDS k_extend(const __grid_constant__ SceneDev S, Pa
                         P.hit[slot] = make_uint4(0xffffffffu, 0xffffffffu, 0u, 0u);
                         const uint32_t key = material_key(S, false, 0);
                         P.key[slot] = key;
-                        warp_count(P.bins, key);
+                        warp_count(bins, key);
                     }
                 }
             }
@@ -286,41 +306,90 @@ __global__ void RTG_TRACE_BOUNDS k_extend(const __grid_constant__ SceneDev S, Pa
                                   : make_uint4(0xffffffffu, 0xffffffffu, 0u, 0u);
                 const uint32_t key = material_key(S, got, T.best_i);
                 P.key[slot] = key;
-                warp_count(P.bins, key);
+                warp_count(bins, key);
             }
         }
     }
     if (err) atomicOr(&P.counters[3], err);
 }
 
-// Exclusive prefix of the key histogram into the scatter cursors; clears the histogram.
-__global__ void k_scan(PathBuffers P) {
-    if (threadIdx.x == 0) {
-        uint32_t acc = 0;
-        for (int k = 0; k < 256; ++k) {
-            uint32_t c = P.bins[k];
-            P.bins[256 + k] = acc;
-            P.bins[k] = 0;
-            acc += c;
+// ---- the order of shading ------------------------------------------------------------------------
+// `out` = the round's n paths of `in` ordered by material key (the order inside a key does not
+// matter: every path's result depends on its own slot only). Each block orders the next SORT_CHUNK
+// of them in shared memory, takes its part of every key's run with one atomic, and writes the runs
+// coalesced; the runs' starts it sums itself from the histogram k_extend left. Sorting only within
+// the chunks a shade block reads would save the pass but not pay: with all blocks in the same few
+// materials at a time the kernel's instructions stay in the caches (1080p frame, chunks of 512, 1024
+// and 2048: 254, 231 and 213 ms; whole queue 193 ms). Against a pass with an atomic per warp and key
+// after a one-thread prefix: 11.1 to 1.8 ms of the 1080p frame's 13 rounds.
+constexpr uint32_t SORT_THREADS = 256, SORT_PER = 8, SORT_CHUNK = SORT_THREADS * SORT_PER;
+static_assert(SORT_THREADS == MATERIAL_KEYS, "a thread per key");
+__device__ __forceinline__ uint32_t block_prefix(uint32_t v, uint32_t* s_warp) {  // exclusive, over SORT_THREADS
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t x = v;
+#pragma unroll
+    for (uint32_t o = 1; o < 32u; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31u) s_warp[warp] = x;
+    __syncthreads();
+    uint32_t before = x - v;
+    for (uint32_t w = 0; w < warp; ++w) before += s_warp[w];
+    __syncthreads();
+    return before;
+}
+__global__ void __launch_bounds__(SORT_THREADS) k_material_sort(PathBuffers P, uint32_t round, const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
+                                                                 uint32_t tail) {
+    __shared__ uint32_t s_slot[SORT_CHUNK], s_to[SORT_CHUNK], s_count[MATERIAL_KEYS], s_run[MATERIAL_KEYS], s_warp[SORT_THREADS / 32];
+    const uint32_t n = round_paths(P, round, tail), tid = threadIdx.x;
+    uint32_t* bins = P.bins + KEY_BINS * (round & 1);
+    uint32_t* cursors = bins + MATERIAL_KEYS;
+    if (blockIdx.x * SORT_CHUNK >= n) return;
+    const uint32_t run = block_prefix(bins[tid], s_warp);  // where this thread's key starts in `out`
+    for (uint32_t base = blockIdx.x * SORT_CHUNK; base < n; base += gridDim.x * SORT_CHUNK) {
+        const uint32_t m = min(SORT_CHUNK, n - base);
+        s_count[tid] = 0;
+        __syncthreads();
+        uint32_t slot[SORT_PER], at[SORT_PER];  // at: the key, and above it the place among the chunk's
+#pragma unroll
+        for (uint32_t j = 0; j < SORT_PER; ++j) {
+            const uint32_t e = j * SORT_THREADS + tid;
+            if (e < m) slot[j] = in[base + e];
         }
+#pragma unroll
+        for (uint32_t j = 0; j < SORT_PER; ++j)
+            if (j * SORT_THREADS + tid < m) at[j] = P.key[slot[j]];
+#pragma unroll
+        for (uint32_t j = 0; j < SORT_PER; ++j)
+            if (j * SORT_THREADS + tid < m) at[j] |= atomicAdd(&s_count[at[j]], 1u) << 8;
+        __syncthreads();
+        const uint32_t count = s_count[tid];
+        const uint32_t local = block_prefix(count, s_warp);
+        s_count[tid] = local;
+        if (count) s_run[tid] = run + atomicAdd(&cursors[tid], count) - local;
+        __syncthreads();
+#pragma unroll
+        for (uint32_t j = 0; j < SORT_PER; ++j)
+            if (j * SORT_THREADS + tid < m) {
+                const uint32_t key = at[j] & 255u, e = s_count[key] + (at[j] >> 8);
+                s_slot[e] = slot[j];
+                s_to[e] = s_run[key];
+            }
+        __syncthreads();
+        for (uint32_t e = tid; e < m; e += SORT_THREADS) out[s_to[e] + e] = s_slot[e];
+        __syncthreads();
     }
 }
-
-// The active queue `in` reordered by material key into `out` (the order inside a key does not
-// matter: every path's result depends on its own slot only).
-__global__ void k_scatter(PathBuffers P, int cur, const uint32_t* __restrict__ in, uint32_t* __restrict__ out) {
-    uint32_t n = *(volatile uint32_t*)&P.counters[cur];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        uint32_t slot = in[i];
-        uint32_t key = P.key[slot];
-        uint32_t mask = __match_any_sync(__activemask(), key);
-        int leader = __ffs((int)mask) - 1;
-        uint32_t base = 0;
-        if ((int)(threadIdx.x & 31) == leader) base = atomicAdd(&P.bins[256 + key], (uint32_t)__popc(mask));
-        base = __shfl_sync(mask, base, leader);
-        uint32_t rank = __popc(mask & ((1u << (threadIdx.x & 31)) - 1u));
-        out[base + rank] = slot;
-    }
+// Calls f(slot) for the n paths of `order`, a path per lane; a thin round's few paths go to the first
+// lanes of all warps. The round's key bins, read for the last time before, are cleared for the next
+// round but one.
+template <class F>
+__device__ __forceinline__ void for_each_path(const PathBuffers& P, const uint32_t* __restrict__ order, uint32_t n, uint32_t round, F f) {
+    if (blockIdx.x == 0)
+        for (uint32_t k = threadIdx.x; k < KEY_BINS; k += blockDim.x) P.bins[KEY_BINS * (round & 1) + k] = 0;
+    const uint32_t lanes = lanes_for(n), warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    for (uint32_t i = lane < lanes ? warp * lanes + lane : n; i < n; i += gridDim.x * (blockDim.x >> 5) * lanes) f(order[i]);
 }
 
 // ---- shade: one vertex of every active path ----------------------------------------------------------
@@ -336,7 +405,7 @@ struct TailShadow {
     float4 o, d, c;
 };
 template <bool PLAIN, class XYI>
-__device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L, const PathBuffers& P, const RaySort& R, uint32_t slot, int cur,
+__device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L, const PathBuffers& P, const RaySort& R, uint32_t slot, uint32_t round,
                                            XYI xyi, uint32_t& rays_local, uint32_t& shadow_local, TailShadow* tail = nullptr) {
     float4 o4 = P.o[slot], d4 = P.d[slot], thr4 = P.thr[slot], sum = P.sum[slot];
     uint32_t flags = P.flags[slot];
@@ -509,7 +578,7 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
                             tail->d = sd;
                             tail->c = sc;
                         } else {
-                            uint32_t k = atomicAdd(&P.counters[2], 1u);
+                            uint32_t k = atomicAdd(&P.counters[round_counter(round, COUNT_SHADOW)], 1u);
                             P.sh_o[k] = so;
                             P.sh_d[k] = sd;
                             P.sh_c[k] = sc;
@@ -568,8 +637,8 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
     P.thr[slot] = make_float4(thr.r, thr.g, thr.b, alpha);
     P.sum[slot] = sum;
     if (alive && !tail) {
-        uint32_t k = atomicAdd(&P.counters[cur ^ 1], 1u);
-        P.queue[cur ^ 1][k] = slot;
+        uint32_t k = atomicAdd(&P.counters[round_counter(round + 1, COUNT_PATHS)], 1u);
+        P.queue[(round + 1) & 1][k] = slot;
         if (P.rbins) {
             const float4 no = P.o[slot], nd = P.d[slot];
             const uint32_t rk = ray_key(R, v3(no.x, no.y, no.z), v3(nd.x, nd.y, nd.z));
@@ -596,23 +665,22 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
 // SM the frame takes 195.4, 198.4, 199.7, 197.7, 192.7 and 202.2 ms.
 // `order`: the active queue in the order to shade it (material-sorted, or as traced).
 template <bool BATCH, bool PLAIN>
-__global__ void __launch_bounds__(128, RTG_SHADE_MIN_BLOCKS) k_shade(const __grid_constant__ SceneDev S, const LightsDev* __restrict__ Lg, PathBuffers P, int cur, WaveDesc w,
+__global__ void __launch_bounds__(128, RTG_SHADE_MIN_BLOCKS) k_shade(const __grid_constant__ SceneDev S, const LightsDev* __restrict__ Lg, PathBuffers P, uint32_t round, WaveDesc w,
                                                   const uint32_t* __restrict__ order, RaySort R) {
-    uint32_t n = *(volatile uint32_t*)&P.counters[cur];
+    const uint32_t n = round_paths(P, round, R.tail_paths);
     uint32_t rays_local = 0, shadow_local = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t slot = order[i];
+    for_each_path(P, order, n, round, [&](uint32_t slot) {
         if constexpr (BATCH) {
             uint32_t job, x, y, index;
             batch_slot(w, slot, job, x, y, index);
             const JobDev& J = w.jobs[job];
-            shade_slot<PLAIN>(J.S, *J.lights, P, R, slot, cur, [&](uint32_t& xx, uint32_t& yy, uint32_t& ii) { xx = x; yy = y; ii = index; },
+            shade_slot<PLAIN>(J.S, *J.lights, P, R, slot, round, [&](uint32_t& xx, uint32_t& yy, uint32_t& ii) { xx = x; yy = y; ii = index; },
                        rays_local, shadow_local);
         } else {
-            shade_slot<PLAIN>(S, *Lg, P, R, slot, cur, [&](uint32_t& xx, uint32_t& yy, uint32_t& ii) { wave_slot(w, slot, xx, yy, ii); },
+            shade_slot<PLAIN>(S, *Lg, P, R, slot, round, [&](uint32_t& xx, uint32_t& yy, uint32_t& ii) { wave_slot(w, slot, xx, yy, ii); },
                        rays_local, shadow_local);
         }
-    }
+    });
     // Ray counts: camera + extension rays in rays[0], shadow rays in rays[1]; one atomic per warp.
     uint32_t total = __reduce_add_sync(0xffffffffu, rays_local);
     uint32_t shadows = __reduce_add_sync(0xffffffffu, shadow_local);
@@ -621,7 +689,7 @@ __global__ void __launch_bounds__(128, RTG_SHADE_MIN_BLOCKS) k_shade(const __gri
 }
 
 // ---- shadow: any hit of every queued shadow ray; the unblocked add their light ----------------------------
-// Persistent warps with lane refill, as k_extend (queue position counter: counters[5]).
+// Persistent warps with lane refill, as k_extend.
 __device__ __forceinline__ void shadow_unblocked(const PathBuffers& P, uint32_t i) {
     const float4 c = P.sh_c[i];
     const uint32_t slot = __float_as_uint(c.w);
@@ -631,26 +699,28 @@ __device__ __forceinline__ void shadow_unblocked(const PathBuffers& P, uint32_t 
 }
 
 // `perm` (may be null): the shadow queue in the order to trace it.
-__global__ void RTG_TRACE_BOUNDS k_shadow(const __grid_constant__ SceneDev S, PathBuffers P, const uint32_t* __restrict__ perm) {
+__global__ void RTG_TRACE_BOUNDS k_shadow(const __grid_constant__ SceneDev S, PathBuffers P, uint32_t round, const uint32_t* __restrict__ perm) {
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
     uint64_t deep[STACK_CAP - SHORT_STACK];
     SplitStack stack{s_stack + threadIdx.x, deep, TRACE_THREADS};
-    const uint32_t n = *(volatile uint32_t*)&P.counters[2];
-    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t n = *(volatile uint32_t*)&P.counters[round_counter(round, COUNT_SHADOW)];
+    if (n == 0) return;
+    uint32_t* position = &P.counters[round_counter(round, NEXT_SHADOW)];
+    const uint32_t lane = threadIdx.x & 31u, lanes = lanes_for(n), enough = min(lanes, (uint32_t)RTG_SHADOW_REFILL_MIN);
     uint32_t err = 0, ray = 0;
     bool busy = false, drained = false;
     Trav T;
     for (;;) {
         if (!drained) {
-            const uint32_t idle = __ballot_sync(0xffffffffu, !busy);
-            if (idle && (RTG_SHADOW_REFILL_MIN <= 1 || __popc(idle) >= RTG_SHADOW_REFILL_MIN || idle == 0xffffffffu)) {
+            const uint32_t idle = __ballot_sync(0xffffffffu, !busy && lane < lanes);
+            if ((uint32_t)__popc(idle) >= enough) {
                 const int leader = __ffs((int)idle) - 1;
                 uint32_t base = 0;
-                if ((int)lane == leader) base = atomicAdd(&P.counters[5], (uint32_t)__popc(idle));
+                if ((int)lane == leader) base = atomicAdd(position, (uint32_t)__popc(idle));
                 base = __shfl_sync(0xffffffffu, base, leader);
                 if (base + (uint32_t)__popc(idle) >= n) drained = true;
                 const uint32_t i = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
-                if (!busy && i < n) {
+                if (!busy && lane < lanes && i < n) {
                     ray = perm ? perm[i] : i;
                     const float4 o = P.sh_o[ray], d = P.sh_d[ray];
                     busy = trav_init(S, T, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 1.0e-3f, o.w, false);
@@ -683,11 +753,11 @@ __global__ void RTG_TRACE_BOUNDS k_shadow(const __grid_constant__ SceneDev S, Pa
 // plane, the studio on the removed side), so the lane refill of the plain kernels does not apply.
 // Launched instead of them for a scene with a section; they write the same records (a cap is a hit
 // with triangle CAP_TRIANGLE).
-__global__ void __launch_bounds__(TRACE_THREADS) k_extend_section(const __grid_constant__ SceneDev S, PathBuffers P, int cur, const uint32_t* __restrict__ order) {
+__global__ void __launch_bounds__(TRACE_THREADS) k_extend_section(const __grid_constant__ SceneDev S, PathBuffers P, uint32_t round, const uint32_t* __restrict__ order, uint32_t tail) {
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
     uint64_t deep[STACK_CAP - SHORT_STACK];
     SplitStack stack{s_stack + threadIdx.x, deep, TRACE_THREADS};
-    const uint32_t n = *(volatile uint32_t*)&P.counters[cur];
+    const uint32_t n = round_paths(P, round, tail);
     uint32_t err = 0;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t slot = order[i];
@@ -699,16 +769,16 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_extend_section(const __grid_c
         P.hit[slot] = got ? make_uint4(res.inst, res.tri, __float_as_uint(res.t), 1u) : make_uint4(0xffffffffu, 0xffffffffu, 0u, 0u);
         const uint32_t key = material_key(S, got, got ? res.inst : 0u);
         P.key[slot] = key;
-        warp_count(P.bins, key);
+        warp_count(P.bins + KEY_BINS * (round & 1), key);
     }
     if (err) atomicOr(&P.counters[3], err);
 }
 
-__global__ void __launch_bounds__(TRACE_THREADS) k_shadow_section(const __grid_constant__ SceneDev S, PathBuffers P, const uint32_t* __restrict__ perm) {
+__global__ void __launch_bounds__(TRACE_THREADS) k_shadow_section(const __grid_constant__ SceneDev S, PathBuffers P, uint32_t round, const uint32_t* __restrict__ perm) {
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
     uint64_t deep[STACK_CAP - SHORT_STACK];
     SplitStack stack{s_stack + threadIdx.x, deep, TRACE_THREADS};
-    const uint32_t n = *(volatile uint32_t*)&P.counters[2];
+    const uint32_t n = *(volatile uint32_t*)&P.counters[round_counter(round, COUNT_SHADOW)];
     uint32_t err = 0;
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
         const uint32_t ray = perm ? perm[j] : j;
@@ -725,11 +795,11 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_shadow_section(const __grid_c
 // behind it, up to 32 crossings; any other surface blocks it. One thread per ray: only scenes with
 // passable instances run it, instead of k_shadow. BATCH: each ray's job gives its materials.
 template <bool BATCH>
-__global__ void __launch_bounds__(TRACE_THREADS) k_shadow_walk(const __grid_constant__ SceneDev S, PathBuffers P, WaveDesc w, const uint32_t* __restrict__ perm) {
+__global__ void __launch_bounds__(TRACE_THREADS) k_shadow_walk(const __grid_constant__ SceneDev S, PathBuffers P, uint32_t round, WaveDesc w, const uint32_t* __restrict__ perm) {
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
     uint64_t deep[STACK_CAP - SHORT_STACK];
     SplitStack stack{s_stack + threadIdx.x, deep, TRACE_THREADS};
-    const uint32_t n = *(volatile uint32_t*)&P.counters[2];
+    const uint32_t n = *(volatile uint32_t*)&P.counters[round_counter(round, COUNT_SHADOW)];
     uint32_t err = 0;
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
         const uint32_t i = perm ? perm[j] : j;
@@ -780,27 +850,31 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_shadow_walk(const __grid_cons
     if (err) atomicOr(&P.counters[3], err);
 }
 
-// ---- tail: the last rounds of a wave, a path per thread -----------------------------------------------
-// When the round's extension queue holds at most `limit` paths, each thread carries its share of
-// them through the wave's remaining `rounds_left` rounds alone: the nearest hit (as k_extend), the
-// vertex (shade_slot), the any hit of its shadow ray and its contribution (as k_shadow), the next
-// ray; each path's arithmetic in the order the wavefront gives it, so its sum has the same bits.
-// A wave whose last rounds hold few paths then pays one launch as long as its slowest path instead
-// of a chain of launches, each as long as its slowest ray. k_tail_end then empties the queue, so
-// the later rounds' launches find no work. Scenes with passable surfaces (shadow walks) and
-// batched waves keep the wavefront.
+// ---- tail: the last rounds of a wave, a path per lane -------------------------------------------------
+// The wave's last launch. From the first round whose extension queue holds at most `limit` paths on,
+// the other kernels do nothing, and here each lane carries its share of those paths through the
+// wave's remaining rounds alone: the nearest hit (as k_extend), the vertex (shade_slot), the any
+// hit of its shadow ray and its contribution (as k_shadow), the next ray; each path's arithmetic in
+// the order the wavefront gives it, so its sum has the same bits. A wave whose last rounds hold few
+// paths then pays one launch as long as its slowest path instead of a chain of launches, each as
+// long as its slowest ray. Scenes with passable surfaces (shadow walks) and batched waves keep the
+// wavefront.
 template <bool PLAIN>
-__global__ void __launch_bounds__(TRACE_THREADS) k_tail(const __grid_constant__ SceneDev S, const LightsDev* __restrict__ Lg, PathBuffers P, int cur, WaveDesc w, uint32_t rounds_left,
+__global__ void __launch_bounds__(TRACE_THREADS) k_tail(const __grid_constant__ SceneDev S, const LightsDev* __restrict__ Lg, PathBuffers P, WaveDesc w, uint32_t rounds,
                                         uint32_t limit) {
-    const uint32_t n = *(volatile uint32_t*)&P.counters[cur];
-    if (n == 0 || n > limit) return;
+    uint32_t round = TAIL_FIRST_ROUND;
+    while (round < rounds && P.counters[round_counter(round, COUNT_PATHS)] > limit) ++round;
+    const uint32_t n = round < rounds ? P.counters[round_counter(round, COUNT_PATHS)] : 0;
+    if (n == 0) return;
+    const uint32_t rounds_left = rounds - round, lanes = lanes_for(n);
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
     uint64_t deep[STACK_CAP - SHORT_STACK];
     SplitStack stack{s_stack + threadIdx.x, deep, TRACE_THREADS};
-    const uint32_t* __restrict__ queue = P.queue[cur];
+    const uint32_t* __restrict__ queue = P.queue[round & 1];
     const RaySort R;  // no coherence keys
     uint32_t err = 0, rays_local = 0, shadow_local = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    for (uint32_t i = lane < lanes ? warp * lanes + lane : n; i < n; i += gridDim.x * (blockDim.x >> 5) * lanes) {
         const uint32_t slot = queue[i];
         for (uint32_t r = 0; r < rounds_left; ++r) {
             const float4 o = P.o[slot], d = P.d[slot];
@@ -811,7 +885,7 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_tail(const __grid_constant__ 
             P.hit[slot] = got ? make_uint4(res.inst, res.tri, __float_as_uint(res.t), 1u) : make_uint4(0xffffffffu, 0xffffffffu, 0u, 0u);
             TailShadow sh;
             sh.on = false;
-            const bool alive = shade_slot<PLAIN>(S, *Lg, P, R, slot, cur, [&](uint32_t& xx, uint32_t& yy, uint32_t& ii) { wave_slot(w, slot, xx, yy, ii); },
+            const bool alive = shade_slot<PLAIN>(S, *Lg, P, R, slot, round, [&](uint32_t& xx, uint32_t& yy, uint32_t& ii) { wave_slot(w, slot, xx, yy, ii); },
                                           rays_local, shadow_local, &sh);
             if (sh.on) {
                 TraceResult unused;
@@ -831,21 +905,6 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_tail(const __grid_constant__ 
     if ((threadIdx.x & 31) == 0 && total) atomicAdd(P.rays, (unsigned long long)total);
     if ((threadIdx.x & 31) == 0 && shadows) atomicAdd(P.rays + 1, (unsigned long long)shadows);
     if (err) atomicOr(&P.counters[3], err);
-}
-
-// After k_tail: a queue it carried to the end is empty for the rest of the wave.
-__global__ void k_tail_end(PathBuffers P, int cur, uint32_t limit) {
-    const uint32_t n = P.counters[cur];
-    if (n > 0 && n <= limit) P.counters[cur] = 0;
-}
-
-__global__ void k_next_round(PathBuffers P, int cur) {
-    // The queue just consumed becomes the next round's output; the shadow queue empties; the
-    // extend and shadow queue positions start again.
-    P.counters[cur] = 0;
-    P.counters[2] = 0;
-    P.counters[4] = 0;
-    P.counters[5] = 0;
 }
 
 // ---- accumulate: film += each pixel's samples in sample-index order (image.rs:82) -------------------------
@@ -1333,59 +1392,58 @@ static void launch_traversal(const RaySort& order, int grid, cudaStream_t st, vo
 static bool tail_on(const SceneDev& S, const RaySort& order, bool batch) {
     return order.tail_paths > 0 && !S.any_passable && !S.section_on && !batch;
 }
+// Blocks of the persistent kernels for a wave of n paths: all that are resident, unless the wave
+// has fewer paths than these have warps.
+static int blocks_of(int resident, uint32_t n, int fallback) {
+    return resident > 0 ? (int)std::min<uint32_t>((uint32_t)resident, (n + TRACE_THREADS / 32 - 1) / (TRACE_THREADS / 32)) : fallback;
+}
 
 uint32_t wave_launches(const SceneDev& S, const RaySort& order, const PathBuffers& P, bool batch) {
     const uint32_t rounds = wave_rounds(S);
     const bool rsort = order.ray_bits > 0 && P.rbins, ssort = rsort && order.shadow_sort && P.sbins;
-    uint32_t per_round = 5 + (order.material_sort ? 1u : 0u) + (ssort ? 2u : 0u);
-    const uint32_t tail = tail_on(S, order, batch) && rounds > TAIL_FIRST_ROUND ? 2u * (rounds - TAIL_FIRST_ROUND) : 0u;
-    return 2 + rounds * per_round + (rsort && rounds > 1 ? 2u * (rounds - 1u) : 0u) + tail;
+    const bool tail = tail_on(S, order, batch) && rounds > TAIL_FIRST_ROUND;
+    return 2 + rounds * (3 + (order.material_sort ? 1u : 0u) + (ssort ? 2u : 0u)) + (rsort ? 2u * (rounds - 1u) : 0u) + (tail ? 1u : 0u);
 }
 
 void launch_wave(const SceneDev& S, const LightsDev* L, const WaveDesc& wave, const PathBuffers& P, const FilmDev* film, cudaStream_t st,
-                 int grid, WaveTiming* timing, const RaySort& order) {
+                 int grid, WaveTiming* timing, const RaySort& tuning) {
     static const int ext_resident = resident_blocks((const void*)k_extend, TRACE_THREADS);
     static const int sh_resident = resident_blocks((const void*)k_shadow, TRACE_THREADS);
     static const int tail_resident = resident_blocks((const void*)k_tail<false>, TRACE_THREADS);
+    static const int shade_resident = resident_blocks((const void*)k_shade<false, false>, 128);
+    static const int sort_resident = resident_blocks((const void*)k_material_sort, SORT_THREADS);
     const WaveDesc w = with_divisors(wave);
     const int g = grid;
-    const int g_ext = ext_resident > 0 && ext_resident < g ? ext_resident : g;
-    const int g_sh = sh_resident > 0 && sh_resident < g ? sh_resident : g;
+    const int g_ext = blocks_of(ext_resident, w.n, g), g_sh = blocks_of(sh_resident, w.n, g), g_shade = blocks_of(shade_resident, w.n, g);
+    const int g_sort = std::min<int>(sort_resident > 0 ? sort_resident : g, (int)((w.n + SORT_CHUNK - 1) / SORT_CHUNK));
     const bool batch = w.segs != nullptr;
+    const uint32_t rounds = wave_rounds(S);
+    RaySort order = tuning;
+    if (!tail_on(S, order, batch) || rounds <= TAIL_FIRST_ROUND) order.tail_paths = 0;
     const bool rsort = order.ray_bits > 0 && order.ray_bits <= RAY_SORT_MAX_BITS && P.rbins;
     const bool ssort = rsort && order.shadow_sort && P.sbins;
     const uint32_t nk = ray_sort_keys(order.ray_bits);
-    if (batch) k_camera<true><<<g, 256, 0, st>>>(S, w, P);
-    else k_camera<false><<<g, 256, 0, st>>>(S, w, P);
-    int cur = 0;
-    const uint32_t rounds = wave_rounds(S);
-    const bool tail = tail_on(S, order, batch);
+    if (batch) k_camera<true><<<g, 256, 0, st>>>(S, w, P, rounds);
+    else k_camera<false><<<g, 256, 0, st>>>(S, w, P, rounds);
     for (uint32_t round = 0; round < rounds; ++round) {
-        if (tail && round >= TAIL_FIRST_ROUND) {
-            (S.plain ? k_tail<true> : k_tail<false>)<<<tail_resident > 0 ? tail_resident : g, TRACE_THREADS, 0, st>>>(S, L, P, cur, w, rounds - round, order.tail_paths);
-            k_tail_end<<<1, 1, 0, st>>>(P, cur, order.tail_paths);
-        }
+        uint32_t* const queue = P.queue[round & 1];
         // The camera rays are traced in pixel order; later rounds' rays in coherence order.
-        const uint32_t* traced = P.queue[cur];
+        const uint32_t* traced = queue;
         if (rsort && round > 0) {
             k_key_scan<<<1, 1024, 0, st>>>(P.rbins, nk);
-            k_key_scatter<<<g, 256, 0, st>>>(P.queue[cur], P.key, P.rbins + nk, &P.counters[cur], P.sorted);
+            k_key_scatter<<<g, 256, 0, st>>>(queue, P.key, P.rbins + nk, &P.counters[round_counter(round, COUNT_PATHS)], P.sorted);
             traced = P.sorted;
         }
-        if (timing && timing->ev_count + 2 <= WaveTiming::MAX_EVENTS) {
-            cudaEventRecord(timing->ev[timing->ev_count++], st);
-            launch_traversal(order, g_ext, st, S.section_on ? k_extend_section : k_extend, S, P, cur, traced);
-            cudaEventRecord(timing->ev[timing->ev_count++], st);
-        } else {
-            launch_traversal(order, g_ext, st, S.section_on ? k_extend_section : k_extend, S, P, cur, traced);
-        }
+        const bool timed = timing && timing->ev_count + 2 <= WaveTiming::MAX_EVENTS;
+        if (timed) cudaEventRecord(timing->ev[timing->ev_count++], st);
+        launch_traversal(order, g_ext, st, S.section_on ? k_extend_section : k_extend, S, P, round, traced, order.tail_paths);
+        if (timed) cudaEventRecord(timing->ev[timing->ev_count++], st);
         if (round == 0 && w.alb && film && !batch) k_albedo_hits<<<g, 256, 0, st>>>(S, L, w, P);
-        k_scan<<<1, 32, 0, st>>>(P);
         // The material-sorted copy goes to whichever list the traversal did not read.
         const uint32_t* shaded = traced;
         if (order.material_sort) {
-            uint32_t* sorted = traced == P.sorted ? P.queue[cur] : P.sorted;
-            k_scatter<<<g, 256, 0, st>>>(P, cur, traced, sorted);
+            uint32_t* sorted = traced == P.sorted ? queue : P.sorted;
+            k_material_sort<<<g_sort, SORT_THREADS, 0, st>>>(P, round, traced, sorted, order.tail_paths);
             shaded = sorted;
         }
         // Keys for the next round's rays (none after the last round) and for this round's shadow rays.
@@ -1393,20 +1451,20 @@ void launch_wave(const SceneDev& S, const LightsDev* L, const WaveDesc& wave, co
         Q.rbins = rsort && round + 1 < rounds ? P.rbins : nullptr;
         Q.sbins = ssort ? P.sbins : nullptr;
         (batch ? (S.plain ? k_shade<true, true> : k_shade<true, false>) : (S.plain ? k_shade<false, true> : k_shade<false, false>))
-            <<<g, 128, 0, st>>>(S, L, Q, cur, w, shaded, order);
-        // queue[cur] is free once shade has read its list: it holds the shadow rays' order.
+            <<<g_shade, 128, 0, st>>>(S, L, Q, round, w, shaded, order);
+        // The round's queue is free once shade has read it: it holds the shadow rays' order.
         const uint32_t* perm = nullptr;
         if (ssort) {
             k_key_scan<<<1, 1024, 0, st>>>(P.sbins, nk);
-            k_key_scatter<<<g, 256, 0, st>>>(nullptr, P.sh_key, P.sbins + nk, &P.counters[2], P.queue[cur]);
-            perm = P.queue[cur];
+            k_key_scatter<<<g, 256, 0, st>>>(nullptr, P.sh_key, P.sbins + nk, &P.counters[round_counter(round, COUNT_SHADOW)], queue);
+            perm = queue;
         }
-        if (!S.any_passable) launch_traversal(order, g_sh, st, S.section_on ? k_shadow_section : k_shadow, S, P, perm);
-        else if (batch) k_shadow_walk<true><<<g, TRACE_THREADS, 0, st>>>(S, P, w, perm);
-        else k_shadow_walk<false><<<g, TRACE_THREADS, 0, st>>>(S, P, w, perm);
-        k_next_round<<<1, 1, 0, st>>>(P, cur);
-        cur ^= 1;
+        if (!S.any_passable) launch_traversal(order, g_sh, st, S.section_on ? k_shadow_section : k_shadow, S, P, round, perm);
+        else if (batch) k_shadow_walk<true><<<g, TRACE_THREADS, 0, st>>>(S, P, round, w, perm);
+        else k_shadow_walk<false><<<g, TRACE_THREADS, 0, st>>>(S, P, round, w, perm);
     }
+    if (order.tail_paths)
+        (S.plain ? k_tail<true> : k_tail<false>)<<<blocks_of(tail_resident, w.n, g), TRACE_THREADS, 0, st>>>(S, L, P, w, rounds, order.tail_paths);
     if (batch) k_accumulate_jobs<<<g, 256, 0, st>>>(w, P);
     else if (film && w.epix) k_accumulate_edges<<<g, 256, 0, st>>>(w, P, *film);
     else if (film) k_accumulate<<<g, 256, 0, st>>>(w, P, *film);
@@ -1443,20 +1501,19 @@ void launch_adjoint_wave(const SceneDev& S, const LightsDev* L, const WaveDesc& 
                          int grid) {
     static const int ext_resident = resident_blocks((const void*)k_extend, TRACE_THREADS);
     static const int sh_resident = resident_blocks((const void*)k_shadow_adjoint, TRACE_THREADS);
+    static const int shade_resident = resident_blocks((const void*)k_shade_adjoint<false>, 128);
+    static const int sort_resident = resident_blocks((const void*)k_material_sort, SORT_THREADS);
     const WaveDesc w = with_divisors(wave);
     const int g = grid;
-    const int g_ext = ext_resident > 0 && ext_resident < g ? ext_resident : g;
-    const int g_sh = sh_resident > 0 && sh_resident < g ? sh_resident : g;
-    k_adjoint_camera<<<g, 256, 0, st>>>(S, w, P, A);
-    int cur = 0;
-    for (uint32_t bounce = 0; bounce <= S.max_depth; ++bounce) {
-        k_extend<<<g_ext, TRACE_THREADS, 0, st>>>(S, P, cur, P.queue[cur]);
-        k_scan<<<1, 32, 0, st>>>(P);
-        k_scatter<<<g, 256, 0, st>>>(P, cur, P.queue[cur], P.sorted);
-        (S.plain ? k_shade_adjoint<true> : k_shade_adjoint<false>)<<<g, 128, 0, st>>>(S, L, P, cur, bounce, w, A);
-        k_shadow_adjoint<<<g_sh, TRACE_THREADS, 0, st>>>(S, P, w, A);
-        k_next_round<<<1, 1, 0, st>>>(P, cur);
-        cur ^= 1;
+    const int g_ext = blocks_of(ext_resident, w.n, g), g_sh = blocks_of(sh_resident, w.n, g), g_shade = blocks_of(shade_resident, w.n, g);
+    const int g_sort = std::min<int>(sort_resident > 0 ? sort_resident : g, (int)((w.n + SORT_CHUNK - 1) / SORT_CHUNK));
+    const uint32_t rounds = S.max_depth + 1;
+    k_adjoint_camera<<<g, 256, 0, st>>>(S, w, P, A, rounds);
+    for (uint32_t bounce = 0; bounce < rounds; ++bounce) {
+        k_extend<<<g_ext, TRACE_THREADS, 0, st>>>(S, P, bounce, P.queue[bounce & 1], 0);
+        k_material_sort<<<g_sort, SORT_THREADS, 0, st>>>(P, bounce, P.queue[bounce & 1], P.sorted, 0);
+        (S.plain ? k_shade_adjoint<true> : k_shade_adjoint<false>)<<<g_shade, 128, 0, st>>>(S, L, P, bounce, w, A);
+        k_shadow_adjoint<<<g_sh, TRACE_THREADS, 0, st>>>(S, P, bounce, w, A);
     }
     k_adjoint_residual<<<g, 256, 0, st>>>(w, P, A);
 }

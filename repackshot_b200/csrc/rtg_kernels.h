@@ -8,6 +8,15 @@ namespace rtg {
 
 struct JobDev;
 
+// Counts of round r, at counters[ROUND_COUNTERS + 4 r]: paths of its extension queue, shadow rays,
+// and how far k_extend and k_shadow have taken them. A wave's camera kernel clears every round's,
+// so no launch between the rounds has to.
+constexpr uint32_t ROUND_COUNTERS = 4, MAX_ROUNDS = 1024 + 1 + 64;
+enum : uint32_t { COUNT_PATHS = 0, COUNT_SHADOW = 1, NEXT_PATH = 2, NEXT_SHADOW = 3 };
+RTG_HD constexpr uint32_t round_counter(uint32_t round, uint32_t which) { return ROUND_COUNTERS + 4 * round + which; }
+constexpr uint32_t MATERIAL_KEYS = 256, KEY_BINS = 2 * MATERIAL_KEYS;  // of two rounds in turn: 2 KEY_BINS words
+constexpr uint32_t COUNTERS_BYTES = (round_counter(MAX_ROUNDS + 1, 0) * 4 + 255) / 256 * 256;
+
 // Rounds of a wave: one per vertex up to the depth, plus, when a material is a cut-out, one per
 // cut-out a path may pass (at most 64; a pass is no vertex).
 inline uint32_t wave_rounds(const SceneDev& S) { return S.max_depth + 1u + (S.any_cutout ? 64u : 0u); }
@@ -105,13 +114,13 @@ struct PathBuffers {
     uint32_t* medium;
     uint4* hit;
     uint32_t* queue[2];
-    uint32_t* sorted;    // the active queue ordered by material key (shade reads it)
+    uint32_t* sorted;    // the active queue in another order: ray-sorted (RaySort) or by material
     uint32_t* key;       // per slot: material of the hit (n_materials: floor or miss)
-    uint32_t* bins;      // [0, 256) key histogram, [256, 512) scatter cursors
+    uint32_t* bins;      // round r's material keys, at bins + KEY_BINS (r & 1): their histogram, then cursors
     float4* sh_o;    // shadow rays: origin, w: t_max
     float4* sh_d;
     float4* sh_c;    // contribution, w: slot
-    uint32_t* counters;  // [0], [1] queue lengths, [2] shadow queue length, [3] error bits
+    uint32_t* counters;  // [3] error bits; ROUND_COUNTERS + 4 r on: round r's counts (round_counters)
     unsigned long long* rays;
     // Coherence sort of the rays before each traversal (RaySort); all null: off.
     uint32_t* rbins;   // extension rays: [0, nk) key histogram, [nk, 2 nk) cursors
@@ -136,7 +145,7 @@ struct RaySort {
     size_t l2_bytes = 0;
     float l2_hit_ratio = 0.0f;
     // tail_paths > 0: from round TAIL_FIRST_ROUND on, a round whose extension queue holds at most
-    // tail_paths paths and every later round run in one launch, a path per thread (k_tail).
+    // tail_paths paths and every later round run in the wave's last launch, a path per lane (k_tail).
     uint32_t tail_paths = 0;
 };
 constexpr uint32_t TAIL_FIRST_ROUND = 2;

@@ -27,8 +27,8 @@ namespace {
 // first-hit albedo of each path (16), which a film with fused guides adds to its guide sums.
 constexpr size_t kBytesPerPath = 10 * 16 + 6 * 4;
 constexpr size_t kPaths = RTG_NOALLOC_MAX_PATHS;
-constexpr size_t kBinsBytes = 512 * 4;
-constexpr size_t kCountersBytes = 64;  // [0], [1] queue lengths, [2] shadow queue, [3] error bits
+constexpr size_t kBinsBytes = 2 * KEY_BINS * 4;
+constexpr size_t kCountersBytes = COUNTERS_BYTES;  // [3] error bits, then the rounds' counts
 constexpr size_t kRaysBytes = 64;      // [0] camera + extension rays, [1] shadow rays
 constexpr size_t kLayoutBytes = kPaths * kBytesPerPath + kBinsBytes + kCountersBytes + kRaysBytes;
 static_assert(kPaths % 64 == 0, "every array must keep 256-byte alignment");
@@ -128,8 +128,8 @@ uint32_t noalloc_render(const NoallocJob& job, NoallocResult& res, const char** 
         uint64_t per = kPaths / bpix;
         if (per > job.count) per = job.count;
         const uint32_t per_wave = (uint32_t)per;
-        // The counters and ray counts are the only part of the array that must start at zero;
-        // the camera kernel writes every path slot of a wave before anything reads it.
+        // The error bits and ray counts must start at zero; the camera kernel writes the rounds'
+        // counts and every path slot of a wave before anything reads them.
         cudaError_t e = cudaMemsetAsync(P.counters, 0, kCountersBytes + kRaysBytes, job.stream);
         if (e != cudaSuccess) { *why = cudaGetErrorString(e); return RTG_STATUS_CUDA_ERROR; }
         for (uint32_t s = 0; s < job.count; s += per_wave) {
