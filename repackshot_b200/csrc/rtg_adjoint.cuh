@@ -6,7 +6,7 @@
 // A forward wave renders every path of the call and leaves each path's radiance L in its slot.
 // k_adjoint_delta turns the film and the target image into the loss and, per pixel, the loss's
 // derivative with respect to one path's radiance. The backward wave (k_adjoint_camera, the forward's
-// k_extend and k_material_sort, then k_shade_adjoint and k_shadow_adjoint per bounce) runs every
+// k_trace and k_material_sort, then k_shade_adjoint and k_shadow_adjoint per bounce) runs every
 // path again from its pixel and sample index (the sampler makes it the same path), carrying
 // L_rem = L - (the contributions met so far), which is the radiance still to come. At each vertex:
 // - a contribution c of area light i adds <dL, c> to light i's scale gradient, and when c is a
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(128, RTG_SHADE_MIN_BLOCKS) k_shade_adjoint(con
 
 // Shadow rays of the backward wave: an unblocked one takes its contribution off its path's
 // radiance still to come and adds its light's and its material's gradients. Persistent warps
-// with lane refill, as k_shadow.
+// with lane refill, as k_trace.
 __device__ __forceinline__ void adjoint_unblocked(const PathBuffers& P, const AdjointDev& A, const WaveDesc& w, float* g, uint32_t i) {
     const float4 c = P.sh_c[i];
     const uint32_t slot = __float_as_uint(c.w);
@@ -435,7 +435,7 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_shadow_adjoint(const __grid_c
     blk.begin(n_params);
     const uint32_t n = *(volatile uint32_t*)&P.counters[round_counter(bounce, COUNT_SHADOW)];
     uint32_t* position = &P.counters[round_counter(bounce, NEXT_SHADOW)];
-    const uint32_t lane = threadIdx.x & 31u, lanes = lanes_for(n), enough = min(lanes, (uint32_t)RTG_SHADOW_REFILL_MIN);
+    const uint32_t lane = threadIdx.x & 31u, lanes = lanes_for(n), enough = min(lanes, (uint32_t)RTG_REFILL_MIN);
     uint32_t err = 0, ray = 0;
     bool busy = false, drained = false;
     Trav T;
@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_shadow_adjoint(const __grid_c
                 ro = v3(o.x, o.y, o.z);
                 rd = v3(d.x, d.y, d.z);
             };
-            if (trav_step<true, true>(S, T, 1.0e-3f, stack, &err, blocked, src)) {
+            if (trav_step<TRACE_ANY, true>(S, T, 1.0e-3f, stack, &err, blocked, src)) {
                 busy = false;
                 if (!blocked) adjoint_unblocked(P, A, w, s_grad, ray);
             }

@@ -493,6 +493,7 @@ uint32_t run_wave(Scene& sc, const WaveDesc& w, const FilmDev* film, const Scene
     launch_wave(Sw, lights ? lights : sc.d_lights, w, sc.P, film, sc.stream, grid_for(w.n, 128), t, sc.order);
     RTG_CHECK(cudaGetLastError());
     sc.launches += wave_launches(Sw, sc.order, sc.P, w.segs != nullptr) - ((film || w.segs) ? 0 : 1) + ((w.alb && film && !w.segs) ? 2 : 0);
+    if (t && !Sw.any_passable && !Sw.section_on) sc.launches += wave_rounds(Sw);  // shadow rays apart
     if (t) {
         RTG_CHECK(cudaStreamSynchronize(sc.stream));
         for (int i = 0; i + 1 < t->ev_count; i += 2) {

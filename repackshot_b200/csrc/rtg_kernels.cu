@@ -17,28 +17,17 @@ __constant__ SobolTable c_sobol;
 
 // Threads per block of the traversal kernels (the stride of their shared stacks).
 constexpr int TRACE_THREADS = 128;
-// RTG_REFILL_MIN (build setting): idle lanes a k_extend warp waits for before it takes new rays
-// (1: every step with an idle lane; a warp whose lanes are all idle always refills). A refill
-// costs the whole warp a ballot, an atomic, a shuffle and two dependent loads, so taking rays for
-// eight lanes at a time beats taking them one by one as rays end: on the 1080p product frame the
-// extend time fell from 145 to 130 ms (4: 134 ms, 10: 130 ms, 12: 130 ms, 16: 133 ms).
+// RTG_REFILL_MIN (build setting): idle lanes a k_trace warp waits for before it takes new rays
+// (1: every step with an idle lane). A refill costs the whole warp a ballot, an atomic, a shuffle
+// and two dependent loads, so taking rays for eight lanes at a time beats taking them one by one as
+// rays end: at 4, 8, 12 and 16 the 1080p product frame took 197.6, 192.7, 193.8 and 196.2 ms.
 #ifndef RTG_REFILL_MIN
 #define RTG_REFILL_MIN 8
 #endif
-// RTG_SHADOW_REFILL_MIN (build setting): the same for k_shadow (frame 312 ms at 1, 308 at 8, 309
-// at 4, 312 at 16).
-#ifndef RTG_SHADOW_REFILL_MIN
-#define RTG_SHADOW_REFILL_MIN 8
-#endif
-// RTG_MIN_LANES (build setting): the fewest lanes of a warp that a thin round fills (lanes_for).
-#ifndef RTG_MIN_LANES
-#define RTG_MIN_LANES 1u
-#endif
-// RTG_TRACE_MIN_BLOCKS (build setting): blocks per SM the traversal kernels (k_extend, k_shadow)
-// are compiled for (0: the compiler's choice of registers, 76). At 8 (64 registers, no spills in
-// k_extend, 40 bytes in k_shadow) the 1080p product frame's extend time fell from 163 to 145 ms
-// and the frame from 349 to 327 ms: more warps hide the node fetches. 7 and 9 blocks measured
-// 337-338 ms, 10 blocks 350 ms.
+// RTG_TRACE_MIN_BLOCKS (build setting): blocks per SM the traversal kernel is compiled for (0: the
+// compiler's choice of registers). At 8 (64 registers, no spills) its warps hide the node fetches
+// best over both workloads: at 7, 8, 9 and 10 blocks the 1080p product frame took 200, 192.7, 190.9
+// and 197 ms, the instanced frame 43.7, 42.7, 43.4 and 45.3 ms.
 #ifndef RTG_TRACE_MIN_BLOCKS
 #define RTG_TRACE_MIN_BLOCKS 8
 #endif
@@ -135,7 +124,7 @@ __device__ __forceinline__ uint32_t round_paths(const PathBuffers& P, uint32_t r
 // and nodes of 31 others.
 __device__ __forceinline__ uint32_t lanes_for(uint32_t n) {
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    return min(32u, max(RTG_MIN_LANES, (n + warps - 1) / warps));
+    return min(32u, (n + warps - 1) / warps);
 }
 
 // ---- camera generation ---------------------------------------------------------------------------
@@ -248,24 +237,44 @@ __global__ void k_key_scatter(const uint32_t* __restrict__ list, const uint32_t*
     }
 }
 
-// ---- extend: nearest hit of every active path ------------------------------------------------------------
-// Persistent warps over the active queue: a lane whose ray has finished takes the next queue entry
-// (one atomic per warp on the round's position) while the rest of the warp keeps traversing, so no
-// lane idles until the slowest ray of its warp is done. In a thin round only lanes_for lanes take rays.
-// `order`: the active queue in the order to trace it (the round's queue, or its ray-sorted copy).
-__global__ void RTG_TRACE_BOUNDS k_extend(const __grid_constant__ SceneDev S, PathBuffers P, uint32_t round, const uint32_t* __restrict__ order, uint32_t tail) {
+// ---- trace: the nearest hit of every active path, the any hit of every shadow ray --------------------
+// An unblocked shadow ray adds its light to its path.
+__device__ __forceinline__ void shadow_unblocked(const PathBuffers& P, uint32_t i) {
+    const float4 c = P.sh_c[i];
+    const uint32_t slot = __float_as_uint(c.w);
+    float4 s = P.sum[slot];
+    s.x = s.x + c.x; s.y = s.y + c.y; s.z = s.z + c.z;
+    P.sum[slot] = s;
+}
+// Persistent warps over the extension queue of round `round` (EXTEND, SHADOW_TOO) and the shadow rays
+// of the round before it (SHADOW_TOO) or of `round` itself (SHADOW): a lane whose ray has finished
+// takes the next one (one atomic per warp on the round's position) while the rest of the warp keeps
+// traversing, so no lane idles until the slowest ray of its warp is done. In a thin round only
+// lanes_for lanes take rays. A round's shadow rays and the next round's extension rays depend on
+// nothing of each other (a path's radiance waits for its shadow ray only at the next vertex), so one
+// launch traces both: its end, where the slowest rays keep a few warps busy, comes once.
+// `order`: the active queue in the order to trace it (the round's queue, or its ray-sorted copy);
+// `perm` (may be null): the shadow queue in the order to trace it.
+enum TraceRays { EXTEND, SHADOW, SHADOW_TOO };
+template <TraceRays RAYS>
+__global__ void RTG_TRACE_BOUNDS k_trace(const __grid_constant__ SceneDev S, PathBuffers P, uint32_t round, const uint32_t* __restrict__ order,
+                                         const uint32_t* __restrict__ perm, uint32_t tail) {
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
     uint64_t deep[STACK_CAP - SHORT_STACK];
     SplitStack stack{s_stack + threadIdx.x, deep, TRACE_THREADS};
-    const uint32_t n = round_paths(P, round, tail);
+    constexpr TraceMode MODE = RAYS == EXTEND ? TRACE_NEAREST : (RAYS == SHADOW ? TRACE_ANY : TRACE_EITHER);
+    const uint32_t paths = RAYS == SHADOW ? 0 : round_paths(P, round, tail);
+    const uint32_t shadows = RAYS == EXTEND ? 0 : *(volatile uint32_t*)&P.counters[round_counter(RAYS == SHADOW ? round : round - 1, COUNT_SHADOW)];
+    const uint32_t n = paths + shadows;
     if (n == 0) return;
-    uint32_t* position = &P.counters[round_counter(round, NEXT_PATH)];
+    uint32_t* position = &P.counters[round_counter(round, RAYS == SHADOW ? NEXT_SHADOW : NEXT_PATH)];
     uint32_t* bins = P.bins + KEY_BINS * (round & 1);
     const uint32_t lane = threadIdx.x & 31u, lanes = lanes_for(n), enough = min(lanes, (uint32_t)RTG_REFILL_MIN);
-    uint32_t err = 0, slot = 0;
+    uint32_t err = 0, ray = 0;  // the path's slot or the shadow ray
     bool busy = false, drained = false;
     Trav T;
     for (;;) {
+        bool done = false, hit = false;
         if (!drained) {
             const uint32_t idle = __ballot_sync(0xffffffffu, !busy && lane < lanes);
             if ((uint32_t)__popc(idle) >= enough) {
@@ -276,39 +285,51 @@ __global__ void RTG_TRACE_BOUNDS k_extend(const __grid_constant__ SceneDev S, Pa
                 if (base + (uint32_t)__popc(idle) >= n) drained = true;
                 const uint32_t i = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
                 if (!busy && lane < lanes && i < n) {
-                    slot = order[i];
-                    const float4 o = P.o[slot], d = P.d[slot];
-                    const uint32_t pf = P.flags[slot];
-                    busy = !(pf & PF_NOTHING) && trav_init(S, T, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 1.0e-3f, f_inf(), (pf & PF_PRIMARY) != 0);
-                    if (!busy) {
-                        P.hit[slot] = make_uint4(0xffffffffu, 0xffffffffu, 0u, 0u);
-                        const uint32_t key = material_key(S, false, 0);
-                        P.key[slot] = key;
-                        warp_count(bins, key);
+                    float4 o, d;
+                    bool camera = false, sees = true;
+                    float tmax = f_inf();
+                    if (RAYS == EXTEND || (RAYS == SHADOW_TOO && i < paths)) {
+                        ray = order[i];
+                        o = P.o[ray];
+                        d = P.d[ray];
+                        const uint32_t pf = P.flags[ray];
+                        camera = (pf & PF_PRIMARY) != 0;
+                        sees = !(pf & PF_NOTHING);
+                        T.any = false;
+                    } else {
+                        ray = perm ? perm[i - paths] : i - paths;
+                        o = P.sh_o[ray];
+                        d = P.sh_d[ray];
+                        tmax = o.w;
+                        T.any = true;
                     }
+                    busy = sees && trav_init(S, T, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 1.0e-3f, tmax, camera);
+                    done = !busy;
                 }
             }
         }
-        if (!__any_sync(0xffffffffu, busy)) {
-            if (drained) break;
-            continue;
-        }
         if (busy) {
-            bool got = false;
             const auto src = [&](V3& ro, V3& rd) {
-                const float4 o = P.o[slot], d = P.d[slot];
+                const bool any = MODE == TRACE_ANY || (MODE == TRACE_EITHER && T.any);
+                const float4 o = any ? P.sh_o[ray] : P.o[ray], d = any ? P.sh_d[ray] : P.d[ray];
                 ro = v3(o.x, o.y, o.z);
                 rd = v3(d.x, d.y, d.z);
             };
-            if (trav_step<false, true>(S, T, 1.0e-3f, stack, &err, got, src)) {
-                busy = false;
-                P.hit[slot] = got ? make_uint4(T.best_i, T.best_tri, __float_as_uint(T.best_t), 1u)
-                                  : make_uint4(0xffffffffu, 0xffffffffu, 0u, 0u);
-                const uint32_t key = material_key(S, got, T.best_i);
-                P.key[slot] = key;
+            done = trav_step<MODE, true>(S, T, 1.0e-3f, stack, &err, hit, src);
+            busy = !done;
+        }
+        if (done) {
+            if (MODE == TRACE_ANY || (MODE == TRACE_EITHER && T.any)) {
+                if (!hit) shadow_unblocked(P, ray);
+            } else {
+                P.hit[ray] = hit ? make_uint4(T.best_i, T.best_tri, __float_as_uint(T.best_t), 1u)
+                                 : make_uint4(0xffffffffu, 0xffffffffu, 0u, 0u);
+                const uint32_t key = material_key(S, hit, T.best_i);
+                P.key[ray] = key;
                 warp_count(bins, key);
             }
         }
+        if (drained && !__any_sync(0xffffffffu, busy)) break;
     }
     if (err) atomicOr(&P.counters[3], err);
 }
@@ -317,7 +338,7 @@ __global__ void RTG_TRACE_BOUNDS k_extend(const __grid_constant__ SceneDev S, Pa
 // `out` = the round's n paths of `in` ordered by material key (the order inside a key does not
 // matter: every path's result depends on its own slot only). Each block orders the next SORT_CHUNK
 // of them in shared memory, takes its part of every key's run with one atomic, and writes the runs
-// coalesced; the runs' starts it sums itself from the histogram k_extend left. Sorting only within
+// coalesced; the runs' starts it sums itself from the histogram k_trace left. Sorting only within
 // the chunks a shade block reads would save the pass but not pay: with all blocks in the same few
 // materials at a time the kernel's instructions stay in the caches (1080p frame, chunks of 512, 1024
 // and 2048: 254, 231 and 213 ms; whole queue 193 ms). Against a pass with an atomic per warp and key
@@ -381,15 +402,14 @@ __global__ void __launch_bounds__(SORT_THREADS) k_material_sort(PathBuffers P, u
         __syncthreads();
     }
 }
-// Calls f(slot) for the n paths of `order`, a path per lane; a thin round's few paths go to the first
-// lanes of all warps. The round's key bins, read for the last time before, are cleared for the next
-// round but one.
+// Calls f(slot) for the n paths of `order`, a path per lane (of whole warps also in thin rounds:
+// the paths of one material share their code). The round's key bins, read for the last time before,
+// are cleared for the next round but one.
 template <class F>
 __device__ __forceinline__ void for_each_path(const PathBuffers& P, const uint32_t* __restrict__ order, uint32_t n, uint32_t round, F f) {
     if (blockIdx.x == 0)
         for (uint32_t k = threadIdx.x; k < KEY_BINS; k += blockDim.x) P.bins[KEY_BINS * (round & 1) + k] = 0;
-    const uint32_t lanes = lanes_for(n), warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
-    for (uint32_t i = lane < lanes ? warp * lanes + lane : n; i < n; i += gridDim.x * (blockDim.x >> 5) * lanes) f(order[i]);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) f(order[i]);
 }
 
 // ---- shade: one vertex of every active path ----------------------------------------------------------
@@ -688,71 +708,11 @@ __global__ void __launch_bounds__(128, RTG_SHADE_MIN_BLOCKS) k_shade(const __gri
     if ((threadIdx.x & 31) == 0 && shadows) atomicAdd(P.rays + 1, (unsigned long long)shadows);
 }
 
-// ---- shadow: any hit of every queued shadow ray; the unblocked add their light ----------------------------
-// Persistent warps with lane refill, as k_extend.
-__device__ __forceinline__ void shadow_unblocked(const PathBuffers& P, uint32_t i) {
-    const float4 c = P.sh_c[i];
-    const uint32_t slot = __float_as_uint(c.w);
-    float4 s = P.sum[slot];
-    s.x = s.x + c.x; s.y = s.y + c.y; s.z = s.z + c.z;
-    P.sum[slot] = s;
-}
-
-// `perm` (may be null): the shadow queue in the order to trace it.
-__global__ void RTG_TRACE_BOUNDS k_shadow(const __grid_constant__ SceneDev S, PathBuffers P, uint32_t round, const uint32_t* __restrict__ perm) {
-    __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
-    uint64_t deep[STACK_CAP - SHORT_STACK];
-    SplitStack stack{s_stack + threadIdx.x, deep, TRACE_THREADS};
-    const uint32_t n = *(volatile uint32_t*)&P.counters[round_counter(round, COUNT_SHADOW)];
-    if (n == 0) return;
-    uint32_t* position = &P.counters[round_counter(round, NEXT_SHADOW)];
-    const uint32_t lane = threadIdx.x & 31u, lanes = lanes_for(n), enough = min(lanes, (uint32_t)RTG_SHADOW_REFILL_MIN);
-    uint32_t err = 0, ray = 0;
-    bool busy = false, drained = false;
-    Trav T;
-    for (;;) {
-        if (!drained) {
-            const uint32_t idle = __ballot_sync(0xffffffffu, !busy && lane < lanes);
-            if ((uint32_t)__popc(idle) >= enough) {
-                const int leader = __ffs((int)idle) - 1;
-                uint32_t base = 0;
-                if ((int)lane == leader) base = atomicAdd(position, (uint32_t)__popc(idle));
-                base = __shfl_sync(0xffffffffu, base, leader);
-                if (base + (uint32_t)__popc(idle) >= n) drained = true;
-                const uint32_t i = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
-                if (!busy && lane < lanes && i < n) {
-                    ray = perm ? perm[i] : i;
-                    const float4 o = P.sh_o[ray], d = P.sh_d[ray];
-                    busy = trav_init(S, T, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 1.0e-3f, o.w, false);
-                    if (!busy) shadow_unblocked(P, ray);
-                }
-            }
-        }
-        if (!__any_sync(0xffffffffu, busy)) {
-            if (drained) break;
-            continue;
-        }
-        if (busy) {
-            bool blocked = false;
-            const auto src = [&](V3& ro, V3& rd) {
-                const float4 o = P.sh_o[ray], d = P.sh_d[ray];
-                ro = v3(o.x, o.y, o.z);
-                rd = v3(d.x, d.y, d.z);
-            };
-            if (trav_step<true, true>(S, T, 1.0e-3f, stack, &err, blocked, src)) {
-                busy = false;
-                if (!blocked) shadow_unblocked(P, ray);
-            }
-        }
-    }
-    if (err) atomicOr(&P.counters[3], err);
-}
-
-// ---- the section view: k_extend and k_shadow through the section's queries (geometry/section.rs) -------
+// ---- the section view: k_trace through the section's queries (geometry/section.rs) --------------------
 // One ray per thread: a query may be several traversals (the kept part, the cap's probe beyond the
-// plane, the studio on the removed side), so the lane refill of the plain kernels does not apply.
-// Launched instead of them for a scene with a section; they write the same records (a cap is a hit
-// with triangle CAP_TRIANGLE).
+// plane, the studio on the removed side), so the lane refill of k_trace does not apply. Launched
+// instead of it for a scene with a section; they write the same records (a cap is a hit with
+// triangle CAP_TRIANGLE).
 __global__ void __launch_bounds__(TRACE_THREADS) k_extend_section(const __grid_constant__ SceneDev S, PathBuffers P, uint32_t round, const uint32_t* __restrict__ order, uint32_t tail) {
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
     uint64_t deep[STACK_CAP - SHORT_STACK];
@@ -793,7 +753,7 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_shadow_section(const __grid_c
 // Nearest hits along the ray: a passable surface multiplies what arrives by its straight
 // transmittance (a thin wall's) times its opacity plus 1 - opacity, and the ray goes on from just
 // behind it, up to 32 crossings; any other surface blocks it. One thread per ray: only scenes with
-// passable instances run it, instead of k_shadow. BATCH: each ray's job gives its materials.
+// passable instances run it, instead of k_trace's any hits. BATCH: each ray's job gives its materials.
 template <bool BATCH>
 __global__ void __launch_bounds__(TRACE_THREADS) k_shadow_walk(const __grid_constant__ SceneDev S, PathBuffers P, uint32_t round, WaveDesc w, const uint32_t* __restrict__ perm) {
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
@@ -853,8 +813,8 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_shadow_walk(const __grid_cons
 // ---- tail: the last rounds of a wave, a path per lane -------------------------------------------------
 // The wave's last launch. From the first round whose extension queue holds at most `limit` paths on,
 // the other kernels do nothing, and here each lane carries its share of those paths through the
-// wave's remaining rounds alone: the nearest hit (as k_extend), the vertex (shade_slot), the any
-// hit of its shadow ray and its contribution (as k_shadow), the next ray; each path's arithmetic in
+// wave's remaining rounds alone: the nearest hit (as k_trace), the vertex (shade_slot), the any
+// hit of its shadow ray and its contribution, the next ray; each path's arithmetic in
 // the order the wavefront gives it, so its sum has the same bits. A wave whose last rounds hold few
 // paths then pays one launch as long as its slowest path instead of a chain of launches, each as
 // long as its slowest ray. Scenes with passable surfaces (shadow walks) and batched waves keep the
@@ -866,7 +826,10 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_tail(const __grid_constant__ 
     while (round < rounds && P.counters[round_counter(round, COUNT_PATHS)] > limit) ++round;
     const uint32_t n = round < rounds ? P.counters[round_counter(round, COUNT_PATHS)] : 0;
     if (n == 0) return;
-    const uint32_t rounds_left = rounds - round, lanes = lanes_for(n);
+    // Up to four paths a warp run spread over all warps; more run in full warps, which meet each
+    // other's code less often (at 4, spread against full: a 64 x 64 tile 0.51 and 0.56 ms, a 720p
+    // viewport 4.74 and 4.39 ms, whose tail holds up to 16,384 paths).
+    const uint32_t rounds_left = rounds - round, spread = lanes_for(n), lanes = spread <= 4u ? spread : 32u;
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
     uint64_t deep[STACK_CAP - SHORT_STACK];
     SplitStack stack{s_stack + threadIdx.x, deep, TRACE_THREADS};
@@ -1402,19 +1365,19 @@ uint32_t wave_launches(const SceneDev& S, const RaySort& order, const PathBuffer
     const uint32_t rounds = wave_rounds(S);
     const bool rsort = order.ray_bits > 0 && P.rbins, ssort = rsort && order.shadow_sort && P.sbins;
     const bool tail = tail_on(S, order, batch) && rounds > TAIL_FIRST_ROUND;
-    return 2 + rounds * (3 + (order.material_sort ? 1u : 0u) + (ssort ? 2u : 0u)) + (rsort ? 2u * (rounds - 1u) : 0u) + (tail ? 1u : 0u);
+    const bool apart = S.any_passable || S.section_on;
+    return 2 + rounds * (2 + (apart ? 1u : 0u) + (order.material_sort ? 1u : 0u) + (ssort ? 2u : 0u)) + (rsort ? 2u * (rounds - 1u) : 0u) + (tail ? 1u : 0u);
 }
 
 void launch_wave(const SceneDev& S, const LightsDev* L, const WaveDesc& wave, const PathBuffers& P, const FilmDev* film, cudaStream_t st,
                  int grid, WaveTiming* timing, const RaySort& tuning) {
-    static const int ext_resident = resident_blocks((const void*)k_extend, TRACE_THREADS);
-    static const int sh_resident = resident_blocks((const void*)k_shadow, TRACE_THREADS);
+    static const int trace_resident = resident_blocks((const void*)k_trace<SHADOW_TOO>, TRACE_THREADS);
     static const int tail_resident = resident_blocks((const void*)k_tail<false>, TRACE_THREADS);
     static const int shade_resident = resident_blocks((const void*)k_shade<false, false>, 128);
     static const int sort_resident = resident_blocks((const void*)k_material_sort, SORT_THREADS);
     const WaveDesc w = with_divisors(wave);
     const int g = grid;
-    const int g_ext = blocks_of(ext_resident, w.n, g), g_sh = blocks_of(sh_resident, w.n, g), g_shade = blocks_of(shade_resident, w.n, g);
+    const int g_trace = blocks_of(trace_resident, w.n, g), g_shade = blocks_of(shade_resident, w.n, g);
     const int g_sort = std::min<int>(sort_resident > 0 ? sort_resident : g, (int)((w.n + SORT_CHUNK - 1) / SORT_CHUNK));
     const bool batch = w.segs != nullptr;
     const uint32_t rounds = wave_rounds(S);
@@ -1425,6 +1388,14 @@ void launch_wave(const SceneDev& S, const LightsDev* L, const WaveDesc& wave, co
     const uint32_t nk = ray_sort_keys(order.ray_bits);
     if (batch) k_camera<true><<<g, 256, 0, st>>>(S, w, P, rounds);
     else k_camera<false><<<g, 256, 0, st>>>(S, w, P, rounds);
+    // Each round's shadow rays are traced with the next round's extension rays. The last round has
+    // none: its vertices are at the greatest depth (only cut-outs, which are passable, shift that).
+    // Timed waves trace them apart, so that the events are around extension rays only.
+    // So do waves of more than 2^25 paths: their launches' ends weigh little, and shadow rays visit
+    // children in slot order there, which needs no sort (132.7 M paths: 180.6 ms apart, 181.7
+    // together; 8.4 M paths: 31.1 and 29.6; 0.9 M paths: 5.05 and 4.71).
+    const bool together = !S.any_passable && !S.section_on && !timing && w.n <= (1u << 25);
+    const uint32_t* perm = nullptr;  // the last round's shadow rays in the order to trace them (null: as queued)
     for (uint32_t round = 0; round < rounds; ++round) {
         uint32_t* const queue = P.queue[round & 1];
         // The camera rays are traced in pixel order; later rounds' rays in coherence order.
@@ -1436,7 +1407,8 @@ void launch_wave(const SceneDev& S, const LightsDev* L, const WaveDesc& wave, co
         }
         const bool timed = timing && timing->ev_count + 2 <= WaveTiming::MAX_EVENTS;
         if (timed) cudaEventRecord(timing->ev[timing->ev_count++], st);
-        launch_traversal(order, g_ext, st, S.section_on ? k_extend_section : k_extend, S, P, round, traced, order.tail_paths);
+        if (S.section_on) launch_traversal(order, g_trace, st, k_extend_section, S, P, round, traced, order.tail_paths);
+        else launch_traversal(order, g_trace, st, together && round > 0 ? k_trace<SHADOW_TOO> : k_trace<EXTEND>, S, P, round, traced, perm, order.tail_paths);
         if (timed) cudaEventRecord(timing->ev[timing->ev_count++], st);
         if (round == 0 && w.alb && film && !batch) k_albedo_hits<<<g, 256, 0, st>>>(S, L, w, P);
         // The material-sorted copy goes to whichever list the traversal did not read.
@@ -1453,15 +1425,15 @@ void launch_wave(const SceneDev& S, const LightsDev* L, const WaveDesc& wave, co
         (batch ? (S.plain ? k_shade<true, true> : k_shade<true, false>) : (S.plain ? k_shade<false, true> : k_shade<false, false>))
             <<<g_shade, 128, 0, st>>>(S, L, Q, round, w, shaded, order);
         // The round's queue is free once shade has read it: it holds the shadow rays' order.
-        const uint32_t* perm = nullptr;
+        perm = nullptr;
         if (ssort) {
             k_key_scan<<<1, 1024, 0, st>>>(P.sbins, nk);
             k_key_scatter<<<g, 256, 0, st>>>(nullptr, P.sh_key, P.sbins + nk, &P.counters[round_counter(round, COUNT_SHADOW)], queue);
             perm = queue;
         }
-        if (!S.any_passable) launch_traversal(order, g_sh, st, S.section_on ? k_shadow_section : k_shadow, S, P, round, perm);
-        else if (batch) k_shadow_walk<true><<<g, TRACE_THREADS, 0, st>>>(S, P, round, w, perm);
-        else k_shadow_walk<false><<<g, TRACE_THREADS, 0, st>>>(S, P, round, w, perm);
+        if (S.any_passable) (batch ? k_shadow_walk<true> : k_shadow_walk<false>)<<<g, TRACE_THREADS, 0, st>>>(S, P, round, w, perm);
+        else if (S.section_on) launch_traversal(order, g_trace, st, k_shadow_section, S, P, round, perm);
+        else if (!together) launch_traversal(order, g_trace, st, k_trace<SHADOW>, S, P, round, traced, perm, 0u);
     }
     if (order.tail_paths)
         (S.plain ? k_tail<true> : k_tail<false>)<<<blocks_of(tail_resident, w.n, g), TRACE_THREADS, 0, st>>>(S, L, P, w, rounds, order.tail_paths);
@@ -1499,7 +1471,7 @@ void launch_adjoint_delta(const FilmDev& F, const float* target, float4* dpath, 
 }
 void launch_adjoint_wave(const SceneDev& S, const LightsDev* L, const WaveDesc& wave, const PathBuffers& P, const AdjointDev& A, cudaStream_t st,
                          int grid) {
-    static const int ext_resident = resident_blocks((const void*)k_extend, TRACE_THREADS);
+    static const int ext_resident = resident_blocks((const void*)k_trace<EXTEND>, TRACE_THREADS);
     static const int sh_resident = resident_blocks((const void*)k_shadow_adjoint, TRACE_THREADS);
     static const int shade_resident = resident_blocks((const void*)k_shade_adjoint<false>, 128);
     static const int sort_resident = resident_blocks((const void*)k_material_sort, SORT_THREADS);
@@ -1510,7 +1482,7 @@ void launch_adjoint_wave(const SceneDev& S, const LightsDev* L, const WaveDesc& 
     const uint32_t rounds = S.max_depth + 1;
     k_adjoint_camera<<<g, 256, 0, st>>>(S, w, P, A, rounds);
     for (uint32_t bounce = 0; bounce < rounds; ++bounce) {
-        k_extend<<<g_ext, TRACE_THREADS, 0, st>>>(S, P, bounce, P.queue[bounce & 1], 0);
+        k_trace<EXTEND><<<g_ext, TRACE_THREADS, 0, st>>>(S, P, bounce, P.queue[bounce & 1], nullptr, 0);
         k_material_sort<<<g_sort, SORT_THREADS, 0, st>>>(P, bounce, P.queue[bounce & 1], P.sorted, 0);
         (S.plain ? k_shade_adjoint<true> : k_shade_adjoint<false>)<<<g_shade, 128, 0, st>>>(S, L, P, bounce, w, A);
         k_shadow_adjoint<<<g_sh, TRACE_THREADS, 0, st>>>(S, P, bounce, w, A);

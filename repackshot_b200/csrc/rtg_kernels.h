@@ -9,7 +9,7 @@ namespace rtg {
 struct JobDev;
 
 // Counts of round r, at counters[ROUND_COUNTERS + 4 r]: paths of its extension queue, shadow rays,
-// and how far k_extend and k_shadow have taken them. A wave's camera kernel clears every round's,
+// and how far k_trace has taken them. A wave's camera kernel clears every round's,
 // so no launch between the rounds has to.
 constexpr uint32_t ROUND_COUNTERS = 4, MAX_ROUNDS = 1024 + 1 + 64;
 enum : uint32_t { COUNT_PATHS = 0, COUNT_SHADOW = 1, NEXT_PATH = 2, NEXT_SHADOW = 3 };

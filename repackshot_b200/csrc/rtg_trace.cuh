@@ -98,8 +98,8 @@ struct TraceResult { uint32_t inst, tri; float t; };
 // every ray stays within the shared part.
 // A build may set RTG_SHORT_STACK to trade shared memory (8 bytes x 128 threads per entry and
 // block) against spills to the deeper part. 16 entries (16 KB a block) leave 128 KB of the SM's
-// shared memory to L1 at 8 blocks per SM, where the node fetches hit; on the 1080p product frame
-// 12, 16 and 20 entries measured within 1% of each other, 24 entries 3% slower.
+// shared memory to L1 at 8 blocks per SM, where the node fetches hit; 10, 16 and 24 entries measured
+// 193.1, 192.7 and 193.4 ms on the 1080p product frame.
 #ifndef RTG_SHORT_STACK
 #define RTG_SHORT_STACK 16
 #endif
@@ -126,6 +126,7 @@ struct Trav {
     int kz;                // its major axis; the other two follow in cyclic order
     bool flip;             // the direction runs down the major axis: the reference swaps the other two
     bool camera;
+    bool any;              // TRACE_EITHER: this ray's query is any-hit
     float best_t;          // nearest hit so far (any-hit queries: t_max)
     uint32_t best_i, best_tri, cur;
     uint32_t blas;         // the BLAS being walked: index << 3 | moved << 2 | flags; TLAS_LEVEL: none
@@ -308,11 +309,11 @@ RTG_D void sort8(uint32_t k[8]) {
 
 // One step of the two-level traversal: the slab test of one node, or the triangles of one leaf,
 // then the next node (a child, or the nearest entry of the stack that is still in range).
-// `ANY`: stop at the first hit in [t_min, t_max] (shadow rays; children in slot order, leaves first).
-// Otherwise the nearest hit with the reference's tie-break, children nearest first. `POS`: t_min is
-// known to be positive. `src(o, d)` gives the query's world ray. Returns true when the query is
-// over; `hit` then says whether it found one (nearest: in T.best_*). A stack that would overflow
-// sets *err bit 0 and ends the query as a miss.
+// `MODE`: the nearest hit with the reference's tie-break, children nearest first; or any hit in
+// [t_min, t_max], which ends the query (children in slot order, leaves first); or either, as T.any
+// says, children nearest first. `POS`: t_min is known to be positive. `src(o, d)` gives the query's
+// world ray. Returns true when the query is over; `hit` then says whether it found one (nearest: in
+// T.best_*). A stack that would overflow sets *err bit 0 and ends the query as a miss.
 //
 // What bounds it is instruction issue (and, in thin rounds, the chain of one ray's steps), not
 // memory: the tree stays in L2. So a node step is kept short: two instructions a plane, 32-bit keys
@@ -320,9 +321,11 @@ RTG_D void sort8(uint32_t k[8]) {
 // planes (five instructions each), a 64-bit selection per pushed child and a greedy collapse, the
 // 1080p product frame went from 312.7 to 229.0 ms, the instanced frame (10 M triangles, 4 spp) from
 // 66.4 to 46.1 ms, a 64 x 64 tile from 1.35 to 0.88 ms; films bit-equal.
-template <bool ANY, bool POS, class Stack, class Src>
+enum TraceMode { TRACE_NEAREST, TRACE_ANY, TRACE_EITHER };
+template <TraceMode MODE, bool POS, class Stack, class Src>
 RTG_D bool trav_step(const SceneDev& S, Trav& T, float tmin, Stack& stack, uint32_t* err, bool& hit, const Src& src) {
     const uint32_t cur = T.cur;
+    const bool any = MODE == TRACE_ANY || (MODE == TRACE_EITHER && T.any);
     if ((cur & NODE_LEAF) == 0) {
         const QNode* node = S.nodes + cur;
         const NodeHead h = load_head(node);
@@ -345,7 +348,7 @@ RTG_D bool trav_step(const SceneDev& S, Trav& T, float tmin, Stack& stack, uint3
                                         plane_t(c < 4 ? Z.n0 : Z.n1, k, Z.a, Z.b_near)), tmin);
             const float f = fminf(fminf(fminf(plane_t(c < 4 ? X.f0 : X.f1, k, X.a, X.b_far), plane_t(c < 4 ? Y.f0 : Y.f1, k, Y.a, Y.b_far)),
                                         plane_t(c < 4 ? Z.f0 : Z.f1, k, Z.a, Z.b_far)), tmax);
-            if (ANY) {
+            if (MODE == TRACE_ANY) {
                 // Slot order, the highest slot (leaves come last) next, the others pushed.
                 if (n <= f) {
                     if (next != 0xffffffffu) stack.put(T.sp++, (uint64_t)next);
@@ -355,7 +358,7 @@ RTG_D bool trav_step(const SceneDev& S, Trav& T, float tmin, Stack& stack, uint3
                 key[c] = n <= f ? ((ordered_bits<POS>(n) & ~7u) | c) : 0xffffffffu;
             }
         }
-        if (!ANY) {
+        if (MODE != TRACE_ANY) {
             // Nearest next, the others pushed farthest first: a sorting network of 19 exchanges.
             sort8(key);
             if (key[0] != 0xffffffffu) {
@@ -426,7 +429,7 @@ RTG_D bool trav_step(const SceneDev& S, Trav& T, float tmin, Stack& stack, uint3
                 if (!(t >= tmin && t <= T.best_t)) continue;
                 const uint32_t tri = __float_as_uint(a.w);
                 uint32_t inst = __float_as_uint(b.w);
-                if (!ANY) {
+                if (!any) {
                     if (inst == 0xffffffffu) inst = __ldg(&S.blas[T.blas >> 3].instance);
                     if (!(t < T.best_t || inst < T.best_i || (inst == T.best_i && tri < T.best_tri))) continue;
                 }
@@ -439,7 +442,7 @@ RTG_D bool trav_step(const SceneDev& S, Trav& T, float tmin, Stack& stack, uint3
                     src(o, d);
                     if (!hit_kept(S.blas, S.leaf_boxes, o, d, T.blas, flags >> TRI_LEAF_SHIFT, tmin, T.best_t)) continue;
                 }
-                if (ANY) { hit = true; return true; }
+                if (any) { hit = true; return true; }
                 T.best_t = t;
                 T.best_i = inst;
                 T.best_tri = tri;
@@ -448,7 +451,7 @@ RTG_D bool trav_step(const SceneDev& S, Trav& T, float tmin, Stack& stack, uint3
     }
     for (;;) {
         if (T.sp == 0) {
-            hit = !ANY && T.best_i != 0xffffffffu;
+            hit = MODE != TRACE_ANY && T.best_i != 0xffffffffu;  // no any-hit query sets it
             return true;
         }
         const uint64_t e = stack.get(--T.sp);
@@ -462,7 +465,7 @@ RTG_D bool trav_step(const SceneDev& S, Trav& T, float tmin, Stack& stack, uint3
             T.blas = TLAS_LEVEL;
             continue;
         }
-        if (ANY || __uint_as_float((uint32_t)(e >> 32)) <= T.best_t * RTG_ROBUST) { T.cur = ref; return false; }
+        if (MODE == TRACE_ANY || __uint_as_float((uint32_t)(e >> 32)) <= T.best_t * RTG_ROBUST) { T.cur = ref; return false; }
     }
 }
 
@@ -479,7 +482,7 @@ RTG_D bool traverse(const SceneDev& S, V3 o, V3 d, float tmin, float tmax, bool 
     if (!trav_init(S, T, o, d, tmin, tmax, camera)) return false;
     bool hit = false;
     const HeldRay src{o, d};
-    while (!trav_step<ANY, POS>(S, T, tmin, stack, err, hit, src)) {
+    while (!trav_step<ANY ? TRACE_ANY : TRACE_NEAREST, POS>(S, T, tmin, stack, err, hit, src)) {
     }
     if (hit && !ANY) { res.inst = T.best_i; res.tri = T.best_tri; res.t = T.best_t; }
     return hit;
