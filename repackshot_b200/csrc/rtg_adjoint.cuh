@@ -214,12 +214,11 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
             s_point = point; s_hit = point; s_normal = nn; s_geom = nn;
         } else {
             HitInfo h;
-            uint4 idx;
-            if (!hit_details<PLAIN>(S, ro, rd, 1.0e-3f, f_inf(), hit.x, hit.y, __uint_as_float(hit.z), h, I, idx)) break;
+            if (!hit_details<PLAIN>(S, ro, rd, 1.0e-3f, f_inf(), hit.x, hit.y, __uint_as_float(hit.z), h, I)) break;
             V3 ng = h.geometric, nrm = h.normal;
             if (dot(nrm, ng) < 0.0f) nrm = -nrm;
             if (dot(nrm, rd) >= -1.0e-4f) nrm = ng;
-            s_point = terminator_point(S, I, idx, h);
+            s_point = terminator_point(S, I, h);
             s_hit = h.point;
             s_normal = nrm;
             s_geom = ng;

@@ -56,7 +56,7 @@ struct alignas(16) DevInstance {
     float to_local[12];
     float to_world[12];
     uint32_t identity, active, material, mesh;
-    uint32_t flags, inside_out, has_normals, tri_base;  // tri_base: first global triangle of its mesh
+    uint32_t flags, inside_out, has_normals, pad0;
     uint32_t tangent_on, passable, emitter, solid;  // passable: shadow rays cross it (cut-out or thin wall);
                                                     // emitter: its mesh light's index in lights[] + 1, or 0;
                                                     // solid: the section caps it, 1 wound outward, 2 inward (0 not)
@@ -166,9 +166,10 @@ struct SceneDev {
     const BlasInst* blas;
     const float* leaf_boxes;  // 8 floats per leaf: its triangles' box, lower corner in [0, 3), upper in [4, 7)
     const DevInstance* instances;
-    const float4* positions;  // xyz per vertex (global)
-    const float4* normals;    // xyz per vertex (global)
-    const uint4* tri_index;   // global vertex indices per global triangle
+    // The three corners' normals (xyz, as the mesh gives them) of each leaf triangle, three float4s;
+    // null when no mesh has normals. A hit names its leaf triangle, so shading reads the corners from
+    // `tris`, where traversal has just been, and these, with no vertex indices in between.
+    const float4* tri_normals;
     const DevMaterial* materials;
     // Bsdf::surface of every material seen from outside (2 m) and from inside (2 m + 1), and the
     // floor's Lambert lobe (2 n_materials): built once on the host, the same bits.

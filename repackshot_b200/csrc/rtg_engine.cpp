@@ -242,11 +242,6 @@ uint32_t upload(BufSet& set, const std::vector<T>& v, const T*& out) {
 // What traversal reads (nodes, leaf triangles, top-level leaves) lies first, in one allocation,
 // so that one L2 access-policy window can cover it (its size in *hot_bytes).
 uint32_t upload_geometry(const Flat& F, BufSet& set, SceneDev& S, size_t* hot_bytes = nullptr) {
-    std::vector<float4> pos(F.positions.size() / 4), nrm(F.normals.size() / 4);
-    std::memcpy(pos.data(), F.positions.data(), F.positions.size() * 4);
-    std::memcpy(nrm.data(), F.normals.data(), F.normals.size() * 4);
-    std::vector<uint4> ti(F.tri_index.size() / 4);
-    std::memcpy(ti.data(), F.tri_index.data(), F.tri_index.size() * 4);
     auto round = [](size_t b) { return (b + 255) / 256 * 256; };
     const size_t b_nodes = F.nodes.size() * sizeof(QNode), b_tris = F.tris.size() * sizeof(TriRec), b_blas = F.blas.size() * sizeof(BlasInst);
     const size_t hot = round(b_nodes) + round(b_tris) + round(b_blas);
@@ -268,9 +263,10 @@ uint32_t upload_geometry(const Flat& F, BufSet& set, SceneDev& S, size_t* hot_by
         if (b_blas) S.blas = (const BlasInst*)(p + round(b_nodes) + round(b_tris));
     }
     uint32_t st;
-    if ((st = upload(set, pos, S.positions)) || (st = upload(set, nrm, S.normals)) || (st = upload(set, ti, S.tri_index)) ||
-        (st = upload(set, F.leaf_boxes, S.leaf_boxes)))
+    const float* normals = nullptr;
+    if ((st = upload(set, F.tri_normals, normals)) || (st = upload(set, F.leaf_boxes, S.leaf_boxes)))
         return st;
+    S.tri_normals = reinterpret_cast<const float4*>(normals);
     return RTG_STATUS_OK;
 }
 
@@ -328,7 +324,7 @@ void keep_shading(Scene& sc, const HScene& hs, const Flat& F) {
 SceneDev compose(const SceneDev& constants, const SceneDev& geom, const SceneDev& shade) {
     SceneDev S = constants;
     S.nodes = geom.nodes; S.tris = geom.tris; S.blas = geom.blas; S.leaf_boxes = geom.leaf_boxes;
-    S.positions = geom.positions; S.normals = geom.normals; S.tri_index = geom.tri_index;
+    S.tri_normals = geom.tri_normals;
     S.tlas_root = geom.tlas_root; S.single_blas = geom.single_blas; S.stack_need = geom.stack_need;
     S.instances = shade.instances; S.materials = shade.materials; S.bsdfs = shade.bsdfs; S.plate = shade.plate;
     S.exempt_boxes = shade.exempt_boxes;

@@ -322,7 +322,7 @@ __global__ void RTG_TRACE_BOUNDS k_trace(const __grid_constant__ SceneDev S, Pat
             if (MODE == TRACE_ANY || (MODE == TRACE_EITHER && T.any)) {
                 if (!hit) shadow_unblocked(P, ray);
             } else {
-                P.hit[ray] = hit ? make_uint4(T.best_i, T.best_tri, __float_as_uint(T.best_t), 1u)
+                P.hit[ray] = hit ? make_uint4(T.best_i, T.best_k, __float_as_uint(T.best_t), 1u)
                                  : make_uint4(0xffffffffu, 0xffffffffu, 0u, 0u);
                 const uint32_t key = material_key(S, hit, T.best_i);
                 P.key[ray] = key;
@@ -489,13 +489,12 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
             s_point = point; s_hit = point; s_normal = nn; s_geom = nn;
         } else {
             HitInfo h;
-            uint4 idx;
-            if (!hit_details<PLAIN>(S, ro, rd, 1.0e-3f, f_inf(), hit.x, hit.y, __uint_as_float(hit.z), h, I, idx)) break;
+            if (!hit_details<PLAIN>(S, ro, rd, 1.0e-3f, f_inf(), hit.x, hit.y, __uint_as_float(hit.z), h, I)) break;
             // bevel.rs:232 shading_point without a bevel
             V3 ng = h.geometric, nrm = h.normal;
             if (dot(nrm, ng) < 0.0f) nrm = -nrm;
             if (dot(nrm, rd) >= -1.0e-4f) nrm = ng;
-            s_point = terminator_point(S, I, idx, h);
+            s_point = terminator_point(S, I, h);
             s_hit = h.point;
             s_normal = nrm;
             s_geom = ng;
@@ -783,9 +782,8 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_shadow_walk(const __grid_cons
             if (!trace_q<false>(J, o, d, 1.0e-3f, tmax, false, res, &err, stack)) { arrives = true; break; }
             if (res.inst >= J.n_instances || !J.instances[res.inst].passable) break;
             HitInfo h;
-            uint4 idx;
             const DevInstance* I = nullptr;
-            if (!hit_details(J, o, d, 1.0e-3f, f_inf(), res.inst, res.tri, res.t, h, I, idx)) break;
+            if (!hit_details(J, o, d, 1.0e-3f, f_inf(), res.inst, res.tri, res.t, h, I)) break;
             const uint32_t m = I->material;
             const float opacity = rclamp(J.materials[m].opacity, 0.0f, 1.0f);
             keep = keep * (straight_transmittance(J.bsdfs[2 * m], dot(h.geometric, d)) * opacity + splat(1.0f - opacity));
@@ -972,9 +970,8 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_edge_exact(const __grid_const
                 e.x = e.y = 0xffffffffu;
             } else {
                 HitInfo h;
-                uint4 idx;
                 const DevInstance* I = nullptr;
-                ok = hit_details(S, o, d, 1.0e-3f, f_inf(), res.inst, res.tri, res.t, h, I, idx) && I != nullptr;
+                ok = hit_details(S, o, d, 1.0e-3f, f_inf(), res.inst, res.tri, res.t, h, I) && I != nullptr;
                 if (ok) {
                     e.x = res.inst + 1u;
                     e.y = I->material < S.n_materials ? I->material + 1u : 0u;
@@ -1020,9 +1017,8 @@ static __device__ __noinline__ void first_hit_passes(const SceneDev& S, const Li
         albedo = rgb(S.floor_color[0], S.floor_color[1], S.floor_color[2]);
     } else {
         HitInfo h;
-        uint4 idx;
         const DevInstance* I = nullptr;
-        if (!(hit_details(S, o, d, 1.0e-3f, f_inf(), res.inst, res.tri, res.t, h, I, idx) && I != nullptr)) return;
+        if (!(hit_details(S, o, d, 1.0e-3f, f_inf(), res.inst, res.tri, res.t, h, I) && I != nullptr)) return;
         e.x = res.inst + 1u;
         const bool known = I->material < S.n_materials;
         e.y = known ? I->material + 1u : 0u;
@@ -1146,9 +1142,8 @@ __global__ void k_albedo_hits(const __grid_constant__ SceneDev S, const LightsDe
                 a = make_float4(S.floor_color[0], S.floor_color[1], S.floor_color[2], 0.0f);
             } else {
                 HitInfo h;
-                uint4 idx;
                 const DevInstance* I = nullptr;
-                if (hit_details(S, o, d, 1.0e-3f, f_inf(), hit.x, hit.y, __uint_as_float(hit.z), h, I, idx) && I != nullptr) {
+                if (hit_details(S, o, d, 1.0e-3f, f_inf(), hit.x, hit.y, __uint_as_float(hit.z), h, I) && I != nullptr) {
                     if (I->material < S.n_materials) {
                         const float* b = S.materials[I->material].base;
                         a = make_float4(b[0], b[1], b[2], 0.0f);
@@ -1300,7 +1295,7 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_trace_batch(const __grid_cons
         } else {
             bool got = trace_q<false>(S, o, d, r[6], r[7], (mode & 1u) != 0, res, &err, stack);
             out[3 * i] = got ? res.inst : 0xffffffffu;
-            out[3 * i + 1] = got ? res.tri : 0xffffffffu;
+            out[3 * i + 1] = got && res.tri != CAP_TRIANGLE ? __ldg(&S.tris[res.tri].tri) : 0xffffffffu;
             out[3 * i + 2] = got ? __float_as_uint(res.t) : 0u;
         }
     }

@@ -963,38 +963,6 @@ static bool flatten(const HScene& s, Flat& F, std::string& error, bool geometry,
     auto t0 = std::chrono::steady_clock::now();
     F = Flat();
     const size_t ni = s.instances.size();
-    // Vertices, normals and triangle indices, global.
-    std::vector<uint32_t> vtx_base(s.meshes.size()), tri_base(s.meshes.size());
-    uint32_t nv = 0, nt = 0;
-    for (size_t m = 0; m < s.meshes.size(); ++m) {
-        vtx_base[m] = nv;
-        tri_base[m] = nt;
-        nv += (uint32_t)s.meshes[m].positions.size();
-        nt += (uint32_t)s.meshes[m].triangles();
-    }
-    if (geometry) {
-        F.positions.resize((size_t)nv * 4);
-        F.normals.assign((size_t)nv * 4, 0.0f);
-        F.tri_index.resize((size_t)nt * 4);
-        for (size_t m = 0; m < s.meshes.size(); ++m) {
-            const HMesh& M = s.meshes[m];
-            for (size_t v = 0; v < M.positions.size(); ++v) {
-                float* p = &F.positions[((size_t)vtx_base[m] + v) * 4];
-                p[0] = M.positions[v].x; p[1] = M.positions[v].y; p[2] = M.positions[v].z; p[3] = 0;
-                if (!M.normals.empty()) {
-                    float* n = &F.normals[((size_t)vtx_base[m] + v) * 4];
-                    n[0] = M.normals[v].x; n[1] = M.normals[v].y; n[2] = M.normals[v].z;
-                }
-            }
-            for (size_t t = 0; t < M.triangles(); ++t) {
-                uint32_t* ti = &F.tri_index[((size_t)tri_base[m] + t) * 4];
-                ti[0] = vtx_base[m] + M.indices[3 * t];
-                ti[1] = vtx_base[m] + M.indices[3 * t + 1];
-                ti[2] = vtx_base[m] + M.indices[3 * t + 2];
-                ti[3] = (uint32_t)m;
-            }
-        }
-    }
     // Instances.
     Box scene_box;
     std::vector<Xf> xf(ni), inv(ni);
@@ -1018,7 +986,6 @@ static bool flatten(const HScene& s, Flat& F, std::string& error, bool geometry,
         d.flags = in.flags;
         d.inside_out = M.inside_out;
         d.has_normals = !M.normals.empty();
-        d.tri_base = tri_base[in.mesh];
         const HMaterial& mat = s.materials[in.material_id];
         // Shadow rays cross cut-outs and thin walls (integrator/mod.rs:371).
         const bool thin = (mat.flags & MATERIAL_FLAG_THIN) != 0;
@@ -1106,8 +1073,11 @@ static bool flatten(const HScene& s, Flat& F, std::string& error, bool geometry,
             std::memcpy(to, v, sizeof(v));
         };
         F.leaf_boxes.assign(8, 0.0f);
-        // Appends the leaf of the triangles `p` as record(p) gives them.
-        auto emit_leaf = [&](const uint32_t* p, uint32_t n, const Box& box, auto&& record) {
+        bool any_normals = false;
+        for (const HMesh& M : s.meshes) any_normals |= !M.normals.empty();
+        if (any_normals) F.tri_normals.assign(12, 0.0f);
+        // Appends the leaf of the triangles `p` as record(p), of mesh(p), gives them.
+        auto emit_leaf = [&](const uint32_t* p, uint32_t n, const Box& box, auto&& record, auto&& mesh) {
             const uint32_t first = (uint32_t)F.tris.size(), leaf = (uint32_t)(F.leaf_boxes.size() / 8);
             F.leaf_boxes.resize(F.leaf_boxes.size() + 8);
             put_box(&F.leaf_boxes[8 * (size_t)leaf], box);
@@ -1115,6 +1085,15 @@ static bool flatten(const HScene& s, Flat& F, std::string& error, bool geometry,
                 TriRec r = record(p[k]);
                 r.flags |= (leaf << TRI_LEAF_SHIFT) | (k + 1 == n ? TRI_LAST : 0u);
                 F.tris.push_back(r);
+                if (!any_normals) continue;
+                const HMesh& M = mesh(p[k]);
+                F.tri_normals.resize(F.tri_normals.size() + 12, 0.0f);
+                if (M.normals.empty()) continue;
+                float* to = &F.tri_normals[F.tri_normals.size() - 12];
+                for (int c = 0; c < 3; ++c) {
+                    const V3& v = M.normals[M.indices[3 * (size_t)r.tri + c]];
+                    to[4 * c] = v.x; to[4 * c + 1] = v.y; to[4 * c + 2] = v.z;
+                }
             }
             return first;
         };
@@ -1146,6 +1125,8 @@ static bool flatten(const HScene& s, Flat& F, std::string& error, bool geometry,
                     cents[k] = b.centroid();
                     all = all.uni(b);
                 }
+                F.tris.reserve(F.tris.size() + prims.size());
+                if (any_normals) F.tri_normals.reserve(F.tri_normals.size() + 12 * prims.size());
                 SahBuilder sb{boxes, cents, 4, 8, {}, {}};
                 sb.order.resize(prims.size());
                 for (size_t k = 0; k < prims.size(); ++k) sb.order[k] = (uint32_t)k;
@@ -1153,9 +1134,8 @@ static bool flatten(const HScene& s, Flat& F, std::string& error, bool geometry,
                 fl.bn = &sb.nodes;
                 fl.order = &sb.order;
                 fl.emit = [&](const uint32_t* p, uint32_t n, const Box& box) {
-                    return emit_leaf(p, n, box, [&](uint32_t k) {
-                        return triangle(s.meshes[s.instances[prims[k].first].mesh], prims[k].second, prims[k].first, seen(prims[k].first));
-                    });
+                    auto mesh = [&](uint32_t k) -> const HMesh& { return s.meshes[s.instances[prims[k].first].mesh]; };
+                    return emit_leaf(p, n, box, [&](uint32_t k) { return triangle(mesh(k), prims[k].second, prims[k].first, seen(prims[k].first)); }, mesh);
                 };
                 BlasInst bi;
                 std::memset(&bi, 0, sizeof(bi));
@@ -1188,7 +1168,8 @@ static bool flatten(const HScene& s, Flat& F, std::string& error, bool geometry,
                 fl.bn = &sb.nodes;
                 fl.order = &sb.order;
                 fl.emit = [&](const uint32_t* p, uint32_t cnt, const Box& box) {
-                    return emit_leaf(p, cnt, box, [&](uint32_t t) { return triangle(M, t, 0xffffffffu, 0u); });
+                    return emit_leaf(p, cnt, box, [&](uint32_t t) { return triangle(M, t, 0xffffffffu, 0u); },
+                                     [&](uint32_t) -> const HMesh& { return M; });
                 };
                 mesh_root[m] = fl.flatten();
                 blas_depth = std::max(blas_depth, fl.max_depth);

@@ -144,8 +144,7 @@ struct Flat {
     std::vector<BlasInst> blas;
     std::vector<float> leaf_boxes;  // 8 per leaf
     std::vector<DevInstance> instances;
-    std::vector<float> positions, normals;  // 4 floats per vertex
-    std::vector<uint32_t> tri_index;        // 4 per triangle
+    std::vector<float> tri_normals;  // 12 floats per leaf triangle (empty: no mesh has normals)
     std::vector<DevMaterial> materials;
     std::vector<Bsdf> bsdfs;  // 2 per material (entering, leaving), then the floor's
     LightsDev lights;

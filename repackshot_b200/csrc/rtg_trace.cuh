@@ -91,7 +91,7 @@ RTG_D V3 xf_transpose(const float* m, V3 v) {
     return v3(m[0] * v.x + m[4] * v.y + m[8] * v.z, m[1] * v.x + m[5] * v.y + m[9] * v.z, m[2] * v.x + m[6] * v.y + m[10] * v.z);
 }
 
-struct TraceResult { uint32_t inst, tri; float t; };
+struct TraceResult { uint32_t inst, tri; float t; };  // tri: the leaf triangle (SceneDev::tris)
 
 // A traversal stack whose first SHORT_STACK entries sit in shared memory, interleaved by thread
 // (entry k of thread i at sm[k * stride + i]), and the deeper ones in a per-thread array. Almost
@@ -128,7 +128,7 @@ struct Trav {
     bool camera;
     bool any;              // TRACE_EITHER: this ray's query is any-hit
     float best_t;          // nearest hit so far (any-hit queries: t_max)
-    uint32_t best_i, best_tri, cur;
+    uint32_t best_i, best_k, cur;  // its instance and leaf triangle
     uint32_t blas;         // the BLAS being walked: index << 3 | moved << 2 | flags; TLAS_LEVEL: none
     int sp;
 };
@@ -164,7 +164,7 @@ RTG_D bool trav_init(const SceneDev& S, Trav& T, V3 o, V3 d, float tmin, float t
     if (!(tmin <= T.best_t)) return false;
     trav_ray(T, o, d);
     T.best_i = 0xffffffffu;
-    T.best_tri = 0xffffffffu;
+    T.best_k = 0xffffffffu;
     T.sp = 0;
     T.camera = camera;
     T.cur = S.tlas_root;
@@ -427,11 +427,10 @@ RTG_D bool trav_step(const SceneDev& S, Trav& T, float tmin, Stack& stack, uint3
                 const float az = T.sz * a_z, bz = T.sz * b_z, cz = T.sz * c_z;
                 const float t = (u * az + v * bz + w * cz) / det;
                 if (!(t >= tmin && t <= T.best_t)) continue;
-                const uint32_t tri = __float_as_uint(a.w);
                 uint32_t inst = __float_as_uint(b.w);
                 if (!any) {
                     if (inst == 0xffffffffu) inst = __ldg(&S.blas[T.blas >> 3].instance);
-                    if (!(t < T.best_t || inst < T.best_i || (inst == T.best_i && tri < T.best_tri))) continue;
+                    if (!(t < T.best_t || inst < T.best_i || (inst == T.best_i && __float_as_uint(a.w) < __ldg(&S.tris[T.best_k].tri)))) continue;
                 }
                 // Within the rounding of t (a generous 2^-14 of the corners' distances) of an end of
                 // the interval, the reference's boxes decide; and where t may be negative, which
@@ -445,7 +444,7 @@ RTG_D bool trav_step(const SceneDev& S, Trav& T, float tmin, Stack& stack, uint3
                 if (any) { hit = true; return true; }
                 T.best_t = t;
                 T.best_i = inst;
-                T.best_tri = tri;
+                T.best_k = k - 1;
             } while (!(flags & TRI_LAST));
         }
     }
@@ -484,7 +483,7 @@ RTG_D bool traverse(const SceneDev& S, V3 o, V3 d, float tmin, float tmax, bool 
     const HeldRay src{o, d};
     while (!trav_step<ANY ? TRACE_ANY : TRACE_NEAREST, POS>(S, T, tmin, stack, err, hit, src)) {
     }
-    if (hit && !ANY) { res.inst = T.best_i; res.tri = T.best_tri; res.t = T.best_t; }
+    if (hit && !ANY) { res.inst = T.best_i; res.tri = T.best_k; res.t = T.best_t; }
     return hit;
 }
 
@@ -517,13 +516,13 @@ RTG_D bool section_hidden(const SceneDev& S, bool camera, uint32_t inst) {
     return camera && inst < S.n_instances && (S.instances[inst].flags & 4u) != 0;  // INSTANCE_NO_CAMERA
 }
 
-// True when triangle `tri` of capped instance `inst` is met by direction d from inside its solid.
+// True when leaf triangle `tri` of capped instance `inst` is met by direction d from inside its solid.
 RTG_D bool section_met_from_inside(const SceneDev& S, V3 d, uint32_t inst, uint32_t tri) {
     if (inst >= S.n_instances) return false;
     const DevInstance* I = S.instances + inst;
     if (!I->active || I->solid == 0u) return false;
-    const uint4 idx = __ldg(S.tri_index + I->tri_base + tri);
-    const float4 q0 = __ldg(S.positions + idx.x), q1 = __ldg(S.positions + idx.y), q2 = __ldg(S.positions + idx.z);
+    const float4* rec = reinterpret_cast<const float4*>(S.tris + tri);
+    const float4 q0 = __ldg(rec), q1 = __ldg(rec + 1), q2 = __ldg(rec + 2);
     const V3 p0 = v3(q0.x, q0.y, q0.z), p1 = v3(q1.x, q1.y, q1.z), p2 = v3(q2.x, q2.y, q2.z);
     V3 w = cross(p1 - p0, p2 - p0);
     if (!I->identity) w = xf_transpose(I->to_local, w);
@@ -650,12 +649,13 @@ struct HitInfo {
     float bary[3];
     bool front, outside;
     bool cap;  // on a section's cap: no triangle, the plane's normal
+    uint32_t tri;  // the leaf triangle
 };
 
 // geometry/mod.rs:731 hit_details for an instance hit. `P`: a plain scene (SceneDev::plain), no section.
 template <bool P = false>
 RTG_D_NI bool hit_details(const SceneDev& S, V3 o, V3 d, float tmin, float tmax, uint32_t inst, uint32_t tri, float t_hit,
-                       HitInfo& h, const DevInstance*& I_out, uint4& idx_out) {
+                       HitInfo& h, const DevInstance*& I_out) {
     if (inst >= S.n_instances) return false;
     const DevInstance* I = S.instances + inst;
     I_out = I;
@@ -672,12 +672,11 @@ RTG_D_NI bool hit_details(const SceneDev& S, V3 o, V3 d, float tmin, float tmax,
         h.bary[0] = 1.0f;
         h.bary[1] = h.bary[2] = 0.0f;
         h.outside = h.front;
-        idx_out = make_uint4(0u, 0u, 0u, 0u);
         return true;
     }
-    uint4 idx = __ldg(S.tri_index + I->tri_base + tri);
-    idx_out = idx;
-    float4 q0 = __ldg(S.positions + idx.x), q1 = __ldg(S.positions + idx.y), q2 = __ldg(S.positions + idx.z);
+    h.tri = tri;
+    const float4* rec = reinterpret_cast<const float4*>(S.tris + tri);
+    const float4 q0 = __ldg(rec), q1 = __ldg(rec + 1), q2 = __ldg(rec + 2);
     V3 p0 = v3(q0.x, q0.y, q0.z), p1 = v3(q1.x, q1.y, q1.z), p2 = v3(q2.x, q2.y, q2.z);
     bool identity = I->identity != 0;
     PRay r = identity ? prepare_ray(o, d, tmin, tmax) : prepare_ray(xf_point(I->to_local, o), xf_vector(I->to_local, d), tmin, tmax);
@@ -696,7 +695,8 @@ RTG_D_NI bool hit_details(const SceneDev& S, V3 o, V3 d, float tmin, float tmax,
     h.front = dot(winding, d) < 0.0f;
     V3 smooth = v3(0, 0, 0);
     if (I->has_normals) {
-        float4 m0 = __ldg(S.normals + idx.x), m1 = __ldg(S.normals + idx.y), m2 = __ldg(S.normals + idx.z);
+        const float4* nr = S.tri_normals + 3 * (size_t)tri;
+        const float4 m0 = __ldg(nr), m1 = __ldg(nr + 1), m2 = __ldg(nr + 2);
         V3 s = v3(m0.x, m0.y, m0.z) * h.bary[0] + v3(m1.x, m1.y, m1.z) * h.bary[1] + v3(m2.x, m2.y, m2.z) * h.bary[2];
         smooth = identity ? s : xf_transpose(I->to_local, s);
     }
@@ -709,10 +709,10 @@ RTG_D_NI bool hit_details(const SceneDev& S, V3 o, V3 d, float tmin, float tmax,
 }
 
 // geometry/mod.rs:682 terminator_point (Hanika 2021).
-RTG_D_NI V3 terminator_point(const SceneDev& S, const DevInstance* I, uint4 idx, const HitInfo& h) {
+RTG_D_NI V3 terminator_point(const SceneDev& S, const DevInstance* I, const HitInfo& h) {
     if (h.cap || !I->has_normals) return h.point;
-    float4 q[3] = {__ldg(S.positions + idx.x), __ldg(S.positions + idx.y), __ldg(S.positions + idx.z)};
-    float4 m[3] = {__ldg(S.normals + idx.x), __ldg(S.normals + idx.y), __ldg(S.normals + idx.z)};
+    const float4 *rec = reinterpret_cast<const float4*>(S.tris + h.tri), *nr = S.tri_normals + 3 * (size_t)h.tri;
+    const float4 q[3] = {__ldg(rec), __ldg(rec + 1), __ldg(rec + 2)}, m[3] = {__ldg(nr), __ldg(nr + 1), __ldg(nr + 2)};
     V3 c[3], n[3];
     for (int k = 0; k < 3; ++k) { c[k] = v3(q[k].x, q[k].y, q[k].z); n[k] = v3(m[k].x, m[k].y, m[k].z); }
     float b0 = h.bary[0], b1 = h.bary[1], b2 = h.bary[2];

@@ -60,7 +60,7 @@ extern "C" uint32_t host_trace(void* l, const float* rays, uint64_t n, int any, 
             out[i] = hit;
         } else {
             out[3 * i] = hit ? res.inst : 0xffffffffu;
-            out[3 * i + 1] = hit ? res.tri : 0xffffffffu;
+            out[3 * i + 1] = hit ? S.tris[res.tri].tri : 0xffffffffu;
             out[3 * i + 2] = hit ? fbits(res.t) : 0u;
         }
     }
