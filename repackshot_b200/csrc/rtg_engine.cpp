@@ -434,10 +434,7 @@ uint32_t ensure_capacity(Scene& sc, uint32_t paths) {
     uint8_t* p = (uint8_t*)sc.path_mem.p;
     auto take = [&](size_t each) { uint8_t* r = p; p += ((n * each + 255) / 256) * 256; return r; };
     // (sizes rounded to 256 bytes; `bytes` above leaves room for the rounding of 14 arrays)
-    sc.P.o = (float4*)take(16);
-    sc.P.d = (float4*)take(16);
-    sc.P.thr = (float4*)take(16);
-    sc.P.sum = (float4*)take(16);
+    place_records(sc.P, take(64));
     sc.P.sel = (float4*)take(16);
     sc.P.flags = (uint32_t*)take(4);
     sc.P.medium = (uint32_t*)take(4);
@@ -1547,20 +1544,20 @@ uint32_t rtg_render_paths(uint32_t handle, const uint32_t* xys, uint32_t n, floa
     WaveDesc wd{0, 0, 1, 1, 0, n, d_xys};
     st = run_wave(*sc, wd, nullptr);
     if (st) return st;
-    std::vector<float4> sum(n), thr(n);
+    std::vector<float4> record(4 * (size_t)n);
     std::vector<uint32_t> flags(n);
-    RTG_CHECK(cudaMemcpyAsync(sum.data(), sc->P.sum, (size_t)n * 16, cudaMemcpyDeviceToHost, sc->stream));
-    RTG_CHECK(cudaMemcpyAsync(thr.data(), sc->P.thr, (size_t)n * 16, cudaMemcpyDeviceToHost, sc->stream));
+    RTG_CHECK(cudaMemcpyAsync(record.data(), sc->P.o.p, record.size() * 16, cudaMemcpyDeviceToHost, sc->stream));
     RTG_CHECK(cudaMemcpyAsync(flags.data(), sc->P.flags, (size_t)n * 4, cudaMemcpyDeviceToHost, sc->stream));
     st = finish(*sc, nullptr);
     if (st) return st;
     for (uint32_t i = 0; i < n; ++i) {
         // a panoramic camera's sample that sees nothing weighs black (render.rs:465)
         const float k = (flags[i] & 8u) ? 0.0f : 1.0f;
-        out5[5 * i] = k == 1.0f ? sum[i].x : sum[i].x * k;
-        out5[5 * i + 1] = k == 1.0f ? sum[i].y : sum[i].y * k;
-        out5[5 * i + 2] = k == 1.0f ? sum[i].z : sum[i].z * k;
-        out5[5 * i + 3] = thr[i].w;
+        const float4 thr = record[4 * (size_t)i + 2], sum = record[4 * (size_t)i + 3];
+        out5[5 * i] = k == 1.0f ? sum.x : sum.x * k;
+        out5[5 * i + 1] = k == 1.0f ? sum.y : sum.y * k;
+        out5[5 * i + 2] = k == 1.0f ? sum.z : sum.z * k;
+        out5[5 * i + 3] = thr.w;
         out5[5 * i + 4] = 0.0f;
     }
     return RTG_STATUS_OK;

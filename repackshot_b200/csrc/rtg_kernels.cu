@@ -127,6 +127,18 @@ __device__ __forceinline__ uint32_t lanes_for(uint32_t n) {
     return min(32u, (n + warps - 1) / warps);
 }
 
+// Two neighbouring float4s of a path's record (o and d, or thr and sum): one 32-byte sector, one access.
+__device__ __forceinline__ void load_pair(const PathField& f, uint32_t slot, float4& a, float4& b) {
+    uint64_t v[4];
+    asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]) : "l"(&f[slot]) : "memory");
+    a = make_float4(__uint_as_float((uint32_t)v[0]), __uint_as_float((uint32_t)(v[0] >> 32)), __uint_as_float((uint32_t)v[1]), __uint_as_float((uint32_t)(v[1] >> 32)));
+    b = make_float4(__uint_as_float((uint32_t)v[2]), __uint_as_float((uint32_t)(v[2] >> 32)), __uint_as_float((uint32_t)v[3]), __uint_as_float((uint32_t)(v[3] >> 32)));
+}
+__device__ __forceinline__ uint64_t pack2(float x, float y) { return ((uint64_t)__float_as_uint(y) << 32) | __float_as_uint(x); }
+__device__ __forceinline__ void store_pair(const PathField& f, uint32_t slot, float4 a, float4 b) {
+    asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(&f[slot]), "l"(pack2(a.x, a.y)), "l"(pack2(a.z, a.w)), "l"(pack2(b.x, b.y)), "l"(pack2(b.z, b.w)) : "memory");
+}
+
 // ---- camera generation ---------------------------------------------------------------------------
 // BATCH: the slots belong to the jobs of a batched wave, each with its own camera.
 template <bool BATCH>
@@ -143,10 +155,8 @@ __global__ void k_camera(const __grid_constant__ SceneDev S, WaveDesc w, PathBuf
             wave_slot(w, slot, x, y, index);
             sees = camera_ray(S, c_sobol, x, y, index, o, d);
         }
-        P.o[slot] = make_float4(o.x, o.y, o.z, 0.0f);  // w: distance since the last scattering vertex
-        P.d[slot] = make_float4(d.x, d.y, d.z, 0.0f);  // w: density of the BSDF sample
-        P.thr[slot] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);  // w: alpha
-        P.sum[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        store_pair(P.o, slot, make_float4(o.x, o.y, o.z, 0.0f), make_float4(d.x, d.y, d.z, 0.0f));
+        store_pair(P.thr, slot, make_float4(1.0f, 1.0f, 1.0f, 1.0f), make_float4(0.0f, 0.0f, 0.0f, 0.0f));
         P.flags[slot] = PF_PRIMARY | (sees ? 0u : PF_NOTHING);
         P.queue[0][slot] = slot;
     }
@@ -290,8 +300,7 @@ __global__ void RTG_TRACE_BOUNDS k_trace(const __grid_constant__ SceneDev S, Pat
                     float tmax = f_inf();
                     if (RAYS == EXTEND || (RAYS == SHADOW_TOO && i < paths)) {
                         ray = order[i];
-                        o = P.o[ray];
-                        d = P.d[ray];
+                        load_pair(P.o, ray, o, d);
                         const uint32_t pf = P.flags[ray];
                         camera = (pf & PF_PRIMARY) != 0;
                         sees = !(pf & PF_NOTHING);
@@ -427,7 +436,9 @@ struct TailShadow {
 template <bool PLAIN, class XYI>
 __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L, const PathBuffers& P, const RaySort& R, uint32_t slot, uint32_t round,
                                            XYI xyi, uint32_t& rays_local, uint32_t& shadow_local, TailShadow* tail = nullptr) {
-    float4 o4 = P.o[slot], d4 = P.d[slot], thr4 = P.thr[slot], sum = P.sum[slot];
+    float4 o4, d4, thr4, sum;
+    load_pair(P.o, slot, o4, d4);
+    load_pair(P.thr, slot, thr4, sum);
     uint32_t flags = P.flags[slot];
     const uint32_t bounce = (flags & PF_BOUNCE_MASK) >> PF_BOUNCE_SHIFT;
     uint4 hit = P.hit[slot];
@@ -648,13 +659,11 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
                 }
             }
         }
-        P.o[slot] = make_float4(next_origin.x, next_origin.y, next_origin.z, offset);
-        P.d[slot] = make_float4(wi.x, wi.y, wi.z, pdf);
+        store_pair(P.o, slot, make_float4(next_origin.x, next_origin.y, next_origin.z, offset), make_float4(wi.x, wi.y, wi.z, pdf));
         P.flags[slot] = (flags & ~PF_BOUNCE_MASK) | ((bounce + 1u) << PF_BOUNCE_SHIFT);
         alive = true;
     } while (false);
-    P.thr[slot] = make_float4(thr.r, thr.g, thr.b, alpha);
-    P.sum[slot] = sum;
+    store_pair(P.thr, slot, make_float4(thr.r, thr.g, thr.b, alpha), sum);
     if (alive && !tail) {
         uint32_t k = atomicAdd(&P.counters[round_counter(round + 1, COUNT_PATHS)], 1u);
         P.queue[(round + 1) & 1][k] = slot;

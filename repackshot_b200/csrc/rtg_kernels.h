@@ -103,12 +103,20 @@ inline WaveDesc with_divisors(WaveDesc w) {
     return w;
 }
 
-// Structure-of-arrays path state of one wave (device pointers).
+// One float4 of the path records.
+struct PathField {
+    float4* p;
+    RTG_HD float4& operator[](size_t slot) const { return p[4 * slot]; }
+};
+// Path state of one wave (device pointers). What a vertex reads and writes of a path together lies
+// together, in a 64-byte record (o, d, thr, sum): shading visits the slots in material order, and
+// of a separate float4 per field it would use half of each 32-byte sector that it moves (1080p frame
+// 179.4 -> 169.0 ms, instanced frame 38.4 -> 37.5 ms).
 struct PathBuffers {
-    float4* o;       // origin, w: distance since the last scattering vertex (straight events)
-    float4* d;       // direction, w: density of the BSDF sample that produced it
-    float4* thr;     // throughput, w: alpha
-    float4* sum;     // radiance
+    PathField o;       // origin, w: distance since the last scattering vertex (straight events)
+    PathField d;       // direction, w: density of the BSDF sample that produced it
+    PathField thr;     // throughput, w: alpha
+    PathField sum;     // radiance
     float4* sel;     // point of the light selection the MIS weights use
     uint32_t* flags;
     uint32_t* medium;
@@ -193,6 +201,14 @@ struct AdjointDev {
     uint32_t* sh_ids;     // material + 1 (0: none) | (light + 1) << 16 (0: environment)
 };
 constexpr uint32_t ADJ_NONE = 0xffffffffu;
+
+inline void place_records(PathBuffers& P, void* base) {
+    float4* p = (float4*)base;
+    P.o.p = p;
+    P.d.p = p + 1;
+    P.thr.p = p + 2;
+    P.sum.p = p + 3;
+}
 
 // CUDA events bracketing every extend launch of a wave (optional).
 struct WaveTiming {

@@ -45,10 +45,7 @@ PathBuffers carve(void* base, float4** albedo) {
     unsigned char* p = static_cast<unsigned char*>(base);
     auto take = [&](size_t each) { unsigned char* r = p; p += kPaths * each; return r; };
     PathBuffers P{};
-    P.o = (float4*)take(16);
-    P.d = (float4*)take(16);
-    P.thr = (float4*)take(16);
-    P.sum = (float4*)take(16);
+    place_records(P, take(64));
     P.sel = (float4*)take(16);
     P.flags = (uint32_t*)take(4);
     P.medium = (uint32_t*)take(4);
