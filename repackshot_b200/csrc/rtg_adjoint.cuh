@@ -65,16 +65,14 @@ __global__ void k_adjoint_camera(const __grid_constant__ SceneDev S, WaveDesc w,
         wave_slot(w, slot, x, y, index);
         V3 o, d;
         const bool sees = camera_ray(S, c_sobol, x, y, index, o, d);
-        P.o[slot] = make_float4(o.x, o.y, o.z, 0.0f);
-        P.d[slot] = make_float4(d.x, d.y, d.z, 0.0f);
+        const float4 L = sees ? P.sum[slot] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        store_pair(P.o, slot, make_float4(o.x, o.y, o.z, __uint_as_float(PF_PRIMARY | (sees ? 0u : PF_NOTHING))), make_float4(d.x, d.y, d.z, 0.0f));
         // A panoramic camera's sample that sees nothing added nothing to the film: it replays with
         // no throughput and no radiance to come, so it adds no gradient.
         const float w0 = sees ? 1.0f : 0.0f;
-        P.thr[slot] = make_float4(w0, w0, w0, 1.0f);
-        P.flags[slot] = PF_PRIMARY | (sees ? 0u : PF_NOTHING);
+        store_pair(P.thr, slot, make_float4(w0, w0, w0, 1.0f), make_float4(0.0f, 0.0f, 0.0f, 0.0f));
         P.queue[0][slot] = slot;
-        float4 L = sees ? P.sum[slot] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        A.rem[slot] = L;
+        A.rem[slot] = make_float4(L.x, L.y, L.z, 0.0f);
         A.pend[slot] = ADJ_NONE;
         all += absf(L.x) + absf(L.y) + absf(L.z);
     }
@@ -113,11 +111,14 @@ __device__ __noinline__ Rgb adjoint_spheres(const LightsDev& L, Rgb crossed, V3 
 template <bool PLAIN>
 __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const LightsDev& L, const PathBuffers& P, const AdjointDev& A, float* g,
                                                    uint32_t slot, uint32_t bounce, const WaveDesc& w) {
-    float4 o4 = P.o[slot], d4 = P.d[slot], thr4 = P.thr[slot];
-    uint32_t flags = P.flags[slot];
-    uint4 hit = P.hit[slot];
+    float4 o4, d4, thr4, sum4, sel4;  // of the sum only w, the path's distance
+    load_pair(P.o, slot, o4, d4);
+    load_pair(P.thr, slot, thr4, sum4);
+    uint4 hit;
+    load_vertex(P, slot, hit, sel4);
+    uint32_t flags = __float_as_uint(o4.w);
     V3 ro = v3(o4.x, o4.y, o4.z), rd = v3(d4.x, d4.y, d4.z);
-    float offset = o4.w, pdf = d4.w;
+    float offset = sum4.w, pdf = d4.w;
     bool has_pdf = (flags & PF_HAS_PDF) != 0, primary = (flags & PF_PRIMARY) != 0;
     Rgb thr = rgb(thr4.x, thr4.y, thr4.z);
     uint32_t x, y, index;
@@ -158,7 +159,6 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
             }
         }
     }
-    float4 sel4 = P.sel[slot];
     Sel from;
     from.p = v3(sel4.x, sel4.y, sel4.z);
     from.by_flux = !(L.per_point && L.n_entries > 0);
@@ -374,12 +374,11 @@ __device__ __forceinline__ void shade_adjoint_slot(const SceneDev& S, const Ligh
                 }
             }
         }
-        P.o[slot] = make_float4(next_origin.x, next_origin.y, next_origin.z, offset);
-        P.d[slot] = make_float4(wi.x, wi.y, wi.z, pdf);
-        P.flags[slot] = flags;
+        store_pair(P.o, slot, make_float4(next_origin.x, next_origin.y, next_origin.z, __uint_as_float(flags)), make_float4(wi.x, wi.y, wi.z, pdf));
         alive = true;
     } while (false);
-    P.thr[slot] = make_float4(thr.r, thr.g, thr.b, thr4.w);
+    sum4.w = offset;
+    store_pair(P.thr, slot, make_float4(thr.r, thr.g, thr.b, thr4.w), sum4);
     A.rem[slot] = make_float4(rem.r, rem.g, rem.b, 0.0f);
     if (alive) {
         uint32_t k = atomicAdd(&P.counters[round_counter(bounce + 1, COUNT_PATHS)], 1u);

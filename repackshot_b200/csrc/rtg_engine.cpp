@@ -334,9 +334,9 @@ SceneDev compose(const SceneDev& constants, const SceneDev& geom, const SceneDev
     return S;
 }
 
-// Device bytes of one path slot: o, d, thr, sum, sel, hit, sh_o, sh_d, sh_c (16 each), flags,
-// medium, queue[0], queue[1], sorted, key, sh_key (4 each).
-constexpr size_t PATH_BYTES = 9 * 16 + 7 * 4;
+// Device bytes of one path slot: o, d, thr, sum, sel, hit, sh_o, sh_d, sh_c (16 each), medium,
+// queue[0], queue[1], sorted, key, sh_key (4 each).
+constexpr size_t PATH_BYTES = 9 * 16 + 6 * 4;
 // The ray sort's two key histograms with their cursors, at the largest key count.
 constexpr size_t SORT_BINS_BYTES = 2 * 2 * (size_t)(8u << (3u * RAY_SORT_MAX_BITS)) * 4;
 // The default tuning: no ray sort, material-sorted shading. On the 1080p product frame the sort
@@ -434,11 +434,9 @@ uint32_t ensure_capacity(Scene& sc, uint32_t paths) {
     uint8_t* p = (uint8_t*)sc.path_mem.p;
     auto take = [&](size_t each) { uint8_t* r = p; p += ((n * each + 255) / 256) * 256; return r; };
     // (sizes rounded to 256 bytes; `bytes` above leaves room for the rounding of 14 arrays)
-    place_records(sc.P, take(64));
-    sc.P.sel = (float4*)take(16);
-    sc.P.flags = (uint32_t*)take(4);
+    void* state = take(64);
+    place_records(sc.P, state, take(32));
     sc.P.medium = (uint32_t*)take(4);
-    sc.P.hit = (uint4*)take(16);
     sc.P.queue[0] = (uint32_t*)take(4);
     sc.P.queue[1] = (uint32_t*)take(4);
     sc.P.sorted = (uint32_t*)take(4);
@@ -1545,14 +1543,12 @@ uint32_t rtg_render_paths(uint32_t handle, const uint32_t* xys, uint32_t n, floa
     st = run_wave(*sc, wd, nullptr);
     if (st) return st;
     std::vector<float4> record(4 * (size_t)n);
-    std::vector<uint32_t> flags(n);
     RTG_CHECK(cudaMemcpyAsync(record.data(), sc->P.o.p, record.size() * 16, cudaMemcpyDeviceToHost, sc->stream));
-    RTG_CHECK(cudaMemcpyAsync(flags.data(), sc->P.flags, (size_t)n * 4, cudaMemcpyDeviceToHost, sc->stream));
     st = finish(*sc, nullptr);
     if (st) return st;
     for (uint32_t i = 0; i < n; ++i) {
         // a panoramic camera's sample that sees nothing weighs black (render.rs:465)
-        const float k = (flags[i] & 8u) ? 0.0f : 1.0f;
+        const float k = (fbits(record[4 * (size_t)i].w) & 8u) ? 0.0f : 1.0f;
         const float4 thr = record[4 * (size_t)i + 2], sum = record[4 * (size_t)i + 3];
         out5[5 * i] = k == 1.0f ? sum.x : sum.x * k;
         out5[5 * i + 1] = k == 1.0f ? sum.y : sum.y * k;

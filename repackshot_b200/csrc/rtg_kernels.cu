@@ -127,12 +127,22 @@ __device__ __forceinline__ uint32_t lanes_for(uint32_t n) {
     return min(32u, (n + warps - 1) / warps);
 }
 
-// Two neighbouring float4s of a path's record (o and d, or thr and sum): one 32-byte sector, one access.
+// Two neighbouring fields of a path's records (o and d, thr and sum, hit and sel): one 32-byte sector,
+// one access.
+__device__ __forceinline__ void load_sector(const void* p, uint64_t v[4]) {
+    asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]) : "l"(p) : "memory");
+}
 __device__ __forceinline__ void load_pair(const PathField& f, uint32_t slot, float4& a, float4& b) {
     uint64_t v[4];
-    asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]) : "l"(&f[slot]) : "memory");
+    load_sector(&f[slot], v);
     a = make_float4(__uint_as_float((uint32_t)v[0]), __uint_as_float((uint32_t)(v[0] >> 32)), __uint_as_float((uint32_t)v[1]), __uint_as_float((uint32_t)(v[1] >> 32)));
     b = make_float4(__uint_as_float((uint32_t)v[2]), __uint_as_float((uint32_t)(v[2] >> 32)), __uint_as_float((uint32_t)v[3]), __uint_as_float((uint32_t)(v[3] >> 32)));
+}
+__device__ __forceinline__ void load_vertex(const PathBuffers& P, uint32_t slot, uint4& hit, float4& sel) {
+    uint64_t v[4];
+    load_sector(&P.hit[slot], v);
+    hit = make_uint4((uint32_t)v[0], (uint32_t)(v[0] >> 32), (uint32_t)v[1], (uint32_t)(v[1] >> 32));
+    sel = make_float4(__uint_as_float((uint32_t)v[2]), __uint_as_float((uint32_t)(v[2] >> 32)), __uint_as_float((uint32_t)v[3]), __uint_as_float((uint32_t)(v[3] >> 32)));
 }
 __device__ __forceinline__ uint64_t pack2(float x, float y) { return ((uint64_t)__float_as_uint(y) << 32) | __float_as_uint(x); }
 __device__ __forceinline__ void store_pair(const PathField& f, uint32_t slot, float4 a, float4 b) {
@@ -155,9 +165,8 @@ __global__ void k_camera(const __grid_constant__ SceneDev S, WaveDesc w, PathBuf
             wave_slot(w, slot, x, y, index);
             sees = camera_ray(S, c_sobol, x, y, index, o, d);
         }
-        store_pair(P.o, slot, make_float4(o.x, o.y, o.z, 0.0f), make_float4(d.x, d.y, d.z, 0.0f));
+        store_pair(P.o, slot, make_float4(o.x, o.y, o.z, __uint_as_float(PF_PRIMARY | (sees ? 0u : PF_NOTHING))), make_float4(d.x, d.y, d.z, 0.0f));
         store_pair(P.thr, slot, make_float4(1.0f, 1.0f, 1.0f, 1.0f), make_float4(0.0f, 0.0f, 0.0f, 0.0f));
-        P.flags[slot] = PF_PRIMARY | (sees ? 0u : PF_NOTHING);
         P.queue[0][slot] = slot;
     }
     start_rounds(P, rounds, w.n);
@@ -301,7 +310,7 @@ __global__ void RTG_TRACE_BOUNDS k_trace(const __grid_constant__ SceneDev S, Pat
                     if (RAYS == EXTEND || (RAYS == SHADOW_TOO && i < paths)) {
                         ray = order[i];
                         load_pair(P.o, ray, o, d);
-                        const uint32_t pf = P.flags[ray];
+                        const uint32_t pf = __float_as_uint(o.w);
                         camera = (pf & PF_PRIMARY) != 0;
                         sees = !(pf & PF_NOTHING);
                         T.any = false;
@@ -439,11 +448,13 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
     float4 o4, d4, thr4, sum;
     load_pair(P.o, slot, o4, d4);
     load_pair(P.thr, slot, thr4, sum);
-    uint32_t flags = P.flags[slot];
+    uint4 hit;
+    float4 sel4;
+    load_vertex(P, slot, hit, sel4);
+    uint32_t flags = __float_as_uint(o4.w);
     const uint32_t bounce = (flags & PF_BOUNCE_MASK) >> PF_BOUNCE_SHIFT;
-    uint4 hit = P.hit[slot];
     V3 ro = v3(o4.x, o4.y, o4.z), rd = v3(d4.x, d4.y, d4.z);
-    float offset = o4.w, pdf = d4.w;
+    float offset = sum.w, pdf = d4.w;
     bool has_pdf = (flags & PF_HAS_PDF) != 0, primary = (flags & PF_PRIMARY) != 0;
     Rgb thr = rgb(thr4.x, thr4.y, thr4.z);
     float alpha = thr4.w;
@@ -460,7 +471,6 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
         const DevMaterial& mm = S.materials[P.medium[slot]];
         thr = thr * rgb(fexp(-mm.sigma[0] * t_nearest), fexp(-mm.sigma[1] * t_nearest), fexp(-mm.sigma[2] * t_nearest));
     }
-    float4 sel4 = P.sel[slot];
     Sel from;
     from.p = v3(sel4.x, sel4.y, sel4.z);
     from.by_flux = !(L.per_point && L.n_entries > 0);
@@ -534,8 +544,7 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
                 if (u >= rmax(mat->opacity, 0.0f)) {
                     const V3 o2 = offset_origin(h.point, -ng);
                     offset += dot(o2 - ro, rd);
-                    P.o[slot] = make_float4(o2.x, o2.y, o2.z, offset);
-                    P.flags[slot] = flags;
+                    P.o[slot] = make_float4(o2.x, o2.y, o2.z, __uint_as_float(flags));
                     alive = true;
                     break;
                 }
@@ -659,10 +668,11 @@ __device__ __forceinline__ bool shade_slot(const SceneDev& S, const LightsDev& L
                 }
             }
         }
-        store_pair(P.o, slot, make_float4(next_origin.x, next_origin.y, next_origin.z, offset), make_float4(wi.x, wi.y, wi.z, pdf));
-        P.flags[slot] = (flags & ~PF_BOUNCE_MASK) | ((bounce + 1u) << PF_BOUNCE_SHIFT);
+        flags = (flags & ~PF_BOUNCE_MASK) | ((bounce + 1u) << PF_BOUNCE_SHIFT);
+        store_pair(P.o, slot, make_float4(next_origin.x, next_origin.y, next_origin.z, __uint_as_float(flags)), make_float4(wi.x, wi.y, wi.z, pdf));
         alive = true;
     } while (false);
+    sum.w = offset;
     store_pair(P.thr, slot, make_float4(thr.r, thr.g, thr.b, alpha), sum);
     if (alive && !tail) {
         uint32_t k = atomicAdd(&P.counters[round_counter(round + 1, COUNT_PATHS)], 1u);
@@ -730,7 +740,7 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_extend_section(const __grid_c
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t slot = order[i];
         const float4 o = P.o[slot], d = P.d[slot];
-        const uint32_t pf = P.flags[slot];
+        const uint32_t pf = __float_as_uint(o.w);
         TraceResult res;
         const bool got = !(pf & PF_NOTHING) &&
                          trace_q<false>(S, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 1.0e-3f, f_inf(), (pf & PF_PRIMARY) != 0, res, &err, stack);
@@ -848,7 +858,7 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_tail(const __grid_constant__ 
         const uint32_t slot = queue[i];
         for (uint32_t r = 0; r < rounds_left; ++r) {
             const float4 o = P.o[slot], d = P.d[slot];
-            const uint32_t pf = P.flags[slot];
+            const uint32_t pf = __float_as_uint(o.w);
             TraceResult res;
             const bool got = !(pf & PF_NOTHING) &&
                              traverse<false, true>(S, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 1.0e-3f, f_inf(), (pf & PF_PRIMARY) != 0, res, &err, stack);
@@ -879,23 +889,23 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_tail(const __grid_constant__ 
 
 // ---- accumulate: film += each pixel's samples in sample-index order (image.rs:82) -------------------------
 // A sample's radiance times its camera weight (render.rs:465): white, or black for a panoramic
-// camera's sample that sees nothing.
-__device__ __forceinline__ float4 sample_sum(const PathBuffers& P, uint32_t slot) {
+// camera's (`dark`) sample that sees nothing.
+__device__ __forceinline__ float4 sample_sum(const PathBuffers& P, uint32_t slot, bool dark) {
     const float4 c = P.sum[slot];
-    if (!(P.flags[slot] & PF_NOTHING)) return c;
+    if (!dark || !(__float_as_uint(P.o[slot].w) & PF_NOTHING)) return c;
     return make_float4(c.x * 0.0f, c.y * 0.0f, c.z * 0.0f, c.w);
 }
 // Film pixel (x, y) += the ns samples in slots slot0, slot0 + stride, ..., in that order
 // (Film::splat_alpha, image.rs:82).
 __device__ __forceinline__ void accumulate_pixel(const FilmDev& F, uint32_t x, uint32_t y, const PathBuffers& P, uint32_t slot0, uint32_t stride,
-                                                 uint32_t ns) {
+                                                 uint32_t ns, bool dark) {
     if (x < F.ox || y < F.oy || x - F.ox >= F.w || y - F.oy >= F.h) return;
     size_t fi = (size_t)(y - F.oy) * F.w + (x - F.ox);
     float r = F.rgb[3 * fi], g = F.rgb[3 * fi + 1], b = F.rgb[3 * fi + 2];
     float wt = F.weight[fi], al = F.alpha[fi], l2 = F.lum2[fi];
     for (uint32_t s = 0; s < ns; ++s) {
         uint32_t slot = slot0 + s * stride;
-        float4 c = sample_sum(P, slot);
+        float4 c = sample_sum(P, slot, dark);
         r = r + c.x; g = g + c.y; b = b + c.z;
         wt = wt + 1.0f;
         al = al + P.thr[slot].w;
@@ -912,7 +922,7 @@ __global__ void k_accumulate(WaveDesc w, PathBuffers P, FilmDev F) {
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += gridDim.x * blockDim.x) {
         const uint32_t x = w.x0 + p % w.w, y = w.y0 + p / w.w;
         if (w.edge && w.edge[(size_t)y * w.edge_stride + x]) continue;  // splatted by the edge waves
-        accumulate_pixel(F, x, y, P, p, npix, ns);
+        accumulate_pixel(F, x, y, P, p, npix, ns, w.dark);
     }
 }
 
@@ -931,7 +941,7 @@ __global__ void k_accumulate_edges(WaveDesc w, PathBuffers P, FilmDev F) {
             float sr = 0.0f, sg = 0.0f, sb = 0.0f, cov = 0.0f;
             for (uint32_t j = 0; j < k; ++j) {
                 const uint32_t slot = (s * w.ne + e) * k + j;
-                const float4 c = sample_sum(P, slot);
+                const float4 c = sample_sum(P, slot, w.dark);
                 sr = sr + c.x; sg = sg + c.y; sb = sb + c.z;
                 cov = cov + P.thr[slot].w;
             }
@@ -1140,7 +1150,7 @@ __global__ void k_albedo_hits(const __grid_constant__ SceneDev S, const LightsDe
         const bool got = hit.w != 0u;
         const float t_geometry = got ? __uint_as_float(hit.z) : f_inf();
         float t_floor = f_inf();
-        if (S.floor_mode == 1 && d.z != 0.0f && !(P.flags[slot] & PF_NOTHING)) {
+        if (S.floor_mode == 1 && d.z != 0.0f && !(__float_as_uint(of.w) & PF_NOTHING)) {
             const float t = (S.floor_z - o.z) / d.z;
             if (t > 1.0e-3f && t < f_inf()) t_floor = t;
         }
@@ -1257,7 +1267,7 @@ __global__ void k_accumulate_jobs(WaveDesc w, PathBuffers P) {
         }
         const SegDev& g = w.segs[lo];
         uint32_t local = p - g.pix_begin, npix = g.w * g.h;
-        accumulate_pixel(w.jobs[g.job].film, local % g.w, g.y0 + local / g.w, P, g.slot_begin + local, npix, g.ns);
+        accumulate_pixel(w.jobs[g.job].film, local % g.w, g.y0 + local / g.w, P, g.slot_begin + local, npix, g.ns, w.jobs[g.job].S.projection != 0);
     }
 }
 
@@ -1379,7 +1389,8 @@ void launch_wave(const SceneDev& S, const LightsDev* L, const WaveDesc& wave, co
     static const int tail_resident = resident_blocks((const void*)k_tail<false>, TRACE_THREADS);
     static const int shade_resident = resident_blocks((const void*)k_shade<false, false>, 128);
     static const int sort_resident = resident_blocks((const void*)k_material_sort, SORT_THREADS);
-    const WaveDesc w = with_divisors(wave);
+    WaveDesc w = with_divisors(wave);
+    w.dark = S.projection != 0;
     const int g = grid;
     const int g_trace = blocks_of(trace_resident, w.n, g), g_shade = blocks_of(shade_resident, w.n, g);
     const int g_sort = std::min<int>(sort_resident > 0 ? sort_resident : g, (int)((w.n + SORT_CHUNK - 1) / SORT_CHUNK));

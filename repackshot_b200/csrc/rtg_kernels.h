@@ -86,6 +86,7 @@ struct WaveDesc {
     // `edge_stride`); its pixels splat from the edge waves, not from this one.
     const uint8_t* edge;
     uint32_t edge_stride;
+    bool dark;  // the camera is panoramic: some samples see nothing and weigh black (PF_NOTHING)
     // Guides taken from the wave itself (the film's albedo pass, passes.rs:209): when `alb` is set
     // (one float4 a path slot), the albedo of each camera ray's first hit is read from the first
     // extend, and after the film's accumulate each pixel adds its samples' albedo (an edge pixel
@@ -103,24 +104,25 @@ inline WaveDesc with_divisors(WaveDesc w) {
     return w;
 }
 
-// One float4 of the path records.
-struct PathField {
-    float4* p;
-    RTG_HD float4& operator[](size_t slot) const { return p[4 * slot]; }
+// One 16-byte field of records of N.
+template <class T, int N>
+struct RecordField {
+    T* p;
+    RTG_HD T& operator[](size_t slot) const { return p[N * slot]; }
 };
+using PathField = RecordField<float4, 4>;
 // Path state of one wave (device pointers). What a vertex reads and writes of a path together lies
-// together, in a 64-byte record (o, d, thr, sum): shading visits the slots in material order, and
+// together, in a record of 64 bytes (o, d, thr, sum) and one of 32 (hit, sel): shading visits the slots in material order, and
 // of a separate float4 per field it would use half of each 32-byte sector that it moves (1080p frame
 // 179.4 -> 169.0 ms, instanced frame 38.4 -> 37.5 ms).
 struct PathBuffers {
-    PathField o;       // origin, w: distance since the last scattering vertex (straight events)
+    PathField o;       // origin, w: flags (bits)
     PathField d;       // direction, w: density of the BSDF sample that produced it
     PathField thr;     // throughput, w: alpha
-    PathField sum;     // radiance
-    float4* sel;     // point of the light selection the MIS weights use
-    uint32_t* flags;
+    PathField sum;     // radiance, w: distance since the last scattering vertex (straight events)
+    RecordField<uint4, 2> hit;   // instance, leaf triangle, t (bits), whether there is one
+    RecordField<float4, 2> sel;  // point of the light selection the MIS weights use, w: its sum of weights
     uint32_t* medium;
-    uint4* hit;
     uint32_t* queue[2];
     uint32_t* sorted;    // the active queue in another order: ray-sorted (RaySort) or by material
     uint32_t* key;       // per slot: material of the hit (n_materials: floor or miss)
@@ -202,12 +204,14 @@ struct AdjointDev {
 };
 constexpr uint32_t ADJ_NONE = 0xffffffffu;
 
-inline void place_records(PathBuffers& P, void* base) {
-    float4* p = (float4*)base;
+inline void place_records(PathBuffers& P, void* state, void* vertex) {
+    float4* p = (float4*)state;
     P.o.p = p;
     P.d.p = p + 1;
     P.thr.p = p + 2;
     P.sum.p = p + 3;
+    P.hit.p = (uint4*)vertex;
+    P.sel.p = (float4*)vertex + 1;
 }
 
 // CUDA events bracketing every extend launch of a wave (optional).

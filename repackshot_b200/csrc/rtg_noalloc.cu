@@ -23,9 +23,9 @@ namespace rtg {
 namespace {
 
 // Bytes per path of the structure-of-arrays state (PathBuffers): o, d, thr, sum, sel, hit, sh_o,
-// sh_d, sh_c (16 each), flags, medium, queue[0], queue[1], sorted, key (4 each); then the
+// sh_d, sh_c (16 each), medium, queue[0], queue[1], sorted, key (4 each); then the
 // first-hit albedo of each path (16), which a film with fused guides adds to its guide sums.
-constexpr size_t kBytesPerPath = 10 * 16 + 6 * 4;
+constexpr size_t kBytesPerPath = 10 * 16 + 5 * 4;
 constexpr size_t kPaths = RTG_NOALLOC_MAX_PATHS;
 constexpr size_t kBinsBytes = 2 * KEY_BINS * 4;
 constexpr size_t kCountersBytes = COUNTERS_BYTES;  // [3] error bits, then the rounds' counts
@@ -45,11 +45,9 @@ PathBuffers carve(void* base, float4** albedo) {
     unsigned char* p = static_cast<unsigned char*>(base);
     auto take = [&](size_t each) { unsigned char* r = p; p += kPaths * each; return r; };
     PathBuffers P{};
-    place_records(P, take(64));
-    P.sel = (float4*)take(16);
-    P.flags = (uint32_t*)take(4);
+    void* state = take(64);
+    place_records(P, state, take(32));
     P.medium = (uint32_t*)take(4);
-    P.hit = (uint4*)take(16);
     P.queue[0] = (uint32_t*)take(4);
     P.queue[1] = (uint32_t*)take(4);
     P.sorted = (uint32_t*)take(4);
