@@ -5,11 +5,11 @@
 // The answer of a nearest-hit query is the smallest (t, instance, triangle) in lexicographic
 // order over the triangles the ray meets in [t_min, t_max] whose enclosing boxes pass the
 // reference's slab test. Those boxes are conservative except where a computed t lies within its
-// rounding of an end of the interval: a ray that starts within about 1e-3 of a large axis-aligned
-// quad can see its flat box end just before t_min while the triangle test alone would accept the
-// hit, and the reference drops that hit. So the tree is walked with a cheaper slab test that
-// passes every box the reference's passes (and a few more), and a hit whose t is that close to an
-// end of the interval is put to the reference's own test of its leaf's exact box (hit_kept).
+// rounding of t_min: a ray that starts within about 1e-3 of a large axis-aligned quad can see its
+// flat box end just before t_min while the triangle test alone would accept the hit, and the
+// reference drops that hit. So the tree is walked with a cheaper slab test that passes every box
+// the reference's passes (and a few more), and a hit whose t is that close to t_min is put to the
+// reference's own test of its leaf's exact box (hit_kept).
 #pragma once
 #include "rtg_dev.h"
 
@@ -172,11 +172,11 @@ RTG_D bool trav_init(const SceneDev& S, Trav& T, V3 o, V3 d, float tmin, float t
     return true;
 }
 
-// The reference's slab test of one box with the ray (o, d) over [tmin, tmax], its operations in its
-// order (traverse.rs:184).
-RTG_D bool box_passes(const float* __restrict__ box, V3 o, V3 d, float tmin, float tmax) {
+// The reference's slab test of one box with the ray (o, d) from tmin on, its operations in its order
+// (traverse.rs:184).
+RTG_D bool box_passes(const float* __restrict__ box, V3 o, V3 d, float tmin) {
     const float org[3] = {o.x, o.y, o.z}, inv[3] = {__frcp_rn(d.x), __frcp_rn(d.y), __frcp_rn(d.z)};
-    float n = tmin, f = tmax;
+    float n = tmin, f = F_MAX;
     for (int a = 0; a < 3; ++a) {
         const bool neg = signbitf(inv[a]);
         const float lo = __ldg(box + a), hi = __ldg(box + 4 + a);
@@ -185,22 +185,22 @@ RTG_D bool box_passes(const float* __restrict__ box, V3 o, V3 d, float tmin, flo
     }
     return n <= f * RTG_ROBUST;
 }
-// Whether the reference's boxes keep a hit of leaf `leaf` while [tmin, tmax] is its interval: the
+// Whether the reference's boxes keep a hit of leaf `leaf` near the start of the query's interval: the
 // leaf's exact box with the ray of its tree and, in a transformed instance, the instance's world box
 // with the world ray (o, d). Boxes further up contain these, and rounding is monotonic, so they
 // pass when these pass.
 RTG_D_NI bool hit_kept(const BlasInst* __restrict__ blases, const float* __restrict__ leaf_boxes, V3 o, V3 d, uint32_t blas, uint32_t leaf,
-                       float tmin, float tmax) {
+                       float tmin) {
     if (blas & BLAS_MOVED) {
         const BlasInst* bi = blases + (blas >> 3);
-        if (!box_passes(bi->box, o, d, tmin, tmax)) return false;
+        if (!box_passes(bi->box, o, d, tmin)) return false;
         float m[12];
         for (int k = 0; k < 12; ++k) m[k] = __ldg(&bi->to_local[k]);
         const V3 lo = xf_point(m, o), ld = xf_vector(m, d);
         o = lo;
         d = ld;
     }
-    return box_passes(leaf_boxes + 8 * (size_t)leaf, o, d, tmin, tmax);
+    return box_passes(leaf_boxes + 8 * (size_t)leaf, o, d, tmin);
 }
 
 // Child `c` of a node whose first `inner` children are nodes: their index, or a leaf reference.
@@ -432,14 +432,15 @@ RTG_D bool trav_step(const SceneDev& S, Trav& T, float tmin, Stack& stack, uint3
                     if (inst == 0xffffffffu) inst = __ldg(&S.blas[T.blas >> 3].instance);
                     if (!(t < T.best_t || inst < T.best_i || (inst == T.best_i && __float_as_uint(a.w) < __ldg(&S.tris[T.best_k].tri)))) continue;
                 }
-                // Within the rounding of t (a generous 2^-14 of the corners' distances) of an end of
-                // the interval, the reference's boxes decide; and where t may be negative, which
-                // turns its factor 1 + 4 eps against the far planes.
+                // Within the rounding of t (a generous 2^-14 of the corners' distances) of t_min, the
+                // reference's boxes decide; and where t may be negative, which turns its factor
+                // 1 + 4 eps against the far planes. (At the far end they only cull what a nearer hit,
+                // computed in whatever order, hides: there the nearest of the hits stands.)
                 const float near = (absf(az) + absf(bz) + absf(cz)) * 6.103515625e-5f;
                 if (!(t - tmin > near) || (!POS && tmin <= 0.0f)) {
                     V3 o, d;
                     src(o, d);
-                    if (!hit_kept(S.blas, S.leaf_boxes, o, d, T.blas, flags >> TRI_LEAF_SHIFT, tmin, T.best_t)) continue;
+                    if (!hit_kept(S.blas, S.leaf_boxes, o, d, T.blas, flags >> TRI_LEAF_SHIFT, tmin)) continue;
                 }
                 if (any) { hit = true; return true; }
                 T.best_t = t;
