@@ -28,7 +28,8 @@ DEVICE_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-fmad=false", "-prec-div=true
                 "-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off", "-Xptxas", "-v"]
 # RTG_SHADE_MIN_BLOCKS (environment): blocks per SM the shade kernels are compiled for (default 8);
 # RTG_SHORT_STACK (environment): traversal stack entries kept in shared memory (default 16).
-# RTG_TRACE_MIN_BLOCKS (environment): blocks per SM the traversal kernels are compiled for (default 8).
+# RTG_TRACE_MIN_BLOCKS (environment): blocks per SM all traversal kernels are compiled for (default 9,
+# and 8 for the one that traces both kinds of rays).
 # RTG_REFILL_MIN (environment): idle lanes a k_trace warp waits for before it refills (default 8).
 for _name in ("RTG_SHADE_MIN_BLOCKS", "RTG_SHORT_STACK", "RTG_TRACE_MIN_BLOCKS", "RTG_REFILL_MIN"):
     if os.environ.get(_name, "").isdigit():

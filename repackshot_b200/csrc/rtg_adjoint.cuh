@@ -466,7 +466,10 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_shadow_adjoint(const __grid_c
                 ro = v3(o.x, o.y, o.z);
                 rd = v3(d.x, d.y, d.z);
             };
-            if (trav_step<TRACE_ANY, true>(S, T, 1.0e-3f, stack, &err, blocked, src)) {
+            bool over = false;
+            if (!trav_at_leaf(T)) over = trav_node<TRACE_ANY, true>(S, T, 1.0e-3f, stack, &err, blocked, src);
+            if (!over && trav_at_leaf(T)) over = trav_leaf<TRACE_ANY, true>(S, T, 1.0e-3f, stack, &err, blocked, src);
+            if (over) {
                 busy = false;
                 if (!blocked) adjoint_unblocked(P, A, w, s_grad, ray);
             }

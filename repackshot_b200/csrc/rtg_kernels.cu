@@ -24,17 +24,15 @@ constexpr int TRACE_THREADS = 128;
 #ifndef RTG_REFILL_MIN
 #define RTG_REFILL_MIN 8
 #endif
-// RTG_TRACE_MIN_BLOCKS (build setting): blocks per SM the traversal kernel is compiled for (0: the
-// compiler's choice of registers). At 8 (64 registers, no spills) its warps hide the node fetches
-// best over both workloads: at 7, 8, 9 and 10 blocks the 1080p product frame took 200, 192.7, 190.9
-// and 197 ms, the instanced frame 43.7, 42.7, 43.4 and 45.3 ms.
-#ifndef RTG_TRACE_MIN_BLOCKS
-#define RTG_TRACE_MIN_BLOCKS 8
-#endif
-#if RTG_TRACE_MIN_BLOCKS > 0
-#define RTG_TRACE_BOUNDS __launch_bounds__(TRACE_THREADS, RTG_TRACE_MIN_BLOCKS)
+// Blocks per SM the traversal kernels are compiled for (56 registers at 9, 64 at 8, no spills): more
+// warps hide the node fetches until registers spill. All kernels at 7, 8, 9 and 10 blocks: 1080p
+// product frame 154.4, 148.8, 145.8 and 150.6 ms, instanced frame 32.6, 31.7, 31.2 and 33.0 ms, adaptive
+// frame (thin rounds) 70.2 at 8, 71.8 at 9, 73.3 ms at 10. So the kernel of the smaller waves, which
+// traces both kinds of rays, takes 8 and the others 9. RTG_TRACE_MIN_BLOCKS (build setting): both.
+#ifdef RTG_TRACE_MIN_BLOCKS
+#define RTG_TRACE_BLOCKS(together) RTG_TRACE_MIN_BLOCKS
 #else
-#define RTG_TRACE_BOUNDS __launch_bounds__(TRACE_THREADS)
+#define RTG_TRACE_BLOCKS(together) ((together) ? 8 : 9)
 #endif
 // Blocks of 128 threads per SM that the shade kernels are compiled for (their register cap:
 // 65536 / (128 x this)); a build may set it (RTG_SHADE_MIN_BLOCKS) to compare occupancies.
@@ -276,7 +274,7 @@ __device__ __forceinline__ void shadow_unblocked(const PathBuffers& P, uint32_t 
 // `perm` (may be null): the shadow queue in the order to trace it.
 enum TraceRays { EXTEND, SHADOW, SHADOW_TOO };
 template <TraceRays RAYS>
-__global__ void RTG_TRACE_BOUNDS k_trace(const __grid_constant__ SceneDev S, PathBuffers P, uint32_t round, const uint32_t* __restrict__ order,
+__global__ void __launch_bounds__(TRACE_THREADS, RTG_TRACE_BLOCKS(RAYS == SHADOW_TOO)) k_trace(const __grid_constant__ SceneDev S, PathBuffers P, uint32_t round, const uint32_t* __restrict__ order,
                                          const uint32_t* __restrict__ perm, uint32_t tail) {
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
     uint64_t deep[STACK_CAP - SHORT_STACK];
@@ -326,16 +324,16 @@ __global__ void RTG_TRACE_BOUNDS k_trace(const __grid_constant__ SceneDev S, Pat
                 }
             }
         }
-        if (busy) {
-            const auto src = [&](V3& ro, V3& rd) {
-                const bool any = MODE == TRACE_ANY || (MODE == TRACE_EITHER && T.any);
-                const float4 o = any ? P.sh_o[ray] : P.o[ray], d = any ? P.sh_d[ray] : P.d[ray];
-                ro = v3(o.x, o.y, o.z);
-                rd = v3(d.x, d.y, d.z);
-            };
-            done = trav_step<MODE, true>(S, T, 1.0e-3f, stack, &err, hit, src);
-            busy = !done;
-        }
+        const auto src = [&](V3& ro, V3& rd) {
+            const bool any = MODE == TRACE_ANY || (MODE == TRACE_EITHER && T.any);
+            const float4 o = any ? P.sh_o[ray] : P.o[ray], d = any ? P.sh_d[ray] : P.d[ray];
+            ro = v3(o.x, o.y, o.z);
+            rd = v3(d.x, d.y, d.z);
+        };
+        if (busy && !trav_at_leaf(T)) done = trav_node<MODE, true>(S, T, 1.0e-3f, stack, &err, hit, src);
+        busy = busy && !done;
+        if (busy && trav_at_leaf(T)) done = trav_leaf<MODE, true>(S, T, 1.0e-3f, stack, &err, hit, src);
+        busy = busy && !done;
         if (done) {
             if (MODE == TRACE_ANY || (MODE == TRACE_EITHER && T.any)) {
                 if (!hit) shadow_unblocked(P, ray);
@@ -1385,14 +1383,15 @@ uint32_t wave_launches(const SceneDev& S, const RaySort& order, const PathBuffer
 
 void launch_wave(const SceneDev& S, const LightsDev* L, const WaveDesc& wave, const PathBuffers& P, const FilmDev* film, cudaStream_t st,
                  int grid, WaveTiming* timing, const RaySort& tuning) {
-    static const int trace_resident = resident_blocks((const void*)k_trace<SHADOW_TOO>, TRACE_THREADS);
+    static const int ext_resident = resident_blocks((const void*)k_trace<EXTEND>, TRACE_THREADS);
+    static const int both_resident = resident_blocks((const void*)k_trace<SHADOW_TOO>, TRACE_THREADS);
     static const int tail_resident = resident_blocks((const void*)k_tail<false>, TRACE_THREADS);
     static const int shade_resident = resident_blocks((const void*)k_shade<false, false>, 128);
     static const int sort_resident = resident_blocks((const void*)k_material_sort, SORT_THREADS);
     WaveDesc w = with_divisors(wave);
     w.dark = S.projection != 0;
     const int g = grid;
-    const int g_trace = blocks_of(trace_resident, w.n, g), g_shade = blocks_of(shade_resident, w.n, g);
+    const int g_trace = blocks_of(ext_resident, w.n, g), g_both = blocks_of(both_resident, w.n, g), g_shade = blocks_of(shade_resident, w.n, g);
     const int g_sort = std::min<int>(sort_resident > 0 ? sort_resident : g, (int)((w.n + SORT_CHUNK - 1) / SORT_CHUNK));
     const bool batch = w.segs != nullptr;
     const uint32_t rounds = wave_rounds(S);
@@ -1423,7 +1422,8 @@ void launch_wave(const SceneDev& S, const LightsDev* L, const WaveDesc& wave, co
         const bool timed = timing && timing->ev_count + 2 <= WaveTiming::MAX_EVENTS;
         if (timed) cudaEventRecord(timing->ev[timing->ev_count++], st);
         if (S.section_on) launch_traversal(order, g_trace, st, k_extend_section, S, P, round, traced, order.tail_paths);
-        else launch_traversal(order, g_trace, st, together && round > 0 ? k_trace<SHADOW_TOO> : k_trace<EXTEND>, S, P, round, traced, perm, order.tail_paths);
+        else if (together && round > 0) launch_traversal(order, g_both, st, k_trace<SHADOW_TOO>, S, P, round, traced, perm, order.tail_paths);
+        else launch_traversal(order, g_trace, st, k_trace<EXTEND>, S, P, round, traced, perm, order.tail_paths);
         if (timed) cudaEventRecord(timing->ev[timing->ev_count++], st);
         if (round == 0 && w.alb && film && !batch) k_albedo_hits<<<g, 256, 0, st>>>(S, L, w, P);
         // The material-sorted copy goes to whichever list the traversal did not read.
