@@ -483,8 +483,7 @@ uint32_t run_wave(Scene& sc, const WaveDesc& w, const FilmDev* film, const Scene
     }
     launch_wave(Sw, lights ? lights : sc.d_lights, w, sc.P, film, sc.stream, grid_for(w.n, 128), t, sc.order);
     RTG_CHECK(cudaGetLastError());
-    sc.launches += wave_launches(Sw, sc.order, sc.P, w.segs != nullptr) - ((film || w.segs) ? 0 : 1) + ((w.alb && film && !w.segs) ? 2 : 0);
-    if (t && !Sw.any_passable && !Sw.section_on) sc.launches += wave_rounds(Sw);  // shadow rays apart
+    sc.launches += wave_launches(Sw, sc.order, sc.P, w.n, w.segs != nullptr, t != nullptr) - ((film || w.segs) ? 0 : 1) + ((w.alb && film && !w.segs) ? 2 : 0);
     if (t) {
         RTG_CHECK(cudaStreamSynchronize(sc.stream));
         for (int i = 0; i + 1 < t->ev_count; i += 2) {
@@ -1034,7 +1033,7 @@ uint32_t rtg_render_progressive_noalloc(uint32_t handle, uint32_t film, uint32_t
     const char* why = "";
     uint32_t st = noalloc_render(job, res, &why);
     if (st) { g_error = why; return st; }
-    sc->launches += res.waves * (wave_launches(sc->S, RaySort(), PathBuffers{}, false) + (job.guide_sum ? 2 : 0));
+    sc->launches += res.waves * (wave_launches(sc->S, RaySort(), PathBuffers{}, 0, false, false) + (job.guide_sum ? 2 : 0));
     sc->rays += res.extend_rays + res.shadow_rays;
     sc->extend_rays += res.extend_rays;
     sc->shadow_rays += res.shadow_rays;

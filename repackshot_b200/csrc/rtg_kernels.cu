@@ -263,6 +263,47 @@ __device__ __forceinline__ void shadow_unblocked(const PathBuffers& P, uint32_t 
     s.x = s.x + c.x; s.y = s.y + c.y; s.z = s.z + c.z;
     P.sum[slot] = s;
 }
+// A shadow ray on its way through cut-outs and thin walls (integrator/mod.rs:629-690): nearest hits
+// along the ray; a passable surface multiplies what arrives by its straight transmittance (a thin
+// wall's) times its opacity plus 1 - opacity, and the ray goes on from just behind it, up to 32
+// crossings (MAX_SHADOW_CROSSINGS); any other surface blocks it.
+struct ShadowWalk {
+    V3 o;  // where its present part starts
+    float travelled;
+    Rgb keep;
+    uint32_t crossings;
+};
+enum : int { WALK_BLOCKED, WALK_ARRIVES, WALK_GOES_ON };
+// The walk's surface at (inst, tri, t): blocked, at the light, or on from behind it for up to `next`.
+__device__ __noinline__ int shadow_crossing(const SceneDev& S, ShadowWalk& walk, V3 d, float t_max, uint32_t inst, uint32_t tri, float t, float& next) {
+    if (inst >= S.n_instances || !S.instances[inst].passable) return WALK_BLOCKED;
+    HitInfo h;
+    const DevInstance* I = nullptr;
+    if (!hit_details(S, walk.o, d, 1.0e-3f, f_inf(), inst, tri, t, h, I)) return WALK_BLOCKED;
+    const uint32_t m = I->material;
+    const float opacity = rclamp(S.materials[m].opacity, 0.0f, 1.0f);
+    walk.keep = walk.keep * (straight_transmittance(S.bsdfs[2 * m], dot(h.geometric, d)) * opacity + splat(1.0f - opacity));
+    if (rmax(rmax(walk.keep.r, walk.keep.g), walk.keep.b) <= 0.0f) return WALK_BLOCKED;
+    const V3 origin = offset_origin(h.point, -h.geometric);
+    walk.travelled += dot(origin - walk.o, d);
+    next = t_max - walk.travelled;
+    if (next != next || next <= 1.0e-3f) return WALK_ARRIVES;
+    walk.o = origin;
+    return ++walk.crossings < 32u ? WALK_GOES_ON : WALK_BLOCKED;
+}
+// A walked shadow ray that arrives adds its light, less what it crossed, to its path.
+__device__ __forceinline__ void shadow_arrived(const SceneDev& S, const PathBuffers& P, float4 c4, bool indirect, Rgb keep) {
+    if (!(peak(keep) > 0.0f)) return;
+    const uint32_t slot = __float_as_uint(c4.w);
+    Rgb c = rgb(c4.x, c4.y, c4.z) * keep;
+    if (indirect && S.clamp_indirect > 0.0f) {
+        const float p = rmax(rmax(c.r, c.g), c.b);
+        if (p > S.clamp_indirect) c = c * (S.clamp_indirect / p);
+    }
+    float4 s4 = P.sum[slot];
+    s4.x = s4.x + c.r; s4.y = s4.y + c.g; s4.z = s4.z + c.b;
+    P.sum[slot] = s4;
+}
 // Persistent warps over the extension queue of round `round` (EXTEND, SHADOW_TOO) and the shadow rays
 // of the round before it (SHADOW_TOO) or of `round` itself (SHADOW): a lane whose ray has finished
 // takes the next one (one atomic per warp on the round's position) while the rest of the warp keeps
@@ -270,26 +311,32 @@ __device__ __forceinline__ void shadow_unblocked(const PathBuffers& P, uint32_t 
 // lanes_for lanes take rays. A round's shadow rays and the next round's extension rays depend on
 // nothing of each other (a path's radiance waits for its shadow ray only at the next vertex), so one
 // launch traces both: its end, where the slowest rays keep a few warps busy, comes once.
+// WALK and WALK_TOO: as SHADOW and SHADOW_TOO where surfaces are passable; a lane walks its shadow ray
+// on from crossing to crossing (against a launch a round with a thread per ray, whose warps wait for
+// their longest walk: studio frame 800x600 of glass and cut-outs 16.0 to 15.1 ms; 6 blocks an SM
+// 15.4).
 // `order`: the active queue in the order to trace it (the round's queue, or its ray-sorted copy);
 // `perm` (may be null): the shadow queue in the order to trace it.
-enum TraceRays { EXTEND, SHADOW, SHADOW_TOO };
+enum TraceRays { EXTEND, SHADOW, SHADOW_TOO, WALK, WALK_TOO };
 template <TraceRays RAYS>
-__global__ void __launch_bounds__(TRACE_THREADS, RTG_TRACE_BLOCKS(RAYS == SHADOW_TOO)) k_trace(const __grid_constant__ SceneDev S, PathBuffers P, uint32_t round, const uint32_t* __restrict__ order,
+__global__ void __launch_bounds__(TRACE_THREADS, RTG_TRACE_BLOCKS(RAYS != EXTEND && RAYS != SHADOW)) k_trace(const __grid_constant__ SceneDev S, PathBuffers P, uint32_t round, const uint32_t* __restrict__ order,
                                          const uint32_t* __restrict__ perm, uint32_t tail) {
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
     uint64_t deep[STACK_CAP - SHORT_STACK];
     SplitStack stack{s_stack + threadIdx.x, deep, TRACE_THREADS};
-    constexpr TraceMode MODE = RAYS == EXTEND ? TRACE_NEAREST : (RAYS == SHADOW ? TRACE_ANY : TRACE_EITHER);
-    const uint32_t paths = RAYS == SHADOW ? 0 : round_paths(P, round, tail);
-    const uint32_t shadows = RAYS == EXTEND ? 0 : *(volatile uint32_t*)&P.counters[round_counter(RAYS == SHADOW ? round : round - 1, COUNT_SHADOW)];
+    constexpr bool WALKS = RAYS == WALK || RAYS == WALK_TOO, TOO = RAYS == SHADOW_TOO || RAYS == WALK_TOO, ALONE = RAYS == SHADOW || RAYS == WALK;
+    constexpr TraceMode MODE = RAYS == EXTEND || WALKS ? TRACE_NEAREST : (RAYS == SHADOW ? TRACE_ANY : TRACE_EITHER);
+    const uint32_t paths = ALONE ? 0 : round_paths(P, round, tail);
+    const uint32_t shadows = RAYS == EXTEND ? 0 : *(volatile uint32_t*)&P.counters[round_counter(ALONE ? round : round - 1, COUNT_SHADOW)];
     const uint32_t n = paths + shadows;
     if (n == 0) return;
-    uint32_t* position = &P.counters[round_counter(round, RAYS == SHADOW ? NEXT_SHADOW : NEXT_PATH)];
+    uint32_t* position = &P.counters[round_counter(round, ALONE ? NEXT_SHADOW : NEXT_PATH)];
     uint32_t* bins = P.bins + KEY_BINS * (round & 1);
     const uint32_t lane = threadIdx.x & 31u, lanes = lanes_for(n), enough = min(lanes, (uint32_t)RTG_REFILL_MIN);
     uint32_t err = 0, ray = 0;  // the path's slot or the shadow ray
     bool busy = false, drained = false;
     Trav T;
+    ShadowWalk walk;
     for (;;) {
         bool done = false, hit = false;
         if (!drained) {
@@ -305,7 +352,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, RTG_TRACE_BLOCKS(RAYS == SHADOW
                     float4 o, d;
                     bool camera = false, sees = true;
                     float tmax = f_inf();
-                    if (RAYS == EXTEND || (RAYS == SHADOW_TOO && i < paths)) {
+                    if (RAYS == EXTEND || (TOO && i < paths)) {
                         ray = order[i];
                         load_pair(P.o, ray, o, d);
                         const uint32_t pf = __float_as_uint(o.w);
@@ -318,6 +365,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, RTG_TRACE_BLOCKS(RAYS == SHADOW
                         d = P.sh_d[ray];
                         tmax = o.w;
                         T.any = true;
+                        if (WALKS) walk = {v3(o.x, o.y, o.z), 0.0f, splat(1.0f), 0u};
                     }
                     busy = sees && trav_init(S, T, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 1.0e-3f, tmax, camera);
                     done = !busy;
@@ -325,17 +373,23 @@ __global__ void __launch_bounds__(TRACE_THREADS, RTG_TRACE_BLOCKS(RAYS == SHADOW
             }
         }
         const auto src = [&](V3& ro, V3& rd) {
-            const bool any = MODE == TRACE_ANY || (MODE == TRACE_EITHER && T.any);
+            const bool any = RAYS != EXTEND && (ALONE || T.any);
             const float4 o = any ? P.sh_o[ray] : P.o[ray], d = any ? P.sh_d[ray] : P.d[ray];
-            ro = v3(o.x, o.y, o.z);
+            ro = WALKS && any ? walk.o : v3(o.x, o.y, o.z);
             rd = v3(d.x, d.y, d.z);
         };
         if (busy && !trav_at_leaf(T)) done = trav_node<MODE, true>(S, T, 1.0e-3f, stack, &err, hit, src);
         busy = busy && !done;
         if (busy && trav_at_leaf(T)) done = trav_leaf<MODE, true>(S, T, 1.0e-3f, stack, &err, hit, src);
         busy = busy && !done;
-        if (done) {
-            if (MODE == TRACE_ANY || (MODE == TRACE_EITHER && T.any)) {
+        if (WALKS && done && (ALONE || T.any)) {
+            float next = 0.0f;
+            const float4 d4 = P.sh_d[ray];
+            const int crossed = hit ? shadow_crossing(S, walk, v3(d4.x, d4.y, d4.z), P.sh_o[ray].w, T.best_i, T.best_k, T.best_t, next) : WALK_ARRIVES;
+            busy = crossed == WALK_GOES_ON && trav_init(S, T, walk.o, v3(d4.x, d4.y, d4.z), 1.0e-3f, next, false);
+            if (!busy && crossed != WALK_BLOCKED) shadow_arrived(S, P, P.sh_c[ray], d4.w != 0.0f, walk.keep);
+        } else if (done) {
+            if (RAYS == SHADOW || (RAYS == SHADOW_TOO && T.any)) {
                 if (!hit) shadow_unblocked(P, ray);
             } else {
                 P.hit[ray] = hit ? make_uint4(T.best_i, T.best_k, __float_as_uint(T.best_t), 1u)
@@ -765,11 +819,10 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_shadow_section(const __grid_c
     if (err) atomicOr(&P.counters[3], err);
 }
 
-// ---- shadow walk: shadow rays through cut-outs and thin walls (integrator/mod.rs:629-690) ------------
-// Nearest hits along the ray: a passable surface multiplies what arrives by its straight
-// transmittance (a thin wall's) times its opacity plus 1 - opacity, and the ray goes on from just
-// behind it, up to 32 crossings; any other surface blocks it. One thread per ray: only scenes with
-// passable instances run it, instead of k_trace's any hits. BATCH: each ray's job gives its materials.
+// ---- shadow walks of sections and batched waves ------------------------------------------------------
+// Shadow rays through cut-outs and thin walls where k_trace's walk cannot take them: each part of a
+// section's walk is several queries, and in a batched wave (BATCH) each ray's job gives its
+// materials. One thread per ray.
 template <bool BATCH>
 __global__ void __launch_bounds__(TRACE_THREADS) k_shadow_walk(const __grid_constant__ SceneDev S, PathBuffers P, uint32_t round, WaveDesc w, const uint32_t* __restrict__ perm) {
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
@@ -790,37 +843,15 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_shadow_walk(const __grid_cons
         const SceneDev& J = *Sp;
         const V3 d = v3(d4.x, d4.y, d4.z);
         const float t_max = o4.w;
-        V3 o = v3(o4.x, o4.y, o4.z);
-        float tmax = t_max, travelled = 0.0f;
-        Rgb keep = splat(1.0f);
-        bool arrives = false;
-        for (uint32_t k = 0; k < 32; ++k) {  // MAX_SHADOW_CROSSINGS
+        ShadowWalk walk = {v3(o4.x, o4.y, o4.z), 0.0f, splat(1.0f), 0u};
+        float tmax = t_max;
+        int crossed = WALK_GOES_ON;
+        while (crossed == WALK_GOES_ON) {
             TraceResult res;
-            if (!trace_q<false>(J, o, d, 1.0e-3f, tmax, false, res, &err, stack)) { arrives = true; break; }
-            if (res.inst >= J.n_instances || !J.instances[res.inst].passable) break;
-            HitInfo h;
-            const DevInstance* I = nullptr;
-            if (!hit_details(J, o, d, 1.0e-3f, f_inf(), res.inst, res.tri, res.t, h, I)) break;
-            const uint32_t m = I->material;
-            const float opacity = rclamp(J.materials[m].opacity, 0.0f, 1.0f);
-            keep = keep * (straight_transmittance(J.bsdfs[2 * m], dot(h.geometric, d)) * opacity + splat(1.0f - opacity));
-            if (rmax(rmax(keep.r, keep.g), keep.b) <= 0.0f) break;
-            const V3 origin = offset_origin(h.point, -h.geometric);
-            travelled += dot(origin - o, d);
-            const float next = t_max - travelled;
-            if (next != next || next <= 1.0e-3f) { arrives = true; break; }
-            o = origin;
-            tmax = next;
+            crossed = trace_q<false>(J, walk.o, d, 1.0e-3f, tmax, false, res, &err, stack)
+                          ? shadow_crossing(J, walk, d, t_max, res.inst, res.tri, res.t, tmax) : WALK_ARRIVES;
         }
-        if (!(arrives && peak(keep) > 0.0f)) continue;
-        Rgb c = rgb(c4.x, c4.y, c4.z) * keep;
-        if (d4.w != 0.0f && J.clamp_indirect > 0.0f) {
-            const float p = rmax(rmax(c.r, c.g), c.b);
-            if (p > J.clamp_indirect) c = c * (J.clamp_indirect / p);
-        }
-        float4 s4 = P.sum[slot];
-        s4.x = s4.x + c.r; s4.y = s4.y + c.g; s4.z = s4.z + c.b;
-        P.sum[slot] = s4;
+        if (crossed == WALK_ARRIVES) shadow_arrived(J, P, c4, d4.w != 0.0f, walk.keep);
     }
     if (err) atomicOr(&P.counters[3], err);
 }
@@ -1373,12 +1404,22 @@ static int blocks_of(int resident, uint32_t n, int fallback) {
     return resident > 0 ? (int)std::min<uint32_t>((uint32_t)resident, (n + TRACE_THREADS / 32 - 1) / (TRACE_THREADS / 32)) : fallback;
 }
 
-uint32_t wave_launches(const SceneDev& S, const RaySort& order, const PathBuffers& P, bool batch) {
+// Shadow rays through passable surfaces are walked inside k_trace, except a section's and a batch's.
+static bool walks_on(const SceneDev& S, bool batch) { return S.any_passable && !S.section_on && !batch; }
+// Whether a wave of n paths traces each round's shadow rays with the next round's extension rays.
+// Timed waves trace them apart, so that the events are around extension rays only. So do waves of
+// more than 2^25 paths: their launches' ends weigh little, and shadow rays visit children in slot
+// order there, which needs no sort (132.7 M paths: 180.6 ms apart, 181.7 together; 8.4 M paths: 31.1
+// and 29.6; 0.9 M paths: 5.05 and 4.71).
+static bool together_on(const SceneDev& S, uint32_t n, bool batch, bool timed) {
+    return !S.section_on && (!S.any_passable || walks_on(S, batch)) && !timed && n <= (1u << 25);
+}
+uint32_t wave_launches(const SceneDev& S, const RaySort& order, const PathBuffers& P, uint32_t n, bool batch, bool timed) {
     const uint32_t rounds = wave_rounds(S);
     const bool rsort = order.ray_bits > 0 && P.rbins, ssort = rsort && order.shadow_sort && P.sbins;
     const bool tail = tail_on(S, order, batch) && rounds > TAIL_FIRST_ROUND;
-    const bool apart = S.any_passable || S.section_on;
-    return 2 + rounds * (2 + (apart ? 1u : 0u) + (order.material_sort ? 1u : 0u) + (ssort ? 2u : 0u)) + (rsort ? 2u * (rounds - 1u) : 0u) + (tail ? 1u : 0u);
+    const uint32_t shadows = !together_on(S, n, batch, timed) ? rounds : (walks_on(S, batch) ? 1u : 0u);
+    return 2 + rounds * (2 + (order.material_sort ? 1u : 0u) + (ssort ? 2u : 0u)) + shadows + (rsort ? 2u * (rounds - 1u) : 0u) + (tail ? 1u : 0u);
 }
 
 void launch_wave(const SceneDev& S, const LightsDev* L, const WaveDesc& wave, const PathBuffers& P, const FilmDev* film, cudaStream_t st,
@@ -1402,13 +1443,9 @@ void launch_wave(const SceneDev& S, const LightsDev* L, const WaveDesc& wave, co
     const uint32_t nk = ray_sort_keys(order.ray_bits);
     if (batch) k_camera<true><<<g, 256, 0, st>>>(S, w, P, rounds);
     else k_camera<false><<<g, 256, 0, st>>>(S, w, P, rounds);
-    // Each round's shadow rays are traced with the next round's extension rays. The last round has
-    // none: its vertices are at the greatest depth (only cut-outs, which are passable, shift that).
-    // Timed waves trace them apart, so that the events are around extension rays only.
-    // So do waves of more than 2^25 paths: their launches' ends weigh little, and shadow rays visit
-    // children in slot order there, which needs no sort (132.7 M paths: 180.6 ms apart, 181.7
-    // together; 8.4 M paths: 31.1 and 29.6; 0.9 M paths: 5.05 and 4.71).
-    const bool together = !S.any_passable && !S.section_on && !timing && w.n <= (1u << 25);
+    // Traced with the next round's extension rays, the last round's shadow rays need a launch of their
+    // own where there are any: its vertices are at the greatest depth, unless cut-outs shift that.
+    const bool walks = walks_on(S, batch), together = together_on(S, w.n, batch, timing != nullptr);
     const uint32_t* perm = nullptr;  // the last round's shadow rays in the order to trace them (null: as queued)
     for (uint32_t round = 0; round < rounds; ++round) {
         uint32_t* const queue = P.queue[round & 1];
@@ -1422,7 +1459,7 @@ void launch_wave(const SceneDev& S, const LightsDev* L, const WaveDesc& wave, co
         const bool timed = timing && timing->ev_count + 2 <= WaveTiming::MAX_EVENTS;
         if (timed) cudaEventRecord(timing->ev[timing->ev_count++], st);
         if (S.section_on) launch_traversal(order, g_trace, st, k_extend_section, S, P, round, traced, order.tail_paths);
-        else if (together && round > 0) launch_traversal(order, g_both, st, k_trace<SHADOW_TOO>, S, P, round, traced, perm, order.tail_paths);
+        else if (together && round > 0) launch_traversal(order, g_both, st, walks ? k_trace<WALK_TOO> : k_trace<SHADOW_TOO>, S, P, round, traced, perm, order.tail_paths);
         else launch_traversal(order, g_trace, st, k_trace<EXTEND>, S, P, round, traced, perm, order.tail_paths);
         if (timed) cudaEventRecord(timing->ev[timing->ev_count++], st);
         if (round == 0 && w.alb && film && !batch) k_albedo_hits<<<g, 256, 0, st>>>(S, L, w, P);
@@ -1446,9 +1483,11 @@ void launch_wave(const SceneDev& S, const LightsDev* L, const WaveDesc& wave, co
             k_key_scatter<<<g, 256, 0, st>>>(nullptr, P.sh_key, P.sbins + nk, &P.counters[round_counter(round, COUNT_SHADOW)], queue);
             perm = queue;
         }
-        if (S.any_passable) (batch ? k_shadow_walk<true> : k_shadow_walk<false>)<<<g, TRACE_THREADS, 0, st>>>(S, P, round, w, perm);
+        if (together && !(walks && round + 1 == rounds)) continue;
+        if (walks) launch_traversal(order, g_both, st, k_trace<WALK>, S, P, round, traced, perm, 0u);
+        else if (S.any_passable) (batch ? k_shadow_walk<true> : k_shadow_walk<false>)<<<g, TRACE_THREADS, 0, st>>>(S, P, round, w, perm);
         else if (S.section_on) launch_traversal(order, g_trace, st, k_shadow_section, S, P, round, perm);
-        else if (!together) launch_traversal(order, g_trace, st, k_trace<SHADOW>, S, P, round, traced, perm, 0u);
+        else launch_traversal(order, g_trace, st, k_trace<SHADOW>, S, P, round, traced, perm, 0u);
     }
     if (order.tail_paths)
         (S.plain ? k_tail<true> : k_tail<false>)<<<blocks_of(tail_resident, w.n, g), TRACE_THREADS, 0, st>>>(S, L, P, w, rounds, order.tail_paths);

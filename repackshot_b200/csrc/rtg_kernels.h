@@ -224,8 +224,8 @@ struct WaveTiming {
 void set_sobol(const SobolTable& t, cudaStream_t s);
 void launch_wave(const SceneDev& S, const LightsDev* L, const WaveDesc& w, const PathBuffers& P, const FilmDev* film, cudaStream_t st,
                  int grid, WaveTiming* timing, const RaySort& order = RaySort());
-// Kernel launches of one launch_wave with a film (camera and accumulate included, guides not).
-uint32_t wave_launches(const SceneDev& S, const RaySort& order, const PathBuffers& P, bool batch);
+// Kernel launches of one launch_wave of n paths with a film (camera and accumulate included, guides not).
+uint32_t wave_launches(const SceneDev& S, const RaySort& order, const PathBuffers& P, uint32_t n, bool batch, bool timed);
 // The adjoint: loss and per-pixel path derivatives of a film against a target (w*h*3 floats on
 // the device), then the backward wave: the replay of the wave that rendered the film.
 void launch_adjoint_delta(const FilmDev& F, const float* target, float4* dpath, double* loss, const PathBuffers& P, uint32_t count, cudaStream_t st,
