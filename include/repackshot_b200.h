@@ -376,7 +376,9 @@ uint32_t rtg_render_tile_alpha(uint32_t handle, uint32_t x, uint32_t y, uint32_t
  * (width*(y1-y0)*4 floats) to `out`. `preset` 0 is the full filter, 1 the viewport's; `strength`
  * (0..1, NaN: 1) blends noisy x (1 - s) + denoised x s per colour channel, and at 0 no filter runs.
  * RTG_STATUS_NULL_POINTER, or RTG_STATUS_BAD_DENOISE when the preset, the sizes, the band or its
- * halo do not fit. The filter runs on the GPU with the reference's bits. */
+ * halo do not fit. The filter runs on the GPU with the reference's bits. The library keeps the
+ * call's device memory, up to 256 MB, and 8 MB of pinned memory for the next one; freeing the last
+ * scene gives both back, and the device memory goes to any allocation that does not fit beside it. */
 uint32_t rtg_denoise(uint32_t width, uint32_t height, uint32_t origin_y, uint32_t rows, uint32_t samples, uint32_t y0, uint32_t y1,
                      const uint8_t* in, float* out);
 uint32_t rtg_denoise_with(uint32_t preset, float strength, uint32_t width, uint32_t height, uint32_t origin_y, uint32_t rows, uint32_t samples,

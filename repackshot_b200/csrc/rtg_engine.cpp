@@ -14,6 +14,7 @@
 
 #include "../../include/repackshot_b200.h"
 #include "rtg_adaptive.h"
+#include "rtg_copy.h"
 #include "rtg_denoise.h"
 #include "rtg_kernels.h"
 #include "rtg_noalloc.h"
@@ -47,6 +48,48 @@ struct DevBuf {
     size_t bytes = 0;
     void release() { if (p) cudaFree(p); p = nullptr; bytes = 0; }
 };
+
+// The device block a call on host planes leaves for the next one (allocating and freeing 130 MB takes
+// 3 to 5 ms): at most KEPT_MOST bytes, given back with the last scene and to an allocation that
+// does not fit beside it. Every call on it has ended with a synchronous copy.
+constexpr size_t KEPT_MOST = 256u << 20;
+DevBuf g_kept;
+int g_kept_device = -1;
+cudaError_t dev_alloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && g_kept.p) {
+        cudaGetLastError();
+        g_kept.release();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+template <class T>
+cudaError_t dev_alloc(T** p, size_t bytes) { return dev_alloc((void**)p, bytes); }
+// A block of at least `bytes` on the current device for one call, which gives it back by lent_return.
+cudaError_t lent_block(size_t bytes, DevBuf& b) {
+    int device = -1;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    if (g_kept.p && g_kept_device == device && g_kept.bytes >= bytes) {
+        b = g_kept;
+        g_kept = DevBuf{};
+        return cudaSuccess;
+    }
+    g_kept.release();
+    e = dev_alloc(&b.p, bytes);
+    if (e == cudaSuccess) b.bytes = bytes;
+    return e;
+}
+void lent_return(DevBuf& b) {
+    int device = -1;
+    if (b.p && b.bytes <= KEPT_MOST && !g_kept.p && cudaGetDevice(&device) == cudaSuccess) {
+        g_kept = b;
+        g_kept_device = device;
+        b = DevBuf{};
+    }
+    b.release();
+}
 
 // Device buffers released together.
 struct BufSet {
@@ -214,7 +257,7 @@ uint32_t device_init() {
     const size_t albedo = put_cells(E.albedo), schlick = put_cells(E.schlick), clear_in = put_cells(E.clear_in), clear_out = put_cells(E.clear_out);
     const size_t albedo_avg = put(E.albedo_avg.data(), 32 * 4), schlick_avg = put(E.schlick_avg.data(), 32 * 4);
     const size_t filter = put(blackman_harris_table(), 256 * 4), sobol = put(low.data(), low.size() * 4);
-    RTG_CHECK(cudaMalloc(&g_energy_dev, host.size()));
+    RTG_CHECK(dev_alloc(&g_energy_dev, host.size()));
     RTG_CHECK(cudaMemcpy(g_energy_dev, host.data(), host.size(), cudaMemcpyHostToDevice));
     const uint8_t* d = (const uint8_t*)g_energy_dev;
     g_energy = EnergyTables{(const uint16_t*)(d + albedo), (const uint16_t*)(d + schlick), (const uint16_t*)(d + clear_in),
@@ -231,7 +274,7 @@ uint32_t upload(BufSet& set, const std::vector<T>& v, const T*& out) {
     DevBuf b;
     b.bytes = v.size() * sizeof(T);
     if (b.bytes == 0) { out = nullptr; return RTG_STATUS_OK; }
-    RTG_CHECK(cudaMalloc(&b.p, b.bytes));
+    RTG_CHECK(dev_alloc(&b.p, b.bytes));
     set.bufs.push_back(b);
     RTG_CHECK(cudaMemcpy(b.p, v.data(), b.bytes, cudaMemcpyHostToDevice));
     out = (const T*)b.p;
@@ -252,7 +295,7 @@ uint32_t upload_geometry(const Flat& F, BufSet& set, SceneDev& S, size_t* hot_by
     if (hot) {
         DevBuf b;
         b.bytes = hot;
-        RTG_CHECK(cudaMalloc(&b.p, b.bytes));
+        RTG_CHECK(dev_alloc(&b.p, b.bytes));
         set.bufs.push_back(b);
         uint8_t* p = (uint8_t*)b.p;
         if (b_nodes) RTG_CHECK(cudaMemcpy(p, F.nodes.data(), b_nodes, cudaMemcpyHostToDevice));
@@ -300,7 +343,7 @@ uint32_t upload_shading(const Flat& F, BufSet& set, SceneDev& S) {
     if (F.plate && (st = upload(set, F.plate->texels, S.plate))) return st;
     S.exempt_boxes = nullptr;
     if (!F.exempt_boxes.empty() && (st = upload(set, F.exempt_boxes, S.exempt_boxes))) return st;
-    RTG_CHECK(cudaMalloc(&set.lights, sizeof(LightsDev)));
+    RTG_CHECK(dev_alloc(&set.lights, sizeof(LightsDev)));
     RTG_CHECK(cudaMemcpy(set.lights, &L, sizeof(LightsDev), cudaMemcpyHostToDevice));
     return RTG_STATUS_OK;
 }
@@ -429,7 +472,7 @@ uint32_t ensure_capacity(Scene& sc, uint32_t paths) {
     sc.capacity = 0;
     size_t n = paths;
     size_t bytes = n * PATH_BYTES + 17 * 256 + COUNTERS_BYTES + 2 * KEY_BINS * 4 + 256 + SORT_BINS_BYTES;
-    RTG_CHECK(cudaMalloc(&sc.path_mem.p, bytes));
+    RTG_CHECK(dev_alloc(&sc.path_mem.p, bytes));
     sc.path_mem.bytes = bytes;
     uint8_t* p = (uint8_t*)sc.path_mem.p;
     auto take = [&](size_t each) { uint8_t* r = p; p += ((n * each + 255) / 256) * 256; return r; };
@@ -518,7 +561,7 @@ uint32_t edge_mask_of(Scene& sc, const uint8_t*& mask, uint32_t*& list, uint32_t
     const size_t need = mask_bytes + npix * sizeof(uint4) + npix * 4 + 16;
     if (sc.edge_mem.bytes < need) {
         sc.edge_mem.release();
-        RTG_CHECK(cudaMalloc(&sc.edge_mem.p, need));
+        RTG_CHECK(dev_alloc(&sc.edge_mem.p, need));
         sc.edge_mem.bytes = need;
         sc.edges_ready = false;
     }
@@ -588,7 +631,7 @@ uint32_t render_region(Scene& sc, uint32_t x, uint32_t y, uint32_t w, uint32_t h
         if (st) return st;
         if (guide_sum && sc.alb_mem.bytes < (size_t)sc.capacity * 16) {
             sc.alb_mem.release();
-            RTG_CHECK(cudaMalloc(&sc.alb_mem.p, (size_t)sc.capacity * 16));
+            RTG_CHECK(dev_alloc(&sc.alb_mem.p, (size_t)sc.capacity * 16));
             sc.alb_mem.bytes = (size_t)sc.capacity * 16;
         }
         auto guides = [&](WaveDesc& wd) {
@@ -636,7 +679,7 @@ uint32_t render_region(Scene& sc, uint32_t x, uint32_t y, uint32_t w, uint32_t h
 uint32_t make_film(uint32_t ox, uint32_t oy, uint32_t w, uint32_t h, Film& f) {
     size_t n = (size_t)w * h;
     f.mem.bytes = n * 6 * 4;
-    RTG_CHECK(cudaMalloc(&f.mem.p, f.mem.bytes));
+    RTG_CHECK(dev_alloc(&f.mem.p, f.mem.bytes));
     RTG_CHECK(cudaMemset(f.mem.p, 0, f.mem.bytes));
     float* p = (float*)f.mem.p;
     f.dev = FilmDev{ox, oy, w, h, p, p + 3 * n, p + 4 * n, p + 5 * n};
@@ -966,6 +1009,10 @@ uint32_t rtg_scene_free(uint32_t handle) {
     const bool window = sc->order.l2_persist != 0;
     g_scenes[handle - 1].reset();
     if (window) release_set_aside(dev, nullptr);
+    if (std::none_of(g_scenes.begin(), g_scenes.end(), [](const auto& s) { return s != nullptr; })) {
+        g_kept.release();
+        copy_release();
+    }
     return RTG_STATUS_OK;
 }
 
@@ -1217,7 +1264,7 @@ uint32_t rtg_queue_run(uint32_t queue, uint32_t flags, uint64_t* rays) {
     size_t bytes = jobs_h.size() * sizeof(JobDev) + nseg * sizeof(SegDev);
     if (q->tables.bytes < bytes) {
         q->tables.release();
-        RTG_CHECK(cudaMalloc(&q->tables.p, bytes));
+        RTG_CHECK(dev_alloc(&q->tables.p, bytes));
         q->tables.bytes = bytes;
     }
     std::vector<uint8_t> host(bytes);
@@ -1363,7 +1410,7 @@ uint32_t rtg_render_adjoint(uint32_t scene, uint32_t film, const float* target, 
     size_t bytes = off_shi + span(4);
     if (sc->adjoint_mem.bytes < bytes) {
         sc->adjoint_mem.release();
-        RTG_CHECK(cudaMalloc(&sc->adjoint_mem.p, bytes));
+        RTG_CHECK(dev_alloc(&sc->adjoint_mem.p, bytes));
         sc->adjoint_mem.bytes = bytes;
     }
     uint8_t* base = (uint8_t*)sc->adjoint_mem.p;
@@ -1448,13 +1495,13 @@ uint32_t film_encode(uint32_t film, float ev, uint32_t tonemap, uint32_t bits, v
     size_t bytes = (size_t)f->dev.w * f->dev.h * 3 * (bits / 8);
     if (f->encoded.bytes < bytes) {
         f->encoded.release();
-        RTG_CHECK(cudaMalloc(&f->encoded.p, bytes));
+        RTG_CHECK(dev_alloc(&f->encoded.p, bytes));
         f->encoded.bytes = bytes;
     }
     launch_film_encode(f->dev, ev, tonemap, bits, f->encoded.p, s, grid_for(f->dev.w * f->dev.h, 256));
     RTG_CHECK(cudaGetLastError());
-    RTG_CHECK(cudaMemcpyAsync(out, f->encoded.p, bytes, cudaMemcpyDeviceToHost, s));
-    RTG_CHECK(cudaStreamSynchronize(s));
+    const CopyPart part{out, f->encoded.p, bytes};
+    RTG_CHECK(copy_planes(&part, 1, false, s));
     return RTG_STATUS_OK;
 }
 }  // namespace
@@ -1487,7 +1534,7 @@ uint32_t rtg_encode_planes(const float* rgb, const float* weight, uint32_t width
     DevBuf m;
     struct Release { DevBuf& b; ~Release() { b.release(); } } release{m};
     m.bytes = rgb_bytes + weight_bytes + out_bytes;
-    RTG_CHECK(cudaMalloc(&m.p, m.bytes));
+    RTG_CHECK(dev_alloc(&m.p, m.bytes));
     uint8_t* base = (uint8_t*)m.p;
     FilmDev F{0, 0, width, height, (float*)base, (float*)(base + rgb_bytes), nullptr, nullptr};
     void* d_out = base + rgb_bytes + weight_bytes;
@@ -1506,11 +1553,13 @@ uint32_t rtg_film_read(uint32_t film, float* rgb, float* weight, float* alpha, f
     Scene* sc = scene_of(f->scene);
     cudaStream_t s = sc ? sc->stream : 0;
     size_t n = (size_t)f->dev.w * f->dev.h;
-    if (rgb) RTG_CHECK(cudaMemcpyAsync(rgb, f->dev.rgb, n * 12, cudaMemcpyDeviceToHost, s));
-    if (weight) RTG_CHECK(cudaMemcpyAsync(weight, f->dev.weight, n * 4, cudaMemcpyDeviceToHost, s));
-    if (alpha) RTG_CHECK(cudaMemcpyAsync(alpha, f->dev.alpha, n * 4, cudaMemcpyDeviceToHost, s));
-    if (lum2) RTG_CHECK(cudaMemcpyAsync(lum2, f->dev.lum2, n * 4, cudaMemcpyDeviceToHost, s));
-    RTG_CHECK(cudaStreamSynchronize(s));
+    CopyPart parts[4];
+    int count = 0;
+    if (rgb) parts[count++] = {rgb, f->dev.rgb, n * 12};
+    if (weight) parts[count++] = {weight, f->dev.weight, n * 4};
+    if (alpha) parts[count++] = {alpha, f->dev.alpha, n * 4};
+    if (lum2) parts[count++] = {lum2, f->dev.lum2, n * 4};
+    RTG_CHECK(copy_planes(parts, count, false, s));
     return RTG_STATUS_OK;
 }
 uint32_t rtg_film_device(uint32_t film, float** rgb, float** weight, float** alpha, float** lum2) {
@@ -1533,7 +1582,7 @@ uint32_t rtg_render_paths(uint32_t handle, const uint32_t* xys, uint32_t n, floa
     uint32_t st = ensure_capacity(*sc, n);
     if (st) return st;
     uint32_t* d_xys = nullptr;
-    RTG_CHECK(cudaMalloc(&d_xys, (size_t)n * 12));
+    RTG_CHECK(dev_alloc(&d_xys, (size_t)n * 12));
     std::unique_ptr<uint32_t, void (*)(uint32_t*)> guard(d_xys, [](uint32_t* p) { cudaFree(p); });
     RTG_CHECK(cudaMemcpyAsync(d_xys, xys, (size_t)n * 12, cudaMemcpyHostToDevice, sc->stream));
     RTG_CHECK(cudaMemsetAsync(sc->P.counters, 0, 16, sc->stream));
@@ -1592,7 +1641,7 @@ uint32_t rtg_trace_rays(uint32_t handle, const float* rays, uint32_t n, uint32_t
     if (st) return st;
     size_t words = (mode & 2u) ? n : (size_t)n * 3;
     void* mem = nullptr;
-    RTG_CHECK(cudaMalloc(&mem, (size_t)n * 32 + words * 4));
+    RTG_CHECK(dev_alloc(&mem, (size_t)n * 32 + words * 4));
     std::unique_ptr<void, void (*)(void*)> guard(mem, [](void* p) { cudaFree(p); });
     float* d_rays = (float*)mem;
     uint32_t* d_out = (uint32_t*)((uint8_t*)mem + (size_t)n * 32);
@@ -1838,7 +1887,7 @@ uint32_t rtg_adaptive_decide(uint32_t width, uint32_t height, float ev, float ta
     struct Release { DevBuf& b; ~Release() { b.release(); } } release{m};
     const size_t sums_bytes = npix * 16, lum_bytes = (npix * 4 + 255) & ~(size_t)255, nb_bytes = (nb * 4 + 255) & ~(size_t)255;
     m.bytes = sums_bytes + lum_bytes + 2 * nb_bytes;
-    RTG_CHECK(cudaMalloc(&m.p, m.bytes));
+    RTG_CHECK(dev_alloc(&m.p, m.bytes));
     uint8_t* base = (uint8_t*)m.p;
     float* d_sums = (float*)base;
     float* d_lum2 = (float*)(base + sums_bytes);
@@ -1895,7 +1944,7 @@ uint32_t rtg_adaptive_create(uint32_t scene, uint32_t film, uint32_t cap) {
     auto round_up = [](size_t b) { return (b + 255) & ~(size_t)255; };
     const size_t nb4 = round_up(nb * 4), list = round_up(npix * 4);
     a->mem.bytes = 2 * nb4 + round_up(nb * sizeof(AdEntry)) + round_up(nb * 8) + 4 * list;
-    if (cudaMalloc(&a->mem.p, a->mem.bytes) != cudaSuccess) {
+    if (dev_alloc(&a->mem.p, a->mem.bytes) != cudaSuccess) {
         a->mem.p = nullptr;
         g_error = "rtg_adaptive_create: out of device memory";
         return 0;
@@ -1996,7 +2045,7 @@ uint32_t rtg_render_tile_passes(uint32_t handle, uint32_t x, uint32_t y, uint32_
     DevBuf m;
     struct Release { DevBuf& b; ~Release() { b.release(); } } release{m};
     m.bytes = px * 24;
-    RTG_CHECK(cudaMalloc(&m.p, m.bytes));
+    RTG_CHECK(dev_alloc(&m.p, m.bytes));
     float* normal = (float*)m.p;
     float* depth = normal + 3 * px;
     uint32_t* part = (uint32_t*)(depth + px);
@@ -2051,7 +2100,7 @@ uint32_t rtg_render_tile_albedo(uint32_t handle, uint32_t x, uint32_t y, uint32_
     DevBuf m;
     struct Release { DevBuf& b; ~Release() { b.release(); } } release{m};
     m.bytes = px * 16;
-    RTG_CHECK(cudaMalloc(&m.p, m.bytes));
+    RTG_CHECK(dev_alloc(&m.p, m.bytes));
     RTG_CHECK(cudaMemsetAsync(m.p, 0, m.bytes, sc->stream));
     float* sum = (float*)m.p;
     RTG_CHECK(launch_albedo_pass(sc->S, sc->d_lights, mask, x, y, w, h, sample_index, 1, sum, sum + 3 * px, nullptr, sc->stream,
@@ -2078,7 +2127,7 @@ uint32_t rtg_render_tile_alpha(uint32_t handle, uint32_t x, uint32_t y, uint32_t
     DevBuf m;
     struct Release { DevBuf& b; ~Release() { b.release(); } } release{m};
     m.bytes = px * 20;
-    RTG_CHECK(cudaMalloc(&m.p, m.bytes));
+    RTG_CHECK(dev_alloc(&m.p, m.bytes));
     RTG_CHECK(cudaMemsetAsync(m.p, 0, m.bytes, sc->stream));
     float* sum = (float*)m.p;
     float* alpha = sum + 4 * px;
@@ -2099,7 +2148,7 @@ uint32_t rtg_film_guides(uint32_t scene, uint32_t film, uint32_t first_sample, u
     const size_t n = f->pixels();
     if (!f->guides.p) {
         f->guides.bytes = n * 10 * 4;
-        RTG_CHECK(cudaMalloc(&f->guides.p, f->guides.bytes));
+        RTG_CHECK(dev_alloc(&f->guides.p, f->guides.bytes));
         RTG_CHECK(cudaMemsetAsync(f->guides.p, 0, f->guides.bytes, sc->stream));
     }
     const uint8_t* mask = nullptr;
@@ -2130,7 +2179,7 @@ uint32_t rtg_film_guides_fused(uint32_t scene, uint32_t film, uint32_t enable) {
     const size_t n = f->pixels();
     if (!f->guides.p) {
         f->guides.bytes = n * 10 * 4;
-        RTG_CHECK(cudaMalloc(&f->guides.p, f->guides.bytes));
+        RTG_CHECK(dev_alloc(&f->guides.p, f->guides.bytes));
         RTG_CHECK(cudaMemsetAsync(f->guides.p, 0, f->guides.bytes, sc->stream));
     }
     const FilmDev& d = f->dev;
@@ -2161,7 +2210,7 @@ uint32_t rtg_film_denoise(uint32_t film, uint32_t preset, float strength, uint32
     const size_t need = dn_scratch_bytes(n) + n * 16 + n * 20;
     if (f->denoise.bytes < need) {
         f->denoise.release();
-        RTG_CHECK(cudaMalloc(&f->denoise.p, need));
+        RTG_CHECK(dev_alloc(&f->denoise.p, need));
         f->denoise.bytes = need;
     }
     float* result = (float*)((uint8_t*)f->denoise.p + dn_scratch_bytes(n));
@@ -2187,8 +2236,8 @@ uint32_t rtg_film_denoise(uint32_t film, uint32_t preset, float strength, uint32
             noisy.resize(4 * n);
             RTG_CHECK(cudaMemcpyAsync(noisy.data(), rgba, n * 16, cudaMemcpyDeviceToHost, sc->stream));
         }
-        if (s > 0.0f) RTG_CHECK(cudaMemcpyAsync(out, result, n * 16, cudaMemcpyDeviceToHost, sc->stream));
-        RTG_CHECK(cudaStreamSynchronize(sc->stream));
+        const CopyPart part{out, result, n * 16};
+        RTG_CHECK(copy_planes(&part, s > 0.0f ? 1 : 0, false, sc->stream));
         if (s <= 0.0f) {
             std::memcpy(out, noisy.data(), n * 16);
         } else if (s < 1.0f) {
@@ -2226,21 +2275,21 @@ uint32_t rtg_denoise_with(uint32_t preset, float strength, uint32_t width, uint3
     uint32_t st = device_init();
     if (st) return st;
     DevBuf m;
-    struct Release { DevBuf& bb; ~Release() { bb.release(); } } release{m};
+    struct Return { DevBuf& bb; ~Return() { lent_return(bb); } } give_back{m};
     const size_t in_bytes = n * 14 * 4, scratch = dn_scratch_bytes(n);
-    m.bytes = ((in_bytes + 255) & ~(size_t)255) + scratch + n * 16;
-    RTG_CHECK(cudaMalloc(&m.p, m.bytes));
+    RTG_CHECK(lent_block(((in_bytes + 255) & ~(size_t)255) + scratch + n * 16, m));
     uint8_t* base = (uint8_t*)m.p;
     const float* words = (const float*)base;
     void* scr = base + ((in_bytes + 255) & ~(size_t)255);
     float* result = (float*)((uint8_t*)scr + scratch);
-    RTG_CHECK(cudaMemcpy(base, in, in_bytes, cudaMemcpyHostToDevice));
+    const CopyPart up{const_cast<uint8_t*>(in), base, in_bytes}, down{out, result + a, (b - a) * 4};
+    RTG_CHECK(copy_planes(&up, 1, true, 0));
     // rt-wasm/src/lib.rs:448-455: sums (4), lum2, albedo (3), normal (3), depth, part, material
     const DnSrc src{words, 4, words + 3, 4, words + n * 4, words + n * 5, nullptr, words + n * 8, words + n * 11,
                     (const uint32_t*)(words + n * 12), (const uint32_t*)(words + n * 13), nullptr};
     uint64_t launches = 0;
     RTG_CHECK(denoise_band(src, width, rows, samples, pr, scr, result, 0, grid_for((uint32_t)n, 256), launches));
-    RTG_CHECK(cudaMemcpy(out, result + a, (b - a) * 4, cudaMemcpyDeviceToHost));
+    RTG_CHECK(copy_planes(&down, 1, false, 0));
     if (s < 1.0f) {
         std::vector<float> noisy(b - a);
         std::memcpy(noisy.data(), in + a * 4, (b - a) * 4);
