@@ -859,9 +859,14 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_shadow_walk(const __grid_cons
 // ---- tail: the last rounds of a wave, a path per lane -------------------------------------------------
 // The wave's last launch. From the first round whose extension queue holds at most `limit` paths on,
 // the other kernels do nothing, and here each lane carries its share of those paths through the
-// wave's remaining rounds alone: the nearest hit (as k_trace), the vertex (shade_slot), the any
-// hit of its shadow ray and its contribution, the next ray; each path's arithmetic in
-// the order the wavefront gives it, so its sum has the same bits. A wave whose last rounds hold few
+// wave's remaining rounds alone: the nearest hit (as k_trace), the vertex (shade_slot), the next
+// ray; each path's arithmetic in the order the wavefront gives it, so its sum has the same bits.
+// What bounds it is the chain of one path's rays and vertices, so warps work in pairs: lane for lane,
+// the second warp traces the vertices' shadow rays and adds their light while the first traces the
+// paths' next rays; they meet twice a vertex. Against one lane for both rays in turn: 720p viewport
+// 4.60 to 4.20 ms, 617x351 crop 3.46 to 3.25, small fit 2.13 to 2.05, adaptive frame 70.3 to 68.7;
+// with the shadow rays in the upper half of the same warp, whose vertices then come from twice the
+// warps, the viewport gained half of that and a 256x256 frame lost 2 %. A wave whose last rounds hold few
 // paths then pays one launch as long as its slowest path instead of a chain of launches, each as
 // long as its slowest ray. Scenes with passable surfaces (shadow walks) and batched waves keep the
 // wavefront.
@@ -872,43 +877,85 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_tail(const __grid_constant__ 
     while (round < rounds && P.counters[round_counter(round, COUNT_PATHS)] > limit) ++round;
     const uint32_t n = round < rounds ? P.counters[round_counter(round, COUNT_PATHS)] : 0;
     if (n == 0) return;
-    // Up to four paths a warp run spread over all warps; more run in full warps, which meet each
-    // other's code less often (at 4, spread against full: a 64 x 64 tile 0.51 and 0.56 ms, a 720p
-    // viewport 4.74 and 4.39 ms, whose tail holds up to 16,384 paths).
-    const uint32_t rounds_left = rounds - round, spread = lanes_for(n), lanes = spread <= 4u ? spread : 32u;
+    // Up to eight paths a pair run spread over all pairs; more run in full warps, which meet each
+    // other's code less often (with a warp for both kinds of rays, spread against full: a 64 x 64 tile
+    // 0.51 and 0.56 ms, a 720p viewport, whose tail holds up to 16,384 paths, 4.74 and 4.39 ms; up to
+    // 2, 4 and 8 a pair: adaptive frame 68.7, 69.0 and 68.7 ms, tile 0.52, 0.51 and 0.51 ms).
+    const uint32_t pairs = gridDim.x * (TRACE_THREADS / 64), spread = (n + pairs - 1) / pairs;
+    const uint32_t rounds_left = rounds - round, lanes = spread <= 8u ? spread : 32u;
     __shared__ uint64_t s_stack[SHORT_STACK * TRACE_THREADS];
+    __shared__ TailShadow s_shadow[TRACE_THREADS / 2];
+    __shared__ bool s_more[TRACE_THREADS / 64];
     uint64_t deep[STACK_CAP - SHORT_STACK];
     SplitStack stack{s_stack + threadIdx.x, deep, TRACE_THREADS};
     const uint32_t* __restrict__ queue = P.queue[round & 1];
     const RaySort R;  // no coherence keys
     uint32_t err = 0, rays_local = 0, shadow_local = 0;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
-    for (uint32_t i = lane < lanes ? warp * lanes + lane : n; i < n; i += gridDim.x * (blockDim.x >> 5) * lanes) {
-        const uint32_t slot = queue[i];
-        for (uint32_t r = 0; r < rounds_left; ++r) {
-            const float4 o = P.o[slot], d = P.d[slot];
-            const uint32_t pf = __float_as_uint(o.w);
+    const uint32_t pair = threadIdx.x >> 6, lane = threadIdx.x & 31u, first = blockIdx.x * (TRACE_THREADS / 64) + pair;
+    TailShadow& sh = s_shadow[pair * 32 + lane];
+    const auto meet = [&] {
+        if (pair) asm volatile("bar.sync 2, 64;" ::: "memory");
+        else asm volatile("bar.sync 1, 64;" ::: "memory");
+    };
+    static_assert(TRACE_THREADS == 128, "two pairs of warps a block");
+    if (!(threadIdx.x & 32u)) {
+        uint32_t i = lane < lanes ? first * lanes + lane : n, slot = 0, r = 0;
+        for (bool more = true; more;) {
+            if (i < n && r == 0) slot = queue[i];
             TraceResult res;
-            const bool got = !(pf & PF_NOTHING) &&
-                             traverse<false, true>(S, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 1.0e-3f, f_inf(), (pf & PF_PRIMARY) != 0, res, &err, stack);
-            P.hit[slot] = got ? make_uint4(res.inst, res.tri, __float_as_uint(res.t), 1u) : make_uint4(0xffffffffu, 0xffffffffu, 0u, 0u);
-            TailShadow sh;
-            sh.on = false;
-            const bool alive = shade_slot<PLAIN>(S, *Lg, P, R, slot, round, [&](uint32_t& xx, uint32_t& yy, uint32_t& ii) { wave_slot(w, slot, xx, yy, ii); },
-                                          rays_local, shadow_local, &sh);
-            if (sh.on) {
-                TraceResult unused;
-                if (!traverse<true, true>(S, v3(sh.o.x, sh.o.y, sh.o.z), v3(sh.d.x, sh.d.y, sh.d.z), 1.0e-3f, sh.o.w, false, unused, &err, stack)) {
-                    float4 sum = P.sum[slot];  // shadow_unblocked's addition
-                    sum.x = sum.x + sh.c.x;
-                    sum.y = sum.y + sh.c.y;
-                    sum.z = sum.z + sh.c.z;
-                    P.sum[slot] = sum;
+            bool got = false;
+            if (i < n) {
+                float4 o, d;
+                load_pair(P.o, slot, o, d);
+                const uint32_t pf = __float_as_uint(o.w);
+                got = !(pf & PF_NOTHING) &&
+                      traverse<false, true>(S, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), 1.0e-3f, f_inf(), (pf & PF_PRIMARY) != 0, res, &err, stack);
+                P.hit[slot] = got ? make_uint4(res.inst, res.tri, __float_as_uint(res.t), 1u) : make_uint4(0xffffffffu, 0xffffffffu, 0u, 0u);
+            }
+            __syncwarp();
+            meet();  // the last vertices' shadow rays have added their light
+            TailShadow next;
+            next.on = false;
+            if (i < n) {
+                const bool alive = shade_slot<PLAIN>(S, *Lg, P, R, slot, round, [&](uint32_t& xx, uint32_t& yy, uint32_t& ii) { wave_slot(w, slot, xx, yy, ii); },
+                                                     rays_local, shadow_local, &next);
+                if (alive && r + 1 < rounds_left) {
+                    ++r;
+                } else {
+                    r = 0;
+                    i += pairs * lanes;
                 }
             }
-            if (!alive) break;
+            if (next.on) sh = next;
+            else sh.on = false;
+            more = __any_sync(0xffffffffu, i < n || next.on);
+            if (lane == 0) s_more[pair] = more;
+            __syncwarp();
+            meet();
+        }
+    } else {
+        TailShadow ray;
+        ray.on = false;
+        for (bool more = true; more;) {
+            if (ray.on) {
+                TraceResult unused;
+                if (!traverse<true, true>(S, v3(ray.o.x, ray.o.y, ray.o.z), v3(ray.d.x, ray.d.y, ray.d.z), 1.0e-3f, ray.o.w, false, unused, &err, stack)) {
+                    float4* const to = &P.sum[__float_as_uint(ray.c.w)];  // shadow_unblocked's addition
+                    float4 sum = *to;
+                    sum.x = sum.x + ray.c.x;
+                    sum.y = sum.y + ray.c.y;
+                    sum.z = sum.z + ray.c.z;
+                    *to = sum;
+                }
+            }
+            __syncwarp();
+            meet();
+            meet();  // the vertices' next shadow rays are there
+            ray = sh;
+            more = s_more[pair];
         }
     }
+    __syncwarp();
     uint32_t total = __reduce_add_sync(0xffffffffu, rays_local);
     uint32_t shadows = __reduce_add_sync(0xffffffffu, shadow_local);
     if ((threadIdx.x & 31) == 0 && total) atomicAdd(P.rays, (unsigned long long)total);

@@ -58,3 +58,12 @@ def test_shadow_rays_together_and_apart_have_the_same_bits(name, size, tail):
     films = [_film(SHADOWS[name](), *size, timed=timed, tail_paths=tail) for timed in (False, True)]
     for a, b in zip(*films):
         assert np.array_equal(a, b)
+
+
+# One path, a warp less and more than full, and more paths than all pairs of warps hold at once.
+@pytest.mark.parametrize("name", ["plain", "light kinds"])
+@pytest.mark.parametrize("size", [(1, 1, 1), (31, 1, 1), (65, 1, 1), (67, 41, 3), (160, 120, 3)])
+def test_the_tail_has_the_wavefronts_bits(name, size):
+    films = [_film(SHADOWS[name](), *size, tail_paths=tail) for tail in (0, 1 << 20)]
+    for a, b in zip(*films):
+        assert np.array_equal(a, b)
