@@ -573,15 +573,15 @@ def run_ours(args, world, rank, local, dist):
         "dtype": "f32", "data": DATA,
         "config": {"workload": WORKLOAD, "width": WIDTH, "height": HEIGHT, "spp": SPP, "max_depth": DEPTH,
                    "triangles": scene.triangles, "paths_per_step_per_gpu": paths_step,
-                   "l2": "flushed between steps (512 MiB write); the per-step working set (172 B of path state per path, "
-                         "23 GB for the frame) exceeds L2",
+                   "l2": "flushed between steps (512 MiB write); the per-step working set (168 B of path state per path, "
+                         "22 GB for the frame) exceeds L2",
                    "parallelism": f"replicas x{world}: each rank renders its own sample range of the frame",
                    "scene_gen_s": round(gen_s, 3), "scene_load_s": round(load_s, 3), "bvh_build_s": round(scene.build_seconds, 3),
                    "tuning": tuned["chosen"]},
         "autotune": {"seconds": round(tune_s, 3), "workload": "the frame at its 64 spp per candidate (a warm-up and three timed renders, the median counts)",
                      "tried": tuned["tried"]},
         "mrays_per_s": world * rays / (total_ms / 1e3) / 1e6 if rank == 0 else None,
-        "roofline": {"kernel": "k_extend (nearest-hit traversal)", "bound": "hbm", "achieved": achieved, "peak": hbm_peak,
+        "roofline": {"kernel": "k_trace<EXTEND> (nearest-hit traversal)", "bound": "hbm", "achieved": achieved, "peak": hbm_peak,
                      "unit": "GB/s", "frac": achieved / hbm_peak, "peak_source": peak_src,
                      "traffic": DRAM_BYTES_PER_EXTEND_RAY * ext_rays / max(ext_launches, 1),
                      "traffic_note": "dram read + write bytes per extend launch: the ncu figure per ray (a 4 Mi-path "
