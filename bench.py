@@ -41,9 +41,9 @@ WORKLOAD = ("1080p product scene: 1920x1080, 64 spp, max depth 12, seeded displa
 DATA = "synthetic (seeded procedural scene; no dataset)"
 FALLBACK_HBM_GBS = 6650.0
 BYTES_RAY_IO = 32 + 12  # ray in, hit out
-# DRAM bytes (read + write) per extend ray, from one ncu capture of k_extend on this scene (round 0
-# of a 4 Mi-path wave: 341 MB for 4,147,200 rays). Scaled to a launch by the rays it traces.
-DRAM_BYTES_PER_EXTEND_RAY = 82.0
+# DRAM bytes (read + write) per extend ray, from one ncu capture of k_trace<EXTEND> on this scene (round 0
+# of a 4 Mi-path wave: 588 MB for 4,147,200 rays). Scaled to a launch by the rays it traces.
+DRAM_BYTES_PER_EXTEND_RAY = 142.0
 
 
 def peaks():
