@@ -22,8 +22,8 @@
 namespace rtg {
 namespace {
 
-// Bytes per path of the structure-of-arrays state (PathBuffers): o, d, thr, sum, sel, hit, sh_o,
-// sh_d, sh_c (16 each), medium, queue[0], queue[1], sorted, key (4 each); then the
+// Bytes per path of the state (PathBuffers): the records of 64 and 32 bytes, sh_o, sh_d, sh_c
+// (16 each), medium, queue[0], queue[1], sorted, key (4 each); then the
 // first-hit albedo of each path (16), which a film with fused guides adds to its guide sums.
 constexpr size_t kBytesPerPath = 10 * 16 + 5 * 4;
 constexpr size_t kPaths = RTG_NOALLOC_MAX_PATHS;
