@@ -3,6 +3,7 @@
 #pragma once
 #include <vector_types.h>
 
+#include <cstddef>
 #include <cstdint>
 
 #include "rtg_bsdf.cuh"
@@ -50,6 +51,7 @@ struct alignas(16) BlasInst {
     uint32_t flags;       // bit 0 one-sided, bit 1 hidden to camera rays
     float box[8];         // its world box: lower corner in [0, 3), upper in [4, 7)
 };
+static_assert(sizeof(BlasInst) == 96 && offsetof(BlasInst, box) == 64, "the box is read in one 32-byte load");
 
 // Per instance, what hit details and shading read.
 struct alignas(16) DevInstance {

@@ -500,7 +500,7 @@ struct SahBuilder {
 
 // Splits the builder's leaves into runs of at most `most` primitives with boxes of their own (the best
 // of all splits in centroid order, as a leaf holds eight at most): a ray then tests the triangles it
-// passes near, not a whole leaf. The primitives keep their leaf, whose box decides hits (hit_kept). A
+// passes near, not a whole leaf. The primitives keep their leaf, whose box decides hits (box_kept). A
 // run's box is grown by 2^-12 of its size, inside its leaf's: the triangle test's t is rounded, and
 // where it lies on the far side of a tight box's plane the reference, which looks at the leaf's box
 // only, still counts the hit.

@@ -4,12 +4,12 @@
 //
 // The answer of a nearest-hit query is the smallest (t, instance, triangle) in lexicographic
 // order over the triangles the ray meets in [t_min, t_max] whose enclosing boxes pass the
-// reference's slab test. Those boxes are conservative except where a computed t lies within its
-// rounding of t_min: a ray that starts within about 1e-3 of a large axis-aligned quad can see its
-// flat box end just before t_min while the triangle test alone would accept the hit, and the
-// reference drops that hit. So the tree is walked with a cheaper slab test that passes every box
-// the reference's passes (and a few more), and a hit whose t is that close to t_min is put to the
-// reference's own test of its leaf's exact box (hit_kept).
+// reference's slab test. Those boxes are not always conservative: a computed t may lie inside the
+// interval while its triangle's flat box begins past t_max or ends before t_min, and the reference
+// drops that hit. So the tree is walked with a cheaper slab test that passes every box the
+// reference's passes (and a few more), and a leaf's first hit puts the leaf's exact box to the
+// reference's own test (box_kept); an instance's world box is put to it before its tree is walked.
+// Boxes further up contain these, and rounding is monotonic, so they pass when these pass.
 #pragma once
 #include "rtg_dev.h"
 
@@ -134,6 +134,7 @@ struct Trav {
 };
 constexpr uint32_t BLAS_MOVED = 4u;  // its ray is in a transformed instance's object space
 
+constexpr float INV_MOST = 1.152921504606847e18f;  // 2^60
 // Sets the state's ray. The slab test's reciprocals are clamped to 2^60 times the major axis's, so
 // that a zero component gives no 0 x inf: such an axis then bounds t by planes 2^60 times as far as
 // the ray's major axis goes, which only a box the origin's coordinate lies outside of can fail.
@@ -145,7 +146,7 @@ RTG_D void trav_ray(Trav& T, V3 o, V3 d) {
                 dy = kz == 0 ? d.z : (kz == 1 ? d.x : d.y);
     const float sz = kz == 0 ? i0 : (kz == 1 ? i1 : i2);
     T.org[0] = o.x; T.org[1] = o.y; T.org[2] = o.z;
-    const float most = absf(sz) * 1.152921504606847e18f;
+    const float most = absf(sz) * INV_MOST;
     T.inv[0] = copysign_(smin_(absf(i0), most), i0);
     T.inv[1] = copysign_(smin_(absf(i1), most), i1);
     T.inv[2] = copysign_(smin_(absf(i2), most), i2);
@@ -172,35 +173,59 @@ RTG_D bool trav_init(const SceneDev& S, Trav& T, V3 o, V3 d, float tmin, float t
     return true;
 }
 
-// The reference's slab test of one box with the ray (o, d) from tmin on, its operations in its order
-// (traverse.rs:184).
-RTG_D bool box_passes(const float* __restrict__ box, V3 o, V3 d, float tmin) {
-    const float org[3] = {o.x, o.y, o.z}, inv[3] = {__frcp_rn(d.x), __frcp_rn(d.y), __frcp_rn(d.z)};
-    float n = tmin, f = F_MAX;
-    for (int a = 0; a < 3; ++a) {
-        const bool neg = signbitf(inv[a]);
-        const float lo = __ldg(box + a), hi = __ldg(box + 4 + a);
-        n = smax_(((neg ? hi : lo) - org[a]) * inv[a], n);
-        f = smin_(((neg ? lo : hi) - org[a]) * inv[a], f);
+// 32 bytes, a whole sector, in one load.
+RTG_D void load32(const void* p, uint32_t v[8]) {
+#ifdef __CUDA_ARCH__
+    uint64_t d[4];
+    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(d[0]), "=l"(d[1]), "=l"(d[2]), "=l"(d[3]) : "l"(p));
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        v[2 * k] = (uint32_t)d[k];
+        v[2 * k + 1] = (uint32_t)(d[k] >> 32);
     }
+#else
+    std::memcpy(v, p, 32);
+#endif
+}
+// The reference's slab test of the box [lo, hi] over [tmin, tmax], its operations in its order
+// (traverse.rs:184).
+RTG_D bool slab_passes(V3 lo, V3 hi, V3 org, V3 inv, float tmin, float tmax) {
+    float n = tmin, f = tmax;
+    const auto axis = [&](float l, float h, float o, float i) {
+        const bool neg = signbitf(i);
+        n = smax_(((neg ? h : l) - o) * i, n);
+        f = smin_(((neg ? l : h) - o) * i, f);
+    };
+    axis(lo.x, hi.x, org.x, inv.x);
+    axis(lo.y, hi.y, org.y, inv.y);
+    axis(lo.z, hi.z, org.z, inv.z);
     return n <= f * RTG_ROBUST;
 }
-// Whether the reference's boxes keep a hit of leaf `leaf` near the start of the query's interval: the
-// leaf's exact box with the ray of its tree and, in a transformed instance, the instance's world box
-// with the world ray (o, d). Boxes further up contain these, and rounding is monotonic, so they
-// pass when these pass.
-RTG_D_NI bool hit_kept(const BlasInst* __restrict__ blases, const float* __restrict__ leaf_boxes, V3 o, V3 d, uint32_t blas, uint32_t leaf,
-                       float tmin) {
-    if (blas & BLAS_MOVED) {
-        const BlasInst* bi = blases + (blas >> 3);
-        if (!box_passes(bi->box, o, d, tmin)) return false;
+// The same for a ray with a clamped reciprocal (trav_ray), from its direction: the query's, `d`,
+// taken into the tree of `blas`. Out of line: such rays run almost along a plane of the axes.
+RTG_D_NI bool slab_passes_axial(const BlasInst* __restrict__ blases, V3 lo, V3 hi, V3 org, V3 d, uint32_t blas, float tmin, float tmax) {
+    if (blas != TLAS_LEVEL && (blas & BLAS_MOVED)) {
         float m[12];
-        for (int k = 0; k < 12; ++k) m[k] = __ldg(&bi->to_local[k]);
-        const V3 lo = xf_point(m, o), ld = xf_vector(m, d);
-        o = lo;
-        d = ld;
+        for (int k = 0; k < 12; ++k) m[k] = __ldg(&blases[blas >> 3].to_local[k]);
+        d = xf_vector(m, d);
     }
-    return box_passes(leaf_boxes + 8 * (size_t)leaf, o, d, tmin);
+    return slab_passes(lo, hi, org, v3(__frcp_rn(d.x), __frcp_rn(d.y), __frcp_rn(d.z)), tmin, tmax);
+}
+// Whether the reference's slab test passes the box at `at` (lower corner in [0, 3), upper in [4, 7))
+// for the ray of the tree being walked.
+template <class Src>
+RTG_D bool box_kept(const SceneDev& S, const Trav& T, const float* at, float tmin, float tmax, const Src& src) {
+    uint32_t v[8];
+    load32(at, v);
+    const V3 lo = v3(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]));
+    const V3 hi = v3(__uint_as_float(v[4]), __uint_as_float(v[5]), __uint_as_float(v[6]));
+    const V3 org = v3(T.org[0], T.org[1], T.org[2]), inv = v3(T.inv[0], T.inv[1], T.inv[2]);
+    if (!(fmaxf(fmaxf(absf(inv.x), absf(inv.y)), absf(inv.z)) < absf(T.sz) * INV_MOST)) {
+        V3 o, d;
+        src(o, d);
+        return slab_passes_axial(S.blas, lo, hi, org, d, T.blas, tmin, tmax);
+    }
+    return slab_passes(lo, hi, org, inv, tmin, tmax);
 }
 
 // Child `c` of a node whose first `inner` children are nodes: their index, or a leaf reference.
@@ -216,19 +241,6 @@ struct NodeHead {
 struct NodePlanes {
     uint32_t w[12], off_lo, off_hi, inner;
 };
-RTG_D void load32(const void* p, uint32_t v[8]) {
-#ifdef __CUDA_ARCH__
-    uint64_t d[4];
-    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(d[0]), "=l"(d[1]), "=l"(d[2]), "=l"(d[3]) : "l"(p));
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        v[2 * k] = (uint32_t)d[k];
-        v[2 * k + 1] = (uint32_t)(d[k] >> 32);
-    }
-#else
-    std::memcpy(v, p, 32);
-#endif
-}
 RTG_D NodeHead load_head(const QNode* node) {
     uint32_t v[8];
     load32(node, v);
@@ -409,7 +421,7 @@ RTG_D bool trav_leaf(const SceneDev& S, Trav& T, float tmin, Stack& stack, uint3
         if (T.blas == TLAS_LEVEL) {
             const BlasInst* bi = S.blas + k;
             const uint4 b = load_blas(bi);  // root, identity, instance, flags
-            if (!(T.camera && (b.w & 2u))) {
+            if (!(T.camera && (b.w & 2u)) && (b.y || box_kept(S, T, bi->box, tmin, T.best_t, src))) {
                 if (T.sp + 1 > STACK_CAP) { *err |= 1u; hit = false; return true; }
                 stack.put(T.sp++, stack_key(0.0f, STACK_RETURN));
                 T.blas = (k << 3) | (b.w & 3u);
@@ -426,6 +438,8 @@ RTG_D bool trav_leaf(const SceneDev& S, Trav& T, float tmin, Stack& stack, uint3
                 return false;
             }
         } else {
+            const float range = T.best_t;  // what the reference holds the leaf's box against
+            bool kept = false;
             uint32_t flags;
             do {
                 const float4* tr = reinterpret_cast<const float4*>(S.tris + k);
@@ -463,16 +477,8 @@ RTG_D bool trav_leaf(const SceneDev& S, Trav& T, float tmin, Stack& stack, uint3
                     if (inst == 0xffffffffu) inst = __ldg(&S.blas[T.blas >> 3].instance);
                     if (!(t < T.best_t || inst < T.best_i || (inst == T.best_i && __float_as_uint(a.w) < __ldg(&S.tris[T.best_k].tri)))) continue;
                 }
-                // Within the rounding of t (a generous 2^-14 of the corners' distances) of t_min, the
-                // reference's boxes decide; and where t may be negative, which turns its factor
-                // 1 + 4 eps against the far planes. (At the far end they only cull what a nearer hit,
-                // computed in whatever order, hides: there the nearest of the hits stands.)
-                const float near = (absf(az) + absf(bz) + absf(cz)) * 6.103515625e-5f;
-                if (!(t - tmin > near) || (!POS && tmin <= 0.0f)) {
-                    V3 o, d;
-                    src(o, d);
-                    if (!hit_kept(S.blas, S.leaf_boxes, o, d, T.blas, flags >> TRI_LEAF_SHIFT, tmin)) continue;
-                }
+                if (!kept && !box_kept(S, T, S.leaf_boxes + 8 * (size_t)(flags >> TRI_LEAF_SHIFT), tmin, range, src)) break;
+                kept = true;
                 if (any) { hit = true; return true; }
                 T.best_t = t;
                 T.best_i = inst;
