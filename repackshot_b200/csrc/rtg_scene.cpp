@@ -374,7 +374,7 @@ Box instance_box(const HMesh& m, const Xf& x) {
 
 // ---- binned SAH build (geometry/bvh.rs:246-420) ------------------------------------------------
 constexpr int BINS = 16;
-struct BNode { Box box; uint32_t left = 0, right = 0, first = 0, count = 0, leaf = 0; };  // leaf: the builder's leaf it is in
+struct BNode { Box box; uint32_t left = 0, right = 0, first = 0, count = 0; };
 struct SahBuilder {
     const std::vector<Box>& boxes;
     const std::vector<V3>& cents;
@@ -498,76 +498,6 @@ struct SahBuilder {
     }
 };
 
-// Splits the builder's leaves into runs of at most `most` primitives with boxes of their own (the best
-// of all splits in centroid order, as a leaf holds eight at most): a ray then tests the triangles it
-// passes near, not a whole leaf. The primitives keep their leaf, whose box decides hits (box_kept). A
-// run's box is grown by 2^-12 of its size, inside its leaf's: the triangle test's t is rounded, and
-// where it lies on the far side of a tight box's plane the reference, which looks at the leaf's box
-// only, still counts the hit.
-// Whole leaves, runs of 3, 2 and 1: 1080p product frame 164.4, 161.1, 158.8 and 171.4 ms, instanced
-// frame 37.1, 35.6, 34.8 and 34.7 ms, studio still 19.3, 18.9, 18.9 and 19.3 ms.
-constexpr uint32_t LEAF_RUN = 2;
-struct LeafSplitter {
-    SahBuilder& sb;
-    uint32_t most;
-    void run() {
-        const size_t n = sb.nodes.size();
-        for (size_t k = 0; k < n; ++k) {
-            sb.nodes[k].leaf = (uint32_t)k;
-            if (sb.nodes[k].count > most) split((uint32_t)k);
-        }
-    }
-    void split(uint32_t at) {
-        const uint32_t b = sb.nodes[at].first, n = sb.nodes[at].count;
-        uint32_t* o = sb.order.data() + b;
-        uint32_t best[16], order[16];
-        Box lo[16], hi[16];
-        float cost = f_inf();
-        uint32_t cut = n / 2;
-        std::copy(o, o + n, best);
-        for (int a = 0; a < 3; ++a) {
-            std::copy(o, o + n, order);
-            std::sort(order, order + n, [&](uint32_t x, uint32_t y) {
-                const float cx = comp(sb.cents[x], a), cy = comp(sb.cents[y], a);
-                return cx < cy || (cx == cy && x < y);
-            });
-            lo[0] = sb.boxes[order[0]];
-            for (uint32_t k = 1; k < n; ++k) lo[k] = lo[k - 1].uni(sb.boxes[order[k]]);
-            hi[n - 1] = sb.boxes[order[n - 1]];
-            for (uint32_t k = n - 1; k-- > 0;) hi[k] = hi[k + 1].uni(sb.boxes[order[k]]);
-            for (uint32_t k = 1; k < n; ++k) {
-                const float c = lo[k - 1].area() * (float)k + hi[k].area() * (float)(n - k);
-                if (c < cost) {
-                    cost = c;
-                    cut = k;
-                    std::copy(order, order + n, best);
-                }
-            }
-        }
-        std::copy(best, best + n, o);
-        const uint32_t leaf = sb.nodes[at].leaf;
-        for (int side = 0; side < 2; ++side) {
-            BNode c;
-            c.first = side ? b + cut : b;
-            c.count = side ? n - cut : cut;
-            c.leaf = leaf;
-            for (uint32_t k = 0; k < c.count; ++k) c.box = c.box.uni(sb.boxes[sb.order[c.first + k]]);
-            const V3 size = c.box.hi - c.box.lo;
-            const float pad = rmax(rmax(size.x, size.y), size.z) * (1.0f / 4096.0f);
-            const Box& in = sb.nodes[leaf].box;
-            c.box.lo = v3(rmax(c.box.lo.x - pad, in.lo.x), rmax(c.box.lo.y - pad, in.lo.y), rmax(c.box.lo.z - pad, in.lo.z));
-            c.box.hi = v3(rmin(c.box.hi.x + pad, in.hi.x), rmin(c.box.hi.y + pad, in.hi.y), rmin(c.box.hi.z + pad, in.hi.z));
-            const uint32_t index = (uint32_t)sb.nodes.size();
-            sb.nodes.push_back(c);
-            if (side) sb.nodes[at].right = index;
-            else sb.nodes[at].left = index;
-        }
-        sb.nodes[at].count = 0;
-        for (uint32_t c : {sb.nodes[at].left, sb.nodes[at].right})
-            if (sb.nodes[c].count > most) split(c);
-    }
-};
-
 // ---- 8-wide collapse and quantisation ---------------------------------------------------------------
 // The binary tree's leaves are the wide tree's; which of its inner nodes become wide nodes is chosen
 // for the smallest total surface area of the wide nodes, the expected number of node steps of a ray
@@ -579,7 +509,7 @@ struct Flattener {
     const std::vector<BNode>* bn = nullptr;
     const std::vector<uint32_t>* order = nullptr;
     // Appends a leaf's primitives: the index of the first.
-    std::function<uint32_t(const uint32_t*, uint32_t, uint32_t)> emit;  // (primitives, count, builder's leaf)
+    std::function<uint32_t(const uint32_t*, uint32_t, const Box&)> emit;
     uint32_t max_depth = 0;
     uint32_t dummy = 0;  // what the empty slots of a node without leaves lead to
     // Always open the child with the largest box instead: a shallower tree where the least area goes
@@ -681,7 +611,7 @@ struct Flattener {
     // Emits the tree under binary node 0: the reference of its root.
     uint32_t flatten() {
         max_depth = 0;
-        if ((*bn)[0].count > 0) return make_leaf(emit(order->data() + (*bn)[0].first, (*bn)[0].count, (*bn)[0].leaf));
+        if ((*bn)[0].count > 0) return make_leaf(emit(order->data() + (*bn)[0].first, (*bn)[0].count, (*bn)[0].box));
         if (!widest) choose();
         const uint32_t root = (uint32_t)F.nodes.size();
         F.nodes.push_back(QNode());
@@ -710,7 +640,7 @@ struct Flattener {
                 q.off[q.inner++] = (uint8_t)s;
                 continue;
             }
-            const uint32_t first = emit(order->data() + k.first, k.count, k.leaf);
+            const uint32_t first = emit(order->data() + k.first, k.count, k.box);
             if (s == (int)q.inner) q.leaf_base = first;
             q.off[s] = (uint8_t)(first - q.leaf_base);
         }
@@ -1177,18 +1107,11 @@ static bool flatten(const HScene& s, Flat& F, std::string& error, bool geometry,
         bool any_normals = false;
         for (const HMesh& M : s.meshes) any_normals |= !M.normals.empty();
         if (any_normals) F.tri_normals.assign(12, 0.0f);
-        // Appends the run of the triangles `p` as record(p), of mesh(p), gives them, all of the builder's
-        // leaf `of`, whose number and box are kept once.
-        std::vector<uint32_t> leaf_number;
-        auto emit_leaf = [&](const uint32_t* p, uint32_t n, uint32_t of, auto&& record, auto&& mesh) {
-            const uint32_t first = (uint32_t)F.tris.size();
-            if (leaf_number.size() != fl.bn->size()) leaf_number.assign(fl.bn->size(), 0);
-            if (!leaf_number[of]) {
-                leaf_number[of] = (uint32_t)(F.leaf_boxes.size() / 8);
-                F.leaf_boxes.resize(F.leaf_boxes.size() + 8);
-                put_box(&F.leaf_boxes[8 * (size_t)leaf_number[of]], (*fl.bn)[of].box);
-            }
-            const uint32_t leaf = leaf_number[of];
+        // Appends the leaf of the triangles `p` as record(p), of mesh(p), gives them.
+        auto emit_leaf = [&](const uint32_t* p, uint32_t n, const Box& box, auto&& record, auto&& mesh) {
+            const uint32_t first = (uint32_t)F.tris.size(), leaf = (uint32_t)(F.leaf_boxes.size() / 8);
+            F.leaf_boxes.resize(F.leaf_boxes.size() + 8);
+            put_box(&F.leaf_boxes[8 * (size_t)leaf], box);
             for (uint32_t k = 0; k < n; ++k) {
                 TriRec r = record(p[k]);
                 r.flags |= (leaf << TRI_LEAF_SHIFT) | (k + 1 == n ? TRI_LAST : 0u);
@@ -1237,13 +1160,11 @@ static bool flatten(const HScene& s, Flat& F, std::string& error, bool geometry,
                 if (any_normals) F.tri_normals.reserve(F.tri_normals.size() + 12 * prims.size());
                 SahBuilder sb{boxes, cents, 4, 8, {}, {}};
                 sb.run();
-                LeafSplitter{sb, LEAF_RUN}.run();
-                leaf_number.clear();
                 fl.bn = &sb.nodes;
                 fl.order = &sb.order;
-                fl.emit = [&](const uint32_t* p, uint32_t n, uint32_t of) {
+                fl.emit = [&](const uint32_t* p, uint32_t n, const Box& box) {
                     auto mesh = [&](uint32_t k) -> const HMesh& { return s.meshes[s.instances[prims[k].first].mesh]; };
-                    return emit_leaf(p, n, of, [&](uint32_t k) { return triangle(mesh(k), prims[k].second, prims[k].first, seen(prims[k].first)); }, mesh);
+                    return emit_leaf(p, n, box, [&](uint32_t k) { return triangle(mesh(k), prims[k].second, prims[k].first, seen(prims[k].first)); }, mesh);
                 };
                 BlasInst bi;
                 std::memset(&bi, 0, sizeof(bi));
@@ -1271,12 +1192,10 @@ static bool flatten(const HScene& s, Flat& F, std::string& error, bool geometry,
                 }
                 SahBuilder sb{boxes, cents, 4, 8, {}, {}};
                 sb.run();
-                LeafSplitter{sb, LEAF_RUN}.run();
-                leaf_number.clear();
                 fl.bn = &sb.nodes;
                 fl.order = &sb.order;
-                fl.emit = [&](const uint32_t* p, uint32_t cnt, uint32_t of) {
-                    return emit_leaf(p, cnt, of, [&](uint32_t t) { return triangle(M, t, 0xffffffffu, 0u); },
+                fl.emit = [&](const uint32_t* p, uint32_t cnt, const Box& box) {
+                    return emit_leaf(p, cnt, box, [&](uint32_t t) { return triangle(M, t, 0xffffffffu, 0u); },
                                      [&](uint32_t) -> const HMesh& { return M; });
                 };
                 mesh_root[m] = fl.flatten();
@@ -1307,7 +1226,7 @@ static bool flatten(const HScene& s, Flat& F, std::string& error, bool geometry,
             sb.run();
             fl.bn = &sb.nodes;
             fl.order = &sb.order;
-            fl.emit = [&](const uint32_t* p, uint32_t, uint32_t) {
+            fl.emit = [&](const uint32_t* p, uint32_t, const Box&) {
                 F.blas.push_back(placed[p[0]]);
                 return (uint32_t)F.blas.size() - 1;
             };
