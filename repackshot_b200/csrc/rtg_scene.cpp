@@ -559,6 +559,7 @@ struct Flattener {
         }
     }
 
+    // In the reference's order (bvh.rs:439): of children of one size the first is opened.
     void open_widest(uint32_t n, uint32_t* kids, int& nk) {
         kids[0] = (*bn)[n].left;
         kids[1] = (*bn)[n].right;
@@ -567,8 +568,10 @@ struct Flattener {
             for (int s = 0; s < nk; ++s)
                 if ((*bn)[kids[s]].count == 0 && (at < 0 || (*bn)[kids[s]].box.area() > (*bn)[kids[at]].box.area())) at = s;
             if (at < 0) break;
-            kids[nk] = (*bn)[kids[at]].right;
-            kids[at] = (*bn)[kids[at]].left;
+            const BNode& opened = (*bn)[kids[at]];
+            for (int s = nk; s > at + 1; --s) kids[s] = kids[s - 1];
+            kids[at] = opened.left;
+            kids[at + 1] = opened.right;
         }
     }
 
@@ -1233,6 +1236,7 @@ static bool flatten(const HScene& s, Flat& F, std::string& error, bool geometry,
             F.tlas_root = fl.flatten();
             tlas_depth = fl.max_depth;
         }
+        // Seven entries a level whatever the nodes hold, as an empty slot may pass by rounding (QNode).
         F.stack_need = 7 * (tlas_depth + blas_depth) + 2;
         if (F.stack_need > 96 && !widest) return flatten(s, F, error, geometry, true);
         if (F.stack_need > 96) { error = "unsupported: BVH too deep for the traversal stack"; return false; }
