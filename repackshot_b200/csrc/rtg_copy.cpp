@@ -65,7 +65,8 @@ cudaError_t copy_planes(const CopyPart* parts, int n, bool to_device, cudaStream
     }
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     int device = 0;
-    if (total < LEAST || !ours || cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone ||
+    // cudaStreamPerThread names another stream in each thread: its order is the calling thread's alone.
+    if (total < LEAST || !ours || stream == cudaStreamPerThread || cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone ||
         cudaGetDevice(&device) != cudaSuccess) {
         cudaGetLastError();
         return plain(parts, n, to_device, stream);
