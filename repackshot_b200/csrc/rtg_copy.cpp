@@ -10,7 +10,7 @@
 #include <atomic>
 #include <cstdint>
 #include <cstring>
-#include <system_error>
+#include <exception>
 #include <thread>
 
 namespace rtg {
@@ -132,7 +132,7 @@ cudaError_t copy_planes(const CopyPart* parts, int n, bool to_device, cudaStream
     for (int k = 1; k < LANES; ++k) {
         try {
             more[k - 1] = std::thread(lane, k);
-        } catch (const std::system_error&) {
+        } catch (const std::exception&) {  // no thread, or no memory for one
             break;  // the other lanes take its pieces
         }
     }

@@ -22,3 +22,8 @@ def copies(tmp_path_factory):
 def test_copies_arrive_in_the_streams_order(copies, mode, size):
     r = subprocess.run([str(copies), mode, str(size)], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout.strip() == "0", (r.returncode, r.stdout, r.stderr)
+
+
+def test_no_memory_for_the_threads(copies):
+    r = subprocess.run([str(copies), "no-memory"], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout.strip() == "0", (r.returncode, r.stdout, r.stderr)
