@@ -71,10 +71,17 @@ cudaError_t copy_planes(const CopyPart* parts, int n, bool to_device, cudaStream
         cudaGetLastError();
         return plain(parts, n, to_device, stream);
     }
+    if (!g_pinned) {
+        // A read takes no memory otherwise, and may go on beside another thread's capture: so in the mode
+        // that an allocation does not break one in.
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (cudaHostAlloc((void**)&g_pinned, 2 * LANES * SLOT, cudaHostAllocPortable) != cudaSuccess) g_pinned = nullptr;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+    }
     Events ev;
     // A stream of another device takes no event of this one.
-    if ((!g_pinned && cudaHostAlloc((void**)&g_pinned, 2 * LANES * SLOT, cudaHostAllocPortable) != cudaSuccess) || !ev.create() ||
-        cudaEventRecord(ev.e[0], stream) != cudaSuccess) {
+    if (!g_pinned || !ev.create() || cudaEventRecord(ev.e[0], stream) != cudaSuccess) {
         cudaGetLastError();
         return plain(parts, n, to_device, stream);
     }

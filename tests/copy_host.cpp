@@ -46,6 +46,11 @@ void drain(const std::pair<cudaStream_t, std::thread::id>& s) {
 }
 }  // namespace
 
+// Another thread captures a stream of its own in the global mode: an allocation outside the relaxed mode
+// breaks that capture.
+static bool g_captured_elsewhere = false, g_capture_broken = false;
+static thread_local cudaStreamCaptureMode t_capture_mode = cudaStreamCaptureModeGlobal;
+
 // Memory for threads runs out on request; this program's own bookkeeping keeps its.
 static thread_local bool t_mine = false;
 struct Mine {
@@ -100,7 +105,12 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) {
     return cudaSuccess;
 }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode* mode) {
+    std::swap(t_capture_mode, *mode);
+    return cudaSuccess;
+}
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
+    if (t_capture_mode != cudaStreamCaptureModeRelaxed) g_capture_broken = g_captured_elsewhere;
     *p = std::malloc(n);
     return cudaSuccess;
 }
@@ -123,6 +133,7 @@ int main(int argc, char** argv) {
     const std::string mode = argc > 1 ? argv[1] : "stream";
     const size_t n = argc > 2 ? std::strtoull(argv[2], nullptr, 10) : (9u << 20) + 12345;
     const cudaStream_t stream = mode == "per-thread" ? cudaStreamPerThread : (cudaStream_t)(uintptr_t)64;
+    g_captured_elsewhere = mode == "captured-elsewhere";
     size_t wrong = 0;
     for (const bool to_device : {false, true}) {
         std::vector<uint8_t> from(n, 1), to(n, 0);
@@ -139,6 +150,7 @@ int main(int argc, char** argv) {
         for (size_t k = 0; k < n; ++k) wrong += to[k] != (uint8_t)(k * 7 + k / 251);
     }
     rtg::copy_release();
+    if (g_capture_broken || t_capture_mode != cudaStreamCaptureModeGlobal) return 3;
     std::printf("%zu\n", wrong);
     return 0;
 }

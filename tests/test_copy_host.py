@@ -27,3 +27,8 @@ def test_copies_arrive_in_the_streams_order(copies, mode, size):
 def test_no_memory_for_the_threads(copies):
     r = subprocess.run([str(copies), "no-memory"], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout.strip() == "0", (r.returncode, r.stdout, r.stderr)
+
+
+def test_another_threads_capture_goes_on(copies):
+    r = subprocess.run([str(copies), "captured-elsewhere"], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout.strip() == "0", (r.returncode, r.stdout, r.stderr)
