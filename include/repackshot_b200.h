@@ -378,7 +378,8 @@ uint32_t rtg_render_tile_alpha(uint32_t handle, uint32_t x, uint32_t y, uint32_t
  * RTG_STATUS_NULL_POINTER, or RTG_STATUS_BAD_DENOISE when the preset, the sizes, the band or its
  * halo do not fit. The filter runs on the GPU with the reference's bits. The library keeps the
  * call's device memory, up to 256 MB, and 8 MB of pinned memory for the next one; freeing the last
- * scene gives both back, and the device memory goes to any allocation that does not fit beside it. */
+ * scene or rtg_release_memory gives both back, and the device memory goes to any allocation that
+ * does not fit beside it. */
 uint32_t rtg_denoise(uint32_t width, uint32_t height, uint32_t origin_y, uint32_t rows, uint32_t samples, uint32_t y0, uint32_t y1,
                      const uint8_t* in, float* out);
 uint32_t rtg_denoise_with(uint32_t preset, float strength, uint32_t width, uint32_t height, uint32_t origin_y, uint32_t rows, uint32_t samples,
@@ -386,6 +387,9 @@ uint32_t rtg_denoise_with(uint32_t preset, float strength, uint32_t width, uint3
 /* rt_denoise_halo (ffi.rs:685-691): rows a band of `preset` holds above and below the rows it
  * computes (72 for the full filter, 24 for the viewport's), 0 for an unknown preset. */
 uint32_t rtg_denoise_halo(uint32_t preset);
+/* Gives back what the library keeps between calls of these entries and of the film reads (no
+ * counterpart in the reference); the next call takes it again. */
+uint32_t rtg_release_memory(void);
 /* No counterpart in the reference (its hosts render the passes tile by tile and hand the planes
  * to rt_denoise): the guide passes of a film on the device. Writes the exact passes of the film's
  * pixels and adds the albedo of samples [first_sample, first_sample + count) to the film's albedo

@@ -89,6 +89,7 @@ ABI = {
     "rtg_denoise": (_u32, [_u32, _u32, _u32, _u32, _u32, _u32, _u32, _f, _f]),
     "rtg_denoise_with": (_u32, [_u32, ctypes.c_float, _u32, _u32, _u32, _u32, _u32, _u32, _u32, _f, _f]),
     "rtg_denoise_halo": (_u32, [_u32]),
+    "rtg_release_memory": (_u32, []),
     "rtg_film_guides": (_u32, [_u32, _u32, _u32, _u32]),
     "rtg_film_guides_fused": (_u32, [_u32, _u32, _u32]),
     "rtg_film_denoise": (_u32, [_u32, _u32, ctypes.c_float, _u32, _f]),
@@ -419,6 +420,11 @@ def denoise(words, width: int, height: int, samples: int, preset: int = 0, stren
     out = np.zeros(max((y1 - y0) * width * 4, 1), np.float32)
     _check(lib().rtg_denoise_with(preset, float(strength), width, height, origin_y, rows, samples, y0, y1, _ptr(words), _ptr(out)))
     return out[:(y1 - y0) * width * 4]
+
+
+def release_memory():
+    """Gives back the device and pinned memory that the library keeps between calls (denoise and reads)."""
+    _check(lib().rtg_release_memory())
 
 
 def tile_passes(handle: int, x: int, y: int, w: int, h: int, mask: int = 0x3E):

@@ -50,8 +50,8 @@ struct DevBuf {
 };
 
 // The device block a call on host planes leaves for the next one (allocating and freeing 130 MB takes
-// 3 to 5 ms): at most KEPT_MOST bytes, given back with the last scene and to an allocation that
-// does not fit beside it. Every call on it has ended with a synchronous copy.
+// 3 to 5 ms): at most KEPT_MOST bytes, given back with the last scene, on request (a process may
+// denoise without scenes) and to an allocation that does not fit beside it. Every call on it has ended with a synchronous copy.
 constexpr size_t KEPT_MOST = 256u << 20;
 DevBuf g_kept;
 int g_kept_device = -1;
@@ -89,6 +89,11 @@ void lent_return(DevBuf& b) {
         b = DevBuf{};
     }
     b.release();
+}
+
+void release_kept() {
+    g_kept.release();
+    copy_release();
 }
 
 // Device buffers released together.
@@ -1009,10 +1014,13 @@ uint32_t rtg_scene_free(uint32_t handle) {
     const bool window = sc->order.l2_persist != 0;
     g_scenes[handle - 1].reset();
     if (window) release_set_aside(dev, nullptr);
-    if (std::none_of(g_scenes.begin(), g_scenes.end(), [](const auto& s) { return s != nullptr; })) {
-        g_kept.release();
-        copy_release();
-    }
+    if (std::none_of(g_scenes.begin(), g_scenes.end(), [](const auto& s) { return s != nullptr; })) release_kept();
+    return RTG_STATUS_OK;
+}
+
+uint32_t rtg_release_memory(void) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    release_kept();
     return RTG_STATUS_OK;
 }
 
