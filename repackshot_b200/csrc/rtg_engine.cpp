@@ -920,7 +920,7 @@ uint32_t rtg_scene_load(const uint8_t* bytes, uint32_t len) {
     sc->bitmaps = std::move(hs.bitmaps);
     sc->build_seconds = F.build_seconds;
     sc->nodes = F.nodes.size();
-    sc->tris = F.tris.size();
+    sc->tris = F.leaf_triangles;
     sc->instanced_triangles = F.instanced_triangles;
     sc->width = F.scene.width;
     sc->height = F.scene.height;
@@ -975,7 +975,7 @@ uint32_t rtg_scene_update(uint32_t handle, const uint8_t* bytes, uint32_t len) {
         sc->geometry.release();
         sc->geometry = std::move(geometry);
         sc->nodes = F.nodes.size();
-        sc->tris = F.tris.size();
+        sc->tris = F.leaf_triangles;
         sc->build_seconds = F.build_seconds;
     }
     sc->shading.release();

@@ -1240,7 +1240,8 @@ static bool flatten(const HScene& s, Flat& F, std::string& error, bool geometry,
         F.stack_need = 7 * (tlas_depth + blas_depth) + 2;
         if (F.stack_need > 96 && !widest) return flatten(s, F, error, geometry, true);
         if (F.stack_need > 96) { error = "unsupported: BVH too deep for the traversal stack"; return false; }
-        if (F.tris.size() >= (1u << 27) - 16) { error = "unsupported: more than 2^27 triangles"; return false; }
+        F.leaf_triangles = F.tris.size() - 1;
+        if (F.leaf_triangles >= (1u << 27) - 16) { error = "unsupported: more than 2^27 triangles"; return false; }
     }
     if (!prepare_lights(s, scene_box, F.lights, F, error)) return false;
 

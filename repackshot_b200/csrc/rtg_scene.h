@@ -153,6 +153,7 @@ struct Flat {
     uint32_t stack_need = 0;
     float box_lo[3] = {0, 0, 0}, box_hi[3] = {0, 0, 0};  // the ray sort's box (empty: lo > hi)
     uint64_t instanced_triangles = 0;
+    uint64_t leaf_triangles = 0;  // of the trees: `tris` without its empty first one
     double build_seconds = 0;
 };
 // Builds the BVHs and the device layout. Returns false with `error` when a limit is exceeded.
