@@ -269,8 +269,11 @@ RTG_D uint4 load_blas(const BlasInst* bi) { return __ldg(reinterpret_cast<const 
 // Slab planes of one axis for a node: t of the plane of byte q is fma(1 + q 2^-15, a, b). The byte
 // becomes 1 + q 2^-15 by one permute into the second-lowest byte of 1.0f's pattern, so a plane
 // costs two instructions. The near planes take `b_near` and the far ones `b_far`, moved apart by
-// 2^-20 |m| + 2^-21 |a|: at least four times what the roundings here and in the reference's test
-// (its factor 1 + 4 eps included) can move a plane, so every box that test passes, this one passes.
+// 2^-19 |m| + 2^-21 |a|, so that every box the reference's test passes, this one passes: with u =
+// 2^-24, the roundings here are at most 5u |m| + 2.1u |a| (two in m, one each in b, in the pad's sum and
+// in the plane's), those of the reference's plane 2u |t|, and its factor 1 + 4 eps with its own
+// rounding moves a far plane by 9u |t| more, where |t| <= |m| + |a| / 128: 16u |m| + 2.2u |a| in all, of a
+// pad of 32u |m| + 8u |a|. (Of half the |m| term random planes needed up to 0.82.)
 struct AxisPlanes {
     float a, b_near, b_far;
     uint32_t n0, n1, f0, f1;  // the near and far planes' bytes
@@ -280,7 +283,7 @@ RTG_D AxisPlanes axis_planes(float p, float scale, float org, float inv, uint32_
     const float m = (p - org) * inv;
     x.a = scale * inv;
     const float b = m - x.a;
-    const float pad = __fmaf_rn(absf(x.a), 4.76837158203125e-7f, absf(m) * 9.5367431640625e-7f);
+    const float pad = __fmaf_rn(absf(x.a), 4.76837158203125e-7f, absf(m) * 1.9073486328125e-6f);
     x.b_near = b - pad;
     x.b_far = b + pad;
     const bool neg = inv < 0.0f;
