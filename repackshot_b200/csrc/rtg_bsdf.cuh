@@ -140,7 +140,7 @@ RTG_HD TabAt tab_at(float x) {
     locate(sqrt_(rmax(x, 0.0f)), NODES_MU, t.i, t.w);
     return t;
 }
-// The four u16 corners of a cell. On the device the tables are stored cell by cell (device_cells),
+// The four u16 corners of a cell. On the device the tables are stored cell by cell (device_init),
 // so that a lookup is one 8-byte load.
 RTG_HD void tab_cell(const uint16_t* t, int slice, int j, int i, float v[4]) {
 #ifdef __CUDA_ARCH__

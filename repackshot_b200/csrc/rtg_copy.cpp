@@ -2,8 +2,10 @@
 // GB/s up, 20 GB/s down, 2 GB/s down into pages never touched, whatever the number of streams (52 MB
 // up in 2 to 16 slices on streams of their own: 4.3 to 4.9 ms; whole 4.4 to 4.9). Here LANES threads
 // each copy through two pinned slots of their own, one filled or emptied while the other is on its
-// way: 52 MB up 1.8 ms, 15 MB down into fresh pages 2.0 instead of 6.5 ms. 8 threads with slots of
-// 1 MB: 2.2 and 1.4 ms, with 512 KB: 2.4 and 1.3 ms.
+// way: 52 MB up 1.8 ms, 15 MB down into fresh pages 2.0 instead of 6.5 ms. 4 threads with slots of 1 MB, 8
+// with 1 MB and 8 with 512 KB: a denoiser call (both copies) 4.02, 4.34 and 4.94 ms, a film of 50 MB read
+// into fresh pages 3.8, 3.2 and 3.4 ms, into used ones 1.95, 1.85 and 2.3 ms. More threads down and fewer
+// up would suit both.
 #include "rtg_copy.h"
 
 #include <algorithm>

@@ -157,7 +157,7 @@ struct SceneDev {
     uint32_t any_passable, any_cutout;
     // The common scene: area lights and the ramp environment only; no emissive, cut-out, absorbing,
     // thin, coated or anisotropic material; no floor plane, background image or section. The shade
-    // kernels have a variant for it (scene_plain).
+    // kernels have a variant for it (flatten_scene decides).
     uint32_t plain;
     uint32_t floor_mode;
     float floor_z;

@@ -15,6 +15,10 @@ namespace rtg {
 
 __constant__ SobolTable c_sobol;
 
+// Figures at a choice compare builds that differ in that one thing, at the time it was made; the 1080p
+// product frame (1 M triangles, 64 spp, depth 12) takes 157 ms now, the instanced frame (10 M triangles,
+// 4 spp) 36 ms.
+
 // Threads per block of the traversal kernels (the stride of their shared stacks).
 constexpr int TRACE_THREADS = 128;
 // RTG_REFILL_MIN (build setting): idle lanes a k_trace warp waits for before it takes new rays
@@ -24,10 +28,12 @@ constexpr int TRACE_THREADS = 128;
 #ifndef RTG_REFILL_MIN
 #define RTG_REFILL_MIN 8
 #endif
-// Blocks per SM the traversal kernels are compiled for (56 registers at 9, 64 at 8, no spills): more
-// warps hide the node fetches until registers spill. All kernels at 7, 8, 9 and 10 blocks: 1080p
-// product frame 154.4, 148.8, 145.8 and 150.6 ms, instanced frame 32.6, 31.7, 31.2 and 33.0 ms, adaptive
-// frame (thin rounds) 70.2 at 8, 71.8 at 9, 73.3 ms at 10. So the kernel of the smaller waves, which
+// Blocks per SM the traversal kernels are compiled for (56 registers at 9, 64 at 8; of the kernels in
+// use 12 bytes are spilled in EXTEND and in the two that walk): more warps hide the node fetches until
+// registers spill. All kernels at 7, 8, 9 and 10 blocks: 1080p product frame 154.4, 148.8, 145.8 and
+// 150.6 ms, instanced frame 32.6, 31.7, 31.2 and 33.0 ms, adaptive frame (thin rounds) 70.2 at 8, 71.8 at
+// 9, 73.3 ms at 10. (With each leaf's box held against its hits, at 8 and 9: 158.6 and 156.9, 37.6 and
+// 36.8 ms.) So the kernel of the smaller waves, which
 // traces both kinds of rays, takes 8 and the others 9. RTG_TRACE_MIN_BLOCKS (build setting): both.
 #ifdef RTG_TRACE_MIN_BLOCKS
 #define RTG_TRACE_BLOCKS(together) RTG_TRACE_MIN_BLOCKS
@@ -1456,8 +1462,8 @@ static bool walks_on(const SceneDev& S, bool batch) { return S.any_passable && !
 // Whether a wave of n paths traces each round's shadow rays with the next round's extension rays.
 // Timed waves trace them apart, so that the events are around extension rays only. So do waves of
 // more than 2^25 paths: their launches' ends weigh little, and shadow rays visit children in slot
-// order there, which needs no sort (132.7 M paths: 180.6 ms apart, 181.7 together; 8.4 M paths: 31.1
-// and 29.6; 0.9 M paths: 5.05 and 4.71).
+// order there, which needs no sort. 1080p product frame apart and together, ms: 8 Mi paths 14.6 and 13.6,
+// 16 Mi 24.6 and 23.6, 32 Mi 43.4 and 43.0, 47 Mi 62.9 and 62.7, 63 Mi 80.6 and 81.6, 127 Mi 154.6 and 159.0.
 static bool together_on(const SceneDev& S, uint32_t n, bool batch, bool timed) {
     return !S.section_on && (!S.any_passable || walks_on(S, batch)) && !timed && n <= (1u << 25);
 }

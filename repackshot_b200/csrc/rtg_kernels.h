@@ -130,7 +130,7 @@ struct PathBuffers {
     float4* sh_o;    // shadow rays: origin, w: t_max
     float4* sh_d;
     float4* sh_c;    // contribution, w: slot
-    uint32_t* counters;  // [3] error bits; ROUND_COUNTERS + 4 r on: round r's counts (round_counters)
+    uint32_t* counters;  // [3] error bits; ROUND_COUNTERS + 4 r on: round r's counts (round_counter)
     unsigned long long* rays;
     // Coherence sort of the rays before each traversal (RaySort); all null: off.
     uint32_t* rbins;   // extension rays: [0, nk) key histogram, [nk, 2 nk) cursors
