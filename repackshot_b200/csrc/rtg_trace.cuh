@@ -300,15 +300,13 @@ RTG_D float plane_t(uint32_t word, uint32_t k, float a, float b) {
     return __fmaf_rn(__uint_as_float(__byte_perm(word, 0x3f800000u, 0x7604u | (k << 4))), a, b);
 }
 
-// The bits of a float as an unsigned number in its order (below 0xffffffff), and back; a positive
-// one's bits are in order as they are.
+// A hit child's key: its entry distance's bits as an unsigned number with the slot in the three lowest
+// bits. That is the reference's order (traverse.rs:47), in which entries before the origin come last, the
+// farthest of them at the end. Back from a key the distance is rounded down, as it only orders children
+// and culls them later.
+RTG_D uint32_t child_key(float n, uint32_t slot) { return (__float_as_uint(n) & ~7u) | slot; }
 template <bool POS>
-RTG_D uint32_t ordered_bits(float x) {
-    const uint32_t b = __float_as_uint(x);
-    return POS ? b : (b & 0x80000000u ? ~b : b | 0x80000000u);
-}
-template <bool POS>
-RTG_D uint32_t ordered_value(uint32_t k) { return POS ? k : (k & 0x80000000u ? k & 0x7fffffffu : ~k); }
+RTG_D uint32_t key_distance(uint32_t k) { return !POS && (k & 0x80000000u) ? k | 7u : k & ~7u; }
 
 // Sorts eight keys, ascending: a network of 19 exchanges.
 RTG_D void exchange(uint32_t& a, uint32_t& b) {
@@ -386,9 +384,8 @@ RTG_D bool trav_node(const SceneDev& S, Trav& T, float tmin, Stack& stack, uint3
     const uint32_t off_lo = q.off_lo, off_hi = q.off_hi, inner = q.inner, leaf_base = h.leaf_base | NODE_LEAF;
     const float tmax = T.best_t * RTG_ROBUST;
     if (T.sp + 7 > STACK_CAP) { *err |= 1u; hit = false; return true; }
-    // A hit child's key: its entry distance with the slot in the three lowest bits (rounded
-    // down: the distance only orders children and culls them later). Every array index is a
-    // constant after unrolling, so the keys stay in registers.
+    // The hit children's keys. Every array index is a constant after unrolling, so the keys stay in
+    // registers.
     uint32_t key[8];
     uint32_t next = 0xffffffffu;
 #pragma unroll
@@ -405,7 +402,7 @@ RTG_D bool trav_node(const SceneDev& S, Trav& T, float tmin, Stack& stack, uint3
                 next = child_ref(inner, h.node_base, leaf_base, off_lo, off_hi, c);
             }
         } else {
-            key[c] = n <= f ? ((ordered_bits<POS>(n) & ~7u) | c) : 0xffffffffu;
+            key[c] = n <= f ? child_key(n, c) : 0xffffffffu;
         }
     }
     if (MODE != TRACE_ANY) {
@@ -415,7 +412,7 @@ RTG_D bool trav_node(const SceneDev& S, Trav& T, float tmin, Stack& stack, uint3
 #pragma unroll
             for (int j = 7; j >= 1; --j)
                 if (key[j] != 0xffffffffu)
-                    stack.put(T.sp++, ((uint64_t)ordered_value<POS>(key[j] & ~7u) << 32) | child_ref(inner, h.node_base, leaf_base, off_lo, off_hi, key[j] & 7u));
+                    stack.put(T.sp++, ((uint64_t)key_distance<POS>(key[j]) << 32) | child_ref(inner, h.node_base, leaf_base, off_lo, off_hi, key[j] & 7u));
             next = child_ref(inner, h.node_base, leaf_base, off_lo, off_hi, key[0] & 7u);
         }
     }
@@ -459,7 +456,8 @@ RTG_D bool trav_leaf(const SceneDev& S, Trav& T, float tmin, Stack& stack, uint3
                 if (T.camera && (see & 2u)) continue;
                 // The scalar watertight test (triangle.rs:123), the reference's operations in its
                 // order. The reference swaps the minor axes for a ray down the major one; that only
-                // negates u, v and w, exactly.
+                // negates u, v and w, exactly (a t of zero, which takes a t_min of zero or less, may have
+                // the other sign).
                 const int kz = T.kz;
                 auto px = [&](float x, float y, float z) { return kz == 0 ? y : (kz == 1 ? z : x); };
                 auto py = [&](float x, float y, float z) { return kz == 0 ? z : (kz == 1 ? x : y); };
